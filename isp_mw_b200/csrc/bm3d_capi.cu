@@ -535,7 +535,7 @@ static int plan_geometry(bm3d_ctx *ctx, StageArgs<T> &a, const bm3d_stage_params
     const int ngcand = sizeof(T) == 4 ? 8 : 6;
     int gi = 0;
     int tx = generic ? gcand[0][0] : ctx->tile_x, ty = generic ? gcand[0][1] : ctx->tile_y;
-    warps = generic ? gcand[0][2] : ctx->warps;
+    warps = generic ? gcand[0][2] : std::min(ctx->warps, stage_max_warps<T>());
     for (;;) {
         const int reach = a.match ? a.range : 0;
         a.region_w = std::min(width, (tx - 1) * a.step + 2 * reach + BS);

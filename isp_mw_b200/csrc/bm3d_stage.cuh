@@ -1293,8 +1293,14 @@ __device__ __forceinline__ void stage_tile_body_seq3(const StageArgs<T> &a, int 
     flush_stats(a, lane, n_sum, n_sq, n_cand, n_fix, n_bad);
 }
 
+// Registers bound the warps of a CTA: FP32 runs 16 of 128 registers a thread.
+// FP64 values take two registers each: at 128 the kernels spill 240-600 bytes a
+// thread, so FP64 runs 8 warps of up to 255 (no spills; lc profile, 640 x 480,
+// both stages: 0.852 -> 0.660 ms).
+template <typename T> __host__ __device__ constexpr int stage_max_warps() { return sizeof(T) == 4 ? 16 : 8; }
+
 template <typename T, bool WIENER, int NPL, int KS>
-__global__ void __launch_bounds__(512, 1) stage_kernel(const StageArgs<T> a)
+__global__ void __launch_bounds__(stage_max_warps<T>() * kWarp, 1) stage_kernel(const StageArgs<T> a)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const unsigned avail = dynamic_smem_bytes();
