@@ -73,7 +73,7 @@ def make_params(d: dict) -> StageParams:
 def build(reference: bool = True) -> None:
     """Compile the restatement, and the reference when its tree is present."""
     targets = ["port"]
-    if reference and os.path.isdir(REFERENCE_TREE):
+    if reference and os.path.isfile(os.path.join(REFERENCE_TREE, "source", "BM3D.cpp")):
         targets.append("ref")
     subprocess.run(["make", "-s", "-C", HERE, f"REF={REFERENCE_TREE}"] + targets, check=True)
 
