@@ -115,7 +115,11 @@ template <> struct SortKey<float> {
     static __device__ __forceinline__ SortKey invalid() { return SortKey{~0ull}; }
     static __device__ __forceinline__ SortKey make(float key, unsigned idx)
     {
-        return SortKey{(static_cast<unsigned long long>(__float_as_uint(key)) << 32) | idx};
+        return pack(__float_as_uint(key), idx);
+    }
+    static __device__ __forceinline__ SortKey pack(unsigned bits, unsigned idx)
+    {
+        return SortKey{(static_cast<unsigned long long>(bits) << 32) | idx};
     }
     __device__ __forceinline__ bool valid() const { return v != ~0ull; }
     __device__ __forceinline__ float key() const { return __uint_as_float(static_cast<unsigned>(v >> 32)); }
@@ -139,7 +143,11 @@ template <> struct SortKey<double> {
     static __device__ __forceinline__ SortKey invalid() { return SortKey{~0ull, ~0ull}; }
     static __device__ __forceinline__ SortKey make(double key, unsigned idx)
     {
-        return SortKey{static_cast<unsigned long long>(__double_as_longlong(key)), idx};
+        return pack(static_cast<unsigned long long>(__double_as_longlong(key)), idx);
+    }
+    static __device__ __forceinline__ SortKey pack(unsigned long long bits, unsigned idx)
+    {
+        return SortKey{bits, idx};
     }
     __device__ __forceinline__ bool valid() const { return k != ~0ull; }
     __device__ __forceinline__ double key() const { return __longlong_as_double(static_cast<long long>(k)); }
@@ -160,21 +168,6 @@ template <> struct SortKey<double> {
     }
 };
 
-// The key part of a SortKey alone (its IEEE bits; an invalid key's are all
-// ones), for the selection threshold, which depends on key values only.
-template <typename B> struct KeyBits {
-    B v;
-    __device__ __forceinline__ bool operator<(const KeyBits &o) const { return v < o.v; }
-    __device__ __forceinline__ KeyBits shfl_xor(int m) const
-    {
-        return KeyBits{__shfl_xor_sync(0xffffffffu, v, m)};
-    }
-    __device__ __forceinline__ KeyBits shfl(int src) const
-    {
-        return KeyBits{__shfl_sync(0xffffffffu, v, src)};
-    }
-};
-
 template <typename K> __device__ __forceinline__ K warp_min(K v)
 {
 #pragma unroll
@@ -183,45 +176,6 @@ template <typename K> __device__ __forceinline__ K warp_min(K v)
         if (o < v) v = o;
     }
     return v;
-}
-
-// Bitonic sort of one key per lane, ascending by lane.
-template <typename K> __device__ __forceinline__ K bitonic32(K v, int lane)
-{
-#pragma unroll
-    for (int k = 2; k <= 32; k <<= 1) {
-#pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            const K p = v.shfl_xor(j);
-            const bool take_min = ((lane & k) == 0) == ((lane & j) == 0);
-            v = (take_min == (p < v)) ? p : v;
-        }
-    }
-    return v;
-}
-
-// Bitonic sort of two keys per lane (element e = lane + 32 s), ascending by e.
-template <typename K> __device__ __forceinline__ void bitonic64(K &v0, K &v1, int lane)
-{
-#pragma unroll
-    for (int k = 2; k <= 64; k <<= 1) {
-#pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            if (j == 32) {
-                if (v1 < v0) {
-                    const K t = v0;
-                    v0 = v1;
-                    v1 = t;
-                }
-            } else {
-                const K p0 = v0.shfl_xor(j), p1 = v1.shfl_xor(j);
-                const bool lower = (lane & j) == 0;
-                const bool up0 = (lane & k) == 0, up1 = ((lane + 32) & k) == 0;
-                v0 = ((up0 == lower) == (p0 < v0)) ? p0 : v0;
-                v1 = ((up1 == lower) == (p1 < v1)) ? p1 : v1;
-            }
-        }
-    }
 }
 
 template <typename T> __device__ __forceinline__ T warp_sum(T v)
@@ -405,7 +359,7 @@ __host__ __device__ inline SmemPlan plan_smem(int nplanes, bool wiener, int alia
         ? sizeof(T) * static_cast<size_t>(gs) * generic_block_stride(bs) *
               (wiener && !generic_one_buffer<T>(wiener, bs) ? 2 : 1)
         : sizeof(T) * kGSMax * kGroupStride;
-    const size_t key_bytes = sizeof(SortKey<T>) * key_slots;
+    const size_t key_bytes = sizeof(T) * key_slots;  // distance bits
     const size_t scratch = group_bytes > key_bytes ? group_bytes : key_bytes;
     s.scratch_bytes = (scratch + 15) / 16 * 16;
     s.refblk_bytes = generic ? (sizeof(T) * bsq + 15) / 16 * 16 : 0;

@@ -187,10 +187,10 @@ __device__ void dct_z_generic(T *G, int n, int bs, int lane, const T *tab, bool 
 // block (include/Block.h:589-611), then the shared ordered selection.
 template <typename T>
 __device__ int match_generic(const StageArgs<T> &a, const Tile<T> &t, int j0, int i0, int lane,
-                             SortKey<T> *keys, T *refblk, SortKey<T> *heap, BlockPos *list,
-                             T *lkeys, unsigned &n_cand, unsigned &n_fix)
+                             typename DistBits<T>::type *dist, T *refblk, SortKey<T> *heap,
+                             BlockPos *list, T *lkeys, unsigned &n_cand, unsigned &n_fix)
 {
-    using K = SortKey<T>;
+    using B = typename DistBits<T>::type;
     if (!a.match) {
         if (lane == 0) {
             list[0] = BlockPos{j0, i0};
@@ -214,14 +214,15 @@ __device__ int match_generic(const StageArgs<T> &a, const Tile<T> &t, int j0, in
         }
     }
     __syncwarp();
+    const unsigned nc_div = div_number(nc);
+    const B limit = dist_limit(a.thSSE);
+    int nvalid = 0;
     for (int c = lane; c <= ngrid; c += kWarp) {
         const T *cand;
         int cp;
-        bool self = false;
         if (c < ngrid) {
-            const int rr = c / nc, cc = c - rr * nc;
+            const int rr = div_magic(c, nc_div), cc = c - rr * nc;
             const int cy = tp + rr * st, cx = l + cc * st;
-            self = (cy == j0 && cx == i0);
             cand = t.refw[0] + (cy - t.ry0) * t.pitch + (cx - t.rx0);
             cp = t.pitch;
         } else {
@@ -243,12 +244,12 @@ __device__ int match_generic(const StageArgs<T> &a, const Tile<T> &t, int j0, in
                     d = add_rn(d, mul_rn(df, df));
                 }
         }
-        const bool ok = !self && d <= a.thSSE && d != T(0);
-        keys[c] = ok ? K::make(key_from_dist(d, a.distMul), static_cast<unsigned>(c)) : K::invalid();
+        dist[c] = accept_dist(DistBits<T>::of(d), limit, nvalid);
     }
     __syncwarp();
     n_cand += static_cast<unsigned>(ngrid);
-    return select_group<T>(a, keys, ngrid, nc, tp, l, st, j0, i0, lane, heap, list, lkeys, n_fix);
+    return select_group<T>(a, dist, ngrid, nc, nc_div, tp, l, st, j0, i0, lane, nvalid, heap, list,
+                           lkeys, n_fix);
 }
 
 // Element e of a group stored [z][y][x]: shifts for BlockSize 8, divisions
@@ -572,7 +573,7 @@ __device__ __forceinline__ void generic_tile_body(const StageArgs<T> &a, int til
     const int gvals = a.group_size * generic_block_stride(bs);
     T *Gs = reinterpret_cast<T *>(wbase);
     T *Gr = Gs + gvals;
-    SortKey<T> *keys = reinterpret_cast<SortKey<T> *>(wbase);
+    auto *dist = reinterpret_cast<typename DistBits<T>::type *>(wbase);
     T *refblk = reinterpret_cast<T *>(wbase + scratch);
     unsigned char *after = wbase + scratch + sp.refblk_bytes;
     SortKey<T> *heap = reinterpret_cast<SortKey<T> *>(after);
@@ -595,9 +596,9 @@ __device__ __forceinline__ void generic_tile_body(const StageArgs<T> &a, int til
         // BlockSize 8 with step 1: the register-resident kernel's strips of
         // four candidates; otherwise one lane per candidate
         const int n = (bs == kBS && a.bm_step == 1)
-                          ? match_block<T, 4>(a, t, j0, i0, lane, keys, heap, list, lkeys, n_cand,
+                          ? match_block<T, 4>(a, t, j0, i0, lane, dist, heap, list, lkeys, n_cand,
                                               n_fix)
-                          : match_generic<T>(a, t, j0, i0, lane, keys, refblk, heap, list, lkeys,
+                          : match_generic<T>(a, t, j0, i0, lane, dist, refblk, heap, list, lkeys,
                                              n_cand, n_fix);
         n_sum += n;
         n_sq += static_cast<unsigned>(n * n);
@@ -649,7 +650,7 @@ __device__ __forceinline__ void generic_tile_body_seq3(const StageArgs<T> &a, in
     const size_t scratch = sp.scratch_bytes;
     T *Gs = reinterpret_cast<T *>(wbase);
     T *Gr = Gs + GS * generic_block_stride(bs);
-    SortKey<T> *keys = reinterpret_cast<SortKey<T> *>(wbase);
+    auto *dist = reinterpret_cast<typename DistBits<T>::type *>(wbase);
     T *refblk = reinterpret_cast<T *>(wbase + scratch);
     unsigned char *after = wbase + scratch + sp.refblk_bytes;
     SortKey<T> *heap = reinterpret_cast<SortKey<T> *>(after);
@@ -671,9 +672,9 @@ __device__ __forceinline__ void generic_tile_body_seq3(const StageArgs<T> &a, in
                 const int ky = ky0 + r / tw, kx = kx0 + r % tw;
                 const int j0 = ref_pos(ky, a.step, bottom), i0 = ref_pos(kx, a.step, right);
                 n = (bs == kBS && a.bm_step == 1)
-                        ? match_block<T, 4>(a, t, j0, i0, lane, keys, heap, list, lkeys, n_cand,
+                        ? match_block<T, 4>(a, t, j0, i0, lane, dist, heap, list, lkeys, n_cand,
                                             n_fix)
-                        : match_generic<T>(a, t, j0, i0, lane, keys, refblk, heap, list, lkeys,
+                        : match_generic<T>(a, t, j0, i0, lane, dist, refblk, heap, list, lkeys,
                                            n_cand, n_fix);
                 n_sum += n;
                 n_sq += static_cast<unsigned>(n * n);

@@ -211,46 +211,110 @@ __device__ __forceinline__ bool block_in_tile(const Tile<T> &t, int py, int px)
     return py >= t.ry0 && px >= t.rx0 && py + t.bs <= t.ry0 + t.rh && px + t.bs <= t.rx0 + t.rw;
 }
 
-// Ordered group of reference block (j0, i0) from its search list: keys[0,
-// ngrid) are the window grid in raster order, keys[ngrid] the trailing (0, 0)
-// slot (invalid keys = rejected or the block itself). Writes list/lkeys in the
+// A warp's search list while a group is selected: the distance bits of every
+// candidate at its place in the reference's list order -- the window grid in
+// raster order, then the trailing (0, 0) slot. A rejected candidate (over the
+// threshold, or equal to the reference block) has all bits set.
+constexpr unsigned kOrdSelf = 0xffffffffu;  // list index that stands for the reference block
+
+template <typename T> struct DistBits;
+template <> struct DistBits<float> {
+    using type = unsigned;
+    static __device__ __forceinline__ unsigned of(float d) { return __float_as_uint(d); }
+    static __device__ __forceinline__ float value(unsigned b) { return __uint_as_float(b); }
+    // keys between 2^-124 and 2^127: normal, with room for the rounding slack
+    static constexpr unsigned kLow = 0x01800000u, kHigh = 0x7f000000u;
+    static __device__ __forceinline__ unsigned warp_max(unsigned v)
+    {
+        return __reduce_max_sync(0xffffffffu, v);
+    }
+};
+template <> struct DistBits<double> {
+    using type = unsigned long long;
+    static __device__ __forceinline__ unsigned long long of(double d)
+    {
+        return static_cast<unsigned long long>(__double_as_longlong(d));
+    }
+    static __device__ __forceinline__ double value(unsigned long long b)
+    {
+        return __longlong_as_double(static_cast<long long>(b));
+    }
+    static constexpr unsigned long long kLow = 0x0040000000000000ull, kHigh = 0x7fe0000000000000ull;
+    static __device__ __forceinline__ unsigned long long warp_max(unsigned long long v)
+    {
+#pragma unroll
+        for (int m = 16; m >= 1; m >>= 1) {
+            const unsigned long long o = __shfl_xor_sync(0xffffffffu, v, m);
+            v = o > v ? o : v;
+        }
+        return v;
+    }
+};
+
+// How many of the n (a multiple of 4) values at p, 16-byte aligned in shared
+// memory, are below v0 / v1: every lane reads the same words (broadcasts), so
+// a lane ranks its values against the whole set with independent compares
+// where a sorting network would chain shuffles.
+__device__ __forceinline__ void count_below(const unsigned *p, int n, unsigned v0, unsigned v1,
+                                            int &c0, int &c1, bool two)
+{
+    c0 = c1 = 0;
+#pragma unroll 2
+    for (int j = 0; j < n; j += 4) {
+        const uint4 q = *reinterpret_cast<const uint4 *>(p + j);
+        c0 += (q.x < v0) + (q.y < v0) + (q.z < v0) + (q.w < v0);
+        if (two) c1 += (q.x < v1) + (q.y < v1) + (q.z < v1) + (q.w < v1);
+    }
+}
+__device__ __forceinline__ void count_below(const unsigned long long *p, int n,
+                                            unsigned long long v0, unsigned long long v1, int &c0,
+                                            int &c1, bool two)
+{
+    c0 = c1 = 0;
+    for (int j = 0; j < n; j += 2) {
+        const ulonglong2 q = *reinterpret_cast<const ulonglong2 *>(p + j);
+        c0 += (q.x < v0) + (q.y < v0);
+        if (two) c1 += (q.x < v1) + (q.y < v1);
+    }
+}
+
+// Unsigned division by a small number d: k / d == div_magic(k, div_number(d))
+// for k * d < 2^32 (d == 1 has no 32-bit number and is passed through).
+__device__ __forceinline__ unsigned div_number(int d) { return d > 1 ? 0xffffffffu / d + 1u : 0u; }
+__device__ __forceinline__ int div_magic(int k, unsigned m)
+{
+    return m ? static_cast<int>(__umulhi(static_cast<unsigned>(k), m)) : k;
+}
+
+// Ordered group of reference block (j0, i0) from its search list `dist` (see
+// above; ngrid = nr x nc window places from (tp, l) in steps of st, plus the
+// slot), of which this lane accepted nvalid. Writes list / lkeys in the
 // reference's group order and returns the group size.
+//
+// What bounds it: latency -- one warp's dependent steps. The list holds
+// 32-bit distances; only the few that can be among the best get a key
+// (key_from_dist is monotone, so the cut is made on distances, with three
+// units in the last place of slack: fewer than that share a key with the
+// cut's). Ranks come from broadcast counts (count_below), two dependent
+// shared-memory passes instead of two 15-stage shuffle networks. Lanes take
+// the list 32 places apart, so that candidates along an edge (one column, or
+// one row) fall to different lanes and the cut stays tight (with the lanes'
+// own strips the compacted set overflowed on such planes: 0.82 -> 1.09 ms).
+// 1080p, sigma 25, against 64-bit keys and two sorting networks: fast basic /
+// final 0.355 / 0.461 -> 0.333 / 0.438 ms, np 2.82 / 6.27 -> 2.00 / 5.86 ms
+// (the smaller list also lets np's basic stage keep 16 warps).
 template <typename T>
-__device__ int select_group(const StageArgs<T> &a, const SortKey<T> *keys, int ngrid, int nc,
-                            int tp, int l, int st, int j0, int i0, int lane, SortKey<T> *heap,
-                            BlockPos *list, T *lkeys, unsigned &n_fix)
+__device__ int select_group(const StageArgs<T> &a, const typename DistBits<T>::type *dist,
+                            int ngrid, int nc, unsigned nc_div, int tp, int l, int st, int j0,
+                            int i0, int lane, int nvalid, SortKey<T> *heap, BlockPos *list,
+                            T *lkeys, unsigned &n_fix)
 {
     using K = SortKey<T>;
+    using DB = DistBits<T>;
+    using B = typename DB::type;
+    const B none = ~B(0);
     const int GS = a.group_size;
-    // Ordered selection of the GS - 1 best candidates by (key, list index).
-    // T = the (take)-th smallest of the lanes' minima bounds the take best
-    // from above (those minima are take distinct candidates). All candidates
-    // whose key value is <= T's -- ties with the cut-off included -- are
-    // compacted and bitonic-sorted; typically 16-24 of ~360. Groups of more
-    // than 17 blocks take T from the lanes' two smallest keys (64 distinct
-    // candidates), which keeps the compacted set within the 64-wide sort.
     const int nkeys = ngrid + 1;
-    const bool two = GS - 1 > kWarp / 2;
-    K lmin = K::invalid(), lmin2 = K::invalid();
-    int nvalid = 0;
-    if (two) {
-        for (int i = lane; i < nkeys; i += kWarp) {
-            const K v = keys[i];
-            nvalid += v.valid() ? 1 : 0;
-            if (v < lmin) {
-                lmin2 = lmin;
-                lmin = v;
-            } else if (v < lmin2) {
-                lmin2 = v;
-            }
-        }
-    } else {
-        for (int i = lane; i < nkeys; i += kWarp) {
-            const K v = keys[i];
-            nvalid += v.valid() ? 1 : 0;
-            if (v < lmin) lmin = v;
-        }
-    }
     const int accepted = __reduce_add_sync(0xffffffffu, nvalid);
     const int take = min(GS - 1, accepted);
     // list[0] is the reference block itself (key 0, include/Block.h:685)
@@ -258,81 +322,151 @@ __device__ int select_group(const StageArgs<T> &a, const SortKey<T> *keys, int n
         list[0] = BlockPos{j0, i0};
         lkeys[0] = T(0);
     }
+    auto place = [&](unsigned idx) {
+        if (idx == kOrdSelf) return BlockPos{j0, i0};
+        if (static_cast<int>(idx) >= ngrid) return BlockPos{0, 0};
+        const int rr = div_magic(static_cast<int>(idx), nc_div);
+        return BlockPos{tp + rr * st, l + (static_cast<int>(idx) - rr * nc) * st};
+    };
     auto put = [&](int rank, const K &m) {  // rank-th best candidate -> list[rank + 1]
-        const int idx = static_cast<int>(m.idx());
-        int y = 0, x = 0;
-        if (idx < ngrid) {
-            const int rr = idx / nc;
-            y = tp + rr * st;
-            x = l + (idx - rr * nc) * st;
-        }
-        list[rank + 1] = BlockPos{y, x};
+        list[rank + 1] = place(m.idx());
         lkeys[rank + 1] = m.key();
+    };
+    auto make = [&](B bits, unsigned idx) {
+        return bits == none ? K::invalid() : K::make(key_from_dist(DB::value(bits), a.distMul), idx);
     };
     bool tie = false;
     if (take > 0) {
-        // The threshold depends on key values only, so the lanes' minima are
-        // sorted by their key bits alone (the (take)-th smallest key value is
-        // the same in (key, index) order).
-        using KB = KeyBits<decltype(lmin.key_bits())>;
-        decltype(lmin.key_bits()) tb;
-        if (two) {  // element take - 1 (< 32) of the 64 sorted sits in lane take - 1's v0
-            KB s0{lmin.key_bits()}, s1{lmin2.key_bits()};
-            bitonic64(s0, s1, lane);
-            tb = s0.shfl(take - 1).v;
-        } else {
-            tb = bitonic32(KB{lmin.key_bits()}, lane).shfl(take - 1).v;
+        // A window of up to kHeld x 32 places (BMrange 9) is read once and
+        // held in registers for both passes; larger ones are read again.
+        constexpr int kHeld = 12;
+        const bool one = nkeys <= kHeld * kWarp;
+        const bool two = GS - 1 > kWarp / 2;
+        B v[kHeld];
+        auto load = [&](int first) {
+#pragma unroll
+            for (int k = 0; k < kHeld; ++k) {
+                const int i = first + k * kWarp + lane;
+                v[k] = i < nkeys ? dist[i] : none;
+            }
+        };
+        // Cut: the (take)-th smallest of the lanes' minima bounds the take best
+        // from above (those minima are take distinct candidates). Groups of
+        // more than 17 blocks use the lanes' two smallest (64 candidates),
+        // which keeps the compacted set within kCand.
+        B lmin = none, lmin2 = none;
+        for (int first = 0; first < nkeys; first += kHeld * kWarp) {
+            load(first);
+#pragma unroll
+            for (int k = 0; k < kHeld; ++k) {
+                if (two) {
+                    const B up = v[k] > lmin ? v[k] : lmin;
+                    lmin2 = up < lmin2 ? up : lmin2;
+                }
+                lmin = v[k] < lmin ? v[k] : lmin;
+            }
         }
-        // One pass counts the keys at or under the threshold (M) and packs the
-        // first kCand of them into heap[] by warp ballot (their order there is
-        // irrelevant: they are sorted next).
-        int M = 0;
-        const unsigned below = (1u << lane) - 1u;
-        for (int first = 0; first < nkeys; first += kWarp) {
-            const int i = first + lane;
-            const K v = i < nkeys ? keys[i] : K::invalid();
-            const bool in = v.valid() && v.key_bits() <= tb;
-            const unsigned m = __ballot_sync(0xffffffffu, in);
-            const int pos = M + __popc(m & below);
-            if (in && pos < kCand) heap[pos] = v;
-            M += __popc(m);
+        B *kb = reinterpret_cast<B *>(heap);
+        kb[lane] = lmin;
+        if (two) kb[lane + kWarp] = lmin2;
+        __syncwarp();
+        int r0, r1;
+        count_below(kb, two ? 2 * kWarp : kWarp, lmin, lmin2, r0, r1, two);
+        B tb = r0 < take ? lmin : B(0);
+        if (two && r1 < take && lmin2 > tb) tb = lmin2;
+        tb = DB::warp_max(tb);
+        B cut = none - 1;  // fewer than take lanes hold a candidate: keep them all
+        bool sure = true;
+        if (tb != none) {
+            const B kt = DB::of(key_from_dist(DB::value(tb), a.distMul));
+            sure = kt >= DB::kLow && kt <= DB::kHigh;  // else the slack does not hold
+            cut = tb + 3;
         }
-        if (M <= kCand) {
+        // Compact the elements at or under the cut into heap[] (any order).
+        int mine = 0;
+        for (int first = 0; first < nkeys; first += kHeld * kWarp) {
+            if (!one) load(first);
+#pragma unroll
+            for (int k = 0; k < kHeld; ++k) mine += v[k] <= cut ? 1 : 0;
+        }
+        int pos = mine;
+#pragma unroll
+        for (int o = 1; o < kWarp; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, pos, o);
+            if (lane >= o) pos += u;
+        }
+        const int M = __shfl_sync(0xffffffffu, pos, kWarp - 1);
+        if (sure && M <= kCand) {
+            pos -= mine;
+            for (int first = 0; first < nkeys; first += kHeld * kWarp) {
+                if (!one) load(first);
+#pragma unroll
+                for (int k = 0; k < kHeld; ++k)
+                    if (v[k] <= cut)
+                        heap[pos++] = K::pack(v[k], static_cast<unsigned>(first + k * kWarp + lane));
+            }
             __syncwarp();
-            K v0 = lane < M ? heap[lane] : K::invalid();
-            K v1 = lane + kWarp < M ? heap[lane + kWarp] : K::invalid();
-            if (M <= kWarp) v0 = bitonic32(v0, lane);
-            else bitonic64(v0, v1, lane);
-            if (lane < take) put(lane, v0);
-            if (lane + kWarp < take) put(lane + kWarp, v1);
-            // equal keys at adjacent ranks r, r + 1 with r < take
-            // (every shuffle runs on all 32 lanes; only the selects below differ)
-            const K n0 = v0.shfl((lane + 1) & (kWarp - 1));
-            const K nx = v1.shfl((lane + 1) & (kWarp - 1));
-            const K f1 = v1.shfl(0);
-            const K next0 = lane < kWarp - 1 ? n0 : f1;
-            const bool t0 = lane < take && lane + 1 < M && next0.key_bits() == v0.key_bits();
-            const bool t1 = lane + kWarp < take && lane + kWarp + 1 < M && lane < kWarp - 1 &&
-                            nx.key_bits() == v1.key_bits();
-            tie = __any_sync(0xffffffffu, t0 || t1);
+            K v0 = K::invalid(), v1 = K::invalid();
+            if (lane < M) v0 = make(heap[lane].key_bits(), heap[lane].idx());
+            if (lane + kWarp < M)
+                v1 = make(heap[lane + kWarp].key_bits(), heap[lane + kWarp].idx());
+            __syncwarp();
+            const bool more = M > kWarp;
+            kb[lane] = v0.key_bits();
+            if (more) kb[lane + kWarp] = v1.key_bits();
+            __syncwarp();
+            count_below(kb, (M + 3) & ~3, v0.key_bits(), v1.key_bits(), r0, r1, more);
+            // the ranks are a permutation of 0 .. M - 1 unless keys are equal
+            unsigned lo = 0, hi = 0;
+            if (lane < M) (r0 < 32 ? lo : hi) |= 1u << (r0 & 31);
+            if (lane + kWarp < M) (r1 < 32 ? lo : hi) |= 1u << (r1 & 31);
+            int distinct = __popc(__reduce_or_sync(0xffffffffu, lo));
+            if (more) distinct += __popc(__reduce_or_sync(0xffffffffu, hi));
+            if (distinct != M) {
+                // equal keys rank by list order; a tie counts when it reaches
+                // the kept set: a kept element with an equal one after it
+                __syncwarp();
+                heap[lane] = v0;
+                heap[lane + kWarp] = v1;
+                __syncwarp();
+                bool e0 = false, e1 = false;
+                for (int j = 0; j < M; ++j) {
+                    const K o = heap[j];
+                    if (o.key_bits() == v0.key_bits()) {
+                        if (o < v0) ++r0;
+                        else if (v0 < o) e0 = true;
+                    }
+                    if (o.key_bits() == v1.key_bits()) {
+                        if (o < v1) ++r1;
+                        else if (v1 < o) e1 = true;
+                    }
+                }
+                const bool t0 = lane < M && e0 && r0 < take;
+                const bool t1 = lane + kWarp < M && e1 && r1 < take;
+                tie = __any_sync(0xffffffffu, t0 || t1);
+            }
+            if (lane < M && r0 < take) put(r0, v0);
+            if (lane + kWarp < M && r1 < take) put(r1, v1);
         } else {
-            // Rare (many candidates share the cut-off): repeated warp minimum,
-            // whose owner lane advances to the next key of its slice.
-            K cur = lmin;
+            // Rare (many candidates share the cut, or keys outside the normal
+            // range): repeated warp minimum, whose owner lane advances to the
+            // next key of its elements.
+            auto next_after = [&](const K &m, bool any) {
+                K nxt = K::invalid();
+                for (int i = lane; i < nkeys; i += kWarp) {
+                    const K u = make(dist[i], static_cast<unsigned>(i));
+                    if ((any || m < u) && u < nxt) nxt = u;
+                }
+                return nxt;
+            };
+            K cur = next_after(K::invalid(), true);
             T prev_key = T(-1);
             for (int k = 0; k < take; ++k) {
                 const K m = warp_min(cur);
                 tie |= (m.key() == prev_key);
                 prev_key = m.key();
                 if (lane == 0) put(k, m);
-                if (cur == m) {
-                    K nxt = K::invalid();
-                    for (int i = lane; i < nkeys; i += kWarp) {
-                        const K v = keys[i];
-                        if (m < v && v < nxt) nxt = v;
-                    }
-                    cur = nxt;
-                }
+                if (cur == m) cur = next_after(m, false);
             }
             const K m = warp_min(cur);
             tie |= (m.valid() && m.key() == prev_key);
@@ -342,73 +476,104 @@ __device__ int select_group(const StageArgs<T> &a, const SortKey<T> *keys, int n
     // More matches than the group holds: the reference keeps GroupSize of them
     // with std::partial_sort (include/Block.h:690-696), whose placement of
     // equal keys is libstdc++'s heap order, not list order. Redo such groups
-    // with that exact algorithm when a tie touches the kept set.
-    if (accepted + 1 > GS && GS > 1) {
-        if (tie) {
-            if (lane == 0) {
-                ++n_fix;
-                // heap[] holds the first GS entries of the reference's match list:
-                // the reference block, then matches in list order.
-                heap[0] = K::make(T(0), 0xffffffffu);
-                int h = 1, i = 0;
-                for (; i < nkeys && h < GS; ++i)
-                    if (keys[i].valid()) heap[h++] = keys[i];
-                auto less = [](const K &p, const K &q) { return p.key() < q.key(); };
-                auto adjust = [&](int hole, int len, K value) {
-                    const int top = hole;
-                    int child = hole;
-                    while (child < (len - 1) / 2) {
-                        child = 2 * (child + 1);
-                        if (less(heap[child], heap[child - 1])) child--;
-                        heap[hole] = heap[child];
-                        hole = child;
-                    }
-                    if ((len & 1) == 0 && child == (len - 2) / 2) {
-                        child = 2 * (child + 1);
-                        heap[hole] = heap[child - 1];
-                        hole = child - 1;
-                    }
-                    int parent = (hole - 1) / 2;
-                    while (hole > top && less(heap[parent], value)) {
-                        heap[hole] = heap[parent];
-                        hole = parent;
-                        parent = (hole - 1) / 2;
-                    }
-                    heap[hole] = value;
-                };
-                for (int parent = (GS - 2) / 2;; --parent) {  // __make_heap
-                    adjust(parent, GS, heap[parent]);
-                    if (parent == 0) break;
-                }
-                for (; i < nkeys; ++i) {  // __heap_select
-                    const K v = keys[i];
-                    if (v.valid() && less(v, heap[0])) adjust(0, GS, v);
-                }
-                for (int last = GS; last > 1;) {  // __sort_heap
-                    --last;
-                    const K v = heap[last];
-                    heap[last] = heap[0];
-                    adjust(0, last, v);
-                }
-                for (int k = 0; k < GS; ++k) {
-                    const unsigned idx = heap[k].idx();
-                    int y = 0, x = 0;
-                    if (idx == 0xffffffffu) {
-                        y = j0;
-                        x = i0;
-                    } else if (static_cast<int>(idx) < ngrid) {
-                        const int rr = static_cast<int>(idx) / nc;
-                        y = tp + rr * st;
-                        x = l + (static_cast<int>(idx) - rr * nc) * st;
-                    }
-                    list[k] = BlockPos{y, x};
-                    lkeys[k] = heap[k].key();
+    // with that exact algorithm when a tie touches the kept set: lane 0 works
+    // the heap, the warp finds the entries that change it (the heap's top only
+    // falls, so an entry not below it once is never below it).
+    if (accepted + 1 > GS && GS > 1 && tie) {
+        auto less = [](const K &p, const K &q) { return p.key() < q.key(); };
+        auto adjust = [&](int hole, int len, K value) {
+            const int top = hole;
+            int child = hole;
+            while (child < (len - 1) / 2) {
+                child = 2 * (child + 1);
+                if (less(heap[child], heap[child - 1])) child--;
+                heap[hole] = heap[child];
+                hole = child;
+            }
+            if ((len & 1) == 0 && child == (len - 2) / 2) {
+                child = 2 * (child + 1);
+                heap[hole] = heap[child - 1];
+                hole = child - 1;
+            }
+            int parent = (hole - 1) / 2;
+            while (hole > top && less(heap[parent], value)) {
+                heap[hole] = heap[parent];
+                hole = parent;
+                parent = (hole - 1) / 2;
+            }
+            heap[hole] = value;
+        };
+        // heap[] starts with the first GS entries of the reference's match
+        // list: the reference block, then matches in list order.
+        if (lane == 0) {
+            ++n_fix;
+            heap[0] = K::make(T(0), kOrdSelf);
+        }
+        int h = 1;
+        for (int first = 0; first < nkeys; first += kWarp) {
+            const int i = first + lane;
+            const K u = i < nkeys ? make(dist[i], static_cast<unsigned>(i)) : K::invalid();
+            unsigned todo = __ballot_sync(0xffffffffu, u.valid());
+            if (h < GS) {
+                const int at = h + __popc(todo & ((1u << lane) - 1u));
+                const bool in = u.valid() && at < GS;
+                if (in) heap[at] = u;
+                const unsigned took = __ballot_sync(0xffffffffu, in);
+                todo &= ~took;
+                h += __popc(took);
+                if (h == GS) {
+                    __syncwarp();
+                    if (lane == 0)
+                        for (int parent = (GS - 2) / 2;; --parent) {  // __make_heap
+                            adjust(parent, GS, heap[parent]);
+                            if (parent == 0) break;
+                        }
                 }
             }
+            while (todo) {  // __heap_select
+                __syncwarp();
+                todo &= __ballot_sync(0xffffffffu, u.valid() && less(u, heap[0]));
+                if (todo == 0) break;
+                const int from = __ffs(todo) - 1;
+                todo &= todo - 1;
+                const K w = u.shfl(from);
+                if (lane == 0) adjust(0, GS, w);
+            }
+        }
+        __syncwarp();
+        if (lane == 0)
+            for (int last = GS; last > 1;) {  // __sort_heap
+                --last;
+                const K u = heap[last];
+                heap[last] = heap[0];
+                adjust(0, last, u);
+            }
+        __syncwarp();
+        if (lane < GS) {
+            list[lane] = place(heap[lane].idx());
+            lkeys[lane] = heap[lane].key();
         }
     }
     __syncwarp();
     return take + 1;
+}
+
+// A candidate's entry in the search list. Distances are sums of squares:
+// >= +0, or NaN, whose bits compare above any threshold. A zero distance (the
+// reference block itself, or an equal block) is rejected like one over the
+// threshold (include/Block.h:606): (bits - 1) wraps to the top for it.
+template <typename B>
+__device__ __forceinline__ B accept_dist(B bits, B limit, int &nvalid)
+{
+    const bool ok = bits - 1 < limit;
+    nvalid += ok ? 1 : 0;
+    return ok ? bits : ~B(0);
+}
+
+// The matching threshold as distance bits: d <= thSSE is bits <= limit.
+template <typename T> __device__ __forceinline__ typename DistBits<T>::type dist_limit(T thSSE)
+{
+    return thSSE > T(0) ? DistBits<T>::of(thSSE) : typename DistBits<T>::type(0);
 }
 
 // ---------------------------------------------------------------------------
@@ -416,11 +581,10 @@ __device__ int select_group(const StageArgs<T> &a, const SortKey<T> *keys, int n
 // with (y, x) in the reference's group order and returns n.
 template <typename T, int KS>
 __device__ int match_block(const StageArgs<T> &a, const Tile<T> &t, int j0, int i0, int lane,
-                           SortKey<T> *keys, SortKey<T> *heap, BlockPos *list, T *lkeys,
-                           unsigned &n_cand, unsigned &n_fix)
+                           typename DistBits<T>::type *dist, SortKey<T> *heap, BlockPos *list,
+                           T *lkeys, unsigned &n_cand, unsigned &n_fix)
 {
-    using K = SortKey<T>;
-    const int GS = a.group_size;
+    using B = typename DistBits<T>::type;
     if (!a.match) {
         if (lane == 0) {
             list[0] = BlockPos{j0, i0};
@@ -433,8 +597,10 @@ __device__ int match_block(const StageArgs<T> &a, const Tile<T> &t, int j0, int 
     const int right = a.width - kBS, bottom = a.height - kBS;
     const int l = search_boundary(i0, 0, R, st), r = search_boundary(i0, right, R, st);
     const int tp = search_boundary(j0, 0, R, st), b = search_boundary(j0, bottom, R, st);
-    const int nr = (b - tp) / st + 1, nc = (r - l) / st + 1;
+    // KS > 1 only with BMstep == 1
+    const int nr = KS > 1 ? b - tp + 1 : (b - tp) / st + 1, nc = KS > 1 ? r - l + 1 : (r - l) / st + 1;
     const int ngrid = nr * nc;
+    const unsigned nc_div = div_number(nc);
 
     // Reference block in registers.
     T refv[kBS][kBS];
@@ -450,15 +616,17 @@ __device__ int match_block(const StageArgs<T> &a, const Tile<T> &t, int j0, int 
     // task for the trailing (0, 0) slot of the reference's search list.
     const int nstrips = (nr + KS - 1) / KS;
     const int ntasks = nstrips * nc;
-    constexpr int ROWS = (KS - 1) + kBS;  // KS > 1 only with BMstep == 1
+    const B limit = dist_limit(a.thSSE);
+    int nvalid = 0;
+    constexpr int ROWS = (KS - 1) + kBS;
     for (int task = lane; task <= ntasks; task += kWarp) {
         const T *base;
-        int bp, nq, rr0 = 0, cc = 0;
+        int bp, nq, at = ngrid;  // the list place of candidate 0
         if (task < ntasks) {
-            const int strip = task / nc;
-            cc = task - strip * nc;
-            rr0 = strip * KS;
-            nq = min(KS, nr - rr0);
+            const int strip = div_magic(task, nc_div);
+            const int cc = task - strip * nc, rr0 = strip * KS;
+            nq = nr - rr0;
+            at = rr0 * nc + cc;
             bp = t.pitch;
             base = t.refw[0] + (tp + rr0 * st - t.ry0) * t.pitch + (l + cc * st - t.rx0);
         } else {
@@ -495,29 +663,15 @@ __device__ int match_block(const StageArgs<T> &a, const Tile<T> &t, int j0, int 
             }
         }
 #pragma unroll
-        for (int q = 0; q < KS; ++q) {
-            if (q < nq) {
-                int idx;
-                bool self;
-                if (task < ntasks) {
-                    const int rr = rr0 + q;
-                    idx = rr * nc + cc;
-                    self = (tp + rr * st == j0) && (l + cc * st == i0);
-                } else {
-                    idx = ngrid;
-                    self = false;
-                }
-                const T d = acc[q];
-                const bool ok = !self && d <= a.thSSE && d != T(0);
-                keys[idx] = ok ? K::make(key_from_dist(d, a.distMul), static_cast<unsigned>(idx))
-                               : K::invalid();
-            }
-        }
+        for (int q = 0; q < KS; ++q)
+            if (q < nq)
+                dist[at + q * nc] = accept_dist(DistBits<T>::of(acc[q]), limit, nvalid);
     }
     __syncwarp();
     n_cand += static_cast<unsigned>(ngrid);  // grid minus self, plus (0, 0)
 
-    return select_group<T>(a, keys, ngrid, nc, tp, l, st, j0, i0, lane, heap, list, lkeys, n_fix);
+    return select_group<T>(a, dist, ngrid, nc, nc_div, tp, l, st, j0, i0, lane, nvalid, heap, list,
+                           lkeys, n_fix);
 }
 
 // ---------------------------------------------------------------------------
@@ -1106,7 +1260,7 @@ __device__ __forceinline__ void stage_tile_body(const StageArgs<T> &a, int tile,
     unsigned char *wbase = smem + sp.off_warps + sp.warp_bytes * warp;
     const size_t scratch = sp.scratch_bytes;
     T *G = reinterpret_cast<T *>(wbase);
-    SortKey<T> *keys = reinterpret_cast<SortKey<T> *>(wbase);
+    auto *dist = reinterpret_cast<typename DistBits<T>::type *>(wbase);
     SortKey<T> *heap = reinterpret_cast<SortKey<T> *>(wbase + scratch);
     BlockPos *list = reinterpret_cast<BlockPos *>(wbase + scratch + sizeof(SortKey<T>) * kCand);
     T *lkeys = reinterpret_cast<T *>(wbase + scratch + sizeof(SortKey<T>) * kCand +
@@ -1125,7 +1279,7 @@ __device__ __forceinline__ void stage_tile_body(const StageArgs<T> &a, int tile,
     for (int r = warp; r < nrefs; r += nwarps) {
         const int ky = ky0 + r / tw, kx = kx0 + r % tw;
         const int j0 = ref_pos(ky, a.step, bottom), i0 = ref_pos(kx, a.step, right);
-        const int n = match_block<T, KS>(a, t, j0, i0, lane, keys, heap, list, lkeys, n_cand, n_fix);
+        const int n = match_block<T, KS>(a, t, j0, i0, lane, dist, heap, list, lkeys, n_cand, n_fix);
         n_sum += n;
         n_sq += static_cast<unsigned>(n * n);
         dump_group(a, ky, kx, n, lane, list, lkeys);
@@ -1241,7 +1395,7 @@ __device__ __forceinline__ void stage_tile_body_seq3(const StageArgs<T> &a, int 
     unsigned char *wbase = smem + sp.off_warps + sp.warp_bytes * warp;
     const size_t scratch = sp.scratch_bytes;
     T *G = reinterpret_cast<T *>(wbase);
-    SortKey<T> *keys = reinterpret_cast<SortKey<T> *>(wbase);
+    auto *dist = reinterpret_cast<typename DistBits<T>::type *>(wbase);
     SortKey<T> *heap = reinterpret_cast<SortKey<T> *>(wbase + scratch);
     BlockPos *list = reinterpret_cast<BlockPos *>(wbase + scratch + sizeof(SortKey<T>) * kCand);
     T *lkeys = reinterpret_cast<T *>(wbase + scratch + sizeof(SortKey<T>) * kCand +
@@ -1261,7 +1415,7 @@ __device__ __forceinline__ void stage_tile_body_seq3(const StageArgs<T> &a, int 
             if (c == 0) {
                 const int ky = ky0 + r / tw, kx = kx0 + r % tw;
                 const int j0 = ref_pos(ky, a.step, bottom), i0 = ref_pos(kx, a.step, right);
-                n = match_block<T, KS>(a, t, j0, i0, lane, keys, heap, list, lkeys, n_cand, n_fix);
+                n = match_block<T, KS>(a, t, j0, i0, lane, dist, heap, list, lkeys, n_cand, n_fix);
                 n_sum += n;
                 n_sq += static_cast<unsigned>(n * n);
                 dump_group(a, ky, kx, n, lane, list, lkeys);

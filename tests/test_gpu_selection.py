@@ -1,0 +1,64 @@
+"""Group selection at the edges of its paths, against the oracle.
+
+The search list of a reference block is selected through a cut on distances,
+a compacted set ranked by counting, and three rarer paths: equal keys, more
+candidates under the cut than the compacted set holds, and keys outside the
+normal range. Groups (positions, order and keys) equal the oracle's exactly:
+both sides evaluate the same correctly rounded operations.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx(bm3d_lib):
+    import isp_mw_b200
+    c = isp_mw_b200.Context(0)
+    yield c
+    c.close()
+
+
+def _plane(kind, h=60, w=53):
+    from isp_mw_b200 import synth
+    noisy = synth.pair(h, w, 20.0, 17)[1]
+    y, x = np.mgrid[0:h, 0:w].astype(np.float32)
+    if kind == "quantised":   # equal keys everywhere
+        return (np.round(noisy * 10) / 10).astype(np.float32)
+    if kind == "columns":     # the best candidates share a column (or a row below)
+        return (np.sin(x) + 0.02 * noisy).astype(np.float32)
+    if kind == "rows":
+        return (np.sin(y) + 0.02 * noisy).astype(np.float32)
+    if kind == "flat":        # many candidates at nearly the cut
+        return (0.5 + 1e-6 * noisy).astype(np.float32)
+    return noisy
+
+
+# list lengths below, at and above the 384 places held in registers
+# (BMrange 9: 362, 10: 442), groups around the one / two minima rule (17, 18)
+@pytest.mark.parametrize("bm_range,group_size", [(1, 16), (9, 2), (9, 16), (9, 17), (9, 18),
+                                                 (10, 16), (16, 32), (20, 32)])
+@pytest.mark.parametrize("kind", ["noisy", "quantised", "columns", "rows", "flat"])
+def test_groups_equal_oracle(ctx, oracle_mod, bm_range, group_size, kind):
+    import isp_mw_b200
+    p = isp_mw_b200.stage_params_default("fast", False, [30.0] * 3)
+    p.bm_range, p.group_size = bm_range, group_size
+    _check(ctx, oracle_mod, p, _plane(kind), 1.0)
+
+
+@pytest.mark.parametrize("value_range", [1e-18, 1e18])
+def test_keys_outside_the_normal_range(ctx, oracle_mod, value_range):
+    """A plane far below its nominal range: keys round to few values or none."""
+    import isp_mw_b200
+    p = isp_mw_b200.stage_params_default("fast", False, [30.0] * 3)
+    _check(ctx, oracle_mod, p, _plane("noisy"), value_range)
+
+
+def _check(ctx, oracle_mod, p, plane, value_range):
+    count, pos, keys = ctx.debug_groups(p, False, plane, value_range)
+    want = oracle_mod.backend("port", np.float32).groups(False, p.as_dict(), plane, value_range)
+    assert np.array_equal(count, want[0])
+    for r, n in enumerate(count):
+        assert np.array_equal(pos[r, :n], want[1][r, :n]), r
+        assert np.array_equal(keys[r, :n], want[2][r, :n]), r
