@@ -58,10 +58,10 @@ __device__ __forceinline__ void zinv_n(T (&a)[kGSMax], T (&b)[kGSMax])
     redft01_pair<T, N>(a, b, DctTab<T>::inv() + O);
 }
 
-template <typename T>
-__device__ __forceinline__ void zbfly8(T (&a)[kGSMax], bool inverse)
+template <typename V>
+__device__ __forceinline__ void zbfly8(V (&a)[kGSMax], bool inverse)
 {
-    T t[8];
+    V t[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) t[i] = a[i];
     if (inverse) redft01_8(t);
@@ -693,14 +693,22 @@ template <> struct Vec4<float> {
     {
         *reinterpret_cast<float4 *>(p) = make_float4(a, b, c, d);
     }
-    static __device__ __forceinline__ void load2(const float *p, float &a, float &b)
+    static __device__ __forceinline__ Pair<float> load2(const float *p)
     {
-        const float2 v = *reinterpret_cast<const float2 *>(p);
-        a = v.x; b = v.y;
+        return Pair<float>{*reinterpret_cast<const unsigned long long *>(p)};
     }
-    static __device__ __forceinline__ void store2(float *p, float a, float b)
+    static __device__ __forceinline__ void store2(float *p, Pair<float> v)
     {
-        *reinterpret_cast<float2 *>(p) = make_float2(a, b);
+        *reinterpret_cast<unsigned long long *>(p) = v.v;
+    }
+    static __device__ __forceinline__ void load4(const float *p, Pair<float> &a, Pair<float> &b)
+    {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(p);
+        a.v = v.x; b.v = v.y;
+    }
+    static __device__ __forceinline__ void store4(float *p, Pair<float> a, Pair<float> b)
+    {
+        *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(a.v, b.v);
     }
 };
 template <> struct Vec4<double> {
@@ -716,14 +724,24 @@ template <> struct Vec4<double> {
         reinterpret_cast<double2 *>(p)[0] = make_double2(a, b);
         reinterpret_cast<double2 *>(p)[1] = make_double2(c, d);
     }
-    static __device__ __forceinline__ void load2(const double *p, double &a, double &b)
+    static __device__ __forceinline__ Pair<double> load2(const double *p)
     {
         const double2 v = *reinterpret_cast<const double2 *>(p);
-        a = v.x; b = v.y;
+        return Pair<double>{v.x, v.y};
     }
-    static __device__ __forceinline__ void store2(double *p, double a, double b)
+    static __device__ __forceinline__ void store2(double *p, Pair<double> v)
     {
-        *reinterpret_cast<double2 *>(p) = make_double2(a, b);
+        *reinterpret_cast<double2 *>(p) = make_double2(v.a, v.b);
+    }
+    static __device__ __forceinline__ void load4(const double *p, Pair<double> &a, Pair<double> &b)
+    {
+        a = load2(p);
+        b = load2(p + 2);
+    }
+    static __device__ __forceinline__ void store4(double *p, Pair<double> a, Pair<double> b)
+    {
+        store2(p, a);
+        store2(p + 2, b);
     }
 };
 
@@ -756,15 +774,13 @@ __device__ __forceinline__ void gather_xy_forward(const Tile<T> &t, const T *win
     }
     __syncwarp();
     if (z < n) {
-        T col[4][8];
+        Pair<T> c01[8], c23[8];  // columns 4h, 4h + 1 and 4h + 2, 4h + 3
 #pragma unroll
-        for (int y = 0; y < 8; ++y)
-            Vec4<T>::load(gz + gidx(y, 4 * h), col[0][y], col[1][y], col[2][y], col[3][y]);
+        for (int y = 0; y < 8; ++y) Vec4<T>::load4(gz + gidx(y, 4 * h), c01[y], c23[y]);
+        redft10_8(c01);
+        redft10_8(c23);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) redft10_8(col[c]);
-#pragma unroll
-        for (int y = 0; y < 8; ++y)
-            Vec4<T>::store(gz + gidx(y, 4 * h), col[0][y], col[1][y], col[2][y], col[3][y]);
+        for (int y = 0; y < 8; ++y) Vec4<T>::store4(gz + gidx(y, 4 * h), c01[y], c23[y]);
     }
     __syncwarp();
 }
@@ -776,15 +792,13 @@ __device__ __forceinline__ void xy_inverse_cols(T *G, int n, int lane)
     const int z = lane >> 1, h = lane & 1;
     T *gz = G + z * kGroupStride;
     if (z < n) {
-        T col[4][8];
+        Pair<T> c01[8], c23[8];  // columns 4h, 4h + 1 and 4h + 2, 4h + 3
 #pragma unroll
-        for (int y = 0; y < 8; ++y)
-            Vec4<T>::load(gz + gidx(y, 4 * h), col[0][y], col[1][y], col[2][y], col[3][y]);
+        for (int y = 0; y < 8; ++y) Vec4<T>::load4(gz + gidx(y, 4 * h), c01[y], c23[y]);
+        redft01_8(c01);
+        redft01_8(c23);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) redft01_8(col[c]);
-#pragma unroll
-        for (int y = 0; y < 8; ++y)
-            Vec4<T>::store(gz + gidx(y, 4 * h), col[0][y], col[1][y], col[2][y], col[3][y]);
+        for (int y = 0; y < 8; ++y) Vec4<T>::store4(gz + gidx(y, 4 * h), c01[y], c23[y]);
     }
     __syncwarp();
 }
@@ -794,26 +808,21 @@ __device__ __forceinline__ void xy_inverse_cols(T *G, int n, int lane)
 __device__ __forceinline__ int pencil_off(int lane) { return gidx(lane >> 2, 2 * (lane & 3)); }
 
 template <typename T>
-__device__ __forceinline__ void load_pencils(const T *G, int n, int lane, T (&a)[kGSMax],
-                                             T (&b)[kGSMax])
-{
-    const int o = pencil_off(lane);
-#pragma unroll
-    for (int z = 0; z < kGSMax; ++z) {
-        a[z] = T(0);
-        b[z] = T(0);
-        if (z < n) Vec4<T>::load2(G + z * kGroupStride + o, a[z], b[z]);
-    }
-}
-
-template <typename T>
-__device__ __forceinline__ void store_pencils(T *G, int n, int lane, const T (&a)[kGSMax],
-                                              const T (&b)[kGSMax])
+__device__ __forceinline__ void load_pencils(const T *G, int n, int lane, Pair<T> (&p)[kGSMax])
 {
     const int o = pencil_off(lane);
 #pragma unroll
     for (int z = 0; z < kGSMax; ++z)
-        if (z < n) Vec4<T>::store2(G + z * kGroupStride + o, a[z], b[z]);
+        p[z] = z < n ? Vec4<T>::load2(G + z * kGroupStride + o) : Pair<T>::make(T(0), T(0));
+}
+
+template <typename T>
+__device__ __forceinline__ void store_pencils(T *G, int n, int lane, const Pair<T> (&p)[kGSMax])
+{
+    const int o = pencil_off(lane);
+#pragma unroll
+    for (int z = 0; z < kGSMax; ++z)
+        if (z < n) Vec4<T>::store2(G + z * kGroupStride + o, p[z]);
 }
 
 // Group-axis transform of the lane's two pencils for the FP32 lengths other
@@ -821,9 +830,10 @@ __device__ __forceinline__ void store_pencils(T *G, int n, int lane, const T (&a
 // order, one runtime loop for every such length (a compact body: groups of
 // varied lengths would otherwise run many unrolled bodies at once).
 __device__ __forceinline__ void zgen(const float *G, int n, int lane, const float *m,
-                                     float (&a)[kGSMax], float (&b)[kGSMax])
+                                     Pair<float> (&p)[kGSMax])
 {
     const int o = pencil_off(lane);
+    float a[kGSMax], b[kGSMax];
 #pragma unroll
     for (int k = 0; k < kGSMax; ++k) {
         a[k] = 0.0f;
@@ -831,8 +841,8 @@ __device__ __forceinline__ void zgen(const float *G, int n, int lane, const floa
     }
 #pragma unroll 1
     for (int j = 0; j < n; ++j) {
-        float xa, xb;
-        Vec4<float>::load2(G + j * kGroupStride + o, xa, xb);
+        const Pair<float> x = Vec4<float>::load2(G + j * kGroupStride + o);
+        const float xa = x.lo(), xb = x.hi();
         const float *mj = m + 16 * j;
 #pragma unroll
         for (int k = 0; k < kGSMax; ++k) {
@@ -840,53 +850,69 @@ __device__ __forceinline__ void zgen(const float *G, int n, int lane, const floa
             b[k] = fmaf(mj[k], xb, b[k]);
         }
     }
+#pragma unroll
+    for (int k = 0; k < kGSMax; ++k) p[k] = Pair<float>::make(a[k], b[k]);
+}
+
+// The compile-time lengths of FP64 on separate pencils.
+template <bool INV>
+__device__ __forceinline__ void zdct2(Pair<double> (&p)[kGSMax], int n)
+{
+    double a[kGSMax], b[kGSMax];
+#pragma unroll
+    for (int k = 0; k < kGSMax; ++k) {
+        a[k] = p[k].a;
+        b[k] = p[k].b;
+    }
+    if constexpr (INV) zdct_inv2(a, b, n);
+    else zdct_fwd2(a, b, n);
+#pragma unroll
+    for (int k = 0; k < kGSMax; ++k) p[k] = Pair<double>{a[k], b[k]};
 }
 
 // Forward group-axis transform of the pencils held in the group buffer.
 template <typename T>
-__device__ __forceinline__ void group_fwd(T *G, int n, int lane, T (&a)[kGSMax], T (&b)[kGSMax])
+__device__ __forceinline__ void group_fwd(T *G, int n, int lane, Pair<T> (&p)[kGSMax])
 {
     if constexpr (sizeof(T) == 4) {
-        if (n != 16 && n != 8) {
-            zgen(G, n, lane, c_dct_pad_fwd + pad_table_offset(n), a, b);
-            return;
-        }
-        load_pencils(G, n, lane, a, b);
         if (n == 16) {
-            redft10_16(a);
-            redft10_16(b);
+            load_pencils(G, 16, lane, p);
+            redft10_16(p);
+        } else if (n == 8) {
+            load_pencils(G, 8, lane, p);
+            zbfly8(p, false);
         } else {
-            zbfly8(a, false);
-            zbfly8(b, false);
+            zgen(G, n, lane, c_dct_pad_fwd + pad_table_offset(n), p);
         }
     } else {
-        load_pencils(G, n, lane, a, b);
-        zdct_fwd2(a, b, n);
+        load_pencils(G, n, lane, p);
+        zdct2<false>(p, n);
     }
 }
 
 // Inverse group-axis transform; the result is left in the group buffer.
 template <typename T>
-__device__ __forceinline__ void group_inv(T *G, int n, int lane, T (&a)[kGSMax], T (&b)[kGSMax])
+__device__ __forceinline__ void group_inv(T *G, int n, int lane, Pair<T> (&p)[kGSMax])
 {
     if constexpr (sizeof(T) == 4) {
-        if (n != 16 && n != 8) {
-            store_pencils(G, n, lane, a, b);
+        if (n == 16) {
+            redft01_16(p);
             __syncwarp();
-            zgen(G, n, lane, c_dct_pad_inv + pad_table_offset(n), a, b);
-            __syncwarp();
-        } else if (n == 16) {
-            redft01_16(a);
-            redft01_16(b);
+            store_pencils(G, 16, lane, p);
+            return;
+        }
+        if (n == 8) {
+            zbfly8(p, true);
         } else {
-            zbfly8(a, true);
-            zbfly8(b, true);
+            store_pencils(G, n, lane, p);
+            __syncwarp();
+            zgen(G, n, lane, c_dct_pad_inv + pad_table_offset(n), p);
         }
     } else {
-        zdct_inv2(a, b, n);
+        zdct2<true>(p, n);
     }
     __syncwarp();
-    store_pencils(G, n, lane, a, b);
+    store_pencils(G, n, lane, p);
 }
 
 // Empirical Wiener weight y^2 / (y^2 + sigma^2) (source/BM3D.cpp:440); the
@@ -955,21 +981,20 @@ __device__ void filter_group(const StageArgs<T> &a, const Tile<T> &t, int p, con
     // p indexes the tile's windows; pt (default p) the plane's threshold /
     // Wiener tables, which differ when planes share one set of windows
     if (pt < 0) pt = p;
-    T sa[kGSMax], sb[kGSMax];
-    T ra[kGSMax], rb[kGSMax];
+    Pair<T> sp[kGSMax], rp[kGSMax];  // the lane's two pencils of src and ref
     if (WIENER) {
         gather_xy_forward(t, t.refw[p], t.ref0[p], list, n, lane, G, n_bad);
-        group_fwd(G, n, lane, ra, rb);
+        group_fwd(G, n, lane, rp);
         __syncwarp();
     }
     gather_xy_forward(t, t.srcw[p], t.src0[p], list, n, lane, G, n_bad);
-    group_fwd(G, n, lane, sa, sb);
+    group_fwd(G, n, lane, sp);
 
     T denW;
     if (!WIENER) {
         // Hard threshold: |x| <= thr -> 0, else retained (source/BM3D.cpp:361-371).
         // thr depends on how many of (x, y, z) are 0 (source/BM3D.cpp:52-67).
-        // pencil a = (lane / 4, 2 (lane % 4)), pencil b = (lane / 4, 2 (lane % 4) + 1)
+        // pencil lo = (lane / 4, 2 (lane % 4)), pencil hi = (lane / 4, 2 (lane % 4) + 1)
         const int fa = ((lane & 3) == 0) + (lane < 4), fb = (lane < 4);
         const T *thr = a.thr[pt][n - 1];
         int kept = 0;
@@ -977,10 +1002,11 @@ __device__ void filter_group(const StageArgs<T> &a, const Tile<T> &t, int p, con
         for (int z = 0; z < kGSMax; ++z) {
             if (z < n) {
                 const T ta = thr[fa + (z == 0)], tb = thr[fb + (z == 0)];
-                const T va = sa[z], vb = sb[z];
+                T va = sp[z].lo(), vb = sp[z].hi();
                 const T aa = va < T(0) ? -va : va, ab = vb < T(0) ? -vb : vb;
-                if (aa <= ta) sa[z] = T(0); else ++kept;
-                if (ab <= tb) sb[z] = T(0); else ++kept;
+                if (aa <= ta) va = T(0); else ++kept;
+                if (ab <= tb) vb = T(0); else ++kept;
+                sp[z] = Pair<T>::make(va, vb);
             }
         }
         const int retained = __reduce_add_sync(0xffffffffu, kept);
@@ -993,10 +1019,10 @@ __device__ void filter_group(const StageArgs<T> &a, const Tile<T> &t, int p, con
 #pragma unroll
         for (int z = 0; z < kGSMax; ++z) {
             if (z < n) {
-                const T ya2 = ra[z] * ra[z], yb2 = rb[z] * rb[z];
+                const T ra = rp[z].lo(), rb = rp[z].hi();
+                const T ya2 = ra * ra, yb2 = rb * rb;
                 const T wa = wiener_weight(ya2, s2), wb = wiener_weight(yb2, s2);
-                sa[z] *= wa;
-                sb[z] *= wb;
+                sp[z] = vmul(sp[z], Pair<T>::make(wa, wb));
                 l2 += wa * wa + wb * wb;
             }
         }
@@ -1005,7 +1031,7 @@ __device__ void filter_group(const StageArgs<T> &a, const Tile<T> &t, int p, con
     }
     const T numW = static_cast<T>(static_cast<double>(denW) / a.finalAMP[n - 1]);
 
-    group_inv(G, n, lane, sa, sb);
+    group_inv(G, n, lane, sp);
     __syncwarp();
     xy_inverse_cols(G, n, lane);
 

@@ -29,46 +29,176 @@ namespace bm3d {
 #define BM3D_C16_6 0.7653668647301797
 #define BM3D_C16_7 0.39018064403225666
 
-// REDFT10 of length 8, in place.
-template <typename T>
-__host__ __device__ __forceinline__ void redft10_8(T (&x)[8])
+// Two values that go through the same operations: FP32 pairs are one 64-bit
+// register pair worked by the packed f32x2 instructions, each half rounded
+// like the scalar operation; FP64 pairs are two doubles. A packed instruction
+// takes one issue slot for two results (the FP32 pipe still spends two cycles
+// on it), which is what pays in kernels that wait for issue slots: with the
+columns and the group axis of the 8 x 8 x 16 groups in pairs the final stage
+issues 268 -> 247 M warp instructions at 1080p and takes 0.427 -> 0.402 ms.
+template <typename T> struct Pair {
+    T a, b;
+    __host__ __device__ __forceinline__ T lo() const { return a; }
+    __host__ __device__ __forceinline__ T hi() const { return b; }
+    static __host__ __device__ __forceinline__ Pair make(T x, T y) { return Pair{x, y}; }
+};
+#ifdef __CUDACC__
+template <> struct Pair<float> {
+    unsigned long long v;
+    __device__ __forceinline__ float lo() const
+    {
+        float x, y;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+        return x;
+    }
+    __device__ __forceinline__ float hi() const
+    {
+        float x, y;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+        return y;
+    }
+    static __device__ __forceinline__ Pair make(float x, float y)
+    {
+        Pair p;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(p.v) : "f"(x), "f"(y));
+        return p;
+    }
+};
+#endif
+
+// The operations of the butterflies on one value or a pair: sums, a constant
+// times a value, and constant * x + y rounded once (on the host, where only
+// tests run them, rounded twice).
+template <typename T> __host__ __device__ __forceinline__ T vadd(T x, T y) { return x + y; }
+template <typename T> __host__ __device__ __forceinline__ T vsub(T x, T y) { return x - y; }
+#ifdef __CUDA_ARCH__
+__device__ __forceinline__ float vmul(double c, float x) { return __fmul_rn(static_cast<float>(c), x); }
+__device__ __forceinline__ double vmul(double c, double x) { return __dmul_rn(c, x); }
+__device__ __forceinline__ float vfma(double c, float x, float y)
 {
-    const T C1 = T(BM3D_C16_1), C2 = T(BM3D_C16_2), C3 = T(BM3D_C16_3), C4 = T(BM3D_C16_4);
-    const T C5 = T(BM3D_C16_5), C6 = T(BM3D_C16_6), C7 = T(BM3D_C16_7);
-    const T u0 = x[0] + x[7], u1 = x[1] + x[6], u2 = x[2] + x[5], u3 = x[3] + x[4];
-    const T v0 = x[0] - x[7], v1 = x[1] - x[6], v2 = x[2] - x[5], v3 = x[3] - x[4];
-    const T a = u0 + u3, b = u1 + u2, c = u0 - u3, d = u1 - u2;
-    x[0] = T(2) * (a + b);
-    x[4] = C4 * (a - b);
-    x[2] = C2 * c + C6 * d;
-    x[6] = C6 * c - C2 * d;
-    x[1] = C1 * v0 + C3 * v1 + C5 * v2 + C7 * v3;
-    x[3] = C3 * v0 - C7 * v1 - C1 * v2 - C5 * v3;
-    x[5] = C5 * v0 - C1 * v1 + C7 * v2 + C3 * v3;
-    x[7] = C7 * v0 - C5 * v1 + C3 * v2 - C1 * v3;
+    return __fmaf_rn(static_cast<float>(c), x, y);
+}
+__device__ __forceinline__ double vfma(double c, double x, double y) { return __fma_rn(c, x, y); }
+#else
+template <typename T> __host__ __device__ inline T vmul(double c, T x) { return static_cast<T>(c) * x; }
+template <typename T> __host__ __device__ inline T vfma(double c, T x, T y)
+{
+    return static_cast<T>(c) * x + y;
+}
+#endif
+#ifdef __CUDACC__
+__device__ __forceinline__ Pair<double> vadd(Pair<double> x, Pair<double> y) { return {x.a + y.a, x.b + y.b}; }
+__device__ __forceinline__ Pair<double> vsub(Pair<double> x, Pair<double> y) { return {x.a - y.a, x.b - y.b}; }
+__device__ __forceinline__ Pair<double> vmul(double c, Pair<double> x)
+{
+    return {vmul(c, x.a), vmul(c, x.b)};
+}
+__device__ __forceinline__ Pair<double> vfma(double c, Pair<double> x, Pair<double> y)
+{
+    return {vfma(c, x.a, y.a), vfma(c, x.b, y.b)};
+}
+__device__ __forceinline__ Pair<float> vadd(Pair<float> x, Pair<float> y)
+{
+    Pair<float> r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(x.v), "l"(y.v));
+    return r;
+}
+__device__ __forceinline__ Pair<float> vsub(Pair<float> x, Pair<float> y)
+{
+    Pair<float> r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(x.v), "l"(y.v));
+    return r;
+}
+__device__ __forceinline__ Pair<float> vmul(Pair<float> x, Pair<float> y)
+{
+    Pair<float> r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(x.v), "l"(y.v));
+    return r;
+}
+__device__ __forceinline__ Pair<double> vmul(Pair<double> x, Pair<double> y)
+{
+    return {x.a * y.a, x.b * y.b};
+}
+__device__ __forceinline__ Pair<float> vmul(double c, Pair<float> x)
+{
+    return vmul(Pair<float>::make(static_cast<float>(c), static_cast<float>(c)), x);
+}
+__device__ __forceinline__ Pair<float> vfma(double c, Pair<float> x, Pair<float> y)
+{
+    Pair<float> r;
+    const Pair<float> k = Pair<float>::make(static_cast<float>(c), static_cast<float>(c));
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(k.v), "l"(x.v), "l"(y.v));
+    return r;
+}
+#endif
+
+// c0 x0 + c1 x1 + c2 x2 + c3 x3 and c0 x0 + c1 x1, in this order of rounding.
+template <typename V>
+__host__ __device__ __forceinline__ V vdot4(double c0, V x0, double c1, V x1, double c2, V x2,
+                                            double c3, V x3)
+{
+    return vfma(c3, x3, vfma(c2, x2, vfma(c0, x0, vmul(c1, x1))));
+}
+template <typename V> __host__ __device__ __forceinline__ V vdot2(double c0, V x0, double c1, V x1)
+{
+    return vfma(c0, x0, vmul(c1, x1));
 }
 
-// REDFT01 of length 8, in place.
-template <typename T>
-__host__ __device__ __forceinline__ void redft01_8(T (&x)[8])
+// REDFT10 of length 8 from the sums u_j = x_j + x_{7-j} and differences
+// v_j = x_j - x_{7-j} (V: a value or a Pair). Returns the fourth output before
+// its scale 2 cos(pi / 4), for sums that take the scale in.
+template <typename V>
+__host__ __device__ __forceinline__ V redft10_8_uv(const V (&u)[4], const V (&v)[4], V (&x)[8])
 {
-    const T C1 = T(BM3D_C16_1), C2 = T(BM3D_C16_2), C3 = T(BM3D_C16_3), C4 = T(BM3D_C16_4);
-    const T C5 = T(BM3D_C16_5), C6 = T(BM3D_C16_6), C7 = T(BM3D_C16_7);
-    const T p = x[0] + C4 * x[4], q = x[0] - C4 * x[4];
-    const T s = C2 * x[2] + C6 * x[6], t = C6 * x[2] - C2 * x[6];
-    const T e0 = p + s, e3 = p - s, e1 = q + t, e2 = q - t;
-    const T o0 = C1 * x[1] + C3 * x[3] + C5 * x[5] + C7 * x[7];
-    const T o1 = C3 * x[1] - C7 * x[3] - C1 * x[5] - C5 * x[7];
-    const T o2 = C5 * x[1] - C1 * x[3] + C7 * x[5] + C3 * x[7];
-    const T o3 = C7 * x[1] - C5 * x[3] + C3 * x[5] - C1 * x[7];
-    x[0] = e0 + o0;
-    x[7] = e0 - o0;
-    x[1] = e1 + o1;
-    x[6] = e1 - o1;
-    x[2] = e2 + o2;
-    x[5] = e2 - o2;
-    x[3] = e3 + o3;
-    x[4] = e3 - o3;
+    constexpr double C1 = BM3D_C16_1, C2 = BM3D_C16_2, C3 = BM3D_C16_3, C4 = BM3D_C16_4;
+    constexpr double C5 = BM3D_C16_5, C6 = BM3D_C16_6, C7 = BM3D_C16_7;
+    const V a = vadd(u[0], u[3]), b = vadd(u[1], u[2]), c = vsub(u[0], u[3]), d = vsub(u[1], u[2]);
+    const V e = vsub(a, b);
+    x[0] = vmul(2.0, vadd(a, b));
+    x[4] = vmul(C4, e);
+    x[2] = vdot2(C6, d, C2, c);
+    x[6] = vdot2(C6, c, -C2, d);
+    x[1] = vdot4(C1, v[0], C3, v[1], C5, v[2], C7, v[3]);
+    x[3] = vdot4(C3, v[0], -C7, v[1], -C1, v[2], -C5, v[3]);
+    x[5] = vdot4(C5, v[0], -C1, v[1], C7, v[2], C3, v[3]);
+    x[7] = vdot4(C7, v[0], -C5, v[1], C3, v[2], -C1, v[3]);
+    return e;
+}
+
+// REDFT10 of length 8, in place.
+template <typename V> __host__ __device__ __forceinline__ V redft10_8_e(V (&x)[8])
+{
+    V u[4], v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        u[j] = vadd(x[j], x[7 - j]);
+        v[j] = vsub(x[j], x[7 - j]);
+    }
+    return redft10_8_uv(u, v, x);
+}
+template <typename V> __host__ __device__ __forceinline__ void redft10_8(V (&x)[8]) { redft10_8_e(x); }
+
+// REDFT01 of length 8, in place.
+template <typename V>
+__host__ __device__ __forceinline__ void redft01_8(V (&x)[8])
+{
+    constexpr double C1 = BM3D_C16_1, C2 = BM3D_C16_2, C3 = BM3D_C16_3, C4 = BM3D_C16_4;
+    constexpr double C5 = BM3D_C16_5, C6 = BM3D_C16_6, C7 = BM3D_C16_7;
+    const V p = vfma(C4, x[4], x[0]), q = vfma(-C4, x[4], x[0]);
+    const V s = vdot2(C2, x[2], C6, x[6]), t = vdot2(C6, x[2], -C2, x[6]);
+    const V e0 = vadd(p, s), e3 = vsub(p, s), e1 = vadd(q, t), e2 = vsub(q, t);
+    const V o0 = vdot4(C1, x[1], C3, x[3], C5, x[5], C7, x[7]);
+    const V o1 = vdot4(C3, x[1], -C7, x[3], -C1, x[5], -C5, x[7]);
+    const V o2 = vdot4(C5, x[1], -C1, x[3], C7, x[5], C3, x[7]);
+    const V o3 = vdot4(C7, x[1], -C5, x[3], C3, x[5], -C1, x[7]);
+    x[0] = vadd(e0, o0);
+    x[7] = vsub(e0, o0);
+    x[1] = vadd(e1, o1);
+    x[6] = vsub(e1, o1);
+    x[2] = vadd(e2, o2);
+    x[5] = vsub(e2, o2);
+    x[3] = vadd(e3, o3);
+    x[4] = vsub(e3, o3);
 }
 
 // D16[m][j] = 2 cos(pi (2j+1)(2m+1) / 32): odd half of the 16-point transforms.
@@ -83,47 +213,47 @@ __host__ __device__ __forceinline__ void redft01_8(T (&x)[8])
      {0.19603428065912154, -0.5805693545089249, 0.942793473651996, -1.2687865683272908, 1.5460209067254753, -1.7638425286967123, 1.9138806714644168, -1.990369453344394}}
 
 // REDFT10 of length 16, in place.
-template <typename T>
-__host__ __device__ __forceinline__ void redft10_16(T (&x)[16])
+template <typename V>
+__host__ __device__ __forceinline__ void redft10_16(V (&x)[16])
 {
     constexpr double D[8][8] = BM3D_D16;
-    T u[8], v[8];
+    V u[8], v[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        u[j] = x[j] + x[15 - j];
-        v[j] = x[j] - x[15 - j];
+        u[j] = vadd(x[j], x[15 - j]);
+        v[j] = vsub(x[j], x[15 - j]);
     }
     redft10_8(u);
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
-        T acc = T(D[m][0]) * v[0];
+        V acc = vdot2(D[m][0], v[0], D[m][1], v[1]);
 #pragma unroll
-        for (int j = 1; j < 8; ++j) acc += T(D[m][j]) * v[j];
+        for (int j = 2; j < 8; ++j) acc = vfma(D[m][j], v[j], acc);
         x[2 * m + 1] = acc;
         x[2 * m] = u[m];
     }
 }
 
 // REDFT01 of length 16, in place.
-template <typename T>
-__host__ __device__ __forceinline__ void redft01_16(T (&x)[16])
+template <typename V>
+__host__ __device__ __forceinline__ void redft01_16(V (&x)[16])
 {
     constexpr double D[8][8] = BM3D_D16;
-    T e[8], o[8];
+    V e[8], o[8];
 #pragma unroll
     for (int m = 0; m < 8; ++m) e[m] = x[2 * m];
     redft01_8(e);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-        T acc = T(D[0][k]) * x[1];
+        V acc = vdot2(D[0][k], x[1], D[1][k], x[3]);
 #pragma unroll
-        for (int m = 1; m < 8; ++m) acc += T(D[m][k]) * x[2 * m + 1];
+        for (int m = 2; m < 8; ++m) acc = vfma(D[m][k], x[2 * m + 1], acc);
         o[k] = acc;
     }
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-        x[k] = e[k] + o[k];
-        x[15 - k] = e[k] - o[k];
+        x[k] = vadd(e[k], o[k]);
+        x[15 - k] = vsub(e[k], o[k]);
     }
 }
 
@@ -150,38 +280,68 @@ __host__ __device__ __forceinline__ void redft01_16(T (&x)[16])
      0.7445362710022986, 0.8393496454155268, 0.9725682378619608, 1.1694399334328847, \
      1.4841646163141662, 2.057781009953411, 3.407608418468719, 10.190008123548033}
 
-template <typename T, int N> __host__ __device__ __forceinline__ void redft10_pow2(T (&x)[N]);
+// REDFT11 (DCT-IV) of length 8, in place. The pre-scales go into the first
+// sums and the scale of output 4 into the last ones (one rounding each).
+template <typename V> __host__ __device__ __forceinline__ void redft11_8(V (&v)[8])
+{
+    constexpr double S[8] = BM3D_S11_8;
+    V u[4], w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        u[j] = vdot2(S[j], v[j], S[7 - j], v[7 - j]);
+        w[j] = vdot2(S[j], v[j], -S[7 - j], v[7 - j]);
+    }
+    const V e = redft10_8_uv(u, w, v);
+#pragma unroll
+    for (int k = 0; k < 7; ++k)
+        v[k] = k == 3 ? vfma(BM3D_C16_4, e, v[3]) : k == 4 ? vfma(BM3D_C16_4, e, v[5]) : vadd(v[k], v[k + 1]);
+}
 
-// REDFT11 (DCT-IV) of length H = 8 or 16, in place.
-template <typename T, int H>
-__host__ __device__ __forceinline__ void redft11_pow2(T (&v)[H])
+// REDFT11 of length 16, in place, likewise.
+template <typename V> __host__ __device__ __forceinline__ void redft11_16(V (&x)[16])
+{
+    constexpr double S[16] = BM3D_S11_16;
+    V u[8], v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        u[j] = vdot2(S[j], x[j], S[15 - j], x[15 - j]);
+        v[j] = vdot2(S[j], x[j], -S[15 - j], x[15 - j]);
+    }
+    const V e = redft10_8_e(u);
+    redft11_8(v);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+        x[2 * m] = u[m];
+        x[2 * m + 1] = v[m];
+    }
+#pragma unroll
+    for (int k = 0; k < 15; ++k)
+        x[k] = k == 7 ? vfma(BM3D_C16_4, e, x[7]) : k == 8 ? vfma(BM3D_C16_4, e, x[9]) : vadd(x[k], x[k + 1]);
+}
+
+template <typename V, int H> __host__ __device__ __forceinline__ void redft11_pow2(V (&v)[H])
 {
     static_assert(H == 8 || H == 16, "DCT-IV lengths 8 and 16");
-    constexpr double S8[8] = BM3D_S11_8;
-    constexpr double S16[16] = BM3D_S11_16;
-#pragma unroll
-    for (int j = 0; j < H; ++j) v[j] *= T(H == 8 ? S8[j] : S16[j]);
-    redft10_pow2<T, H>(v);
-#pragma unroll
-    for (int k = 0; k < H - 1; ++k) v[k] += v[k + 1];
+    if constexpr (H == 8) redft11_8(v);
+    else redft11_16(v);
 }
 
 // REDFT10 of length N = 8, 16 or 32, in place.
-template <typename T, int N>
-__host__ __device__ __forceinline__ void redft10_pow2(T (&x)[N])
+template <typename V, int N>
+__host__ __device__ __forceinline__ void redft10_pow2(V (&x)[N])
 {
     if constexpr (N == 8) {
         redft10_8(x);
     } else {
         constexpr int H = N / 2;
-        T u[H], v[H];
+        V u[H], v[H];
 #pragma unroll
         for (int j = 0; j < H; ++j) {
-            u[j] = x[j] + x[N - 1 - j];
-            v[j] = x[j] - x[N - 1 - j];
+            u[j] = vadd(x[j], x[N - 1 - j]);
+            v[j] = vsub(x[j], x[N - 1 - j]);
         }
-        redft10_pow2<T, H>(u);
-        redft11_pow2<T, H>(v);
+        redft10_pow2<V, H>(u);
+        redft11_pow2<V, H>(v);
 #pragma unroll
         for (int m = 0; m < H; ++m) {
             x[2 * m] = u[m];
@@ -191,25 +351,25 @@ __host__ __device__ __forceinline__ void redft10_pow2(T (&x)[N])
 }
 
 // REDFT01 of length N = 8, 16 or 32, in place.
-template <typename T, int N>
-__host__ __device__ __forceinline__ void redft01_pow2(T (&x)[N])
+template <typename V, int N>
+__host__ __device__ __forceinline__ void redft01_pow2(V (&x)[N])
 {
     if constexpr (N == 8) {
         redft01_8(x);
     } else {
         constexpr int H = N / 2;
-        T e[H], o[H];
+        V e[H], o[H];
 #pragma unroll
         for (int m = 0; m < H; ++m) {
             e[m] = x[2 * m];
             o[m] = x[2 * m + 1];
         }
-        redft01_pow2<T, H>(e);
-        redft11_pow2<T, H>(o);
+        redft01_pow2<V, H>(e);
+        redft11_pow2<V, H>(o);
 #pragma unroll
         for (int j = 0; j < H; ++j) {
-            x[j] = e[j] + o[j];
-            x[N - 1 - j] = e[j] - o[j];
+            x[j] = vadd(e[j], o[j]);
+            x[N - 1 - j] = vsub(e[j], o[j]);
         }
     }
 }
