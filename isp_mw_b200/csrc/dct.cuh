@@ -34,8 +34,8 @@ namespace bm3d {
 // like the scalar operation; FP64 pairs are two doubles. A packed instruction
 // takes one issue slot for two results (the FP32 pipe still spends two cycles
 // on it), which is what pays in kernels that wait for issue slots: with the
-columns and the group axis of the 8 x 8 x 16 groups in pairs the final stage
-issues 268 -> 247 M warp instructions at 1080p and takes 0.427 -> 0.402 ms.
+// columns and the group axis of the 8 x 8 x 16 groups in pairs the final stage
+// issues 268 -> 247 M warp instructions at 1080p and takes 0.427 -> 0.402 ms.
 template <typename T> struct Pair {
     T a, b;
     __host__ __device__ __forceinline__ T lo() const { return a; }
