@@ -292,13 +292,16 @@ struct SmemPlan {
     int n_stage;                 // staged windows (src planes + separate ref planes)
     size_t region_bytes;         // one staged window
     size_t acc_bytes;            // one accumulator window
-    size_t off_acc;              // 2 * planes accumulator windows
+    size_t off_acc;              // an accumulator window (numerator sums) per plane
     size_t off_origin;           // block (0, 0) copies per staged window
     size_t off_origin_acc;       // block (0, 0) accumulators
     size_t off_warps;
     size_t warp_bytes;
-    size_t scratch_bytes;        // group buffer(s) / search list union at the start of a warp's area
-    size_t refblk_bytes;         // generic path: copy of the reference block
+    // within a warp's area: the group buffer(s) start at 0; before a group is
+    // gathered the same bytes hold the search list, the candidate / heap
+    // buffer (which holds the reference block while distances are computed)
+    // and the group's keys; the group list follows
+    size_t off_ref, off_heap, off_keys, off_list;
     size_t off_groups;           // three-plane register-resident path: the tile's group lists
     size_t total;
 };
@@ -351,22 +354,22 @@ __host__ __device__ inline SmemPlan plan_smem(int nplanes, bool wiener, int alia
     s.region_bytes = (static_cast<size_t>(region_h) * region_pitch * sizeof(T) + 15) / 16 * 16;
     s.acc_bytes = (static_cast<size_t>(region_h) * region_pitch * sizeof(Acc) + 15) / 16 * 16;
     s.off_acc = s.region_bytes * s.n_stage;
-    s.off_origin = s.off_acc + s.acc_bytes * 2 * nplanes;
+    s.off_origin = s.off_acc + s.acc_bytes * nplanes;
     // block (0, 0) copies: T per staged window, then (16-byte aligned) Acc per accumulator
     s.off_origin_acc = s.off_origin + (sizeof(T) * bsq * s.n_stage + 15) / 16 * 16;
-    s.off_warps = (s.off_origin_acc + sizeof(Acc) * bsq * 2 * nplanes + 15) / 16 * 16;
+    s.off_warps = (s.off_origin_acc + sizeof(Acc) * bsq * nplanes + 15) / 16 * 16;
     const size_t group_bytes = generic
         ? sizeof(T) * static_cast<size_t>(gs) * generic_block_stride(bs) *
               (wiener && !generic_one_buffer<T>(wiener, bs) ? 2 : 1)
         : sizeof(T) * kGSMax * kGroupStride;
     const size_t key_bytes = sizeof(T) * key_slots;  // distance bits
-    const size_t scratch = group_bytes > key_bytes ? group_bytes : key_bytes;
-    s.scratch_bytes = (scratch + 15) / 16 * 16;
-    s.refblk_bytes = generic ? (sizeof(T) * bsq + 15) / 16 * 16 : 0;
-    // scratch | reference block (generic) | candidate/heap buffer (kCand sort keys) |
-    // group list (kGSTab BlockPos) | group keys (kGSTab T)
-    s.warp_bytes = (s.scratch_bytes + s.refblk_bytes + sizeof(SortKey<T>) * kCand +
-                    sizeof(BlockPos) * kGSTab + sizeof(T) * kGSTab + 15) / 16 * 16;
+    const auto up = [](size_t v) { return (v + 15) / 16 * 16; };
+    const size_t heap_bytes = sizeof(SortKey<T>) * kCand, ref_bytes = sizeof(T) * bsq;
+    s.off_ref = s.off_heap = up(key_bytes);
+    s.off_keys = s.off_heap + up(heap_bytes > ref_bytes ? heap_bytes : ref_bytes);
+    const size_t match_bytes = s.off_keys + sizeof(T) * kGSTab;
+    s.off_list = up(group_bytes > match_bytes ? group_bytes : match_bytes);
+    s.warp_bytes = s.off_list + up(sizeof(BlockPos) * (gs > 1 ? gs : 1));
     s.off_groups = (s.off_warps + s.warp_bytes * nwarps + 15) / 16 * 16;
     const int glist = generic ? gs : kGSMax;  // group-list entries per reference block
     s.total = seq3 ? s.off_groups + static_cast<size_t>(tile_refs) * (2 * glist + 1)

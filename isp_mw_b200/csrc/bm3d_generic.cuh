@@ -336,7 +336,7 @@ __device__ __forceinline__ void aggregate_rows(const StageArgs<T> &a, const Tile
         if (!check && (q.y >= BS || q.x >= BS)) {
 #pragma unroll
             for (int x = 0; x < BS; ++x) acc_add(dn + x, v[x] * numW, scale);
-            if (y == 0) acc_add(block_ptr(t, t.accD[p], t.accD0[p], q.y, q.x, pitch), denW, scale);
+            if (y == 0) weight_add(a.den[pt], a.width, q.y, q.x, denW, scale);
         } else {
             const float scale_c = fixed_scale(a.absmax[pt], a.log2_corner);
             unsigned char *const poison = poison_map(a, pt);
@@ -350,7 +350,7 @@ __device__ __forceinline__ void aggregate_rows(const StageArgs<T> &a, const Tile
             if (y == 0) {
                 const float sd = (q.y == 0 && q.x == 0) ? scale_c : scale;
                 if (mk == nullptr || fabsf(static_cast<float>(denW) * sd) < kFixedLimit)
-                    acc_add(block_ptr(t, t.accD[p], t.accD0[p], q.y, q.x, pitch), denW, sd);
+                    weight_add(a.den[pt], a.width, q.y, q.x, denW, sd);
                 else  // the block's weight reaches all of its pixels
                     for (int i = 0; i < BS * BS; ++i)
                         mk[static_cast<long long>(i / BS) * a.width + i % BS] = 1;
@@ -522,7 +522,7 @@ __device__ void filter_generic(const StageArgs<T> &a, const Tile<T> &t, int p, c
         if (!check && (q.y >= bs || q.x >= bs)) {
             acc_add(dn + y * pitch + x, Gs[z * zs + y * rs + x] * numW, scale);
             if (y == 0 && x == 0)
-                acc_add(block_ptr(t, t.accD[p], t.accD0[p], q.y, q.x, pitch), denW, scale);
+                weight_add(a.den[pt], a.width, q.y, q.x, denW, scale);
         } else {
             // a member reaching block (0, 0)'s pixels (their own scale), or a plane
             // with non-finite pixels (per-term check, marks into the poison map)
@@ -537,7 +537,7 @@ __device__ void filter_generic(const StageArgs<T> &a, const Tile<T> &t, int p, c
             if (y == 0 && x == 0) {
                 const float sd = (q.y == 0 && q.x == 0) ? scale_c : scale;
                 if (mk == nullptr || fabsf(static_cast<float>(denW) * sd) < kFixedLimit)
-                    acc_add(block_ptr(t, t.accD[p], t.accD0[p], q.y, q.x, pitch), denW, sd);
+                    weight_add(a.den[pt], a.width, q.y, q.x, denW, sd);
                 else  // the block's weight reaches all of its pixels
                     for (int i = 0; i < bsq; ++i)
                         mk[static_cast<long long>(i / bs) * a.width + i % bs] = 1;
@@ -569,16 +569,14 @@ __device__ __forceinline__ void generic_tile_body(const StageArgs<T> &a, int til
     stage_tile<T, WIENER, NPL>(a, t);
 
     unsigned char *wbase = smem + sp.off_warps + sp.warp_bytes * warp;
-    const size_t scratch = sp.scratch_bytes;
     const int gvals = a.group_size * generic_block_stride(bs);
     T *Gs = reinterpret_cast<T *>(wbase);
     T *Gr = Gs + gvals;
     auto *dist = reinterpret_cast<typename DistBits<T>::type *>(wbase);
-    T *refblk = reinterpret_cast<T *>(wbase + scratch);
-    unsigned char *after = wbase + scratch + sp.refblk_bytes;
-    SortKey<T> *heap = reinterpret_cast<SortKey<T> *>(after);
-    BlockPos *list = reinterpret_cast<BlockPos *>(after + sizeof(SortKey<T>) * kCand);
-    T *lkeys = reinterpret_cast<T *>(after + sizeof(SortKey<T>) * kCand + sizeof(BlockPos) * kGSTab);
+    T *refblk = reinterpret_cast<T *>(wbase + sp.off_ref);
+    SortKey<T> *heap = reinterpret_cast<SortKey<T> *>(wbase + sp.off_heap);
+    T *lkeys = reinterpret_cast<T *>(wbase + sp.off_keys);
+    BlockPos *list = reinterpret_cast<BlockPos *>(wbase + sp.off_list);
 
     // per-tile counters (small: 32 bits suffice), flushed once per tile
     unsigned n_sum = 0, n_sq = 0, n_cand = 0, n_fix = 0, n_bad = 0;
@@ -647,15 +645,13 @@ __device__ __forceinline__ void generic_tile_body_seq3(const StageArgs<T> &a, in
     unsigned char *gn = reinterpret_cast<unsigned char *>(gpos + a.tile_x * a.tile_y * GS);
 
     unsigned char *wbase = smem + sp.off_warps + sp.warp_bytes * warp;
-    const size_t scratch = sp.scratch_bytes;
     T *Gs = reinterpret_cast<T *>(wbase);
     T *Gr = Gs + GS * generic_block_stride(bs);
     auto *dist = reinterpret_cast<typename DistBits<T>::type *>(wbase);
-    T *refblk = reinterpret_cast<T *>(wbase + scratch);
-    unsigned char *after = wbase + scratch + sp.refblk_bytes;
-    SortKey<T> *heap = reinterpret_cast<SortKey<T> *>(after);
-    BlockPos *list = reinterpret_cast<BlockPos *>(after + sizeof(SortKey<T>) * kCand);
-    T *lkeys = reinterpret_cast<T *>(after + sizeof(SortKey<T>) * kCand + sizeof(BlockPos) * kGSTab);
+    T *refblk = reinterpret_cast<T *>(wbase + sp.off_ref);
+    SortKey<T> *heap = reinterpret_cast<SortKey<T> *>(wbase + sp.off_heap);
+    T *lkeys = reinterpret_cast<T *>(wbase + sp.off_keys);
+    BlockPos *list = reinterpret_cast<BlockPos *>(wbase + sp.off_list);
 
     // per-tile counters (small: 32 bits suffice), flushed once per tile
     unsigned n_sum = 0, n_sq = 0, n_cand = 0, n_fix = 0, n_bad = 0;

@@ -130,8 +130,8 @@ template <typename T> struct Tile {
     const T *refw[kMaxPlanes]; // staged ref windows (refw[0] drives matching)
     const T *src0[kMaxPlanes]; // block (0, 0) of src when outside the window
     const T *ref0[kMaxPlanes];
-    Acc *accN[kMaxPlanes], *accD[kMaxPlanes];
-    Acc *accN0[kMaxPlanes], *accD0[kMaxPlanes];
+    Acc *accN[kMaxPlanes];     // numerator sums over the window
+    Acc *accN0[kMaxPlanes];    // and over block (0, 0) when outside the window
 };
 
 // Adds q to the 64-bit two's-complement sum at p (shared memory). A 64-bit
@@ -185,6 +185,20 @@ __device__ __forceinline__ void acc_flush(long long *p, long long v)
     atomicAdd(reinterpret_cast<unsigned long long *>(p), static_cast<unsigned long long>(v));
 }
 __device__ __forceinline__ void acc_flush(double *p, double v) { atomicAdd(p, v); }
+
+// A block's weight, added at the block's origin (py, px) of a plane's weight
+// sums. It goes straight to global memory: one reduction per group member
+// costs no more than flushing a window of them, and without the window a tile
+// needs a third less shared memory and no second zeroing and flushing pass.
+__device__ __forceinline__ void weight_add(long long *den, int width, int py, int px, float w,
+                                           float scale)
+{
+    acc_flush(den + static_cast<long long>(py) * width + px, __float2ll_rn(w * scale));
+}
+__device__ __forceinline__ void weight_add(double *den, int width, int py, int px, double w, float)
+{
+    acc_flush(den + static_cast<long long>(py) * width + px, w);
+}
 
 // Address of pixel (y, x) of the block at plane position (py, px) inside a
 // staged window, or inside the (0, 0) copy when the block is (0, 0) and the
@@ -962,7 +976,7 @@ __device__ __forceinline__ void aggregate_member_slow(const StageArgs<T> &a, con
     if (h == 0) {
         const float sd = (q.y == 0 && q.x == 0) ? scale_c : scale;
         if (poison == nullptr || fabsf(static_cast<float>(denW) * sd) < kFixedLimit)
-            acc_add(block_ptr(t, t.accD[p], t.accD0[p], q.y, q.x, pitch), denW, sd);
+            weight_add(a.den[plane], a.width, q.y, q.x, denW, sd);
         else  // the block's weight reaches all of its pixels
             for (int i = 0; i < kBS * kBS; ++i)
                 poison[static_cast<long long>(q.y + (i >> 3)) * a.width + q.x + (i & 7)] = 1;
@@ -1057,7 +1071,7 @@ __device__ void filter_group(const StageArgs<T> &a, const Tile<T> &t, int p, con
 #pragma unroll
                 for (int x = 0; x < 8; ++x) acc_add(dn + y * pitch + x, v[x] * numW, scale);
             }
-            if (h == 0) acc_add(block_ptr(t, t.accD[p], t.accD0[p], q.y, q.x, pitch), denW, scale);
+            if (h == 0) weight_add(a.den[pt], a.width, q.y, q.x, denW, scale);
         } else {
             aggregate_member_slow<T>(a, t, p, pt, q, gz, h, numW, denW, scale);
         }
@@ -1136,10 +1150,8 @@ __device__ __forceinline__ void carve_tile(const StageArgs<T> &a, const SmemPlan
     }
     Acc *origin_acc = reinterpret_cast<Acc *>(smem + sp.off_origin_acc);
     for (int p = 0; p < NPL; ++p) {
-        t.accN[p] = reinterpret_cast<Acc *>(smem + sp.off_acc + sp.acc_bytes * (2 * p));
-        t.accD[p] = reinterpret_cast<Acc *>(smem + sp.off_acc + sp.acc_bytes * (2 * p + 1));
-        t.accN0[p] = origin_acc + bsq * (2 * p);
-        t.accD0[p] = origin_acc + bsq * (2 * p + 1);
+        t.accN[p] = reinterpret_cast<Acc *>(smem + sp.off_acc + sp.acc_bytes * p);
+        t.accN0[p] = origin_acc + bsq * p;
     }
 }
 
@@ -1173,10 +1185,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs<T> &a, const Tile<T> 
             const int s = y * t.pitch + x;
             if (need_src || (p == 0 && !ref_sep)) cp_async_elem(const_cast<T *>(t.srcw[p]) + s, a.src[p] + g);
             if (ref_sep) cp_async_elem(const_cast<T *>(t.refw[p]) + s, a.ref[p] + g);
-            if (need_src) {
-                t.accN[p][s] = 0;
-                t.accD[p][s] = 0;
-            }
+            if (need_src) t.accN[p][s] = 0;
         }
         if (!t.origin_inside && (need_src || p == 0)) {
             for (int i = tid; i < bsq; i += blockDim.x) {
@@ -1185,7 +1194,6 @@ __device__ __forceinline__ void stage_tile(const StageArgs<T> &a, const Tile<T> 
                 const_cast<T *>(t.src0[p])[i] = __ldg(a.src[p] + g);
                 if (ref_sep) const_cast<T *>(t.ref0[p])[i] = __ldg(a.ref[p] + g);
                 t.accN0[p][i] = 0;
-                t.accD0[p][i] = 0;
             }
         }
     }
@@ -1193,7 +1201,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs<T> &a, const Tile<T> 
     __syncthreads();
 }
 
-// Flush the accumulator windows into the plane-wide num / den sums.
+// Flush the accumulator windows into the plane-wide numerator sums.
 template <typename T, int NPL>
 __device__ __forceinline__ void flush_tile(const StageArgs<T> &a, const Tile<T> &t)
 {
@@ -1205,18 +1213,16 @@ __device__ __forceinline__ void flush_tile(const StageArgs<T> &a, const Tile<T> 
         for (int i = tid; i < npx; i += blockDim.x) {
             const int y = i / t.rw, x = i - y * t.rw;
             const int s = y * t.pitch + x;
-            const auto nv = t.accN[p][s], d = t.accD[p][s];
+            const auto nv = t.accN[p][s];
             const long long g = static_cast<long long>(t.ry0 + y) * a.width + (t.rx0 + x);
             if (nv != 0) acc_flush(a.num[p] + g, nv);
-            if (d != 0) acc_flush(a.den[p] + g, d);
         }
         if (!t.origin_inside) {
             for (int i = tid; i < bsq; i += blockDim.x) {
-                const auto nv = t.accN0[p][i], d = t.accD0[p][i];
+                const auto nv = t.accN0[p][i];
                 const int y = i / bs, x = i - y * bs;
                 const long long g = static_cast<long long>(y) * a.width + x;
                 if (nv != 0) acc_flush(a.num[p] + g, nv);
-                if (d != 0) acc_flush(a.den[p] + g, d);
             }
         }
     }
@@ -1234,6 +1240,7 @@ __device__ __forceinline__ void dump_group(const StageArgs<T> &a, int ky, int kx
         a.group_pos[(ridx * kGSTab + k) * 2 + 1] = list[k].x;
         a.group_key[ridx * kGSTab + k] = lkeys[k];
     }
+    __syncwarp();  // the keys' bytes become the group buffer
 }
 
 // A CTA whose launch gave it less shared memory than its layout needs does
@@ -1284,13 +1291,11 @@ __device__ __forceinline__ void stage_tile_body(const StageArgs<T> &a, int tile,
 
     // Per-warp scratch.
     unsigned char *wbase = smem + sp.off_warps + sp.warp_bytes * warp;
-    const size_t scratch = sp.scratch_bytes;
     T *G = reinterpret_cast<T *>(wbase);
     auto *dist = reinterpret_cast<typename DistBits<T>::type *>(wbase);
-    SortKey<T> *heap = reinterpret_cast<SortKey<T> *>(wbase + scratch);
-    BlockPos *list = reinterpret_cast<BlockPos *>(wbase + scratch + sizeof(SortKey<T>) * kCand);
-    T *lkeys = reinterpret_cast<T *>(wbase + scratch + sizeof(SortKey<T>) * kCand +
-                                     sizeof(BlockPos) * kGSTab);
+    SortKey<T> *heap = reinterpret_cast<SortKey<T> *>(wbase + sp.off_heap);
+    T *lkeys = reinterpret_cast<T *>(wbase + sp.off_keys);
+    BlockPos *list = reinterpret_cast<BlockPos *>(wbase + sp.off_list);
 
     // per-tile counters (small: 32 bits suffice), flushed once per tile
     unsigned n_sum = 0, n_sq = 0, n_cand = 0, n_fix = 0, n_bad = 0;
@@ -1342,10 +1347,7 @@ __device__ __forceinline__ void stage_plane(const StageArgs<T> &a, const Tile<T>
         const int s = y * t.pitch + x;
         cp_async_elem(const_cast<T *>(t.srcw[0]) + s, a.src[c] + g);
         if (need_ref) cp_async_elem(const_cast<T *>(t.refw[0]) + s, a.ref[c] + g);
-        if (filt) {
-            t.accN[0][s] = 0;
-            t.accD[0][s] = 0;
-        }
+        if (filt) t.accN[0][s] = 0;
     }
     if (!t.origin_inside) {
         for (int i = tid; i < bsq; i += blockDim.x) {
@@ -1354,7 +1356,6 @@ __device__ __forceinline__ void stage_plane(const StageArgs<T> &a, const Tile<T>
             const_cast<T *>(t.src0[0])[i] = __ldg(a.src[c] + g);
             if (need_ref) const_cast<T *>(t.ref0[0])[i] = __ldg(a.ref[c] + g);
             t.accN0[0][i] = 0;
-            t.accD0[0][i] = 0;
         }
     }
     cp_async_wait_all();
@@ -1371,18 +1372,16 @@ __device__ __forceinline__ void flush_plane(const StageArgs<T> &a, const Tile<T>
     for (int i = tid; i < npx; i += blockDim.x) {
         const int y = i / t.rw, x = i - y * t.rw;
         const int s = y * t.pitch + x;
-        const auto nv = t.accN[0][s], d = t.accD[0][s];
+        const auto nv = t.accN[0][s];
         const long long g = static_cast<long long>(t.ry0 + y) * a.width + (t.rx0 + x);
         if (nv != 0) acc_flush(a.num[c] + g, nv);
-        if (d != 0) acc_flush(a.den[c] + g, d);
     }
     if (!t.origin_inside) {
         for (int i = tid; i < bsq; i += blockDim.x) {
-            const auto nv = t.accN0[0][i], d = t.accD0[0][i];
+            const auto nv = t.accN0[0][i];
             const int y = i / bs, x = i - y * bs;
             const long long g = static_cast<long long>(y) * a.width + x;
             if (nv != 0) acc_flush(a.num[c] + g, nv);
-            if (d != 0) acc_flush(a.den[c] + g, d);
         }
     }
 }
@@ -1419,13 +1418,11 @@ __device__ __forceinline__ void stage_tile_body_seq3(const StageArgs<T> &a, int 
     unsigned char *gn = reinterpret_cast<unsigned char *>(gpos + a.tile_x * a.tile_y * kGSMax);
 
     unsigned char *wbase = smem + sp.off_warps + sp.warp_bytes * warp;
-    const size_t scratch = sp.scratch_bytes;
     T *G = reinterpret_cast<T *>(wbase);
     auto *dist = reinterpret_cast<typename DistBits<T>::type *>(wbase);
-    SortKey<T> *heap = reinterpret_cast<SortKey<T> *>(wbase + scratch);
-    BlockPos *list = reinterpret_cast<BlockPos *>(wbase + scratch + sizeof(SortKey<T>) * kCand);
-    T *lkeys = reinterpret_cast<T *>(wbase + scratch + sizeof(SortKey<T>) * kCand +
-                                     sizeof(BlockPos) * kGSTab);
+    SortKey<T> *heap = reinterpret_cast<SortKey<T> *>(wbase + sp.off_heap);
+    T *lkeys = reinterpret_cast<T *>(wbase + sp.off_keys);
+    BlockPos *list = reinterpret_cast<BlockPos *>(wbase + sp.off_list);
 
     // per-tile counters (small: 32 bits suffice), flushed once per tile
     unsigned n_sum = 0, n_sq = 0, n_cand = 0, n_fix = 0, n_bad = 0;
