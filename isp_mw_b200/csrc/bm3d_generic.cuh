@@ -594,7 +594,7 @@ __device__ __forceinline__ void generic_tile_body(const StageArgs<T> &a, int til
         // BlockSize 8 with step 1: the register-resident kernel's strips of
         // four candidates; otherwise one lane per candidate
         const int n = (bs == kBS && a.bm_step == 1)
-                          ? match_block<T, 4>(a, t, j0, i0, lane, dist, heap, list, lkeys, n_cand,
+                          ? match_block<T, 4>(a, t, j0, i0, lane, dist, refblk, heap, list, lkeys, n_cand,
                                               n_fix)
                           : match_generic<T>(a, t, j0, i0, lane, dist, refblk, heap, list, lkeys,
                                              n_cand, n_fix);
@@ -668,7 +668,7 @@ __device__ __forceinline__ void generic_tile_body_seq3(const StageArgs<T> &a, in
                 const int ky = ky0 + r / tw, kx = kx0 + r % tw;
                 const int j0 = ref_pos(ky, a.step, bottom), i0 = ref_pos(kx, a.step, right);
                 n = (bs == kBS && a.bm_step == 1)
-                        ? match_block<T, 4>(a, t, j0, i0, lane, dist, heap, list, lkeys, n_cand,
+                        ? match_block<T, 4>(a, t, j0, i0, lane, dist, refblk, heap, list, lkeys, n_cand,
                                             n_fix)
                         : match_generic<T>(a, t, j0, i0, lane, dist, refblk, heap, list, lkeys,
                                            n_cand, n_fix);
