@@ -331,8 +331,8 @@ __device__ __forceinline__ void aggregate_rows(const StageArgs<T> &a, const Tile
         if constexpr (BS == 8) redft01_8(v);
         else redft01_line<T, BS>(v, c_dct11_inv);
         int pitch;
-        auto *dn = block_ptr(t, t.accN[p], t.accN0[p], q.y, q.x, pitch);
-        dn += y * pitch;
+        AccWin<T> dn = block_acc(t, p, q.y, q.x, pitch);
+        dn = dn + y * pitch;
         if (!check && (q.y >= BS || q.x >= BS)) {
 #pragma unroll
             for (int x = 0; x < BS; ++x) acc_add(dn + x, v[x] * numW, scale);
@@ -518,9 +518,9 @@ __device__ void filter_generic(const StageArgs<T> &a, const Tile<T> &t, int p, c
         const BlockPos q = list[z];
         if (!block_in_tile(t, q.y, q.x)) continue;
         int pitch;
-        auto *dn = block_ptr(t, t.accN[p], t.accN0[p], q.y, q.x, pitch);
+        AccWin<T> dn = block_acc(t, p, q.y, q.x, pitch);
         if (!check && (q.y >= bs || q.x >= bs)) {
-            acc_add(dn + y * pitch + x, Gs[z * zs + y * rs + x] * numW, scale);
+            acc_add(dn + (y * pitch + x), Gs[z * zs + y * rs + x] * numW, scale);
             if (y == 0 && x == 0)
                 weight_add(a.den[pt], a.width, q.y, q.x, denW, scale);
         } else {
@@ -531,7 +531,7 @@ __device__ void filter_generic(const StageArgs<T> &a, const Tile<T> &t, int p, c
             const bool corner = q.y + y < bs && q.x + x < bs;
             unsigned char *mk =
                 poison ? poison + static_cast<long long>(q.y) * a.width + q.x : nullptr;
-            acc_add_checked(dn + y * pitch + x, Gs[z * zs + y * rs + x] * numW,
+            acc_add_checked(dn + (y * pitch + x), Gs[z * zs + y * rs + x] * numW,
                             corner ? scale_c : scale,
                             mk ? mk + static_cast<long long>(y) * a.width + x : nullptr);
             if (y == 0 && x == 0) {

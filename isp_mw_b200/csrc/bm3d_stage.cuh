@@ -119,9 +119,58 @@ __device__ __forceinline__ void zdct_inv2(T (&a)[kGSMax], T (&b)[kGSMax], int n)
 }
 
 // ---------------------------------------------------------------------------
+// Numerator sums in shared memory. FP32 stages keep 64-bit two's-complement
+// sums as two arrays of 32-bit words, the low words at p, the high words `hi`
+// words after them. A 64-bit shared-memory atomic add has no native form (it
+// runs as a compare-and-swap loop), so each word is updated by a native 32-bit
+// atomic: the low word's atomic returns the value it replaced, which tells
+// whether this addition wrapped it, and that carry goes into the high word
+// with the term's own high half. Every wrap of the low word is seen by exactly
+// the addition that caused it, so once all additions are done the two words
+// hold the sum mod 2^64 -- the value a 64-bit atomic add gives -- whatever the
+// order. Nothing reads the sums until the tile's barrier.
+//
+// The words lie in separate arrays because a warp's additions fall on 32
+// unrelated pixels: 32 banks spread them better than the 16 that words of
+// interleaved pairs leave.
+template <typename T> struct AccWin;
+template <> struct AccWin<float> {
+    unsigned *p;
+    int hi;
+    __device__ __forceinline__ AccWin operator+(int i) const { return AccWin{p + i, hi}; }
+    __device__ __forceinline__ void zero(int i) const
+    {
+        p[i] = 0;
+        p[i + hi] = 0;
+    }
+    __device__ __forceinline__ long long get(int i) const
+    {
+        return static_cast<long long>(static_cast<unsigned long long>(p[i + hi]) << 32 | p[i]);
+    }
+    __device__ __forceinline__ void add(long long q) const
+    {
+        const unsigned lo = static_cast<unsigned>(q);
+        const unsigned up = static_cast<unsigned>(static_cast<unsigned long long>(q) >> 32);
+        const unsigned old = atomicAdd(p, lo);
+        atomicAdd(p + hi, up + (old + lo < old ? 1u : 0u));
+    }
+};
+template <> struct AccWin<double> {
+    double *p;
+    __device__ __forceinline__ AccWin operator+(int i) const { return AccWin{p + i}; }
+    __device__ __forceinline__ void zero(int i) const { p[i] = 0.0; }
+    __device__ __forceinline__ double get(int i) const { return p[i]; }
+};
+// n sums at p, as carved by plan_smem (FP32: n low words, then n high words).
+template <typename T> __device__ __forceinline__ AccWin<T> make_acc(void *p, int n)
+{
+    if constexpr (sizeof(T) == 4) return AccWin<T>{static_cast<unsigned *>(p), n};
+    else return AccWin<T>{static_cast<double *>(p)};
+}
+
+// ---------------------------------------------------------------------------
 // One CTA's view of its staged windows.
 template <typename T> struct Tile {
-    using Acc = typename AccOf<T>::type;
     int ry0, rx0, rh, rw;      // staged window origin / size in the plane
     int pitch;
     int bs;                    // block size
@@ -130,35 +179,16 @@ template <typename T> struct Tile {
     const T *refw[kMaxPlanes]; // staged ref windows (refw[0] drives matching)
     const T *src0[kMaxPlanes]; // block (0, 0) of src when outside the window
     const T *ref0[kMaxPlanes];
-    Acc *accN[kMaxPlanes];     // numerator sums over the window
-    Acc *accN0[kMaxPlanes];    // and over block (0, 0) when outside the window
+    AccWin<T> accN[kMaxPlanes];   // numerator sums over the window
+    AccWin<T> accN0[kMaxPlanes];  // and over block (0, 0) when outside the window
 };
 
-// Adds q to the 64-bit two's-complement sum at p (shared memory). A 64-bit
-// shared-memory atomic add has no native form (it runs as a compare-and-swap
-// loop: a load, an add and a CAS round trip per attempt), so the sum is kept
-// as two 32-bit words, low word at p, high word after it, each updated by a
-// native 32-bit atomic. The low word's atomic returns the value it replaced,
-// which tells whether this addition wrapped it; that carry goes into the high
-// word with q's own high half. Every wrap of the low word is seen by exactly
-// the addition that caused it, so once all additions are done the 8 bytes at
-// p hold sum(q) mod 2^64 -- the value the 64-bit atomic add gave -- whatever
-// the order. Nothing reads the slot until the tile's barrier.
-__device__ __forceinline__ void acc_add_fixed(long long *p, long long q)
-{
-    unsigned *w = reinterpret_cast<unsigned *>(p);
-    const unsigned lo = static_cast<unsigned>(q);
-    const unsigned hi = static_cast<unsigned>(static_cast<unsigned long long>(q) >> 32);
-    const unsigned old = atomicAdd(w, lo);
-    atomicAdd(w + 1, hi + (old + lo < old ? 1u : 0u));
-}
-
 // One aggregation term: fixed point for FP32 stages, double for FP64.
-__device__ __forceinline__ void acc_add(long long *p, float v, float scale)
+__device__ __forceinline__ void acc_add(AccWin<float> w, float v, float scale)
 {
-    acc_add_fixed(p, __float2ll_rn(v * scale));
+    w.add(__float2ll_rn(v * scale));
 }
-__device__ __forceinline__ void acc_add(double *p, double v, float) { atomicAdd(p, v); }
+__device__ __forceinline__ void acc_add(AccWin<double> w, double v, float) { atomicAdd(w.p, v); }
 
 // The same for planes with non-finite pixels: a term that has no fixed-point
 // value (NaN, +-Inf, or beyond the 2^62 range) marks its pixel instead, and
@@ -167,18 +197,18 @@ __device__ __forceinline__ void acc_add(double *p, double v, float) { atomicAdd(
 // Finite terms are converted exactly as acc_add does; with no mark they are
 // always converted.
 constexpr float kFixedLimit = 4.0e18f;
-__device__ __forceinline__ void acc_add_checked(long long *p, float v, float scale,
+__device__ __forceinline__ void acc_add_checked(AccWin<float> w, float v, float scale,
                                                 unsigned char *mark)
 {
     const float x = v * scale;
     if (mark == nullptr || fabsf(x) < kFixedLimit)
-        acc_add_fixed(p, __float2ll_rn(x));
+        w.add(__float2ll_rn(x));
     else
         *mark = 1;
 }
-__device__ __forceinline__ void acc_add_checked(double *p, double v, float, unsigned char *)
+__device__ __forceinline__ void acc_add_checked(AccWin<double> w, double v, float, unsigned char *)
 {
-    atomicAdd(p, v);
+    atomicAdd(w.p, v);
 }
 __device__ __forceinline__ void acc_flush(long long *p, long long v)
 {
@@ -213,6 +243,18 @@ __device__ __forceinline__ P *block_ptr(const Tile<T> &t, P *win, P *origin, int
     }
     pitch = t.pitch;
     return win + (py - t.ry0) * t.pitch + (px - t.rx0);
+}
+
+// The same place of the numerator sums of windows p.
+template <typename T>
+__device__ __forceinline__ AccWin<T> block_acc(const Tile<T> &t, int p, int py, int px, int &pitch)
+{
+    if (py == 0 && px == 0 && !t.origin_inside) {
+        pitch = t.bs;
+        return t.accN0[p];
+    }
+    pitch = t.pitch;
+    return t.accN[p] + ((py - t.ry0) * t.pitch + (px - t.rx0));
 }
 
 // True when the block at (py, px) can be addressed: inside the staged window,
@@ -955,7 +997,7 @@ __device__ __forceinline__ void aggregate_member_slow(const StageArgs<T> &a, con
     const float scale_c = fixed_scale(a.absmax[plane], a.log2_corner);
     unsigned char *const poison = poison_map(a, plane);
     int pitch;
-    auto *dn = block_ptr(t, t.accN[p], t.accN0[p], q.y, q.x, pitch);
+    const AccWin<T> dn = block_acc(t, p, q.y, q.x, pitch);
 #pragma unroll 1
     for (int r = 0; r < 4; ++r) {
         const int y = 4 * h + r;
@@ -968,7 +1010,7 @@ __device__ __forceinline__ void aggregate_member_slow(const StageArgs<T> &a, con
             const bool corner = q.y + y < kBS && q.x + x < kBS;
             unsigned char *mk =
                 poison ? poison + static_cast<long long>(q.y + y) * a.width + q.x + x : nullptr;
-            acc_add_checked(dn + y * pitch + x, v[x] * numW, corner ? scale_c : scale, mk);
+            acc_add_checked(dn + (y * pitch + x), v[x] * numW, corner ? scale_c : scale, mk);
         }
     }
     if (h == 0) {
@@ -1058,7 +1100,7 @@ __device__ void filter_group(const StageArgs<T> &a, const Tile<T> &t, int p, con
         const T *gz = G + z * kGroupStride;
         if (!check && (q.y >= kBS || q.x >= kBS)) {
             int pitch;
-            auto *dn = block_ptr(t, t.accN[p], t.accN0[p], q.y, q.x, pitch);
+            const AccWin<T> dn = block_acc(t, p, q.y, q.x, pitch);
 #pragma unroll 1
             for (int r = 0; r < 4; ++r) {
                 const int y = 4 * h + r;
@@ -1067,7 +1109,7 @@ __device__ void filter_group(const StageArgs<T> &a, const Tile<T> &t, int p, con
                 Vec4<T>::load(gz + gidx(y, 4), v[4], v[5], v[6], v[7]);
                 redft01_8(v);
 #pragma unroll
-                for (int x = 0; x < 8; ++x) acc_add(dn + y * pitch + x, v[x] * numW, scale);
+                for (int x = 0; x < 8; ++x) acc_add(dn + (y * pitch + x), v[x] * numW, scale);
             }
             if (h == 0) weight_add(a.den[pt], a.width, q.y, q.x, denW, scale);
         } else {
@@ -1126,7 +1168,6 @@ template <typename T, bool WIENER, int NPL>
 __device__ __forceinline__ void carve_tile(const StageArgs<T> &a, const SmemPlan &sp,
                                            unsigned char *smem, Tile<T> &t)
 {
-    using Acc = typename AccOf<T>::type;
     const int bsq = t.bs * t.bs;
     int s = 0;
     T *origin = reinterpret_cast<T *>(smem + sp.off_origin);
@@ -1146,10 +1187,10 @@ __device__ __forceinline__ void carve_tile(const StageArgs<T> &a, const SmemPlan
             ++s;
         }
     }
-    Acc *origin_acc = reinterpret_cast<Acc *>(smem + sp.off_origin_acc);
     for (int p = 0; p < NPL; ++p) {
-        t.accN[p] = reinterpret_cast<Acc *>(smem + sp.off_acc + sp.acc_bytes * p);
-        t.accN0[p] = origin_acc + bsq * p;
+        t.accN[p] = make_acc<T>(smem + sp.off_acc + sp.acc_bytes * p,
+                                static_cast<int>(sp.acc_bytes / sizeof(typename AccOf<T>::type)));
+        t.accN0[p] = make_acc<T>(smem + sp.off_origin_acc + sizeof(typename AccOf<T>::type) * bsq * p, bsq);
     }
 }
 
@@ -1183,7 +1224,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs<T> &a, const Tile<T> 
             const int s = y * t.pitch + x;
             if (need_src || (p == 0 && !ref_sep)) cp_async_elem(const_cast<T *>(t.srcw[p]) + s, a.src[p] + g);
             if (ref_sep) cp_async_elem(const_cast<T *>(t.refw[p]) + s, a.ref[p] + g);
-            if (need_src) t.accN[p][s] = 0;
+            if (need_src) t.accN[p].zero(s);
         }
         if (!t.origin_inside && (need_src || p == 0)) {
             for (int i = tid; i < bsq; i += blockDim.x) {
@@ -1191,7 +1232,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs<T> &a, const Tile<T> 
                 const long long g = static_cast<long long>(y) * a.stride + x;
                 const_cast<T *>(t.src0[p])[i] = __ldg(a.src[p] + g);
                 if (ref_sep) const_cast<T *>(t.ref0[p])[i] = __ldg(a.ref[p] + g);
-                t.accN0[p][i] = 0;
+                t.accN0[p].zero(i);
             }
         }
     }
@@ -1211,13 +1252,13 @@ __device__ __forceinline__ void flush_tile(const StageArgs<T> &a, const Tile<T> 
         for (int i = tid; i < npx; i += blockDim.x) {
             const int y = i / t.rw, x = i - y * t.rw;
             const int s = y * t.pitch + x;
-            const auto nv = t.accN[p][s];
+            const auto nv = t.accN[p].get(s);
             const long long g = static_cast<long long>(t.ry0 + y) * a.width + (t.rx0 + x);
             if (nv != 0) acc_flush(a.num[p] + g, nv);
         }
         if (!t.origin_inside) {
             for (int i = tid; i < bsq; i += blockDim.x) {
-                const auto nv = t.accN0[p][i];
+                const auto nv = t.accN0[p].get(i);
                 const int y = i / bs, x = i - y * bs;
                 const long long g = static_cast<long long>(y) * a.width + x;
                 if (nv != 0) acc_flush(a.num[p] + g, nv);
@@ -1347,7 +1388,7 @@ __device__ __forceinline__ void stage_plane(const StageArgs<T> &a, const Tile<T>
         const int s = y * t.pitch + x;
         cp_async_elem(const_cast<T *>(t.srcw[0]) + s, a.src[c] + g);
         if (need_ref) cp_async_elem(const_cast<T *>(t.refw[0]) + s, a.ref[c] + g);
-        if (filt) t.accN[0][s] = 0;
+        if (filt) t.accN[0].zero(s);
     }
     if (!t.origin_inside) {
         for (int i = tid; i < bsq; i += blockDim.x) {
@@ -1355,7 +1396,7 @@ __device__ __forceinline__ void stage_plane(const StageArgs<T> &a, const Tile<T>
             const long long g = static_cast<long long>(y) * a.stride + x;
             const_cast<T *>(t.src0[0])[i] = __ldg(a.src[c] + g);
             if (need_ref) const_cast<T *>(t.ref0[0])[i] = __ldg(a.ref[c] + g);
-            t.accN0[0][i] = 0;
+            t.accN0[0].zero(i);
         }
     }
     cp_async_wait_all();
@@ -1372,13 +1413,13 @@ __device__ __forceinline__ void flush_plane(const StageArgs<T> &a, const Tile<T>
     for (int i = tid; i < npx; i += blockDim.x) {
         const int y = i / t.rw, x = i - y * t.rw;
         const int s = y * t.pitch + x;
-        const auto nv = t.accN[0][s];
+        const auto nv = t.accN[0].get(s);
         const long long g = static_cast<long long>(t.ry0 + y) * a.width + (t.rx0 + x);
         if (nv != 0) acc_flush(a.num[c] + g, nv);
     }
     if (!t.origin_inside) {
         for (int i = tid; i < bsq; i += blockDim.x) {
-            const auto nv = t.accN0[0][i];
+            const auto nv = t.accN0[0].get(i);
             const int y = i / bs, x = i - y * bs;
             const long long g = static_cast<long long>(y) * a.width + x;
             if (nv != 0) acc_flush(a.num[c] + g, nv);

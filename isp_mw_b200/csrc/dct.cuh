@@ -47,14 +47,14 @@ template <> struct Pair<float> {
     unsigned long long v;
     __device__ __forceinline__ float lo() const
     {
-        float x, y;
-        asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+        float x;
+        asm("{ .reg .f32 t; mov.b64 {%0, t}, %1; }" : "=f"(x) : "l"(v));
         return x;
     }
     __device__ __forceinline__ float hi() const
     {
-        float x, y;
-        asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+        float y;
+        asm("{ .reg .f32 t; mov.b64 {t, %0}, %1; }" : "=f"(y) : "l"(v));
         return y;
     }
     static __device__ __forceinline__ Pair make(float x, float y)
