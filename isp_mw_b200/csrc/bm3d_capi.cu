@@ -426,7 +426,7 @@ static int launch_one(bm3d_ctx *ctx, StageArgs<T> &a, cudaStream_t s, int warps)
 {
     const void *kern = stage_kernel_fn<T, W, NPL, KS>();
     const SmemPlan sp =
-        plan_smem<T>(NPL, W, a.ref_alias_src, a.region_h, a.region_pitch, a.key_slots, warps,
+        plan_smem<T>(NPL, W, a.ref_alias_src, a.region_h, a.region_pitch, a.span, warps,
                      false, kBS, kGSMax, a.tile_x * a.tile_y);
     CK(ctx, raise_smem_limit(kern, sp.total));
     const int grid = a.tiles_x * ((a.ny + a.tile_y - 1) / a.tile_y);
@@ -457,7 +457,7 @@ static int launch_generic(bm3d_ctx *ctx, StageArgs<T> &a, cudaStream_t s, int wa
 {
     const void *kern = generic_kernel_fn<T, W, NPL>();
     const SmemPlan sp = plan_smem<T>(NPL, W, a.ref_alias_src, a.region_h, a.region_pitch,
-                                     a.key_slots, warps, true, a.block_size, a.group_size,
+                                     a.span, warps, true, a.block_size, a.group_size,
                                      a.tile_x * a.tile_y);
     CK(ctx, raise_smem_limit(kern, sp.total));
     const int grid = a.tiles_x * ((a.ny + a.tile_y - 1) / a.tile_y);
@@ -523,8 +523,7 @@ static int plan_geometry(bm3d_ctx *ctx, StageArgs<T> &a, const bm3d_stage_params
     a.range = p->bm_range / p->bm_step * p->bm_step;
     a.nx = ref_count(width - BS, a.step);
     a.ny = ref_count(height - BS, a.step);
-    const int span = 2 * (a.range / a.bm_step) + 1;
-    a.key_slots = span * span + 1;
+    a.span = 2 * (a.range / a.bm_step) + 1;
     // The generic kernel (launch bounds 384 in FP32, 256 in FP64) takes the
     // first of these (tile_x, tile_y, warps) that fits: reference blocks per
     // tile a multiple of the warps, so no warp idles in a tile's last round.
@@ -544,7 +543,7 @@ static int plan_geometry(bm3d_ctx *ctx, StageArgs<T> &a, const bm3d_stage_params
         // and this residue keeps those lane groups on the fewest shared banks
         a.region_pitch = a.region_w + ((5 - a.region_w % 8) + 8) % 8;
         const SmemPlan sp = plan_smem<T>(nplanes, wiener, a.ref_alias_src, a.region_h,
-                                         a.region_pitch, a.key_slots, warps, generic, BS,
+                                         a.region_pitch, a.span, warps, generic, BS,
                                          p->group_size, std::min(tx, a.nx) * std::min(ty, a.ny));
         if (sp.total <= ctx->smem_optin) break;
         if (generic) {

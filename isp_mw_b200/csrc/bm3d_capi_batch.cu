@@ -173,8 +173,7 @@ int build_stage(bm3d_batch *B, bool wiener, int tx, int ty, int warps, StageBuil
         a.range = p->bm_range / p->bm_step * p->bm_step;
         a.nx = ref_count(a.width - BS, a.step);
         a.ny = ref_count(a.height - BS, a.step);
-        const int span = 2 * (a.range / a.bm_step) + 1;
-        a.key_slots = span * span + 1;
+        a.span = 2 * (a.range / a.bm_step) + 1;
         const int reach = a.match ? a.range : 0;
         a.region_w = std::min(a.width, (tx - 1) * a.step + 2 * reach + BS);
         a.region_h = std::min(a.height, (ty - 1) * a.step + 2 * reach + BS);
@@ -202,7 +201,7 @@ int build_stage(bm3d_batch *B, bool wiener, int tx, int ty, int warps, StageBuil
         a.dct_fwd = ctx->gtab_f;
         a.dct_inv = ctx->gtab_f ? ctx->gtab_f + kDctTableSize : nullptr;
         const SmemPlan sp = plan_smem<float>(npl, wiener, a.ref_alias_src, a.region_h,
-                                             a.region_pitch, a.key_slots, warps, generic, BS,
+                                             a.region_pitch, a.span, warps, generic, BS,
                                              p->group_size, a.tile_x * a.tile_y);
         smem = std::max(smem, sp.total + kBatchHeader);
         args.push_back(a);

@@ -54,6 +54,22 @@ __device__ __forceinline__ float ssd_row8(float acc, const float (&r)[8], const 
     }
     return acc;
 }
+// The same sum up to rounding, in a third fewer operations: squares and sums
+// fused, even and odd columns in the two halves of acc. All terms are >= 0, so
+// it is within 98 * 2^-24 (relative) of the ordered sum -- 65 roundings there,
+// 33 here -- as long as neither is near the subnormal range.
+__device__ __forceinline__ unsigned long long ssd_row8_near(unsigned long long acc,
+                                                            const unsigned long long (&r)[4],
+                                                            const unsigned long long (&c)[4])
+{
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+        unsigned long long d;
+        asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(r[x]), "l"(c[x]));
+        asm("fma.rn.f32x2 %0, %1, %1, %0;" : "+l"(acc) : "l"(d));
+    }
+    return acc;
+}
 __device__ __forceinline__ double ssd_row8(double acc, const double (&r)[8], const double (&c)[8])
 {
 #pragma unroll
@@ -86,6 +102,14 @@ __host__ __device__ __forceinline__ int search_boundary(int pos, int plane_bound
     int b = pos + range;
     if (b > plane_boundary) b -= (b - plane_boundary + step - 1) / step * step;
     return b;
+}
+
+// Rounds of 32 tasks that match a full window of span x span places: strips of
+// kStrip rows of one column, and the trailing slot.
+constexpr int kStrip = 4;
+__host__ __device__ __forceinline__ int task_rounds(int span)
+{
+    return ((span + kStrip - 1) / kStrip * span + 1 + kWarp - 1) / kWarp;
 }
 
 // Reference-block position k along one axis: 0, step, 2 step, ... with the
@@ -258,7 +282,7 @@ template <typename T> struct StageArgs {
     int tiles_x;                // tiles per row of the tile grid
     int region_w, region_h;     // upper bounds of a tile's staged window
     int region_pitch;           // row pitch of staged windows in shared memory
-    int key_slots;              // per-warp search list capacity
+    int span;                   // window places per axis, 2 range / bm_step + 1 (list: span^2 + 1)
     int ref_alias_src;          // bit p set: ref[p] == src[p], stage once
     T thSSE;                    // FLType(thMSE * MSE2SSE)      (include/Block.h:582-584)
     double distMul;             // 1 / MSE2SSE
@@ -295,6 +319,7 @@ struct SmemPlan {
     size_t off_acc;              // an accumulator window (numerator sums) per plane
     size_t off_origin;           // block (0, 0) copies per staged window
     size_t off_origin_acc;       // block (0, 0) accumulators
+    size_t off_tasks;            // strip matching: the tile's task table (task_rounds x 32 words)
     size_t off_warps;
     size_t warp_bytes;
     // within a warp's area: the group buffer(s) start at 0; before a group is
@@ -334,7 +359,7 @@ __host__ __device__ constexpr bool generic_one_buffer(bool wiener, int bs)
 // relative to the window (windows under 255 x 255) and a count byte.
 template <typename T>
 __host__ __device__ inline SmemPlan plan_smem(int nplanes, bool wiener, int alias_mask,
-                                              int region_h, int region_pitch, int key_slots,
+                                              int region_h, int region_pitch, int span,
                                               int nwarps, bool generic = false, int bs = kBS,
                                               int gs = kGSMax, int tile_refs = 0)
 {
@@ -357,12 +382,13 @@ __host__ __device__ inline SmemPlan plan_smem(int nplanes, bool wiener, int alia
     s.off_origin = s.off_acc + s.acc_bytes * nplanes;
     // block (0, 0) copies: T per staged window, then (16-byte aligned) Acc per accumulator
     s.off_origin_acc = s.off_origin + (sizeof(T) * bsq * s.n_stage + 15) / 16 * 16;
-    s.off_warps = (s.off_origin_acc + sizeof(Acc) * bsq * nplanes + 15) / 16 * 16;
+    s.off_tasks = (s.off_origin_acc + sizeof(Acc) * bsq * nplanes + 15) / 16 * 16;
+    s.off_warps = s.off_tasks + (bs == kBS ? sizeof(unsigned) * kWarp * task_rounds(span) : 0);
     const size_t group_bytes = generic
         ? sizeof(T) * static_cast<size_t>(gs) * generic_block_stride(bs) *
               (wiener && !generic_one_buffer<T>(wiener, bs) ? 2 : 1)
         : sizeof(T) * kGSMax * kGroupStride;
-    const size_t key_bytes = sizeof(T) * key_slots;  // distance bits
+    const size_t key_bytes = sizeof(T) * (static_cast<size_t>(span) * span + 1);  // distance bits
     const auto up = [](size_t v) { return (v + 15) / 16 * 16; };
     const size_t heap_bytes = sizeof(SortKey<T>) * kCand, ref_bytes = sizeof(T) * bsq;
     s.off_ref = s.off_heap = up(key_bytes);
@@ -374,6 +400,9 @@ __host__ __device__ inline SmemPlan plan_smem(int nplanes, bool wiener, int alia
     const int glist = generic ? gs : kGSMax;  // group-list entries per reference block
     s.total = seq3 ? s.off_groups + static_cast<size_t>(tile_refs) * (2 * glist + 1)
                    : s.off_warps + s.warp_bytes * nwarps;
+    // the task table's list places and offsets have 16 bits (a list of 256 x 256
+    // would not fit anyway)
+    if (span > 255) s.total = ~size_t(0) >> 1;
     if (seq3 && (region_h > 255 || region_pitch > 255)) s.total = ~size_t(0) >> 1;  // too wide
     return s;
 }

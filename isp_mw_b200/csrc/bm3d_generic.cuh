@@ -248,8 +248,8 @@ __device__ int match_generic(const StageArgs<T> &a, const Tile<T> &t, int j0, in
     }
     __syncwarp();
     n_cand += static_cast<unsigned>(ngrid);
-    return select_group<T>(a, dist, ngrid, nc, nc_div, tp, l, st, j0, i0, lane, nvalid, heap, list,
-                           lkeys, n_fix);
+    return select_group<T, false>(a, dist, limit, [](int) { return B(0); }, ngrid, nc, nc_div, tp, l,
+                                  st, j0, i0, lane, nvalid, heap, list, lkeys, n_fix);
 }
 
 // Element e of a group stored [z][y][x]: shifts for BlockSize 8, divisions
@@ -560,15 +560,19 @@ __device__ __forceinline__ void generic_tile_body(const StageArgs<T> &a, int til
     int kx0, kx1, ky0, ky1;
     tile_window(a, tile, bs, t, kx0, kx1, ky0, ky1);
     const SmemPlan sp = plan_smem<T>(NPL, WIENER, a.ref_alias_src, a.region_h, a.region_pitch,
-                                     a.key_slots, nwarps, true, bs, a.group_size);
+                                     a.span, nwarps, true, bs, a.group_size);
     if (sp.total > avail) {  // launched with less shared memory than the layout needs
         smem_shortfall(a);
         return;
     }
     carve_tile<T, WIENER, NPL>(a, sp, smem, t);
+    unsigned *tasks = reinterpret_cast<unsigned *>(smem + sp.off_tasks);
+    unsigned char *wbase = smem + sp.off_warps + sp.warp_bytes * warp;
+    const bool strips = bs == kBS && a.bm_step == 1;
+    if (strips && warp == 0)
+        build_tasks(tasks, reinterpret_cast<unsigned *>(wbase), a.span, t.pitch, lane);
     stage_tile<T, WIENER, NPL>(a, t);
 
-    unsigned char *wbase = smem + sp.off_warps + sp.warp_bytes * warp;
     const int gvals = a.group_size * generic_block_stride(bs);
     T *Gs = reinterpret_cast<T *>(wbase);
     T *Gr = Gs + gvals;
@@ -593,8 +597,8 @@ __device__ __forceinline__ void generic_tile_body(const StageArgs<T> &a, int til
         const int j0 = ref_pos(ky, a.step, bottom), i0 = ref_pos(kx, a.step, right);
         // BlockSize 8 with step 1: the register-resident kernel's strips of
         // four candidates; otherwise one lane per candidate
-        const int n = (bs == kBS && a.bm_step == 1)
-                          ? match_block<T, 4>(a, t, j0, i0, lane, dist, refblk, heap, list, lkeys, n_cand,
+        const int n = strips
+                          ? match_block<T, kStrip>(a, t, j0, i0, lane, tasks, dist, refblk, heap, list, lkeys, n_cand,
                                               n_fix)
                           : match_generic<T>(a, t, j0, i0, lane, dist, refblk, heap, list, lkeys,
                                              n_cand, n_fix);
@@ -633,7 +637,7 @@ __device__ __forceinline__ void generic_tile_body_seq3(const StageArgs<T> &a, in
     int kx0, kx1, ky0, ky1;
     tile_window(a, tile, bs, t, kx0, kx1, ky0, ky1);
     const SmemPlan sp = plan_smem<T>(3, WIENER, a.ref_alias_src, a.region_h, a.region_pitch,
-                                     a.key_slots, nwarps, true, bs, GS, a.tile_x * a.tile_y);
+                                     a.span, nwarps, true, bs, GS, a.tile_x * a.tile_y);
     if (sp.total > avail) {  // launched with less shared memory than the layout needs
         smem_shortfall(a);
         return;
@@ -644,7 +648,11 @@ __device__ __forceinline__ void generic_tile_body_seq3(const StageArgs<T> &a, in
     unsigned short *gpos = reinterpret_cast<unsigned short *>(smem + sp.off_groups);
     unsigned char *gn = reinterpret_cast<unsigned char *>(gpos + a.tile_x * a.tile_y * GS);
 
+    unsigned *tasks = reinterpret_cast<unsigned *>(smem + sp.off_tasks);
     unsigned char *wbase = smem + sp.off_warps + sp.warp_bytes * warp;
+    const bool strips = bs == kBS && a.bm_step == 1;
+    if (strips && warp == 0)
+        build_tasks(tasks, reinterpret_cast<unsigned *>(wbase), a.span, t.pitch, lane);
     T *Gs = reinterpret_cast<T *>(wbase);
     T *Gr = Gs + GS * generic_block_stride(bs);
     auto *dist = reinterpret_cast<typename DistBits<T>::type *>(wbase);
@@ -667,8 +675,8 @@ __device__ __forceinline__ void generic_tile_body_seq3(const StageArgs<T> &a, in
             if (c == 0) {
                 const int ky = ky0 + r / tw, kx = kx0 + r % tw;
                 const int j0 = ref_pos(ky, a.step, bottom), i0 = ref_pos(kx, a.step, right);
-                n = (bs == kBS && a.bm_step == 1)
-                        ? match_block<T, 4>(a, t, j0, i0, lane, dist, refblk, heap, list, lkeys, n_cand,
+                n = strips
+                        ? match_block<T, kStrip>(a, t, j0, i0, lane, tasks, dist, refblk, heap, list, lkeys, n_cand,
                                             n_fix)
                         : match_generic<T>(a, t, j0, i0, lane, dist, refblk, heap, list, lkeys,
                                            n_cand, n_fix);

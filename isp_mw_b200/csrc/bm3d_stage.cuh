@@ -280,6 +280,12 @@ template <> struct DistBits<float> {
     static __device__ __forceinline__ float value(unsigned b) { return __uint_as_float(b); }
     // keys between 2^-124 and 2^127: normal, with room for the rounding slack
     static constexpr unsigned kLow = 0x01800000u, kHigh = 0x7f000000u;
+    // approximate distances (ssd_row8_near): two that differ by more than kNear
+    // units in the last place are in the order of the exact keys. kNear of them
+    // are at least 256 * 2^-24 of the value; the bounds need 2 (65 + 33) 2^-24
+    // for the two sums and 4 * 2^-24 for keys that round together. All of it
+    // holds above kTiny = 2^-100, far from the subnormal range.
+    static constexpr unsigned kNear = 256u, kTiny = 0x0d800000u;
     static __device__ __forceinline__ unsigned warp_max(unsigned v)
     {
         return __reduce_max_sync(0xffffffffu, v);
@@ -296,6 +302,7 @@ template <> struct DistBits<double> {
         return __longlong_as_double(static_cast<long long>(b));
     }
     static constexpr unsigned long long kLow = 0x0040000000000000ull, kHigh = 0x7fe0000000000000ull;
+    static constexpr unsigned long long kNear = 0, kTiny = 0;
     static __device__ __forceinline__ unsigned long long warp_max(unsigned long long v)
     {
 #pragma unroll
@@ -423,8 +430,16 @@ __device__ __forceinline__ int div_magic(int k, unsigned m)
 // 1080p, sigma 25, against 64-bit keys and two sorting networks: fast basic /
 // final 0.355 / 0.461 -> 0.333 / 0.438 ms, np 2.82 / 6.27 -> 2.00 / 5.86 ms
 // (the smaller list also lets np's basic stage keep 16 warps).
-template <typename T>
-__device__ int select_group(const StageArgs<T> &a, const typename DistBits<T>::type *dist,
+//
+// NEAR: the list holds approximate distances (ssd_row8_near), accepted up to
+// kNear above `limit`. The cut then leaves that much more room, and the
+// approximate order stands when no kept distance is within kNear of the next;
+// else `exact` (list index -> exact distance bits) gives the compacted ones'
+// exact distances. Returns -1 where the whole list has to be exact: a distance
+// at the matching threshold, ties, ranges where the bounds do not hold.
+template <typename T, bool NEAR, typename Exact>
+__device__ __forceinline__ int select_group(const StageArgs<T> &a, const typename DistBits<T>::type *dist,
+                            typename DistBits<T>::type limit, Exact exact,
                             int ngrid, int nc, unsigned nc_div, int tp, int l, int st, int j0,
                             int i0, int lane, int nvalid, SortKey<T> *heap, BlockPos *list,
                             T *lkeys, unsigned &n_fix)
@@ -501,6 +516,19 @@ __device__ int select_group(const StageArgs<T> &a, const typename DistBits<T>::t
             const B kt = DB::of(key_from_dist(DB::value(tb), a.distMul));
             sure = kt >= DB::kLow && kt <= DB::kHigh;  // else the slack does not hold
             cut = tb + 3;
+            if (NEAR) cut += DB::kNear;
+        }
+        if constexpr (NEAR) {
+            if (!sure || limit < DB::kTiny) return -1;
+            // a distance too close to the threshold to tell matters when it can be
+            // kept, or when the group takes every accepted one; either way the cut
+            // is up there
+            if (cut >= limit - DB::kNear) {
+                bool edge = false;
+                for (int i = lane; i < nkeys; i += kWarp)
+                    edge |= dist[i] - (limit - DB::kNear) <= 2 * DB::kNear;
+                if (__any_sync(0xffffffffu, edge)) return -1;
+            }
         }
         // Compact the elements at or under the cut into heap[] (any order).
         int mine = 0;
@@ -516,7 +544,8 @@ __device__ int select_group(const StageArgs<T> &a, const typename DistBits<T>::t
             if (lane >= o) pos += u;
         }
         const int M = __shfl_sync(0xffffffffu, pos, kWarp - 1);
-        if (sure && M <= kCand) {
+        if (NEAR && M > kCand) return -1;
+        if (NEAR || (sure && M <= kCand)) {
             pos -= mine;
             for (int first = 0; first < nkeys; first += kHeld * kWarp) {
                 if (!one) load(first);
@@ -526,44 +555,79 @@ __device__ int select_group(const StageArgs<T> &a, const typename DistBits<T>::t
                         heap[pos++] = K::pack(v[k], static_cast<unsigned>(first + k * kWarp + lane));
             }
             __syncwarp();
-            K v0 = K::invalid(), v1 = K::invalid();
-            if (lane < M) v0 = make(heap[lane].key_bits(), heap[lane].idx());
-            if (lane + kWarp < M)
-                v1 = make(heap[lane + kWarp].key_bits(), heap[lane + kWarp].idx());
-            __syncwarp();
             const bool more = M > kWarp;
-            kb[lane] = v0.key_bits();
-            if (more) kb[lane + kWarp] = v1.key_bits();
-            __syncwarp();
-            count_below(kb, (M + 3) & ~3, v0.key_bits(), v1.key_bits(), r0, r1, more);
-            // the ranks are a permutation of 0 .. M - 1 unless keys are equal
-            unsigned lo = 0, hi = 0;
-            if (lane < M) (r0 < 32 ? lo : hi) |= 1u << (r0 & 31);
-            if (lane + kWarp < M) (r1 < 32 ? lo : hi) |= 1u << (r1 & 31);
-            int distinct = __popc(__reduce_or_sync(0xffffffffu, lo));
-            if (more) distinct += __popc(__reduce_or_sync(0xffffffffu, hi));
-            if (distinct != M) {
-                // equal keys rank by list order; a tie counts when it reaches
-                // the kept set: a kept element with an equal one after it
+            K v0 = lane < M ? heap[lane] : K::invalid();  // distances for now, not keys
+            K v1 = lane + kWarp < M ? heap[lane + kWarp] : K::invalid();
+            bool ranked = false;
+            if constexpr (NEAR) {
+                B *sorted = kb + kCand;
                 __syncwarp();
-                heap[lane] = v0;
-                heap[lane + kWarp] = v1;
+                kb[lane] = v0.key_bits();
+                if (more) kb[lane + kWarp] = v1.key_bits();
                 __syncwarp();
-                bool e0 = false, e1 = false;
-                for (int j = 0; j < M; ++j) {
-                    const K o = heap[j];
-                    if (o.key_bits() == v0.key_bits()) {
-                        if (o < v0) ++r0;
-                        else if (v0 < o) e0 = true;
-                    }
-                    if (o.key_bits() == v1.key_bits()) {
-                        if (o < v1) ++r1;
-                        else if (v1 < o) e1 = true;
-                    }
+                count_below(kb, (M + 3) & ~3, v0.key_bits(), v1.key_bits(), r0, r1, more);
+                // distances that are equal share a rank and leave a later one
+                // unwritten: the slots start at the lanes' own values' ceiling
+                sorted[lane] = none;
+                if (more) sorted[lane + kWarp] = none;
+                __syncwarp();
+                if (lane < M) sorted[r0] = v0.key_bits();
+                if (lane + kWarp < M) sorted[r1] = v1.key_bits();
+                __syncwarp();
+                const B s0 = sorted[lane], n0 = lane + 1 < kCand ? sorted[lane + 1] : none;
+                bool close = lane < take && lane + 1 < M && (s0 == none || n0 == none || n0 - s0 <= DB::kNear);
+                if (more) {
+                    const B s1 = sorted[lane + kWarp];
+                    const B n1 = lane + kWarp + 1 < kCand ? sorted[lane + kWarp + 1] : none;
+                    close |= lane + kWarp < take && lane + kWarp + 1 < M &&
+                             (s1 == none || n1 == none || n1 - s1 <= DB::kNear);
                 }
-                const bool t0 = lane < M && e0 && r0 < take;
-                const bool t1 = lane + kWarp < M && e1 && r1 < take;
-                tie = __any_sync(0xffffffffu, t0 || t1);
+                ranked = !__any_sync(0xffffffffu, close);
+                if (__any_sync(0xffffffffu, v0.key_bits() < DB::kTiny || v1.key_bits() < DB::kTiny))
+                    return -1;
+                if (!ranked) {
+                    if (lane < M) v0 = K::pack(exact(static_cast<int>(v0.idx())), v0.idx());
+                    if (lane + kWarp < M) v1 = K::pack(exact(static_cast<int>(v1.idx())), v1.idx());
+                }
+            }
+            if (!ranked) {
+                if (lane < M) v0 = make(v0.key_bits(), v0.idx());
+                if (lane + kWarp < M) v1 = make(v1.key_bits(), v1.idx());
+                __syncwarp();
+                kb[lane] = v0.key_bits();
+                if (more) kb[lane + kWarp] = v1.key_bits();
+                __syncwarp();
+                count_below(kb, (M + 3) & ~3, v0.key_bits(), v1.key_bits(), r0, r1, more);
+                // the ranks are a permutation of 0 .. M - 1 unless keys are equal
+                unsigned lo = 0, hi = 0;
+                if (lane < M) (r0 < 32 ? lo : hi) |= 1u << (r0 & 31);
+                if (lane + kWarp < M) (r1 < 32 ? lo : hi) |= 1u << (r1 & 31);
+                int distinct = __popc(__reduce_or_sync(0xffffffffu, lo));
+                if (more) distinct += __popc(__reduce_or_sync(0xffffffffu, hi));
+                if (distinct != M) {
+                    // equal keys rank by list order; a tie counts when it reaches
+                    // the kept set: a kept element with an equal one after it
+                    __syncwarp();
+                    heap[lane] = v0;
+                    heap[lane + kWarp] = v1;
+                    __syncwarp();
+                    bool e0 = false, e1 = false;
+                    for (int j = 0; j < M; ++j) {
+                        const K o = heap[j];
+                        if (o.key_bits() == v0.key_bits()) {
+                            if (o < v0) ++r0;
+                            else if (v0 < o) e0 = true;
+                        }
+                        if (o.key_bits() == v1.key_bits()) {
+                            if (o < v1) ++r1;
+                            else if (v1 < o) e1 = true;
+                        }
+                    }
+                    const bool t0 = lane < M && e0 && r0 < take;
+                    const bool t1 = lane + kWarp < M && e1 && r1 < take;
+                    tie = __any_sync(0xffffffffu, t0 || t1);
+                    if (NEAR && tie) return -1;
+                }
             }
             if (lane < M && r0 < take) put(r0, v0);
             if (lane + kWarp < M && r1 < take) put(r1, v1);
@@ -599,7 +663,7 @@ __device__ int select_group(const StageArgs<T> &a, const typename DistBits<T>::t
     // with that exact algorithm when a tie touches the kept set: lane 0 works
     // the heap, the warp finds the entries that change it (the heap's top only
     // falls, so an entry not below it once is never below it).
-    if (accepted + 1 > GS && GS > 1 && tie) {
+    if (!NEAR && accepted + 1 > GS && GS > 1 && tie) {
         auto less = [](const K &p, const K &q) { return p.key() < q.key(); };
         auto adjust = [&](int hole, int len, K value) {
             const int top = hole;
@@ -696,12 +760,63 @@ template <typename T> __device__ __forceinline__ typename DistBits<T>::type dist
     return thSSE > T(0) ? DistBits<T>::of(thSSE) : typename DistBits<T>::type(0);
 }
 
+// Which strip each lane takes in each round over a full window (KS = kStrip):
+// entry [round * 32 + lane] is the strip's list place << 16 | its offset in the
+// staged window, kTaskSlot for the trailing (0, 0) slot or kTaskIdle. A lane's
+// loads of one row touch bank kStrip * pitch * strip + column (+ a constant of
+// the instruction), so handing out the strips in raster order puts two lanes of
+// most rounds on one bank: lane b takes the strips of bank b instead, and only
+// what exceeds the rounds moves to lanes with room. BMrange 9 (95 strips and
+// the slot, 3 rounds): 3 strips move, all into the last round, and the first two
+// rounds read every row in one wavefront instead of two. Built by one warp
+// while the others stage; `spill` is scratch.
+constexpr unsigned kTaskSlot = 0xffffffffu, kTaskIdle = 0xfffffffeu;
+__device__ __forceinline__ void build_tasks(unsigned *tab, unsigned *spill, int span, int pitch,
+                                            int lane)
+{
+    const int nstrips = (span + kStrip - 1) / kStrip, rounds = task_rounds(span);
+    const unsigned below = (1u << lane) - 1u;
+    int mine = 0, moved = 0;
+    for (int s = 0; s < nstrips; ++s) {
+        const int first = (lane - kStrip * pitch * s) & (kWarp - 1);
+        for (int c0 = 0; c0 < span; c0 += kWarp) {
+            const int c = c0 + first;
+            const unsigned task = static_cast<unsigned>(kStrip * s * span + c) << 16 |
+                                  static_cast<unsigned>(kStrip * s * pitch + c);
+            const bool over = c < span && mine >= rounds;
+            if (c < span && !over) tab[mine++ * kWarp + lane] = task;
+            const unsigned m = __ballot_sync(0xffffffffu, over);
+            if (over) spill[moved + __popc(m & below)] = task;
+            moved += __popc(m);
+        }
+    }
+    if (lane == 0) spill[moved] = kTaskSlot;
+    ++moved;
+    __syncwarp();
+    int next = 0;
+    for (int r = 0; r < rounds; ++r) {
+        const bool room = r >= mine;
+        const unsigned m = __ballot_sync(0xffffffffu, room);
+        const int k = next + __popc(m & below);
+        if (room) tab[r * kWarp + lane] = k < moved ? spill[k] : kTaskIdle;
+        next += __popc(m);
+    }
+}
+
 // ---------------------------------------------------------------------------
-// Block matching for reference block (j0, i0) by one warp. Fills list[0..n)
+// Block matching for reference block (j0, i0) by one warp. What bounds it: the
+// FP32 pipe (an ordered, unfused distance is 192 cycles a lane and candidate)
+// and, with the warps of a CTA in step, the shared-memory pipe (88 row loads
+// per strip, two wavefronts each in raster order). So FP32 distances are first
+// taken with fused squares and sums (128 cycles) and strips go to the lanes of
+// their banks (build_tasks); either alone gains nothing, both together take the
+// 1080p basic / final stage from 0.241 / 0.346 to 0.225 / 0.329 ms (4 x 8 tiles)
+// and np on 1283 x 717 from 3.66 to 3.45 ms.
+// Fills list[0..n)
 // with (y, x) in the reference's group order and returns n.
 template <typename T, int KS>
 __device__ int match_block(const StageArgs<T> &a, const Tile<T> &t, int j0, int i0, int lane,
-                           typename DistBits<T>::type *dist, T *refblk, SortKey<T> *heap,
+                           const unsigned *tasks, typename DistBits<T>::type *dist, T *refblk, SortKey<T> *heap,
                            BlockPos *list, T *lkeys, unsigned &n_cand, unsigned &n_fix)
 {
     using B = typename DistBits<T>::type;
@@ -736,33 +851,75 @@ __device__ int match_block(const StageArgs<T> &a, const Tile<T> &t, int j0, int 
     // task for the trailing (0, 0) slot of the reference's search list.
     const int nstrips = (nr + KS - 1) / KS;
     const int ntasks = nstrips * nc;
+    // FP32 lists hold approximate distances first (select_group, NEAR)
+    constexpr bool kNearList = sizeof(T) == 4;
     const B limit = dist_limit(a.thSSE);
+    const B accept = kNearList && limit < static_cast<B>(0x7f800000u) ? limit + DistBits<T>::kNear : limit;
     int nvalid = 0;
     constexpr int ROWS = (KS - 1) + kBS;
-    for (int task = lane; task <= ntasks; task += kWarp) {
+    // a window that the plane's border clips takes its strips in raster order
+    const bool full = KS == kStrip && nr == a.span && nc == a.span;
+    const T *const win = t.refw[0] + (tp - t.ry0) * t.pitch + (l - t.rx0);
+    for (int first = 0; first <= ntasks; first += kWarp) {
         const T *base;
-        int bp, nq, at = ngrid;  // the list place of candidate 0
-        if (task < ntasks) {
-            const int strip = div_magic(task, nc_div);
-            const int cc = task - strip * nc, rr0 = strip * KS;
-            nq = nr - rr0;
-            at = rr0 * nc + cc;
-            bp = t.pitch;
-            base = t.refw[0] + (tp + rr0 * st - t.ry0) * t.pitch + (l + cc * st - t.rx0);
+        int bp = t.pitch, at, end = ngrid;  // list place of candidate 0; end of the valid ones
+        bool slot;
+        if (full) {
+            const unsigned task = tasks[first + lane];
+            if (task == kTaskIdle) break;  // the last round
+            slot = task == kTaskSlot;
+            base = win + (task & 0xffffu);
+            at = static_cast<int>(task >> 16);
         } else {
-            nq = 1;
-            base = block_ptr(t, t.refw[0], t.ref0[0], 0, 0, bp);
+            const int task = first + lane;
+            if (task > ntasks) break;
+            slot = task == ntasks;
+            const int strip = div_magic(task, nc_div), cc = task - strip * nc;
+            base = win + strip * KS * st * t.pitch + cc * st;
+            at = strip * KS * nc + cc;
         }
-        T acc[KS];
+        if (slot) {
+            base = block_ptr(t, t.refw[0], t.ref0[0], 0, 0, bp);
+            at = ngrid;
+            end = ngrid + 1;
+        }
+        // Every strip computes all KS candidates over all ROWS window rows,
+        // with no data-dependent branch; candidates past the window's last row
+        // (at or past `end`) are discarded below. Their rows lie at most KS - 1 rows
+        // past a staged window or the (0, 0) copy, which are always followed by
+        // other parts of the CTA's shared memory.
+        T d[KS];
+        if constexpr (kNearList) {
+            unsigned long long acc[KS], refv[KS][4];  // row y of the reference block in refv[y % KS]
 #pragma unroll
-        for (int q = 0; q < KS; ++q) acc[q] = T(0);
-        T refv[KS][kBS];  // row y of the reference block in refv[y % KS]
-        {
-            // Every strip computes all KS candidates over all ROWS window rows,
-            // with no data-dependent branch; candidates past the window's
-            // last row (q >= nq) are discarded below. Their rows lie at most
-            // KS - 1 rows past a staged window or the (0, 0) copy, which are
-            // always followed by other parts of the CTA's shared memory.
+            for (int q = 0; q < KS; ++q) acc[q] = 0;
+#pragma unroll
+            for (int w = 0; w < ROWS; ++w) {
+                unsigned long long row[4];
+                if (w < kBS) {
+                    unsigned long long (&r)[4] = refv[w % KS];
+                    const ulonglong2 *rr = reinterpret_cast<const ulonglong2 *>(refblk + w * kBS);
+                    const ulonglong2 r01 = rr[0], r23 = rr[1];
+                    r[0] = r01.x; r[1] = r01.y; r[2] = r23.x; r[3] = r23.y;
+                }
+#pragma unroll
+                for (int x = 0; x < 4; ++x)
+                    row[x] = Pair<float>::make(base[w * bp + 2 * x], base[w * bp + 2 * x + 1]).v;
+#pragma unroll
+                for (int q = 0; q < KS; ++q) {
+                    const int y = w - q;
+                    if (y >= 0 && y < kBS) acc[q] = ssd_row8_near(acc[q], refv[y % KS], row);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < KS; ++q) {
+                const Pair<float> s{acc[q]};
+                d[q] = s.lo() + s.hi();
+            }
+        } else {
+            T refv[KS][kBS];
+#pragma unroll
+            for (int q = 0; q < KS; ++q) d[q] = T(0);
 #pragma unroll
             for (int w = 0; w < ROWS; ++w) {
                 T row[kBS];
@@ -776,20 +933,55 @@ __device__ int match_block(const StageArgs<T> &a, const Tile<T> &t, int j0, int 
 #pragma unroll
                 for (int q = 0; q < KS; ++q) {
                     const int y = w - q;
-                    if (y >= 0 && y < kBS) acc[q] = ssd_row8(acc[q], refv[y % KS], row);
+                    if (y >= 0 && y < kBS) d[q] = ssd_row8(d[q], refv[y % KS], row);
                 }
             }
         }
 #pragma unroll
         for (int q = 0; q < KS; ++q)
-            if (q < nq)
-                dist[at + q * nc] = accept_dist(DistBits<T>::of(acc[q]), limit, nvalid);
+            if (at + q * nc < end)
+                dist[at + q * nc] = accept_dist(DistBits<T>::of(d[q]), accept, nvalid);
     }
     __syncwarp();
     n_cand += static_cast<unsigned>(ngrid);  // grid minus self, plus (0, 0)
 
-    return select_group<T>(a, dist, ngrid, nc, nc_div, tp, l, st, j0, i0, lane, nvalid, heap, list,
-                           lkeys, n_fix);
+    // The exact distance of a list place, in the reference's order.
+    auto exact = [&](int i) -> B {
+        const T *cb;
+        int cp = t.pitch;
+        if (i < ngrid) {
+            const int rr = div_magic(i, nc_div);
+            cb = t.refw[0] + (tp + rr * st - t.ry0) * t.pitch + (l + (i - rr * nc) * st - t.rx0);
+        } else {
+            cb = block_ptr(t, t.refw[0], t.ref0[0], 0, 0, cp);
+        }
+        T acc = T(0);
+#pragma unroll 1
+        for (int y = 0; y < kBS; ++y) {
+            T r[kBS], c[kBS];
+#pragma unroll
+            for (int x = 0; x < kBS; ++x) {
+                r[x] = rb[y * t.pitch + x];
+                c[x] = cb[y * cp + x];
+            }
+            acc = ssd_row8(acc, r, c);
+        }
+        return DistBits<T>::of(acc);
+    };
+    if constexpr (kNearList) {
+        if (a.group_key == nullptr) {
+            const int n = select_group<T, true>(a, dist, limit, exact, ngrid, nc, nc_div, tp, l, st, j0,
+                                                i0, lane, nvalid, heap, list, lkeys, n_fix);
+            if (n > 0) return n;
+        }
+        // rare: the whole list exactly
+        __syncwarp();
+        nvalid = 0;
+        for (int i = lane; i <= ngrid; i += kWarp) dist[i] = accept_dist(exact(i), limit, nvalid);
+        __syncwarp();
+    }
+    return select_group<T, false>(a, dist, limit, exact, ngrid, nc, nc_div, tp, l, st, j0, i0, lane,
+                                  nvalid, heap, list, lkeys, n_fix);
 }
 
 // ---------------------------------------------------------------------------
@@ -1320,16 +1512,18 @@ __device__ __forceinline__ void stage_tile_body(const StageArgs<T> &a, int tile,
     int kx0, kx1, ky0, ky1;
     tile_window(a, tile, kBS, t, kx0, kx1, ky0, ky1);
     const SmemPlan sp = plan_smem<T>(NPL, WIENER, a.ref_alias_src, a.region_h, a.region_pitch,
-                                     a.key_slots, nwarps);
+                                     a.span, nwarps);
     if (sp.total > avail) {  // launched with less shared memory than the layout needs
         smem_shortfall(a);
         return;
     }
     carve_tile<T, WIENER, NPL>(a, sp, smem, t);
+    unsigned *tasks = reinterpret_cast<unsigned *>(smem + sp.off_tasks);
+    unsigned char *wbase = smem + sp.off_warps + sp.warp_bytes * warp;  // per-warp scratch
+    if (KS == kStrip && warp == 0)
+        build_tasks(tasks, reinterpret_cast<unsigned *>(wbase), a.span, t.pitch, lane);
     stage_tile<T, WIENER, NPL>(a, t);
 
-    // Per-warp scratch.
-    unsigned char *wbase = smem + sp.off_warps + sp.warp_bytes * warp;
     T *G = reinterpret_cast<T *>(wbase);
     auto *dist = reinterpret_cast<typename DistBits<T>::type *>(wbase);
     T *refblk = reinterpret_cast<T *>(wbase + sp.off_ref);
@@ -1350,7 +1544,7 @@ __device__ __forceinline__ void stage_tile_body(const StageArgs<T> &a, int tile,
     for (int r = warp; r < nrefs; r += nwarps) {
         const int ky = ky0 + r / tw, kx = kx0 + r % tw;
         const int j0 = ref_pos(ky, a.step, bottom), i0 = ref_pos(kx, a.step, right);
-        const int n = match_block<T, KS>(a, t, j0, i0, lane, dist, refblk, heap, list, lkeys, n_cand,
+        const int n = match_block<T, KS>(a, t, j0, i0, lane, tasks, dist, refblk, heap, list, lkeys, n_cand,
                                        n_fix);
         n_sum += n;
         n_sq += static_cast<unsigned>(n * n);
@@ -1446,7 +1640,7 @@ __device__ __forceinline__ void stage_tile_body_seq3(const StageArgs<T> &a, int 
     int kx0, kx1, ky0, ky1;
     tile_window(a, tile, kBS, t, kx0, kx1, ky0, ky1);
     const SmemPlan sp = plan_smem<T>(3, WIENER, a.ref_alias_src, a.region_h, a.region_pitch,
-                                     a.key_slots, nwarps, false, kBS, kGSMax,
+                                     a.span, nwarps, false, kBS, kGSMax,
                                      a.tile_x * a.tile_y);
     if (sp.total > avail) {  // launched with less shared memory than the layout needs
         smem_shortfall(a);
@@ -1458,6 +1652,7 @@ __device__ __forceinline__ void stage_tile_body_seq3(const StageArgs<T> &a, int 
     unsigned short *gpos = reinterpret_cast<unsigned short *>(smem + sp.off_groups);
     unsigned char *gn = reinterpret_cast<unsigned char *>(gpos + a.tile_x * a.tile_y * kGSMax);
 
+    unsigned *tasks = reinterpret_cast<unsigned *>(smem + sp.off_tasks);
     unsigned char *wbase = smem + sp.off_warps + sp.warp_bytes * warp;
     T *G = reinterpret_cast<T *>(wbase);
     auto *dist = reinterpret_cast<typename DistBits<T>::type *>(wbase);
@@ -1465,6 +1660,9 @@ __device__ __forceinline__ void stage_tile_body_seq3(const StageArgs<T> &a, int 
     SortKey<T> *heap = reinterpret_cast<SortKey<T> *>(wbase + sp.off_heap);
     T *lkeys = reinterpret_cast<T *>(wbase + sp.off_keys);
     BlockPos *list = reinterpret_cast<BlockPos *>(wbase + sp.off_list);
+
+    if (KS == kStrip && warp == 0)
+        build_tasks(tasks, reinterpret_cast<unsigned *>(wbase), a.span, t.pitch, lane);
 
     // per-tile counters (small: 32 bits suffice), flushed once per tile
     unsigned n_sum = 0, n_sq = 0, n_cand = 0, n_fix = 0, n_bad = 0;
@@ -1480,7 +1678,7 @@ __device__ __forceinline__ void stage_tile_body_seq3(const StageArgs<T> &a, int 
             if (c == 0) {
                 const int ky = ky0 + r / tw, kx = kx0 + r % tw;
                 const int j0 = ref_pos(ky, a.step, bottom), i0 = ref_pos(kx, a.step, right);
-                n = match_block<T, KS>(a, t, j0, i0, lane, dist, refblk, heap, list, lkeys, n_cand,
+                n = match_block<T, KS>(a, t, j0, i0, lane, tasks, dist, refblk, heap, list, lkeys, n_cand,
                                        n_fix);
                 n_sum += n;
                 n_sq += static_cast<unsigned>(n * n);

@@ -62,3 +62,31 @@ def _check(ctx, oracle_mod, p, plane, value_range):
     for r, n in enumerate(count):
         assert np.array_equal(pos[r, :n], want[1][r, :n]), r
         assert np.array_equal(keys[r, :n], want[2][r, :n]), r
+
+
+# FP32 lists hold approximate distances where their order decides the group.
+# Keys scaled by a power of two to just above the subnormal range keep every
+# mantissa but lie where the approximation is not used, so the same call with
+# value_range * 2^67 and thMSE * 2^-134 takes exact distances throughout.
+@pytest.mark.parametrize("wiener", [False, True])
+@pytest.mark.parametrize("bm_range,group_size,shape", [(1, 2, (40, 41)), (3, 16, (24, 71)),
+                                                       (9, 16, (8, 8)), (9, 16, (75, 91)),
+                                                       (9, 17, (50, 64)), (10, 32, (64, 60)),
+                                                       (16, 32, (70, 83))])
+def test_approximate_order_equals_exact(ctx, bm_range, group_size, shape, wiener):
+    import torch
+    import isp_mw_b200
+    rng = np.random.default_rng(bm_range * 100 + group_size)
+    plane = torch.from_numpy((0.5 + 0.09 * rng.standard_normal(shape)).astype(np.float32)).cuda()
+    out = []
+    for k in (0, 67):
+        p = isp_mw_b200.stage_params_default("fast", wiener, [40.0] * 3)
+        p.bm_range, p.group_size, p.block_step = bm_range, group_size, 3
+        p.thMSE = 1e4 * 2.0 ** (-2 * k)
+        dst = torch.zeros_like(plane)
+        ctx.stage(p, wiener, dst, plane, plane.clone() if wiener else None, 2.0 ** k)
+        out.append(dst)
+        stats = ctx.last_stats()
+        assert stats[0] > 0
+    assert torch.equal(out[0], out[1])
+    assert not torch.equal(out[0], plane)
