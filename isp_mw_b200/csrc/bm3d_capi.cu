@@ -269,6 +269,7 @@ extern "C" const char *bm3d_last_error(const bm3d_ctx *ctx)
 extern "C" int bm3d_set_tiling(bm3d_ctx *ctx, int tile_x, int tile_y, int warps)
 {
     if (!ctx || tile_x < 0 || tile_y < 0 || warps < 0 || warps > 16) return BM3D_ERR_INVALID;
+    if (tile_x || tile_y || warps) ctx->tiling_set = true;
     if (tile_x) ctx->tile_x = tile_x;
     if (tile_y) ctx->tile_y = tile_y;
     if (warps) ctx->warps = warps;
@@ -507,6 +508,59 @@ template <> struct GenericTables<double> {
     static const double *inv(const bm3d_ctx *c) { return c->gtab_d ? c->gtab_d + kDctTableSize : nullptr; }
 };
 
+// Tile shapes offered to a stage: reference blocks per tile (tx x ty, a multiple
+// of the warps, so no warp idles in a tile's last round) and warps per CTA.
+struct TileShape {
+    int tx, ty, warps;
+};
+
+// Window geometry and shared memory of a stage at one tile shape.
+template <typename T>
+static SmemPlan plan_tile(StageArgs<T> &a, const bm3d_stage_params *p, bool wiener, int nplanes,
+                          const TileShape &t)
+{
+    const int BS = p->block_size;
+    const int reach = a.match ? a.range : 0;
+    a.region_w = std::min(a.width, (t.tx - 1) * a.step + 2 * reach + BS);
+    a.region_h = std::min(a.height, (t.ty - 1) * a.step + 2 * reach + BS);
+    a.region_pitch = window_pitch(a.region_w);
+    a.tile_x = std::min(t.tx, a.nx);
+    a.tile_y = std::min(t.ty, a.ny);
+    a.tiles_x = (a.nx + a.tile_x - 1) / a.tile_x;
+    return plan_smem<T>(nplanes, wiener, a.ref_alias_src, a.region_h, a.region_pitch, a.span, t.warps,
+                        !fast_args(BS, p->group_size), BS, p->group_size, a.tile_x * a.tile_y);
+}
+
+// Predicted time of a stage at one tile shape (microseconds; only the order
+// matters). A warp takes 8.5 us for a reference block when its SM runs few
+// warps and 12 us with 16 (fast profile); a tile adds about 10 us of staging,
+// flushing and waiting for its last warp, which other CTAs of the SM overlap;
+// CTAs run in waves, whose rounding up fades once there are several. Measured
+// at 64 x 64 .. 3840 x 2160, one shape for all sizes (8 x 8, 16 warps) against
+// the shapes this picks, basic / final stage: 64 x 64 60 / 67 -> 20 / 23 us,
+// 512 x 512 72 / 88 -> 49 / 65 us, 1280 x 720 128 / 197 -> 113 / 177 us,
+// 1920 x 1080 245 / 343 -> 225 / 329 us.
+template <typename T>
+static double tile_cost(const bm3d_ctx *ctx, const StageArgs<T> &a, const SmemPlan &sp,
+                        const TileShape &t, int nplanes, bool generic)
+{
+    const size_t sm_smem = ctx->smem_optin + 1024;  // an SM's share; 1 KB of it per CTA is reserved
+    const int regs = sizeof(T) == 8 ? 256 : generic ? 168 : 128;
+    const int by_smem = static_cast<int>(sm_smem / (sp.total + 1024));
+    const int by_regs = 65536 / (t.warps * kWarp * regs);
+    const int per_sm = std::max(1, std::min(by_smem, by_regs));
+    const double tiles = static_cast<double>(a.tiles_x) * ((a.ny + a.tile_y - 1) / a.tile_y);
+    const double share = tiles / ctx->sm_count;  // tiles per SM
+    const int busy = std::min(per_sm, std::max(1, static_cast<int>(std::ceil(share)))) * t.warps;
+    // matching is about a third of a block's time at BMrange 9
+    const double work = (0.65 + 0.35 * a.span * a.span / 361.0) * (nplanes == 3 ? 1.9 : 1.0);
+    const double round = (8.5 + 0.22 * busy) * work;
+    const int rounds = (a.tile_x * a.tile_y + t.warps - 1) / t.warps;
+    const double x = share / per_sm;
+    const double waves = x < 4.0 ? std::ceil(x) : x + 0.5;
+    return waves * (rounds * round + (8.0 + rounds + 0.1 * t.warps) * nplanes);
+}
+
 // Geometry, tiling and shared-memory fit.
 template <typename T>
 static int plan_geometry(bm3d_ctx *ctx, StageArgs<T> &a, const bm3d_stage_params *p, bool wiener,
@@ -524,52 +578,59 @@ static int plan_geometry(bm3d_ctx *ctx, StageArgs<T> &a, const bm3d_stage_params
     a.nx = ref_count(width - BS, a.step);
     a.ny = ref_count(height - BS, a.step);
     a.span = 2 * (a.range / a.bm_step) + 1;
-    // The generic kernel (launch bounds 384 in FP32, 256 in FP64) takes the
-    // first of these (tile_x, tile_y, warps) that fits: reference blocks per
-    // tile a multiple of the warps, so no warp idles in a tile's last round.
-    static const int gen32[][3] = {{6, 4, 12}, {4, 3, 12}, {4, 4, 8}, {4, 4, 4},
-                                   {2, 2, 4},  {2, 2, 2},  {1, 1, 2}, {1, 1, 1}};
-    static const int gen64[][3] = {{4, 4, 8}, {4, 4, 4}, {2, 2, 4}, {2, 2, 2}, {1, 1, 2}, {1, 1, 1}};
-    const int (*gcand)[3] = sizeof(T) == 4 ? gen32 : gen64;
-    const int ngcand = sizeof(T) == 4 ? 8 : 6;
-    int gi = 0;
-    int tx = generic ? gcand[0][0] : ctx->tile_x, ty = generic ? gcand[0][1] : ctx->tile_y;
-    warps = generic ? gcand[0][2] : std::min(ctx->warps, stage_max_warps<T>());
-    for (;;) {
-        const int reach = a.match ? a.range : 0;
-        a.region_w = std::min(width, (tx - 1) * a.step + 2 * reach + BS);
-        a.region_h = std::min(height, (ty - 1) * a.step + 2 * reach + BS);
-        // pitch = 5 (mod 8): block matching's lanes read window rows 4 apart,
-        // and this residue keeps those lane groups on the fewest shared banks
-        a.region_pitch = a.region_w + ((5 - a.region_w % 8) + 8) % 8;
-        const SmemPlan sp = plan_smem<T>(nplanes, wiener, a.ref_alias_src, a.region_h,
-                                         a.region_pitch, a.span, warps, generic, BS,
-                                         p->group_size, std::min(tx, a.nx) * std::min(ty, a.ny));
-        if (sp.total <= ctx->smem_optin) break;
-        if (generic) {
-            if (++gi >= ngcand) {
-                ctx->err = "stage does not fit in shared memory";
-                return BM3D_ERR_UNSUPPORTED;
+    // The launch bounds (register-resident 512 threads in FP32, 256 in FP64;
+    // generic 384 and 256) limit the warps; the small shapes are for windows
+    // that leave no room for more.
+    static const TileShape fast[] = {{2, 2, 4}, {4, 2, 8}, {4, 4, 8}, {4, 8, 8}, {6, 4, 8}, {8, 8, 16}};
+    static const TileShape gen[] = {{6, 4, 12}, {4, 3, 12}, {4, 4, 8}, {4, 2, 8}, {2, 2, 4}, {4, 4, 4}};
+    static const TileShape gen_small[] = {{2, 2, 4}, {2, 2, 2}, {1, 1, 2}, {1, 1, 1}};
+    const int max_warps = generic ? (sizeof(T) == 4 ? 12 : 8) : stage_max_warps<T>();
+    if (generic || !ctx->tiling_set) {
+        TileShape best{0, 0, 0};
+        double least = 1e300;
+        auto offer = [&](const TileShape &t) {
+            if (t.warps > max_warps) return;
+            const SmemPlan sp = plan_tile(a, p, wiener, nplanes, t);
+            if (sp.total > ctx->smem_optin) return;
+            const double c = tile_cost(ctx, a, sp, t, nplanes, generic);
+            if (c < least) {
+                least = c;
+                best = t;
             }
-            tx = gcand[gi][0];
-            ty = gcand[gi][1];
-            warps = gcand[gi][2];
-        } else if (warps > 8) {
-            warps /= 2;
-        } else if (ty > 1 && ty >= tx) {
-            --ty;
-        } else if (tx > 1) {
-            --tx;
-        } else if (warps > 1) {
-            warps /= 2;
+        };
+        if (generic) for (const TileShape &t : gen) offer(t);
+        else for (const TileShape &t : fast) offer(t);
+        if (generic && best.warps == 0)
+            for (const TileShape &t : gen_small)
+                if (best.warps == 0) offer(t);
+        if (best.warps != 0) {
+            plan_tile(a, p, wiener, nplanes, best);
+            warps = best.warps;
+            return BM3D_OK;
+        }
+        if (generic) {
+            ctx->err = "stage does not fit in shared memory";
+            return BM3D_ERR_UNSUPPORTED;
+        }
+    }
+    // a set shape, or none of the usual ones fits: the largest that does
+    TileShape t{ctx->tile_x, ctx->tile_y, std::min(ctx->warps, max_warps)};
+    for (;;) {
+        if (plan_tile(a, p, wiener, nplanes, t).total <= ctx->smem_optin) break;
+        if (t.warps > 8) {
+            t.warps /= 2;
+        } else if (t.ty > 1 && t.ty >= t.tx) {
+            --t.ty;
+        } else if (t.tx > 1) {
+            --t.tx;
+        } else if (t.warps > 1) {
+            t.warps /= 2;
         } else {
             ctx->err = "stage does not fit in shared memory";
             return BM3D_ERR_UNSUPPORTED;
         }
     }
-    a.tile_x = std::min(tx, a.nx);
-    a.tile_y = std::min(ty, a.ny);
-    a.tiles_x = (a.nx + a.tile_x - 1) / a.tile_x;
+    warps = t.warps;
     return BM3D_OK;
 }
 

@@ -177,7 +177,7 @@ int build_stage(bm3d_batch *B, bool wiener, int tx, int ty, int warps, StageBuil
         const int reach = a.match ? a.range : 0;
         a.region_w = std::min(a.width, (tx - 1) * a.step + 2 * reach + BS);
         a.region_h = std::min(a.height, (ty - 1) * a.step + 2 * reach + BS);
-        a.region_pitch = a.region_w + ((5 - a.region_w % 8) + 8) % 8;
+        a.region_pitch = window_pitch(a.region_w);
         a.tile_x = std::min(tx, a.nx);
         a.tile_y = std::min(ty, a.ny);
         a.tiles_x = (a.nx + a.tile_x - 1) / a.tile_x;
@@ -355,9 +355,9 @@ int tune_stage(bm3d_batch *B, StageBuild &sbd, const DevBuf &planes, bool autotu
     const bool generic = !fast_args(p.block_size, p.group_size);
     // reference blocks per tile a multiple of the warps where it can be, so
     // the tile's last round keeps every warp busy
-    static const int fast_cand[][3] = {{8, 8, 16}, {7, 7, 16}, {6, 8, 16}, {8, 6, 16},
-                                       {8, 4, 16}, {6, 8, 12}, {8, 6, 12}, {6, 6, 12},
-                                       {4, 4, 4},  {4, 4, 2},  {2, 2, 1}};
+    static const int fast_cand[][3] = {{4, 8, 8}, {8, 4, 8}, {6, 4, 8}, {4, 4, 8}, {8, 8, 16},
+                                       {6, 8, 16}, {8, 6, 12}, {4, 2, 8}, {2, 2, 4}, {4, 4, 4},
+                                       {2, 2, 1}};
     static const int gen_cand[][3] = {{6, 4, 12}, {4, 3, 12}, {4, 4, 8}, {4, 4, 4},
                                       {2, 2, 4},  {2, 2, 2},  {1, 1, 2}, {1, 1, 1}};
     const int (*cand)[3] = generic ? gen_cand : fast_cand;

@@ -47,6 +47,9 @@ struct bm3d_ctx {
     float *gtab_f = nullptr;          // generic path cosine matrices: fwd | inv (float)
     double *gtab_d = nullptr;         // same in double
     cudaStream_t last_stream = nullptr;
+    // tile shape of the register-resident kernel when the caller sets one
+    // (bm3d_set_tiling); else plan_geometry picks per call
+    bool tiling_set = false;
     int tile_x = 8, tile_y = 8, warps = 16;
     // bm3d_full_many's copy pipeline: two slots of device planes, an upload
     // and a download stream, and the events that order slot reuse

@@ -353,6 +353,22 @@ __host__ __device__ constexpr bool generic_one_buffer(bool wiener, int bs)
     return wiener && bs == 8 && sizeof(T) == 4;
 }
 
+// Row pitch of staged windows w wide: 5, 13, 19 or 27 (mod 32) words. Group
+// members cluster along edges and textures, so gathers and aggregation meet
+// small displacements (dy, dx) again and again; two members share a bank where
+// pitch * dy + dx = 0 (mod 32), and for these residues the shortest such
+// displacement is 5 pixels or more ((3, 1) for 21, the residue many windows
+// had: on planes whose texture runs that way a 4K YUV frame took 6.1 instead
+// of 5.4 ms). They also give 4 * pitch = 20 or 12, which spreads block
+// matching's strips over the banks (build_tasks).
+__host__ __device__ inline int window_pitch(int w)
+{
+    for (;; ++w) {
+        const int r = w & 31;
+        if (r == 5 || r == 13 || r == 19 || r == 27) return w;
+    }
+}
+
 // Shared-memory layout of one CTA. The register-resident kernel runs three
 // planes one after another through a single plane's windows: it then also
 // keeps the tile's group lists, per reference block kGSMax 16-bit positions

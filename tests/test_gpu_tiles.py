@@ -1,0 +1,40 @@
+"""The tile shape a call picks from its size changes nothing but the time:
+results equal one fixed shape's bit for bit (sums are exact integers), from
+one block to several waves of tiles, for one and three planes and for the
+profiles of both kernels."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("planes", [1, 3])
+@pytest.mark.parametrize("profile,shape", [("fast", (8, 8)), ("fast", (9, 70)), ("fast", (64, 64)),
+                                           ("fast", (203, 301)), ("fast", (520, 519)),
+                                           ("fast", (720, 1280)), ("lc", (333, 222)),
+                                           ("np", (50, 61)), ("np", (220, 230)), ("vn", (130, 90))])
+def test_picked_shape_equals_fixed_shape(bm3d_lib, profile, shape, planes):
+    import torch
+    import isp_mw_b200
+    from isp_mw_b200 import synth
+    h, w = shape
+    src = [torch.from_numpy(synth.pair(h, w, 20.0, 40 + c)[1]).cuda() for c in range(planes)]
+    sp = [30.0, 20.0, 20.0]
+    b = isp_mw_b200.stage_params_default(profile, False, sp)
+    f = isp_mw_b200.stage_params_default(profile, True, sp)
+    out = []
+    for fixed in (None, (8, 8, 16), (3, 5, 2)):
+        ctx = isp_mw_b200.Context(0)
+        if fixed:
+            ctx.set_tiling(*fixed)
+        dst = [torch.zeros_like(p) for p in src]
+        if planes == 1:
+            ctx.full(b, f, dst[0], src[0])
+        else:
+            ctx.full3(b, f, dst, src)
+        ctx.check()
+        out.append(dst)
+        ctx.close()
+    for other in out[1:]:
+        for p, q in zip(out[0], other):
+            assert torch.equal(p, q)
