@@ -38,3 +38,23 @@ def test_picked_shape_equals_fixed_shape(bm3d_lib, profile, shape, planes):
     for other in out[1:]:
         for p, q in zip(out[0], other):
             assert torch.equal(p, q)
+
+
+@pytest.mark.parametrize("block", [1, 5, 8, 11, 16])
+@pytest.mark.parametrize("shape", [(16, 64), (17, 65), (33, 63), (16, 129), (31, 20), (50, 192)])
+def test_normalisation_tile_edges(bm3d_lib, oracle_mod, shape, block):
+    """One stage at sizes around the normalisation's 64 x 16 tiles, for the
+    block sizes its windows hold, against the oracle."""
+    import isp_mw_b200
+    from isp_mw_b200 import synth
+    h, w = shape
+    noisy = synth.pair(h, w, 20.0, 5)[1]
+    p = isp_mw_b200.stage_params_default("fast", False, [30.0] * 3)
+    p.block_size, p.block_step, p.group_size, p.bm_range = block, max(1, block // 2), 4, 3
+    ctx = isp_mw_b200.Context(0)
+    out = np.empty_like(noisy)
+    ctx.stage(p, False, out, noisy)
+    ctx.close()
+    want = oracle_mod.backend("port", np.float32).stage(False, p.as_dict(), noisy)
+    want = want[1] if isinstance(want, tuple) else want
+    assert np.abs(out - want).max() <= 1e-3
