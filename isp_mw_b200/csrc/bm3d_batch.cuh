@@ -43,61 +43,21 @@ __global__ void __launch_bounds__(GENERIC ? (sizeof(T) == 4 ? 384 : 256) : stage
     }
 }
 
-// One plane of a batch, for the per-pixel kernels.
-template <typename T> struct BatchPlane {
-    typename AccOf<T>::type *num, *den;
-    const T *src;
-    const T *ref;              // counted for non-finite pixels too when not null
-    T *dst;
-    long long src_stride, dst_stride;
-    int width, height;
-    int block_size;
-    float *absmax;
-    int log2_bound, log2_corner;  // fixed-point bounds of the stage (StageArgs)
-    unsigned *nonfinite;       // non-finite src / ref pixels (may be null)
-    unsigned char *poison;     // pixels a non-finite term reached (may be null; all zero
-                               // between stages: normalize_tile clears what it reads)
-};
-
 // Zero each plane's sums, fold its max finite |src| and count its non-finite
 // pixels (grid.y = plane).
-template <typename T>
-__global__ void prep_batch_kernel(const BatchPlane<T> *planes)
+template <typename T> __global__ void prep_batch_kernel(const PlaneJob<T> *planes)
 {
-    const BatchPlane<T> q = planes[blockIdx.y];
-    prep_plane<T>(q.num, q.den, q.src, q.ref, q.src_stride, q.width, q.height, q.absmax,
-                  q.nonfinite, blockIdx.x, gridDim.x);
+    prep_plane<T>(planes[blockIdx.y], blockIdx.x, gridDim.x);
 }
 
-// dst = num / den for every plane (grid.y = plane), each CTA walking the
-// plane's tiles from blockIdx.x in steps of gridDim.x.
+// dst = num / den for every plane (grid.y = plane), a CTA per tile; planes
+// smaller than the grid leave CTAs without one.
 template <typename T>
-__global__ void __launch_bounds__(256) normalize_batch_kernel(const BatchPlane<T> *planes)
+__global__ void __launch_bounds__(256) normalize_batch_kernel(const PlaneJob<T> *planes)
 {
-    const BatchPlane<T> q = planes[blockIdx.y];
-    if constexpr (std::is_same<T, float>::value) {
-        __shared__ FixedSmem sm;
-        const int tx = fixed_tiles_x(q.width), tiles = fixed_tiles(q.width, q.height);
-        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-            const int ty = tile / tx, y0 = ty * kFixH, x0 = (tile - ty * tx) * kFixW;
-            if (q.block_size == kBS)
-                normalize_fixed<kBS>(sm, q.dst, q.dst_stride, q.num, q.den, q.width, q.height, kBS, y0, x0,
-                                     q.poison, q.nonfinite, q.absmax, q.log2_bound, q.log2_corner);
-            else
-                normalize_fixed<0>(sm, q.dst, q.dst_stride, q.num, q.den, q.width, q.height, q.block_size,
-                                   y0, x0, q.poison, q.nonfinite, q.absmax, q.log2_bound,
-                                   q.log2_corner);
-        }
-        return;
-    }
-    const int tx = (q.width + kNormTile - 1) / kNormTile;
-    const int ntiles = tx * ((q.height + kNormTile - 1) / kNormTile);
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int ty = tile / tx, txi = tile - ty * tx;
-        normalize_tile<T>(q.dst, q.dst_stride, q.num, q.den, q.width, q.height, q.block_size,
-                          ty * kNormTile, txi * kNormTile, q.poison, q.nonfinite, q.absmax,
-                          q.log2_bound, q.log2_corner);
-    }
+    const PlaneJob<T> q = planes[blockIdx.y];
+    if (static_cast<int>(blockIdx.x) < normalize_tiles<T>(q.width, q.height))
+        normalize_job(q, static_cast<int>(blockIdx.x));
 }
 
 }  // namespace bm3d

@@ -175,20 +175,16 @@ extern "C" int bm3d_ctx_create(bm3d_ctx **out, int device)
         delete ctx;
         return cuda_fail(nullptr, e, "upload_dct_tables");
     }
-    e = cudaMalloc(&ctx->stats, kStats * sizeof(unsigned long long));
+    e = cudaMalloc(&ctx->head, kHeadBytes);
     if (e != cudaSuccess) {
         delete ctx;
-        return cuda_fail(nullptr, e, "cudaMalloc(stats)");
+        return cuda_fail(nullptr, e, "cudaMalloc(head)");
     }
-    cudaMemset(ctx->stats, 0, kStats * sizeof(unsigned long long));
-    e = cudaMalloc(&ctx->absmax, kMaxPlanes * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->nonfinite, kMaxPlanes * sizeof(unsigned));
-    if (e != cudaSuccess) {
-        cudaFree(ctx->stats);
-        if (ctx->absmax) cudaFree(ctx->absmax);
-        delete ctx;
-        return cuda_fail(nullptr, e, "cudaMalloc(absmax)");
-    }
+    cudaMemset(ctx->head, 0, kHeadBytes);
+    ctx->absmax = reinterpret_cast<float *>(ctx->head);
+    ctx->nonfinite = reinterpret_cast<unsigned *>(ctx->head) + kMaxPlanes;
+    ctx->nonfinite_next = ctx->nonfinite + kMaxPlanes;
+    ctx->stats = reinterpret_cast<unsigned long long *>(ctx->head + kHeadStats);
     // cosine matrices of lengths 1..32 for the generic path
     {
         std::vector<float> tf(2 * kDctTableSize);
@@ -213,9 +209,7 @@ extern "C" int bm3d_ctx_create(bm3d_ctx **out, int device)
         if (e == cudaSuccess)
             e = cudaMemcpy(ctx->gtab_d, td.data(), td.size() * sizeof(double), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) {
-            cudaFree(ctx->stats);
-            cudaFree(ctx->absmax);
-            cudaFree(ctx->nonfinite);
+            cudaFree(ctx->head);
             cudaFree(ctx->gtab_f);
             cudaFree(ctx->gtab_d);
             delete ctx;
@@ -235,6 +229,7 @@ extern "C" void bm3d_ctx_destroy(bm3d_ctx *ctx)
         b.ptr = nullptr;
     };
     for (auto &b : ctx->acc) fr(b);
+    for (auto &b : ctx->den_next) fr(b);
     for (auto &b : ctx->basic) fr(b);
     for (auto &b : ctx->stage_in) fr(b);
     for (auto &b : ctx->stage_ref) fr(b);
@@ -251,9 +246,7 @@ extern "C" void bm3d_ctx_destroy(bm3d_ctx *ctx)
     }
     if (ctx->up) cudaStreamDestroy(ctx->up);
     if (ctx->down) cudaStreamDestroy(ctx->down);
-    if (ctx->stats) cudaFree(ctx->stats);
-    if (ctx->absmax) cudaFree(ctx->absmax);
-    if (ctx->nonfinite) cudaFree(ctx->nonfinite);
+    if (ctx->head) cudaFree(ctx->head);
     if (ctx->gtab_f) cudaFree(ctx->gtab_f);
     if (ctx->gtab_d) cudaFree(ctx->gtab_d);
     drain_timing(ctx);
@@ -634,13 +627,18 @@ static int plan_geometry(bm3d_ctx *ctx, StageArgs<T> &a, const bm3d_stage_params
     return BM3D_OK;
 }
 
+// How a stage call relates to another one: a basic stage that also prepares
+// the final stage that follows on the same planes, and that final stage
+// (PlaneJob's *_next). Saves the final stage's preparation pass and resets.
+enum class Chain { None, Leads, Follows };
+
 // One stage over device-resident planes (all with row pitch `stride`).
 template <typename T>
 static int run_stage_device(bm3d_ctx *ctx, const bm3d_stage_params *p, bool wiener, int nplanes,
                             T *const dst[], const T *const src[], const T *const ref[], int width,
                             int height, size_t stride, double value_range, cudaStream_t s,
-                            int *gcount = nullptr, int *gpos = nullptr, T *gkey = nullptr,
-                            bool bm_only = false)
+                            Chain chain = Chain::None, int *gcount = nullptr, int *gpos = nullptr,
+                            T *gkey = nullptr, bool bm_only = false)
 {
     StageArgs<T> a;
     std::memset(&a, 0, sizeof(a));
@@ -668,51 +666,63 @@ static int run_stage_device(bm3d_ctx *ctx, const bm3d_stage_params *p, bool wien
     // FP32 sums are fixed point: planes with NaN / Inf pixels take the checking
     // aggregation (FP64 sums are doubles and carry them like the reference's)
     constexpr bool kFixed = std::is_same<Acc, long long>::value;
-    a.nonfinite = kFixed ? ctx->nonfinite : nullptr;
-    if (!bm_only) {
-        CK(ctx, cudaMemsetAsync(ctx->absmax, 0, kMaxPlanes * sizeof(float), s));
-        CK(ctx, cudaMemsetAsync(ctx->nonfinite, 0, kMaxPlanes * sizeof(unsigned), s));
-    }
+    const bool follows = chain == Chain::Follows, leads = chain == Chain::Leads;
+    a.nonfinite = !kFixed ? nullptr : follows ? ctx->nonfinite_next : ctx->nonfinite;
+    a.stats = ctx->stats;
+    a.bad = ctx->stats + 4;
+    // per-call state and counters; the invariant counter (stats[4]) is sticky
+    if (!follows) CK(ctx, cudaMemsetAsync(ctx->head, 0, kHeadClear, s));
+    PlaneJobs<T> jobs;
+    std::memset(&jobs, 0, sizeof(jobs));
+    int njobs = 0;
     for (int c = 0; c < nplanes; ++c) {
         if (!(a.active & (1 << c)) && !bm_only) continue;
+        DevBuf &den = follows ? ctx->den_next[c] : ctx->acc[2 * c + 1];
         if ((rc = ensure(ctx, ctx->acc[2 * c], acc_bytes)) != BM3D_OK) return rc;
-        if ((rc = ensure(ctx, ctx->acc[2 * c + 1], acc_bytes)) != BM3D_OK) return rc;
+        if ((rc = ensure(ctx, den, acc_bytes)) != BM3D_OK) return rc;
+        if (leads && (rc = ensure(ctx, ctx->den_next[c], acc_bytes)) != BM3D_OK) return rc;
         a.num[c] = static_cast<Acc *>(ctx->acc[2 * c].ptr);
-        a.den[c] = static_cast<Acc *>(ctx->acc[2 * c + 1].ptr);
+        a.den[c] = static_cast<Acc *>(den.ptr);
         if (kFixed) {  // starts zeroed; normalisation leaves it zero
             const bool grow = ctx->poison[c].bytes < static_cast<size_t>(npx);
             if ((rc = ensure(ctx, ctx->poison[c], static_cast<size_t>(npx))) != BM3D_OK) return rc;
             if (grow) CK(ctx, cudaMemsetAsync(ctx->poison[c].ptr, 0, ctx->poison[c].bytes, s));
             a.poison[c] = static_cast<unsigned char *>(ctx->poison[c].ptr);
         }
-        if (!bm_only) {
-            prep_kernel<T><<<std::min(height, blocks), threads, 0, s>>>(
-                a.num[c], a.den[c], src[c], static_cast<long long>(stride), width, height,
-                ctx->absmax + c, ref[c] != src[c] ? ref[c] : nullptr,
-                kFixed ? ctx->nonfinite + c : nullptr);
-            CK(ctx, cudaGetLastError());
+        PlaneJob<T> &q = jobs.job[njobs++];
+        q.num = a.num[c];
+        q.den = a.den[c];
+        q.src = src[c];
+        q.ref = ref[c] != src[c] ? ref[c] : nullptr;
+        q.dst = dst[c];
+        q.src_stride = q.dst_stride = static_cast<long long>(stride);
+        q.width = width;
+        q.height = height;
+        q.block_size = a.block_size;
+        q.absmax = ctx->absmax + c;
+        q.log2_bound = a.log2_bound;
+        q.log2_corner = a.log2_corner;
+        q.nonfinite = kFixed ? const_cast<unsigned *>(a.nonfinite) + c : nullptr;
+        q.poison = a.poison[c];
+        if (leads) {
+            q.den_next = static_cast<long long *>(ctx->den_next[c].ptr);
+            q.nonfinite_next = ctx->nonfinite_next + c;
+            if (njobs == 1) q.stats = ctx->stats;
         }
+    }
+    if (!bm_only && !follows) {
+        prep_kernel<T><<<dim3(std::min(height, blocks), njobs), threads, 0, s>>>(jobs);
+        CK(ctx, cudaGetLastError());
     }
     a.group_count = gcount;
     a.group_pos = gpos;
     a.group_key = gkey;
     a.bm_only = bm_only ? 1 : 0;
-    a.stats = ctx->stats;
-    a.bad = ctx->stats + 4;
-    // per-stage counters; the invariant counter (stats[4]) is sticky
-    CK(ctx, cudaMemsetAsync(ctx->stats, 0, 4 * sizeof(unsigned long long), s));
     if ((rc = launch_stage(ctx, a, wiener, nplanes, s, warps)) != BM3D_OK) return rc;
     ctx->last_stream = s;
     if (bm_only) return BM3D_OK;
-    for (int c = 0; c < nplanes; ++c) {
-        if (!(a.active & (1 << c))) continue;
-        const dim3 ngrid = normalize_grid<T>(width, height);
-        normalize_kernel<T><<<ngrid, 256, 0, s>>>(dst[c], static_cast<long long>(stride), a.num[c],
-                                                  a.den[c], width, height, a.block_size,
-                                                  a.poison[c], a.nonfinite ? a.nonfinite + c : nullptr,
-                                                  ctx->absmax + c, a.log2_bound, a.log2_corner);
-        CK(ctx, cudaGetLastError());
-    }
+    normalize_kernel<T><<<dim3(normalize_tiles<T>(width, height), njobs), 256, 0, s>>>(jobs);
+    CK(ctx, cudaGetLastError());
     return BM3D_OK;
 }
 
@@ -905,45 +915,50 @@ int bm3d::full_any(bm3d_ctx *ctx, const bm3d_stage_params *basic, const bm3d_sta
         if (own_ref) dr[0] = ref[0];
     }
     // Planes a stage does not filter (sigma <= 0), or a stage whose parameters
-    // the reference's guard rejects, pass src through: the basic estimate and
-    // dst start as copies of src, as in the reference's in-place Frame path
+    // the reference's guard rejects, pass src through: there the basic estimate
+    // and dst are copies of src, as in the reference's in-place Frame path
     // (source/BM3D.cpp:512-521).
+    const Guard gb = check_params(basic, nplanes), gf = check_params(fin, nplanes);
+    auto filtered = [&](const bm3d_stage_params *p, Guard g, int c) {
+        return g == Guard::Run && (nplanes == 1 || p->sigma[c] > 0);
+    };
     for (int c = 0; c < nplanes; ++c) {
-        if ((rc = copy_plane(ctx, tmp[c], dpitch, ds[c], dpitch, width, height,
+        if (!filtered(basic, gb, c) &&
+            (rc = copy_plane(ctx, tmp[c], dpitch, ds[c], dpitch, width, height,
                              cudaMemcpyDeviceToDevice, s)) != BM3D_OK)
             return rc;
-        if (nplanes > 1 || check_params(fin, nplanes) != Guard::Run)
-            if ((rc = copy_plane(ctx, dd[c], dpitch, ds[c], dpitch, width, height,
-                                 cudaMemcpyDeviceToDevice, s)) != BM3D_OK)
-                return rc;
+        if (!filtered(fin, gf, c) &&
+            (rc = copy_plane(ctx, dd[c], dpitch, ds[c], dpitch, width, height,
+                             cudaMemcpyDeviceToDevice, s)) != BM3D_OK)
+            return rc;
     }
-    {
-        const Guard g = check_params(basic, nplanes);
+    auto refused = [&](Guard g) {
         if (g == Guard::Invalid) return BM3D_ERR_INVALID;
         if (g == Guard::Unsupported) {
             ctx->err = "parameters outside this build (BlockSize <= 16, GroupSize <= 32)";
             return BM3D_ERR_UNSUPPORTED;
         }
-        if (g == Guard::Run) {
-            rc = run_stage_device(ctx, basic, false, nplanes, tmp, ds, dr, width, height, dpitch,
-                                  value_range, s);
-            if (rc != BM3D_OK) return rc;
-        }
+        return BM3D_OK;
+    };
+    // both stages on the same planes with fixed-point sums: the basic stage's
+    // passes prepare the final stage
+    bool chained = std::is_same<typename AccOf<T>::type, long long>::value && gb == Guard::Run &&
+                   gf == Guard::Run;
+    for (int c = 0; c < nplanes; ++c)
+        chained = chained && filtered(basic, gb, c) == filtered(fin, gf, c);
+    if ((rc = refused(gb)) != BM3D_OK) return rc;
+    if (gb == Guard::Run) {
+        rc = run_stage_device(ctx, basic, false, nplanes, tmp, ds, dr, width, height, dpitch,
+                              value_range, s, chained ? Chain::Leads : Chain::None);
+        if (rc != BM3D_OK) return rc;
     }
-    {
-        const Guard g = check_params(fin, nplanes);
-        if (g == Guard::Invalid) return BM3D_ERR_INVALID;
-        if (g == Guard::Unsupported) {
-            ctx->err = "parameters outside this build (BlockSize <= 16, GroupSize <= 32)";
-            return BM3D_ERR_UNSUPPORTED;
-        }
+    if ((rc = refused(gf)) != BM3D_OK) return rc;
+    if (gf == Guard::Run) {
         const T *tr[kMaxPlanes];
         for (int c = 0; c < nplanes; ++c) tr[c] = tmp[c];
-        if (g == Guard::Run) {
-            rc = run_stage_device(ctx, fin, true, nplanes, dd, ds, tr, width, height, dpitch,
-                                  value_range, s);
-            if (rc != BM3D_OK) return rc;
-        }
+        rc = run_stage_device(ctx, fin, true, nplanes, dd, ds, tr, width, height, dpitch,
+                              value_range, s, chained ? Chain::Follows : Chain::None);
+        if (rc != BM3D_OK) return rc;
     }
     if (mem == BM3D_MEM_HOST) {
         for (int c = 0; c < nplanes; ++c)
@@ -1014,7 +1029,7 @@ extern "C" int bm3d_debug_groups(bm3d_ctx *ctx, const bm3d_stage_params *p, int 
     float *d[1] = {in};
     const float *sp[1] = {in};
     rc = run_stage_device<float>(ctx, p, wiener != 0, 1, d, sp, sp, width, height, width,
-                                 value_range, s, static_cast<int *>(ctx->groups[0].ptr),
+                                 value_range, s, Chain::None, static_cast<int *>(ctx->groups[0].ptr),
                                  static_cast<int *>(ctx->groups[1].ptr),
                                  static_cast<float *>(ctx->groups[2].ptr), true);
     if (rc != BM3D_OK) return rc;
@@ -1235,16 +1250,28 @@ extern "C" int bm3d_stage_noalloc(const bm3d_stage_params *params, int wiener, f
     // (stats[4]) is left alone so bm3d_noalloc_check sees every call
     if ((e = cudaMemsetAsync(absmax, 0, kNoAllocClearBytes, s)) != cudaSuccess)
         return noalloc_error("cudaMemsetAsync(scratch header)", e);
-    prep_kernel<float><<<std::min(height, blocks), threads, 0, s>>>(
-        num, den, src, a.stride, width, height, absmax, ref != src ? ref : nullptr, nonfinite);
+    PlaneJobs<float> jobs;
+    std::memset(&jobs, 0, sizeof(jobs));
+    PlaneJob<float> &q = jobs.job[0];
+    q.num = num;
+    q.den = den;
+    q.src = src;
+    q.ref = ref != src ? ref : nullptr;
+    q.dst = dst;
+    q.src_stride = q.dst_stride = a.stride;
+    q.width = width;
+    q.height = height;
+    q.block_size = a.block_size;
+    q.absmax = absmax;
+    q.log2_bound = a.log2_bound;
+    q.log2_corner = a.log2_corner;
+    q.nonfinite = nonfinite;
+    q.poison = poison;
+    prep_kernel<float><<<std::min(height, blocks), threads, 0, s>>>(jobs);
     if ((e = cudaGetLastError()) != cudaSuccess) return noalloc_error("prep_kernel", e);
     rc = launch_stage(&info, a, wiener != 0, 1, s, warps);
     if (rc != BM3D_OK) return noalloc_error(info.err.c_str(), cudaSuccess, rc);
-    const dim3 ngrid = normalize_grid<float>(width, height);
-    normalize_kernel<float><<<ngrid, 256, 0, s>>>(
-        dst, a.stride, num, den, width, height,
-                                                  a.block_size, poison, nonfinite, absmax,
-                                                  a.log2_bound, a.log2_corner);
+    normalize_kernel<float><<<normalize_tiles<float>(width, height), 256, 0, s>>>(jobs);
     if ((e = cudaGetLastError()) != cudaSuccess) return noalloc_error("normalize_kernel", e);
     return BM3D_OK;
 }

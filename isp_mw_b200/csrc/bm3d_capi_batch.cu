@@ -121,8 +121,25 @@ struct bm3d_batch {
     std::vector<bm3d_stage_params> pb, pf;
     std::vector<Guard> gb, gf;
     std::vector<size_t> acc_off, basic_off;  // per plane: offsets into acc (int64) and basic (float)
-    DevBuf acc, basic, absmax, counters, planes_b, planes_f;
-    DevBuf nonfinite, poison;  // per plane: non-finite input pixels; pixels they reached
+    std::vector<size_t> next_off;            // and into den_next (int64; even, so 16-byte aligned)
+    DevBuf acc, basic, planes_b, planes_f;
+    // reset at the start of every run, in one piece: per plane |src|'s maximum, the
+    // non-finite pixels of the basic stage's inputs and of the final stage's, then
+    // the two stages' work counters
+    DevBuf head;
+    DevBuf poison;     // per plane: pixels a non-finite term reached
+    DevBuf den_next;   // weight sums of the final stage when the basic stage prepares it
+    bool chained = false;  // every plane is filtered by both stages (PlaneJob's *_next)
+    float *absmax() const { return static_cast<float *>(head.ptr); }
+    unsigned *nonfinite(bool final_stage) const
+    {
+        return static_cast<unsigned *>(head.ptr) + static_cast<size_t>(n) * npl * (final_stage ? 2 : 1);
+    }
+    int *counter(bool final_stage) const
+    {
+        return static_cast<int *>(head.ptr) + static_cast<size_t>(n) * npl * 3 + (final_stage ? 1 : 0);
+    }
+    size_t head_bytes() const { return sizeof(int) * (static_cast<size_t>(n) * npl * 3 + 2); }
     std::vector<size_t> poison_off;  // per plane: offset into poison (bytes)
     // final-stage-only batches: the caller's reference planes (e.g. the learned
     // pilot's estimates) stand in for the basic estimates; empty otherwise
@@ -191,10 +208,12 @@ int build_stage(bm3d_batch *B, bool wiener, int tx, int ty, int warps, StageBuil
                            ? B->ext_ref[k]
                            : static_cast<const float *>(B->basic.ptr) + B->basic_off[k];
             a.num[c] = static_cast<long long *>(B->acc.ptr) + B->acc_off[k];
-            a.den[c] = a.num[c] + static_cast<size_t>(a.width) * a.height;
+            a.den[c] = wiener && B->chained
+                           ? static_cast<long long *>(B->den_next.ptr) + B->next_off[k]
+                           : a.num[c] + static_cast<size_t>(a.width) * a.height;
         }
-        a.absmax = static_cast<float *>(B->absmax.ptr) + i * npl;
-        a.nonfinite = static_cast<const unsigned *>(B->nonfinite.ptr) + i * npl;
+        a.absmax = B->absmax() + i * npl;
+        a.nonfinite = B->nonfinite(wiener) + i * npl;
         for (int c = 0; c < npl; ++c)
             a.poison[c] = static_cast<unsigned char *>(B->poison.ptr) + B->poison_off[i * npl + c];
         fixed_point_bounds(p, a.width, a.height, a.log2_bound, a.log2_corner);
@@ -227,12 +246,13 @@ int build_stage(bm3d_batch *B, bool wiener, int tx, int ty, int warps, StageBuil
     return BM3D_OK;
 }
 
+// The stage's work counter must be zero.
 template <bool W>
-int launch_batch_stage(bm3d_batch *B, StageBuild &sbd, int *counter, cudaStream_t s)
+int launch_batch_stage(bm3d_batch *B, StageBuild &sbd, cudaStream_t s)
 {
     bm3d_ctx *ctx = B->ctx;
     if (sbd.nact == 0) return BM3D_OK;
-    CK(ctx, cudaMemsetAsync(counter, 0, sizeof(int), s));
+    int *counter = B->counter(W);
     const auto *args = static_cast<const StageArgs<float> *>(sbd.args.ptr);
     const int *base = static_cast<const int *>(sbd.base.ptr);
     int nimg = sbd.nact;
@@ -261,12 +281,15 @@ int launch_planes(bm3d_batch *B, const DevBuf &planes, bool prep, cudaStream_t s
     if (count == 0) return BM3D_OK;
     long long maxpx = 0;
     for (int i = 0; i < B->n; ++i) maxpx = std::max(maxpx, static_cast<long long>(B->w[i]) * B->h[i]);
-    // enough CTAs in all to fill the GPU a few times over, at least 64 per plane
-    const long long tiles = (maxpx + kFixW * kFixH - 1) / (kFixW * kFixH);
+    // normalisation: a CTA per tile of the largest plane; preparation: enough CTAs in
+    // all to fill the GPU a few times over, at least 64 per plane
+    int tiles = 1;
+    for (int i = 0; i < B->n; ++i) tiles = std::max(tiles, normalize_tiles<float>(B->w[i], B->h[i]));
     const long long cap = std::max<long long>(64, 8LL * B->ctx->sm_count / count);
-    const dim3 grid(static_cast<unsigned>(std::min<long long>(prep ? (maxpx + 255) / 256 : tiles, cap)),
+    const dim3 grid(prep ? static_cast<unsigned>(std::min<long long>((maxpx + 255) / 256, cap))
+                         : static_cast<unsigned>(tiles),
                     static_cast<unsigned>(count));
-    const auto *q = static_cast<const BatchPlane<float> *>(planes.ptr);
+    const auto *q = static_cast<const PlaneJob<float> *>(planes.ptr);
     if (prep) prep_batch_kernel<float><<<grid, 256, 0, s>>>(q);
     else normalize_batch_kernel<float><<<grid, 256, 0, s>>>(q);
     CK(B->ctx, cudaGetLastError());
@@ -280,7 +303,6 @@ int enqueue_batch(bm3d_batch *B, cudaStream_t s, cudaEvent_t *ev = nullptr)
 {
     bm3d_ctx *ctx = B->ctx;
     int rc;
-    int *counters = static_cast<int *>(B->counters.ptr);
     for (int i = 0; i < B->n; ++i) {  // planes a stage passes through unfiltered
         for (int c = 0; c < B->npl; ++c) {
             const int k = i * B->npl + c;
@@ -296,16 +318,15 @@ int enqueue_batch(bm3d_batch *B, cudaStream_t s, cudaEvent_t *ev = nullptr)
                                           B->w[i] * 4, B->h[i], cudaMemcpyDeviceToDevice, s));
         }
     }
-    CK(ctx, cudaMemsetAsync(B->absmax.ptr, 0, sizeof(float) * B->n * B->npl, s));
-    CK(ctx, cudaMemsetAsync(B->nonfinite.ptr, 0, sizeof(unsigned) * B->n * B->npl, s));
+    CK(ctx, cudaMemsetAsync(B->head.ptr, 0, B->head_bytes(), s));
     if ((rc = launch_planes(B, B->planes_b, true, s)) != BM3D_OK) return rc;
     if (ev) CK(ctx, cudaEventRecord(ev[0], s));
-    if ((rc = launch_batch_stage<false>(B, B->sb, counters, s)) != BM3D_OK) return rc;
+    if ((rc = launch_batch_stage<false>(B, B->sb, s)) != BM3D_OK) return rc;
     if (ev) CK(ctx, cudaEventRecord(ev[1], s));
     if ((rc = launch_planes(B, B->planes_b, false, s)) != BM3D_OK) return rc;
-    if ((rc = launch_planes(B, B->planes_f, true, s)) != BM3D_OK) return rc;
+    if (!B->chained && (rc = launch_planes(B, B->planes_f, true, s)) != BM3D_OK) return rc;
     if (ev) CK(ctx, cudaEventRecord(ev[2], s));
-    if ((rc = launch_batch_stage<true>(B, B->sf, counters + 1, s)) != BM3D_OK) return rc;
+    if ((rc = launch_batch_stage<true>(B, B->sf, s)) != BM3D_OK) return rc;
     if (ev) CK(ctx, cudaEventRecord(ev[3], s));
     if ((rc = launch_planes(B, B->planes_f, false, s)) != BM3D_OK) return rc;
     return BM3D_OK;
@@ -323,10 +344,9 @@ int time_stage(bm3d_batch *B, StageBuild &sbd, const DevBuf &planes, cudaStream_
     ms = 1e30f;
     for (int rep = 0; rep < 3; ++rep) {
         if ((rc = launch_planes(B, planes, true, s)) != BM3D_OK) return rc;
+        CK(ctx, cudaMemsetAsync(B->counter(W), 0, sizeof(int), s));
         CK(ctx, cudaEventRecord(e0, s));
-        if ((rc = launch_batch_stage<W>(B, sbd, static_cast<int *>(B->counters.ptr) + (W ? 1 : 0),
-                                        s)) != BM3D_OK)
-            return rc;
+        if ((rc = launch_batch_stage<W>(B, sbd, s)) != BM3D_OK) return rc;
         CK(ctx, cudaEventRecord(e1, s));
         CK(ctx, cudaEventSynchronize(e1));
         float t = 0;
@@ -410,7 +430,7 @@ static int batch_create_any(bm3d_ctx *ctx, int npl, int count, const bm3d_stage_
         bm3d_batch_destroy(B);
         return rc;
     };
-    size_t acc_total = 0, basic_total = 0;
+    size_t acc_total = 0, basic_total = 0, next_total = 0;
     for (int i = 0; i < count; ++i) {
         const Guard gb = check_params(&basic[i], npl), gf = check_params(&final_[i], npl);
         if (gb == Guard::Invalid || gf == Guard::Invalid) return fail(batch_fail(ctx, "invalid parameters"));
@@ -445,6 +465,8 @@ static int batch_create_any(bm3d_ctx *ctx, int npl, int count, const bm3d_stage_
             B->acc_off.push_back(acc_total);
             B->basic_off.push_back(basic_total);
             B->poison_off.push_back(acc_total / 2);
+            B->next_off.push_back(next_total);
+            next_total += (static_cast<size_t>(width[i]) * height[i] + 1) / 2 * 2;
             acc_total += 2 * static_cast<size_t>(width[i]) * height[i];
             if (!ext_ref) basic_total += stride[i] * height[i];
         }
@@ -452,17 +474,23 @@ static int batch_create_any(bm3d_ctx *ctx, int npl, int count, const bm3d_stage_
     int rc;
     if ((rc = ensure(ctx, B->acc, sizeof(long long) * acc_total)) != BM3D_OK) return fail(rc);
     if ((rc = ensure(ctx, B->basic, sizeof(float) * basic_total)) != BM3D_OK) return fail(rc);
-    if ((rc = ensure(ctx, B->absmax, sizeof(float) * count * npl)) != BM3D_OK) return fail(rc);
-    if ((rc = ensure(ctx, B->nonfinite, sizeof(unsigned) * count * npl)) != BM3D_OK) return fail(rc);
+    if ((rc = ensure(ctx, B->head, B->head_bytes())) != BM3D_OK) return fail(rc);
+    B->chained = !ext_ref;
+    for (int i = 0; i < count; ++i) {
+        B->chained = B->chained && B->gb[i] == Guard::Run && B->gf[i] == Guard::Run;
+        for (int c = 0; npl > 1 && c < npl; ++c)
+            B->chained = B->chained && (basic[i].sigma[c] > 0) == (final_[i].sigma[c] > 0);
+    }
+    if (B->chained && (rc = ensure(ctx, B->den_next, sizeof(long long) * next_total)) != BM3D_OK)
+        return fail(rc);
     if ((rc = ensure(ctx, B->poison, acc_total / 2)) != BM3D_OK) return fail(rc);
     // all zero between stages: the normalisation clears what it reads
     CK(ctx, cudaMemset(B->poison.ptr, 0, acc_total / 2));
-    if ((rc = ensure(ctx, B->counters, 2 * sizeof(int))) != BM3D_OK) return fail(rc);
     if ((rc = ensure(ctx, B->bad, sizeof(unsigned long long))) != BM3D_OK) return fail(rc);
     CK(ctx, cudaMemset(B->bad.ptr, 0, sizeof(unsigned long long)));
     // per-pixel kernels' plane tables, active planes of each stage in batch order
     for (int st = 0; st < 2; ++st) {
-        std::vector<BatchPlane<float>> q;
+        std::vector<PlaneJob<float>> q;
         for (int i = 0; i < count; ++i) {
             if ((st ? B->gf[i] : B->gb[i]) != Guard::Run) continue;
             if (!st && ext_ref) continue;  // no basic stage
@@ -470,9 +498,19 @@ static int batch_create_any(bm3d_ctx *ctx, int npl, int count, const bm3d_stage_
             for (int c = 0; c < npl; ++c) {
                 if (npl > 1 && !(pp.sigma[c] > 0)) continue;  // plane left alone by the stage
                 const int k = i * npl + c;
-                BatchPlane<float> bp;
+                PlaneJob<float> bp;
+                std::memset(&bp, 0, sizeof(bp));
                 bp.num = static_cast<long long *>(B->acc.ptr) + B->acc_off[k];
                 bp.den = bp.num + static_cast<size_t>(width[i]) * height[i];
+                if (B->chained) {
+                    long long *next = static_cast<long long *>(B->den_next.ptr) + B->next_off[k];
+                    if (st) {
+                        bp.den = next;
+                    } else {
+                        bp.den_next = next;
+                        bp.nonfinite_next = B->nonfinite(true) + k;
+                    }
+                }
                 bp.src = src[k];
                 // the final stage's Wiener weights come from the basic estimate
                 bp.ref = !st ? nullptr
@@ -484,9 +522,9 @@ static int batch_create_any(bm3d_ctx *ctx, int npl, int count, const bm3d_stage_
                 bp.width = width[i];
                 bp.height = height[i];
                 bp.block_size = pp.block_size;
-                bp.absmax = static_cast<float *>(B->absmax.ptr) + k;
+                bp.absmax = B->absmax() + k;
                 fixed_point_bounds(&pp, width[i], height[i], bp.log2_bound, bp.log2_corner);
-                bp.nonfinite = static_cast<unsigned *>(B->nonfinite.ptr) + k;
+                bp.nonfinite = B->nonfinite(st != 0) + k;
                 bp.poison = static_cast<unsigned char *>(B->poison.ptr) + B->poison_off[k];
                 q.push_back(bp);
             }
@@ -494,8 +532,8 @@ static int batch_create_any(bm3d_ctx *ctx, int npl, int count, const bm3d_stage_
         DevBuf &dbuf = st ? B->planes_f : B->planes_b;
         (st ? B->nq_f : B->nq_b) = static_cast<int>(q.size());
         if (!q.empty()) {
-            if ((rc = ensure(ctx, dbuf, sizeof(BatchPlane<float>) * q.size())) != BM3D_OK) return fail(rc);
-            CK(ctx, cudaMemcpy(dbuf.ptr, q.data(), sizeof(BatchPlane<float>) * q.size(),
+            if ((rc = ensure(ctx, dbuf, sizeof(PlaneJob<float>) * q.size())) != BM3D_OK) return fail(rc);
+            CK(ctx, cudaMemcpy(dbuf.ptr, q.data(), sizeof(PlaneJob<float>) * q.size(),
                                cudaMemcpyHostToDevice));
         }
     }
@@ -512,9 +550,7 @@ static int batch_create_any(bm3d_ctx *ctx, int npl, int count, const bm3d_stage_
                                   cudaMemcpyDeviceToDevice, B->cap);
             if (e != cudaSuccess) return fail(cuda_fail(ctx, e, "cudaMemcpy2DAsync"));
         }
-    e = cudaMemsetAsync(B->absmax.ptr, 0, sizeof(float) * count * npl, B->cap);
-    if (e == cudaSuccess)
-        e = cudaMemsetAsync(B->nonfinite.ptr, 0, sizeof(unsigned) * count * npl, B->cap);
+    e = cudaMemsetAsync(B->head.ptr, 0, B->head_bytes(), B->cap);
     if (e != cudaSuccess) return fail(cuda_fail(ctx, e, "cudaMemsetAsync"));
     if (!ext_ref && (rc = tune_stage<false>(B, B->sb, B->planes_b, autotune != 0, B->cap,
                                             force_tiling)) != BM3D_OK)
@@ -653,7 +689,7 @@ extern "C" void bm3d_batch_destroy(bm3d_batch *B)
     if (B->exec) cudaGraphExecDestroy(B->exec);
     if (B->graph) cudaGraphDestroy(B->graph);
     if (B->cap) cudaStreamDestroy(B->cap);
-    for (DevBuf *b : {&B->acc, &B->basic, &B->absmax, &B->nonfinite, &B->poison, &B->counters,
+    for (DevBuf *b : {&B->acc, &B->basic, &B->head, &B->poison, &B->den_next,
                       &B->bad, &B->planes_b, &B->planes_f,
                       &B->sb.args, &B->sb.base, &B->sf.args, &B->sf.base})
         if (b->ptr) cudaFree(b->ptr);

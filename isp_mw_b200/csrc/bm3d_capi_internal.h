@@ -41,9 +41,14 @@ struct bm3d_ctx {
     DevBuf conv[3 * kMaxPlanes];      // float working planes of the integer paths: src, ref, dst
     DevBuf ints[3 * kMaxPlanes];      // host-mode staging of integer planes: src, ref, dst
     DevBuf poison[kMaxPlanes];        // per plane: pixels a non-finite term reached (1 B / pixel)
-    unsigned long long *stats = nullptr;
+    DevBuf den_next[kMaxPlanes];      // weight sums of a final stage prepared with its basic stage
+    // one small device block (kHeadBytes): |src| maxima and non-finite counts, the
+    // stage's counters, and the sticky consistency counter after them
+    unsigned char *head = nullptr;
     float *absmax = nullptr;          // per plane max finite |src| of the running stage
     unsigned *nonfinite = nullptr;    // per plane non-finite src / ref pixels of the running stage
+    unsigned *nonfinite_next = nullptr;  // the same of a final stage prepared with its basic stage
+    unsigned long long *stats = nullptr;
     float *gtab_f = nullptr;          // generic path cosine matrices: fwd | inv (float)
     double *gtab_d = nullptr;         // same in double
     cudaStream_t last_stream = nullptr;
@@ -69,6 +74,9 @@ struct bm3d_ctx {
 
 
 constexpr int kStats = 5;
+constexpr size_t kHeadStats = 40;  // offset of the counters: after 3 x 3 words, 8-byte aligned
+constexpr size_t kHeadClear = kHeadStats + 4 * sizeof(unsigned long long);  // all but the sticky one
+constexpr size_t kHeadBytes = kHeadStats + kStats * sizeof(unsigned long long);
 
 namespace bm3d {
 

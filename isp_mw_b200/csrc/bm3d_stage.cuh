@@ -1735,87 +1735,83 @@ __device__ __forceinline__ float ratio(long long n, long long d)
 }
 __device__ __forceinline__ double ratio(double n, double d) { return n / d; }
 
+// One plane of a stage, for the per-pixel kernels.
+template <typename T> struct PlaneJob {
+    typename AccOf<T>::type *num, *den;
+    const T *src;
+    const T *ref;              // counted for non-finite pixels too when not null
+    T *dst;
+    long long src_stride, dst_stride;
+    int width, height;
+    int block_size;
+    float *absmax;
+    int log2_bound, log2_corner;  // fixed-point bounds of the stage (StageArgs)
+    unsigned *nonfinite;       // non-finite src / ref pixels (may be null)
+    unsigned char *poison;     // pixels a non-finite term reached (may be null; all zero
+                               // between stages: the normalisation clears what it reads)
+    // A basic stage that its final stage follows (FP32; null otherwise). The final
+    // stage takes num, zeroed by the normalisation as it reads it, weight sums of
+    // its own, zeroed together with the basic stage's, |src|'s maximum as it is,
+    // and a count of non-finite pixels that starts from the basic stage's and adds
+    // the estimate's: it needs no preparation pass.
+    long long *den_next;
+    unsigned *nonfinite_next;
+    unsigned long long *stats;  // the stage's counters, zeroed for the next
+};
+template <typename T> struct PlaneJobs {
+    PlaneJob<T> job[kMaxPlanes];
+};
+
 // Tile of the normalisation: 32 x 32 pixels per CTA.
 constexpr int kNormTile = 32;
 
-// dst = num / den for the kNormTile^2 pixels at (y0, x0), with den(y, x) the
-// sum of the block weights W at the bs x bs origins whose block covers
-// (y, x): y - bs < oy <= y, x - bs < ox <= x. Separable sums over a
-// shared-memory copy of W; exact for integer sums.
-//
-// FP32 (fixed point): block (0, 0)'s pixels and the weight at origin (0, 0)
-// carry the scale of log2_corner, everything else that of log2_bound
-// (fixed_scale); for those pixels den = (sum of the other weights) * ratio +
-// W(0, 0), ratio = corner scale / general scale (a power of two, exact).
-// On planes whose prep found non-finite inputs (*nonfinite != 0) the pixels
-// marked in `poison` get NaN -- a non-finite term reached them
-// (acc_add_checked) -- and the map is cleared as it is read, so it is all
-// zero again for the next stage; other planes never touch it.
+// FP64 sums: dst = num / den for the kNormTile^2 pixels at (y0, x0), with
+// den(y, x) the sum of the block weights W at the bs x bs origins whose block
+// covers (y, x): y - bs < oy <= y, x - bs < ox <= x. Separable sums over a
+// shared-memory copy of W.
 template <typename T>
-__device__ __forceinline__ void normalize_tile(T *dst, long long dst_stride,
-                                               const typename AccOf<T>::type *num,
-                                               const typename AccOf<T>::type *wsum, int width,
-                                               int height, int bs, int y0, int x0,
-                                               unsigned char *poison = nullptr,
-                                               const unsigned *nonfinite = nullptr,
-                                               const float *absmax = nullptr, int log2_bound = 0,
-                                               int log2_corner = 0)
+__device__ __forceinline__ void normalize_tile(T *dst, long long dst_stride, const T *num,
+                                               const T *wsum, int width, int height, int bs, int y0,
+                                               int x0)
 {
-    using Acc = typename AccOf<T>::type;
-    constexpr bool kFixed = std::is_same<Acc, long long>::value;
     constexpr int N = kNormTile, E = N + kBSMax - 1;
-    __shared__ Acc w[E][E];
-    __shared__ Acc hs[E][N];
+    __shared__ T w[E][E];
+    __shared__ T hs[E][N];
     const int ext = N + bs - 1;
-    // origin (0, 0) is summed apart in fixed point (its own scale)
-    const bool split = kFixed && y0 < bs && x0 < bs;
     for (int i = threadIdx.x; i < ext * ext; i += blockDim.x) {
         const int ly = i / ext, lx = i - ly * ext;
         const int gy = y0 - bs + 1 + ly, gx = x0 - bs + 1 + lx;
-        w[ly][lx] = (gy >= 0 && gx >= 0 && gy < height && gx < width &&
-                     !(split && gy == 0 && gx == 0))
+        w[ly][lx] = (gy >= 0 && gx >= 0 && gy < height && gx < width)
                         ? wsum[static_cast<long long>(gy) * width + gx]
-                        : Acc(0);
+                        : T(0);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < ext * N; i += blockDim.x) {
         const int ly = i / N, lx = i - ly * N;
-        Acc v = 0;
+        T v = 0;
         for (int d = 0; d < bs; ++d) v += w[ly][lx + d];
         hs[ly][lx] = v;
     }
     __syncthreads();
-    const bool marked = poison != nullptr && nonfinite != nullptr && *nonfinite != 0;
-    double cratio = 1.0;
-    if (split) {
-        const float am = absmax != nullptr ? *absmax : 1.0f;
-        cratio = static_cast<double>(fixed_scale(am, log2_corner)) /
-                 static_cast<double>(fixed_scale(am, log2_bound));
-    }
     for (int i = threadIdx.x; i < N * N; i += blockDim.x) {
         const int ly = i / N, lx = i - ly * N;
         const int gy = y0 + ly, gx = x0 + lx;
         if (gy >= height || gx >= width) continue;
-        Acc d = 0;
+        T d = 0;
         for (int k = 0; k < bs; ++k) d += hs[ly + k][lx];
-        const long long g = static_cast<long long>(gy) * width + gx;
-        T out;
-        if (split && gy < bs && gx < bs)  // block (0, 0): covered by origin (0, 0)
-            out = static_cast<T>(static_cast<double>(num[g]) /
-                                 (static_cast<double>(d) * cratio + static_cast<double>(wsum[0])));
-        else
-            out = ratio(num[g], d);
-        if (marked && poison[g]) {
-            out = static_cast<T>(NAN);
-            poison[g] = 0;
-        }
-        dst[gy * dst_stride + gx] = out;
+        dst[gy * dst_stride + gx] = ratio(num[static_cast<long long>(gy) * width + gx], d);
     }
-    __syncthreads();  // before the next tile overwrites w / hs
 }
 
 // Fixed-point normalisation of one kFixW x kFixH tile of pixels at (y0, x0) by
-// 256 threads, exactly normalize_tile's sums and rules. What bounds it: the
+// 256 threads: the same sums, exact. Block (0, 0)'s pixels and the weight at
+// origin (0, 0) carry the scale of log2_corner, everything else that of
+// log2_bound (fixed_scale); for those pixels den = (sum of the other weights) *
+// ratio + W(0, 0), ratio = corner scale / general scale (a power of two, exact).
+// On planes whose prep found non-finite inputs (*nonfinite != 0) the pixels
+// marked in `poison` get NaN -- a non-finite term reached them
+// (acc_add_checked) -- and the map is cleared as it is read, so it is all zero
+// again for the next stage; other planes never touch it. What bounds it: the
 // latency of a tile's dependent steps (its loads, two box sums, a division), so
 // a tile has few of them and many tiles are resident. Each warp takes every
 // eighth row of block weights: all its loads are issued first, then per row a
@@ -1844,14 +1840,12 @@ struct FixedSmem {
 
 // BS: the block size, or 0 to take it from `block_size`.
 template <int BS>
-__device__ __forceinline__ void normalize_fixed(FixedSmem &sm, float *dst, long long dst_stride, const long long *num,
-                                                const long long *wsum, int width, int height,
-                                                int block_size, int y0, int x0, unsigned char *poison,
-                                                const unsigned *nonfinite, const float *absmax,
-                                                int log2_bound, int log2_corner)
+__device__ __forceinline__ void normalize_fixed(FixedSmem &sm, const PlaneJob<float> &q, int y0, int x0)
 {
+    const int width = q.width, height = q.height;
+    const long long *const wsum = q.den;
     constexpr int kMost = BS > 0 ? BS : kBSMax;
-    const int bs = BS > 0 ? BS : block_size;
+    const int bs = BS > 0 ? BS : q.block_size;
     long long *const hs = reinterpret_cast<long long *>(sm.hs);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool split = x0 == 0 && y0 == 0;  // the only tile whose sums reach W(0, 0)
@@ -1861,7 +1855,7 @@ __device__ __forceinline__ void normalize_fixed(FixedSmem &sm, float *dst, long 
     long long n[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-        n[k] = (x < width && yb + k < height) ? num[static_cast<long long>(yb + k) * width + x] : 0;
+        n[k] = (x < width && yb + k < height) ? q.num[static_cast<long long>(yb + k) * width + x] : 0;
     // weight rows warp, warp + 8, ... of the tile's window: columns
     // x0 - bs + 1 .. x0 + kFixW - 1, three words per lane at most
     constexpr int kRows = (kFixH + kMost - 1 + 7) / 8;
@@ -1902,7 +1896,14 @@ __device__ __forceinline__ void normalize_fixed(FixedSmem &sm, float *dst, long 
     }
     __syncthreads();
     if (x < width && yb < height) {
-        const bool marked = poison != nullptr && nonfinite != nullptr && *nonfinite != 0;
+        const bool marked = q.poison != nullptr && q.nonfinite != nullptr && *q.nonfinite != 0;
+        const bool next = q.nonfinite_next != nullptr;
+        unsigned bad = 0;
+        if (next && split && tid == 0) {
+            bad = *q.nonfinite;
+            if (q.stats != nullptr)
+                for (int k = 0; k < 4; ++k) q.stats[k] = 0;
+        }
         const long long *c = hs + (yb - y0) * kFixW + col;
         long long v = 0;
 #pragma unroll
@@ -1914,59 +1915,56 @@ __device__ __forceinline__ void normalize_fixed(FixedSmem &sm, float *dst, long 
             v += c[(k + bs - 1) * kFixW];
             float out;
             if (split && y < bs && x < bs) {  // block (0, 0): covered by origin (0, 0)
-                const float am = absmax != nullptr ? *absmax : 1.0f;
-                const double cratio = static_cast<double>(fixed_scale(am, log2_corner)) /
-                                      static_cast<double>(fixed_scale(am, log2_bound));
+                const float am = *q.absmax;
+                const double cratio = static_cast<double>(fixed_scale(am, q.log2_corner)) /
+                                      static_cast<double>(fixed_scale(am, q.log2_bound));
                 out = static_cast<float>(static_cast<double>(n[k]) /
                                          (static_cast<double>(v) * cratio +
                                           static_cast<double>(wsum[0])));
             } else {
                 out = ratio(n[k], v);
             }
-            if (marked) {
-                const long long g = static_cast<long long>(y) * width + x;
-                if (poison[g]) {
-                    out = NAN;
-                    poison[g] = 0;
-                }
+            const long long g = static_cast<long long>(y) * width + x;
+            if (marked && q.poison[g]) {
+                out = NAN;
+                q.poison[g] = 0;
             }
-            dst[y * dst_stride + x] = out;
+            q.dst[y * q.dst_stride + x] = out;
+            if (next) {
+                q.num[g] = 0;
+                if (!(fabsf(out) <= 3.4028235e38f)) ++bad;
+            }
             v -= c[k * kFixW];
         }
+        if (bad) atomicAdd(q.nonfinite_next, bad);
     }
-    __syncthreads();  // before the next tile overwrites hs
 }
 
-// Grid of the single-plane normalisation: one CTA per tile.
-template <typename T>
-inline dim3 normalize_grid(int width, int height)
+// Tile `tile` of a plane's normalisation (normalize_tiles in all).
+template <typename T> __host__ __device__ inline int normalize_tiles(int width, int height)
 {
-    if (std::is_same<T, float>::value) return dim3(static_cast<unsigned>(fixed_tiles(width, height)));
-    return dim3((width + kNormTile - 1) / kNormTile, (height + kNormTile - 1) / kNormTile);
+    if (sizeof(T) == 4) return fixed_tiles(width, height);
+    return ((width + kNormTile - 1) / kNormTile) * ((height + kNormTile - 1) / kNormTile);
+}
+__device__ __forceinline__ void normalize_job(const PlaneJob<float> &q, int tile)
+{
+    __shared__ FixedSmem sm;
+    const int tx = fixed_tiles_x(q.width), ty = tile / tx;
+    if (q.block_size == kBS) normalize_fixed<kBS>(sm, q, ty * kFixH, (tile - ty * tx) * kFixW);
+    else normalize_fixed<0>(sm, q, ty * kFixH, (tile - ty * tx) * kFixW);
+}
+__device__ __forceinline__ void normalize_job(const PlaneJob<double> &q, int tile)
+{
+    const int tx = (q.width + kNormTile - 1) / kNormTile, ty = tile / tx;
+    normalize_tile<double>(q.dst, q.dst_stride, q.num, q.den, q.width, q.height, q.block_size,
+                           ty * kNormTile, (tile - ty * tx) * kNormTile);
 }
 
-// One plane: grid = normalize_grid<T>(width, height), 256 threads.
+// The planes of one stage call (grid.y), one CTA of 256 threads per tile.
 template <typename T>
-__global__ void __launch_bounds__(256)
-    normalize_kernel(T *dst, long long dst_stride, const typename AccOf<T>::type *num,
-                     const typename AccOf<T>::type *wsum, int width, int height, int bs,
-                     unsigned char *poison = nullptr, const unsigned *nonfinite = nullptr,
-                     const float *absmax = nullptr, int log2_bound = 0, int log2_corner = 0)
+__global__ void __launch_bounds__(256) normalize_kernel(const PlaneJobs<T> jobs)
 {
-    if constexpr (std::is_same<T, float>::value) {
-        __shared__ FixedSmem sm;
-        const int tx = fixed_tiles_x(width), ty = static_cast<int>(blockIdx.x) / tx;
-        const int y0 = ty * kFixH, x0 = (static_cast<int>(blockIdx.x) - ty * tx) * kFixW;
-        if (bs == kBS)
-            normalize_fixed<kBS>(sm, dst, dst_stride, num, wsum, width, height, bs, y0, x0, poison,
-                                 nonfinite, absmax, log2_bound, log2_corner);
-        else
-            normalize_fixed<0>(sm, dst, dst_stride, num, wsum, width, height, bs, y0, x0, poison,
-                               nonfinite, absmax, log2_bound, log2_corner);
-    } else {
-        normalize_tile<T>(dst, dst_stride, num, wsum, width, height, bs, blockIdx.y * kNormTile,
-                          blockIdx.x * kNormTile, poison, nonfinite, absmax, log2_bound, log2_corner);
-    }
+    normalize_job(jobs.job[blockIdx.y], static_cast<int>(blockIdx.x));
 }
 
 // Zero one plane's accumulators and fold the largest finite |src| into
@@ -1976,28 +1974,31 @@ __global__ void __launch_bounds__(256)
 // kernel checks its terms only on such planes. Rows row0, row0 + row_step, ...
 // of the plane, threads along each row.
 template <typename T>
-__device__ __forceinline__ void prep_plane(typename AccOf<T>::type *num,
-                                           typename AccOf<T>::type *den, const T *src,
-                                           const T *ref, long long stride, int width, int height,
-                                           float *absmax, unsigned *nonfinite, int row0,
-                                           int row_step)
+__device__ __forceinline__ void prep_plane(const PlaneJob<T> &q, int row0, int row_step)
 {
+    using Acc = typename AccOf<T>::type;
+    Acc *const num = q.num, *const den = q.den;
+    long long *const den2 = q.den_next;
+    const int width = q.width, height = q.height;
     float m = 0.0f;
     unsigned bad = 0;
     for (int y = row0; y < height; y += row_step) {
         const long long o = static_cast<long long>(y) * width;
-        const T *s = src + static_cast<long long>(y) * stride;
-        const T *r = ref != nullptr ? ref + static_cast<long long>(y) * stride : nullptr;
+        const T *s = q.src + static_cast<long long>(y) * q.src_stride;
+        const T *r = q.ref != nullptr ? q.ref + static_cast<long long>(y) * q.src_stride : nullptr;
         if constexpr (sizeof(T) == 4) {
             // two pixels per thread where the row allows 16-byte sum stores
             // and 8-byte source loads (uniform over the CTA)
             const bool vec = (width % 2 == 0) &&
-                             ((reinterpret_cast<uintptr_t>(num + o) | reinterpret_cast<uintptr_t>(den + o)) & 15) == 0 &&
+                             ((reinterpret_cast<uintptr_t>(num + o) | reinterpret_cast<uintptr_t>(den + o) |
+                               (den2 != nullptr ? reinterpret_cast<uintptr_t>(den2 + o) : 0)) & 15) == 0 &&
                              ((reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(r)) & 7) == 0;
             if (vec) {
                 for (int x = 2 * threadIdx.x; x < width; x += 2 * blockDim.x) {
                     *reinterpret_cast<longlong2 *>(num + o + x) = make_longlong2(0, 0);
                     *reinterpret_cast<longlong2 *>(den + o + x) = make_longlong2(0, 0);
+                    if (den2 != nullptr)
+                        *reinterpret_cast<longlong2 *>(den2 + o + x) = make_longlong2(0, 0);
                     const float2 v2 = *reinterpret_cast<const float2 *>(s + x);
                     const float v0 = fabsf(v2.x), v1 = fabsf(v2.y);
                     if (v0 <= 3.4028235e38f) m = v0 > m ? v0 : m;  // NaN and Inf are skipped
@@ -2016,6 +2017,7 @@ __device__ __forceinline__ void prep_plane(typename AccOf<T>::type *num,
         for (int x = threadIdx.x; x < width; x += blockDim.x) {
             num[o + x] = 0;
             den[o + x] = 0;
+            if (den2 != nullptr) den2[o + x] = 0;
             const float v = fabsf(static_cast<float>(s[x]));
             if (v <= 3.4028235e38f) m = v > m ? v : m;  // NaN and Inf are skipped
             else ++bad;
@@ -2029,19 +2031,15 @@ __device__ __forceinline__ void prep_plane(typename AccOf<T>::type *num,
         bad += __shfl_xor_sync(0xffffffffu, bad, o);
     }
     if ((threadIdx.x & 31) == 0) {
-        if (m > 0.0f) atomicMax(reinterpret_cast<int *>(absmax), __float_as_int(m));
-        if (nonfinite != nullptr && bad) atomicAdd(nonfinite, bad);
+        if (m > 0.0f) atomicMax(reinterpret_cast<int *>(q.absmax), __float_as_int(m));
+        if (q.nonfinite != nullptr && bad) atomicAdd(q.nonfinite, bad);
     }
 }
 
-// One plane, one row per CTA at a time.
-template <typename T>
-__global__ void prep_kernel(typename AccOf<T>::type *num, typename AccOf<T>::type *den,
-                            const T *src, long long stride, int width, int height, float *absmax,
-                            const T *ref = nullptr, unsigned *nonfinite = nullptr)
+// The planes of one stage call (grid.y), one row per CTA at a time.
+template <typename T> __global__ void prep_kernel(const PlaneJobs<T> jobs)
 {
-    prep_plane<T>(num, den, src, ref, stride, width, height, absmax, nonfinite, blockIdx.x,
-                  gridDim.x);
+    prep_plane<T>(jobs.job[blockIdx.y], blockIdx.x, gridDim.x);
 }
 
 }  // namespace bm3d

@@ -1,0 +1,50 @@
+"""The combined call's basic stage prepares its final stage (sums, counts, the
+estimate's non-finite pixels). Results equal the two stages called one after
+the other, bit for bit: with non-finite inputs, planes left out by their noise
+level, a reference of its own, and sizes that change from call to call."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _planes(n, h, w, kind):
+    import torch
+    from isp_mw_b200 import synth
+    out = []
+    for c in range(n):
+        p = synth.pair(h, w, 20.0, 70 + c)[1]
+        if kind == "nan" and c != 1:
+            p = p.copy()
+            p[h // 2, w // 3], p[0, 0], p[-1, -1] = np.nan, np.inf, -np.inf
+        out.append(torch.from_numpy(p).cuda())
+    return out
+
+
+@pytest.mark.parametrize("profile", ["fast", "vn"])
+@pytest.mark.parametrize("kind", ["plain", "nan"])
+@pytest.mark.parametrize("sigma", [[30.0, 20.0, 20.0], [30.0, 0.0, 20.0]])
+def test_combined_equals_stages(bm3d_lib, profile, kind, sigma):
+    import torch
+    import isp_mw_b200
+    ctx = isp_mw_b200.Context(0)
+    b = isp_mw_b200.stage_params_default(profile, False, sigma)
+    f = isp_mw_b200.stage_params_default(profile, True, sigma)
+    same = lambda x, y: np.array_equal(x.cpu().numpy(), y.cpu().numpy(), equal_nan=True)
+    for (h, w) in ((40, 61), (90, 128), (33, 40), (64, 17)):
+        src = _planes(3, h, w, kind)
+        got = [torch.zeros_like(p) for p in src]
+        ctx.full3(b, f, got, src)
+        est, want = [p.clone() for p in src], [p.clone() for p in src]
+        ctx.stage3(b, False, est, src)
+        ctx.stage3(f, True, want, src, est)
+        ctx.check()
+        assert all(same(x, y) for x, y in zip(got, want))
+        ref = _planes(2, h, w, "plain")[1]
+        for r in (None, ref):
+            got1, est1, want1 = (torch.zeros_like(src[0]) for _ in range(3))
+            ctx.full(b, f, got1, src[0], ref=r)
+            ctx.stage(b, False, est1, src[0], r)
+            ctx.stage(f, True, want1, src[0], est1)
+            assert same(got1, want1)
+    ctx.close()
