@@ -10,8 +10,10 @@
 
 namespace bm3d {
 
-// The first 16 bytes of dynamic shared memory hold the CTA's current item.
-constexpr int kBatchHeader = 16;
+// Dynamic shared memory starts with the CTA's current item (16 bytes) and a copy
+// of its image's arguments: the tile body reads them all through, and a
+// shared-memory copy takes one address register and no global loads.
+constexpr int kBatchHeader = 16 + static_cast<int>((sizeof(StageArgs<float>) + 15) / 16 * 16);
 
 template <typename T, bool WIENER, int NPL, int KS, bool GENERIC>
 __global__ void __launch_bounds__(GENERIC ? (sizeof(T) == 4 ? 384 : 256) : stage_max_warps<T>() * kWarp, 1)
@@ -20,6 +22,8 @@ __global__ void __launch_bounds__(GENERIC ? (sizeof(T) == 4 ? 384 : 256) : stage
 {
     extern __shared__ __align__(16) unsigned char smem[];
     int *item = reinterpret_cast<int *>(smem);
+    StageArgs<T> &a = *reinterpret_cast<StageArgs<T> *>(smem + 16);
+    int held = -1;  // the image whose arguments are held
     const int total = tile_base[nimg];
     const unsigned avail = dynamic_smem_bytes() - kBatchHeader;
     for (;;) {
@@ -33,7 +37,15 @@ __global__ void __launch_bounds__(GENERIC ? (sizeof(T) == 4 ? 384 : 256) : stage
             if (tile_base[mid] <= it) lo = mid;
             else hi = mid - 1;
         }
-        const StageArgs<T> &a = args[lo];
+        if (lo != held) {  // uniform over the CTA; no warp reads them between items
+            static_assert(sizeof(StageArgs<T>) % 8 == 0, "copied by 8-byte words");
+            const auto *from = reinterpret_cast<const unsigned long long *>(args + lo);
+            auto *to = reinterpret_cast<unsigned long long *>(&a);
+            for (int i = threadIdx.x; i < static_cast<int>(sizeof(StageArgs<T>) / 8); i += blockDim.x)
+                to[i] = from[i];
+            held = lo;
+            __syncthreads();
+        }
         unsigned char *body = smem + kBatchHeader;
         if constexpr (GENERIC && NPL == 3) generic_tile_body_seq3<T, WIENER>(a, it - tile_base[lo], body, avail);
         else if constexpr (GENERIC) generic_tile_body<T, WIENER, NPL>(a, it - tile_base[lo], body, avail);

@@ -187,7 +187,7 @@ extern "C" int bm3d_ctx_create(bm3d_ctx **out, int device)
     ctx->stats = reinterpret_cast<unsigned long long *>(ctx->head + kHeadStats);
     // cosine matrices of lengths 1..32 for the generic path
     {
-        std::vector<float> tf(2 * kDctTableSize);
+        std::vector<float> tf(2 * kDctTableSize + 2 * kPad32Table, 0.0f);
         std::vector<double> td(2 * kDctTableSize);
         const long double pi = 3.141592653589793238462643383279502884L;
         for (int n = 1; n <= kGSTab; ++n) {
@@ -200,6 +200,11 @@ extern "C" int bm3d_ctx_create(bm3d_ctx **out, int device)
                     tf[kDctTableSize + o + k * n + j] = static_cast<float>(ci);
                     td[o + k * n + j] = static_cast<double>(cf);
                     td[kDctTableSize + o + k * n + j] = static_cast<double>(ci);
+                    if (n < kGSTab) {
+                        const int q = 2 * kDctTableSize + pad32_offset(n) + 32 * j + k;
+                        tf[q] = static_cast<float>(cf);
+                        tf[q + kPad32Table] = static_cast<float>(ci);
+                    }
                 }
         }
         e = cudaMalloc(&ctx->gtab_f, tf.size() * sizeof(float));
@@ -525,14 +530,17 @@ static SmemPlan plan_tile(StageArgs<T> &a, const bm3d_stage_params *p, bool wien
 }
 
 // Predicted time of a stage at one tile shape (microseconds; only the order
-// matters). A warp takes 8.5 us for a reference block when its SM runs few
-// warps and 12 us with 16 (fast profile); a tile adds about 10 us of staging,
-// flushing and waiting for its last warp, which other CTAs of the SM overlap;
-// CTAs run in waves, whose rounding up fades once there are several. Measured
-// at 64 x 64 .. 3840 x 2160, one shape for all sizes (8 x 8, 16 warps) against
-// the shapes this picks, basic / final stage: 64 x 64 60 / 67 -> 20 / 23 us,
-// 512 x 512 72 / 88 -> 49 / 65 us, 1280 x 720 128 / 197 -> 113 / 177 us,
-// 1920 x 1080 245 / 343 -> 225 / 329 us.
+// matters). Fast profile: a warp takes 8.5 us for a reference block when its SM
+// runs few warps and 12 us with 16; about a third of it is matching, the rest
+// follows the group's size. A tile adds staging, flushing and the wait for its last
+// warp: about 10 us where other CTAs of the SM overlap it, or by its window in the
+// generic kernel, whose 12 warps fill an SM. CTAs run in waves, whose rounding up
+// fades once there are several. Measured at 64 x 64 .. 3840 x 2160, one shape for all
+// sizes (8 x 8, 16 warps) against the shapes this picks, basic / final stage:
+// 64 x 64 60 / 67 -> 20 / 23 us, 512 x 512 72 / 88 -> 49 / 65 us, 1280 x 720
+// 128 / 197 -> 113 / 177 us, 1920 x 1080 245 / 343 -> 225 / 329 us; generic kernel
+// (6 x 4, 12 warps before) np final 300 x 200 212 -> 171 us, vn basic 960 x 540
+// 672 -> 650 us.
 template <typename T>
 static double tile_cost(const bm3d_ctx *ctx, const StageArgs<T> &a, const SmemPlan &sp,
                         const TileShape &t, int nplanes, bool generic)
@@ -544,14 +552,17 @@ static double tile_cost(const bm3d_ctx *ctx, const StageArgs<T> &a, const SmemPl
     const int per_sm = std::max(1, std::min(by_smem, by_regs));
     const double tiles = static_cast<double>(a.tiles_x) * ((a.ny + a.tile_y - 1) / a.tile_y);
     const double share = tiles / ctx->sm_count;  // tiles per SM
-    const int busy = std::min(per_sm, std::max(1, static_cast<int>(std::ceil(share)))) * t.warps;
-    // matching is about a third of a block's time at BMrange 9
-    const double work = (0.65 + 0.35 * a.span * a.span / 361.0) * (nplanes == 3 ? 1.9 : 1.0);
-    const double round = (8.5 + 0.22 * busy) * work;
+    const int ctas = std::min(per_sm, std::max(1, static_cast<int>(std::ceil(share))));
+    const double px = a.block_size * a.block_size / 64.0;
+    const double work = px * (0.65 * std::max(16, a.group_size) / 16.0 +
+                              0.35 * a.span * a.span / 361.0) * (nplanes == 3 ? 1.9 : 1.0);
+    const double round = (8.5 + 0.22 * ctas * t.warps) * work;
     const int rounds = (a.tile_x * a.tile_y + t.warps - 1) / t.warps;
     const double x = share / per_sm;
     const double waves = x < 4.0 ? std::ceil(x) : x + 0.5;
-    return waves * (rounds * round + (8.0 + rounds + 0.1 * t.warps) * nplanes);
+    const double window = static_cast<double>(a.region_w) * a.region_h * ctas;
+    const double edge = generic ? 3.0 + 1.05e-3 * window : 8.0 + rounds + 0.1 * t.warps;
+    return waves * (rounds * round + edge * nplanes);
 }
 
 // Geometry, tiling and shared-memory fit.
@@ -575,7 +586,8 @@ static int plan_geometry(bm3d_ctx *ctx, StageArgs<T> &a, const bm3d_stage_params
     // generic 384 and 256) limit the warps; the small shapes are for windows
     // that leave no room for more.
     static const TileShape fast[] = {{2, 2, 4}, {4, 2, 8}, {4, 4, 8}, {4, 8, 8}, {6, 4, 8}, {8, 8, 16}};
-    static const TileShape gen[] = {{6, 4, 12}, {4, 3, 12}, {4, 4, 8}, {4, 2, 8}, {2, 2, 4}, {4, 4, 4}};
+    static const TileShape gen[] = {{6, 6, 12}, {6, 4, 12}, {4, 3, 12}, {3, 2, 6}, {2, 2, 4},
+                                    {4, 4, 8},  {4, 2, 8},  {5, 2, 5},  {4, 4, 4}};
     static const TileShape gen_small[] = {{2, 2, 4}, {2, 2, 2}, {1, 1, 2}, {1, 1, 1}};
     const int max_warps = generic ? (sizeof(T) == 4 ? 12 : 8) : stage_max_warps<T>();
     if (generic || !ctx->tiling_set) {
@@ -655,6 +667,8 @@ static int run_stage_device(bm3d_ctx *ctx, const bm3d_stage_params *p, bool wien
     if (rc != BM3D_OK) return rc;
     a.dct_fwd = GenericTables<T>::fwd(ctx);
     a.dct_inv = GenericTables<T>::inv(ctx);
+    a.pad_fwd = ctx->gtab_f + 2 * kDctTableSize;
+    a.pad_inv = a.pad_fwd + kPad32Table;
     using Acc = typename AccOf<T>::type;
     const size_t acc_bytes = sizeof(Acc) * static_cast<size_t>(width) * height;
     const long long npx = static_cast<long long>(width) * height;

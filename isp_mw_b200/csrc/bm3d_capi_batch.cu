@@ -219,6 +219,8 @@ int build_stage(bm3d_batch *B, bool wiener, int tx, int ty, int warps, StageBuil
         fixed_point_bounds(p, a.width, a.height, a.log2_bound, a.log2_corner);
         a.dct_fwd = ctx->gtab_f;
         a.dct_inv = ctx->gtab_f ? ctx->gtab_f + kDctTableSize : nullptr;
+        a.pad_fwd = ctx->gtab_f + 2 * kDctTableSize;
+        a.pad_inv = a.pad_fwd + kPad32Table;
         const SmemPlan sp = plan_smem<float>(npl, wiener, a.ref_alias_src, a.region_h,
                                              a.region_pitch, a.span, warps, generic, BS,
                                              p->group_size, a.tile_x * a.tile_y);
@@ -375,10 +377,10 @@ int tune_stage(bm3d_batch *B, StageBuild &sbd, const DevBuf &planes, bool autotu
     static const int fast_cand[][3] = {{4, 8, 8}, {8, 4, 8}, {6, 4, 8}, {4, 4, 8}, {8, 8, 16},
                                        {6, 8, 16}, {8, 6, 12}, {4, 2, 8}, {2, 2, 4}, {4, 4, 4},
                                        {2, 2, 1}};
-    static const int gen_cand[][3] = {{6, 4, 12}, {4, 3, 12}, {4, 4, 8}, {4, 4, 4},
-                                      {2, 2, 4},  {2, 2, 2},  {1, 1, 2}, {1, 1, 1}};
+    static const int gen_cand[][3] = {{6, 6, 12}, {6, 4, 12}, {4, 3, 12}, {4, 4, 8},
+                                      {4, 4, 4},  {2, 2, 4},  {2, 2, 2},  {1, 1, 2}, {1, 1, 1}};
     const int (*cand)[3] = generic ? gen_cand : fast_cand;
-    const int ncand = generic ? 8 : 11;
+    const int ncand = generic ? 9 : 11;
     int best = -1;
     float best_ms = 1e30f;
     for (int c = 0; c < ncand; ++c) {

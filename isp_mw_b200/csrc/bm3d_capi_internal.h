@@ -49,7 +49,8 @@ struct bm3d_ctx {
     unsigned *nonfinite = nullptr;    // per plane non-finite src / ref pixels of the running stage
     unsigned *nonfinite_next = nullptr;  // the same of a final stage prepared with its basic stage
     unsigned long long *stats = nullptr;
-    float *gtab_f = nullptr;          // generic path cosine matrices: fwd | inv (float)
+    float *gtab_f = nullptr;          // generic path cosine matrices: fwd | inv (float), then the
+                                      // padded columns: fwd | inv (pad32_offset)
     double *gtab_d = nullptr;         // same in double
     cudaStream_t last_stream = nullptr;
     // tile shape of the register-resident kernel when the caller sets one

@@ -291,6 +291,8 @@ template <typename T> struct StageArgs {
     double finalAMP[kGSTab];       // 2n * 2BS * 2BS                     (source/BM3D.cpp:26)
     const T *dct_fwd;           // generic path: cosine matrices of lengths 1..32 (device),
     const T *dct_inv;           //   length n at offset (n-1) n (2n-1) / 6
+    const float *pad_fwd;       // FP32 groups of 8 x 8 blocks: matrices of lengths 1..31 by
+    const float *pad_inv;       //   columns of 32 rows (pad32_offset)
     // optional outputs
     int *group_count;           // per reference block: group size        (may be null)
     int *group_pos;             // per reference block: kGSTab x (y, x)   (may be null)
@@ -307,6 +309,10 @@ template <typename T> struct StageArgs {
 // generic path: sum_{m < n} m^2.
 __host__ __device__ __forceinline__ int dct_table_offset(int n) { return (n - 1) * n * (2 * n - 1) / 6; }
 constexpr int kDctTableSize = 32 * 33 * 65 / 6;  // lengths 1..32
+// FP32 group-axis matrices of lengths 1..31, column by column of 32 rows, zero
+// past the length: length n starts at pad32_offset(n).
+__host__ __device__ constexpr int pad32_offset(int n) { return 32 * ((n - 1) * n / 2); }
+constexpr int kPad32Table = pad32_offset(32);
 
 // Shared-memory carve-up of one CTA, identical on host and device.
 // `generic` selects the layout of the generic-path kernel (group buffers of

@@ -248,8 +248,23 @@ __device__ int match_generic(const StageArgs<T> &a, const Tile<T> &t, int j0, in
     }
     __syncwarp();
     n_cand += static_cast<unsigned>(ngrid);
-    return select_group<T, false>(a, dist, limit, [](int) { return B(0); }, ngrid, nc, nc_div, tp, l,
-                                  st, j0, i0, lane, nvalid, heap, list, lkeys, n_fix);
+    Search<T> e = {};
+    e.st = st;
+    e.ngrid = ngrid;
+    e.nc = nc;
+    e.nc_div = nc_div;
+    e.tp = tp;
+    e.l = l;
+    e.j0 = j0;
+    e.i0 = i0;
+    e.group_size = a.group_size;
+    e.dist_mul = a.distMul;
+    e.limit = limit;
+    e.dist = dist;
+    e.heap = heap;
+    e.list = list;
+    e.lkeys = lkeys;
+    return select_group<T, false>(e, false, lane, nvalid, n_fix);
 }
 
 // Element e of a group stored [z][y][x]: shifts for BlockSize 8, divisions
@@ -359,50 +374,138 @@ __device__ __forceinline__ void aggregate_rows(const StageArgs<T> &a, const Tile
     }
 }
 
-// Wiener shrinkage of a BlockSize-8 FP32 group with ONE group buffer: the
-// basic estimate's group is transformed in G, each lane keeps the Wiener
-// weights of its two pencils (lane and lane + 32: 2 x 32 registers), then
-// the noisy group is transformed in the same buffer and scaled. Elements,
-// weights and the lane's sum of squared weights come out in exactly the
-// order of the two-buffer form (a lane's elements e = lane + 32 k are pencil
-// lane + 32 (k % 2) at z = k / 2), so results are bit-identical; the warp
-// needs half the shared memory. Returns the lane's sum of w^2.
-template <typename T>
-__device__ __forceinline__ T wiener_one_buffer(const StageArgs<T> &a, const Tile<T> &t, int p,
-                                               int pt, const BlockPos *list, int n, int lane, T *G,
-                                               unsigned &n_bad)
+// Group-axis transform of pencils g0 and g1 (length n < 32, stride kGroupStride)
+// by matrix columns m of 32 rows: y_k = sum_j m[k][j] x_j, j in order, from the
+// buffer into registers. ROWS (16 or 32) bounds n. Sums of all rows advance
+// together, so a step is independent loads and multiply-adds; row by row, each
+// output waited for its own chain of loads and adds, and one short group could
+// take longer than the rest of a tile.
+template <int ROWS>
+__device__ __forceinline__ void pencils_by_columns(const float *g0, const float *g1, int n,
+                                                   const float *m, Pair<float> (&out)[kGSTab])
 {
-    gather_rows<T, 8>(t, t.refw[p], t.ref0[p], list, n, lane, G, static_cast<unsigned *>(nullptr));
-    __syncwarp();
-    dct_cols_z_fwd<T, 8>(G, n, lane, a.dct_fwd);
-    const T s2 = a.wss[pt][n - 1];
-    T *const p0 = G + (lane >> 3) * 9 + (lane & 7);  // pencil lane
-    T *const p1 = p0 + 4 * 9;                        // pencil lane + 32
-    T w0[kGSTab], w1[kGSTab];
-    T l2 = T(0);
+    float a[ROWS], b[ROWS];
 #pragma unroll
-    for (int z = 0; z < kGSTab; ++z) {
-        w0[z] = w1[z] = T(0);
-        if (z < n) {
-            const T y0 = p0[z * 72], y1 = p1[z * 72];
-            w0[z] = wiener_weight(y0 * y0, s2);
-            l2 += w0[z] * w0[z];
-            w1[z] = wiener_weight(y1 * y1, s2);
-            l2 += w1[z] * w1[z];
+    for (int k = 0; k < ROWS; ++k) a[k] = b[k] = 0.0f;
+#pragma unroll 1
+    for (int j = 0; j < n; ++j) {
+        const float x0 = g0[j * kGroupStride], x1 = g1[j * kGroupStride];
+        const float4 *c = reinterpret_cast<const float4 *>(m + 32 * j);
+#pragma unroll
+        for (int k = 0; k < ROWS; k += 4) {
+            const float4 q = __ldg(c + k / 4);
+            const float r[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                a[k + i] = fmaf(r[i], x0, a[k + i]);
+                b[k + i] = fmaf(r[i], x1, b[k + i]);
+            }
         }
     }
-    __syncwarp();
-    gather_rows<T, 8>(t, t.srcw[p], t.src0[p], list, n, lane, G, &n_bad);
-    __syncwarp();
-    dct_cols_z_fwd<T, 8>(G, n, lane, a.dct_fwd);
 #pragma unroll
-    for (int z = 0; z < kGSTab; ++z)
-        if (z < n) {
-            p0[z * 72] *= w0[z];
-            p1[z * 72] *= w1[z];
+    for (int k = 0; k < kGSTab; ++k)
+        out[k] = k < ROWS ? Pair<float>::make(a[k < ROWS ? k : 0], b[k < ROWS ? k : 0])
+                          : Pair<float>::make(0.0f, 0.0f);
+}
+
+// Collaborative filtering of an FP32 group of 8 x 8 blocks, up to 32 of them, in
+// one group buffer of the register-resident kernel's layout and passes (16-byte
+// rows, columns in packed pairs). Each lane owns pencils lane and lane + 32 of
+// the group axis as the halves of pairs: full groups of 32 stay in registers from
+// the last column pass to the first inverse one, and the Wiener weights in 64
+// more while the noisy group takes the buffer; shorter groups go through matrix
+// columns (pencils_by_columns). What bounds it: issue slots and, at 12 warps of 168 registers,
+// latency. Against scalar lines in rows of 9 words (and, for short groups, row by
+// row products): np on 1283 x 717 3.33 -> 2.78 ms, its final stage on 64 x 64
+// 127 -> 53 us.
+template <bool WIENER>
+__device__ void filter_group32(const StageArgs<float> &a, const Tile<float> &t, int p,
+                               const BlockPos *list, int n, int lane, float *G, float scale,
+                               unsigned &n_bad, int pt, bool check)
+{
+    using P = Pair<float>;
+    float *const g0 = G + gidx(lane >> 3, lane & 7);        // pencil lane
+    float *const g1 = G + gidx((lane >> 3) + 4, lane & 7);  // pencil lane + 32
+    auto by_columns = [&](const float *m, P (&v)[kGSTab]) {
+        if (n <= 16) pencils_by_columns<16>(g0, g1, n, m + pad32_offset(n), v);
+        else pencils_by_columns<32>(g0, g1, n, m + pad32_offset(n), v);
+    };
+    auto forward = [&](P (&v)[kGSTab]) {
+        if (n == kGSTab) {
+#pragma unroll
+            for (int z = 0; z < kGSTab; ++z)
+                v[z] = P::make(g0[z * kGroupStride], g1[z * kGroupStride]);
+            redft10_pow2<P, kGSTab>(v);
+        } else {
+            by_columns(a.pad_fwd, v);
         }
+    };
+    auto store = [&](const P (&v)[kGSTab]) {
+#pragma unroll
+        for (int z = 0; z < kGSTab; ++z)
+            if (z < n) {
+                g0[z * kGroupStride] = v[z].lo();
+                g1[z * kGroupStride] = v[z].hi();
+            }
+    };
+    P w[kGSTab];
+    float denW;
+    if (WIENER) {
+        unsigned none = 0;
+        gather_xy_forward<float, kGSTab>(t, t.refw[p], t.ref0[p], list, n, lane, G, none);
+        forward(w);
+        const float s2 = a.wss[pt][n - 1];
+        float l2 = 0.0f;
+#pragma unroll
+        for (int z = 0; z < kGSTab; ++z) {
+            if (z < n) {
+                const float y0 = w[z].lo(), y1 = w[z].hi();
+                const float w0 = wiener_weight(y0 * y0, s2);
+                l2 += w0 * w0;
+                const float w1 = wiener_weight(y1 * y1, s2);
+                l2 += w1 * w1;
+                w[z] = P::make(w0, w1);
+            }
+        }
+        l2 = warp_sum(l2);
+        denW = l2 <= 0.0f ? 1.0f : 1.0f / l2;
+        __syncwarp();
+    }
+    gather_xy_forward<float, kGSTab>(t, t.srcw[p], t.src0[p], list, n, lane, G, n_bad);
+    P v[kGSTab];
+    forward(v);
+    if (WIENER) {
+#pragma unroll
+        for (int z = 0; z < kGSTab; ++z)
+            if (z < n) v[z] = vmul(v[z], w[z]);
+    } else {
+        // hard threshold (source/BM3D.cpp:361-371) with thr by #zero indices
+        const float *thr = a.thr[pt][n - 1];
+        const int f0 = ((lane & 7) == 0) + (lane < 8), f1 = (lane & 7) == 0;
+        int kept = 0;
+#pragma unroll
+        for (int z = 0; z < kGSTab; ++z) {
+            if (z < n) {
+                float x0 = v[z].lo(), x1 = v[z].hi();
+                if (fabsf(x0) <= thr[f0 + (z == 0)]) x0 = 0.0f; else ++kept;
+                if (fabsf(x1) <= thr[f1 + (z == 0)]) x1 = 0.0f; else ++kept;
+                v[z] = P::make(x0, x1);
+            }
+        }
+        const int retained = __reduce_add_sync(0xffffffffu, kept);
+        denW = retained < 1 ? 1.0f : 1.0f / static_cast<float>(retained);
+    }
+    const float numW = static_cast<float>(static_cast<double>(denW) / a.finalAMP[n - 1]);
+    if (n == kGSTab) {
+        redft01_pow2<P, kGSTab>(v);
+    } else {  // a lane reads back only its own pencils
+        store(v);
+        by_columns(a.pad_inv, v);
+    }
+    store(v);
     __syncwarp();
-    return l2;
+    xy_cols<float, kGSTab, true>(G, n, lane);
+    aggregate_group<float, kGSTab>(a, t, p, pt, list, n, lane, G, numW, denW, scale, check);
 }
 
 // Collaborative filtering of one group on plane p (generic sizes).
@@ -414,13 +517,15 @@ __device__ void filter_generic(const StageArgs<T> &a, const Tile<T> &t, int p, c
     // p indexes the tile's windows; pt (default p) the plane's threshold /
     // Wiener tables, which differ when planes share one set of windows
     if (pt < 0) pt = p;
+    if constexpr (sizeof(T) == 4) {
+        if (t.bs == kBS) {
+            filter_group32<WIENER>(a, t, p, list, n, lane, Gs, scale, n_bad, pt, check);
+            return;
+        }
+    }
     const int bs = t.bs, bsq = bs * bs, total = n * bsq;
     const int zs = generic_block_stride(bs), rs = generic_row_stride(bs);
     T denW;
-    if (WIENER && generic_one_buffer<T>(WIENER, bs)) {
-        const T l2 = warp_sum(wiener_one_buffer(a, t, p, pt, list, n, lane, Gs, n_bad));
-        denW = l2 <= T(0) ? T(1) : T(1) / l2;
-    } else {
     if (bs == 8) {
         gather_rows<T, 8>(t, t.srcw[p], t.src0[p], list, n, lane, Gs, &n_bad);
         if (WIENER)
@@ -492,7 +597,6 @@ __device__ void filter_generic(const StageArgs<T> &a, const Tile<T> &t, int p, c
         }
         l2 = warp_sum(l2);
         denW = l2 <= T(0) ? T(1) : T(1) / l2;
-    }
     }
     const T numW = static_cast<T>(static_cast<double>(denW) / a.finalAMP[n - 1]);
     __syncwarp();

@@ -413,10 +413,69 @@ __device__ __forceinline__ int div_magic(int k, unsigned m)
     return m ? static_cast<int>(__umulhi(static_cast<unsigned>(k), m)) : k;
 }
 
-// Ordered group of reference block (j0, i0) from its search list `dist` (see
-// above; ngrid = nr x nc window places from (tp, l) in steps of st, plus the
-// slot), of which this lane accepted nvalid. Writes list / lkeys in the
-// reference's group order and returns the group size.
+// One reference block's search: its window's grid, where its pixels and its
+// candidates' are, and the warp's buffers.
+template <typename T> struct Search {
+    const T *win, *refb, *slot;  // window place (0, 0), reference block, block (0, 0)
+    int pitch, slot_pitch, st;   // row pitches; grid step
+    int ngrid, nc;               // grid places in all, columns
+    unsigned nc_div;
+    int tp, l, j0, i0;           // plane positions of the grid's first place and the block
+    int group_size;
+    double dist_mul;
+    typename DistBits<T>::type limit;  // the matching threshold (dist_limit)
+    typename DistBits<T>::type *dist;
+    SortKey<T> *heap;
+    BlockPos *list;
+    T *lkeys;
+};
+
+// The exact distance of a list place, in the reference's order (BlockSize 8).
+template <typename T>
+__device__ __forceinline__ typename DistBits<T>::type exact_dist(const Search<T> &e, int i)
+{
+    const T *cb = e.slot;
+    int cp = e.slot_pitch;
+    if (i < e.ngrid) {
+        const int rr = div_magic(i, e.nc_div);
+        cb = e.win + rr * e.st * e.pitch + (i - rr * e.nc) * e.st;
+        cp = e.pitch;
+    }
+    T acc = T(0);
+#pragma unroll 1
+    for (int y = 0; y < kBS; ++y) {
+        T r[kBS], c[kBS];
+#pragma unroll
+        for (int x = 0; x < kBS; ++x) {
+            r[x] = e.refb[y * e.pitch + x];
+            c[x] = cb[y * cp + x];
+        }
+        acc = ssd_row8(acc, r, c);
+    }
+    return DistBits<T>::of(acc);
+}
+
+// A candidate's entry in the search list. Distances are sums of squares:
+// >= +0, or NaN, whose bits compare above any threshold. A zero distance (the
+// reference block itself, or an equal block) is rejected like one over the
+// threshold (include/Block.h:606): (bits - 1) wraps to the top for it.
+template <typename B>
+__device__ __forceinline__ B accept_dist(B bits, B limit, int &nvalid)
+{
+    const bool ok = bits - 1 < limit;
+    nvalid += ok ? 1 : 0;
+    return ok ? bits : ~B(0);
+}
+
+// The matching threshold as distance bits: d <= thSSE is bits <= limit.
+template <typename T> __device__ __forceinline__ typename DistBits<T>::type dist_limit(T thSSE)
+{
+    return thSSE > T(0) ? DistBits<T>::of(thSSE) : typename DistBits<T>::type(0);
+}
+
+// Ordered group of a reference block from its search list, of which this lane
+// accepted nvalid. Writes list / lkeys in the reference's group order and
+// returns the group size.
 //
 // What bounds it: latency -- one warp's dependent steps. The list holds
 // 32-bit distances; only the few that can be among the best get a key
@@ -431,44 +490,44 @@ __device__ __forceinline__ int div_magic(int k, unsigned m)
 // final 0.355 / 0.461 -> 0.333 / 0.438 ms, np 2.82 / 6.27 -> 2.00 / 5.86 ms
 // (the smaller list also lets np's basic stage keep 16 warps).
 //
-// NEAR: the list holds approximate distances (ssd_row8_near), accepted up to
+// NEAR, near: the list holds approximate distances (ssd_row8_near), accepted up to
 // kNear above `limit`. The cut then leaves that much more room, and the
 // approximate order stands when no kept distance is within kNear of the next;
-// else `exact` (list index -> exact distance bits) gives the compacted ones'
-// exact distances. Returns -1 where the whole list has to be exact: a distance
+// else exact_dist gives the compacted ones'. Returns -1 where the whole list has to be exact: a distance
 // at the matching threshold, ties, ranges where the bounds do not hold.
-template <typename T, bool NEAR, typename Exact>
-__device__ __forceinline__ int select_group(const StageArgs<T> &a, const typename DistBits<T>::type *dist,
-                            typename DistBits<T>::type limit, Exact exact,
-                            int ngrid, int nc, unsigned nc_div, int tp, int l, int st, int j0,
-                            int i0, int lane, int nvalid, SortKey<T> *heap, BlockPos *list,
-                            T *lkeys, unsigned &n_fix)
+template <typename T, bool NEAR>
+__device__ __forceinline__ int select_once(const Search<T> &e, bool near, int lane, int nvalid,
+                                           unsigned &n_fix)
 {
     using K = SortKey<T>;
     using DB = DistBits<T>;
     using B = typename DB::type;
     const B none = ~B(0);
-    const int GS = a.group_size;
-    const int nkeys = ngrid + 1;
+    const int GS = e.group_size, nkeys = e.ngrid + 1;
+    const B limit = e.limit;
+    const B *const dist = e.dist;
+    SortKey<T> *const heap = e.heap;
+    BlockPos *const list = e.list;
+    T *const lkeys = e.lkeys;
     const int accepted = __reduce_add_sync(0xffffffffu, nvalid);
     const int take = min(GS - 1, accepted);
     // list[0] is the reference block itself (key 0, include/Block.h:685)
     if (lane == 0) {
-        list[0] = BlockPos{j0, i0};
+        list[0] = BlockPos{e.j0, e.i0};
         lkeys[0] = T(0);
     }
     auto place = [&](unsigned idx) {
-        if (idx == kOrdSelf) return BlockPos{j0, i0};
-        if (static_cast<int>(idx) >= ngrid) return BlockPos{0, 0};
-        const int rr = div_magic(static_cast<int>(idx), nc_div);
-        return BlockPos{tp + rr * st, l + (static_cast<int>(idx) - rr * nc) * st};
+        if (idx == kOrdSelf) return BlockPos{e.j0, e.i0};
+        if (static_cast<int>(idx) >= e.ngrid) return BlockPos{0, 0};
+        const int rr = div_magic(static_cast<int>(idx), e.nc_div);
+        return BlockPos{e.tp + rr * e.st, e.l + (static_cast<int>(idx) - rr * e.nc) * e.st};
     };
     auto put = [&](int rank, const K &m) {  // rank-th best candidate -> list[rank + 1]
         list[rank + 1] = place(m.idx());
         lkeys[rank + 1] = m.key();
     };
     auto make = [&](B bits, unsigned idx) {
-        return bits == none ? K::invalid() : K::make(key_from_dist(DB::value(bits), a.distMul), idx);
+        return bits == none ? K::invalid() : K::make(key_from_dist(DB::value(bits), e.dist_mul), idx);
     };
     bool tie = false;
     if (take > 0) {
@@ -510,15 +569,58 @@ __device__ __forceinline__ int select_group(const StageArgs<T> &a, const typenam
         B tb = r0 < take ? lmin : B(0);
         if (two && r1 < take && lmin2 > tb) tb = lmin2;
         tb = DB::warp_max(tb);
-        B cut = none - 1;  // fewer than take lanes hold a candidate: keep them all
-        bool sure = true;
-        if (tb != none) {
-            const B kt = DB::of(key_from_dist(DB::value(tb), a.distMul));
-            sure = kt >= DB::kLow && kt <= DB::kHigh;  // else the slack does not hold
-            cut = tb + 3;
-            if (NEAR) cut += DB::kNear;
+        // The cut leaves slack for distances that share the bound's key. With
+        // fewer than take lanes holding a candidate it keeps them all.
+        const B slack = 3 + (NEAR && near ? DB::kNear : 0);
+        bool sure = true;  // the slack holds (keys are normal)
+        auto cut_at = [&](B bound) {
+            if (bound >= none - slack) return static_cast<B>(none - 1);
+            const B kt = DB::of(key_from_dist(DB::value(bound), e.dist_mul));
+            sure = kt >= DB::kLow && kt <= DB::kHigh;
+            return static_cast<B>(bound + slack);
+        };
+        auto count = [&](B top) {  // this lane's elements at or under top
+            int c = 0;
+            for (int first = 0; first < nkeys; first += kHeld * kWarp) {
+                if (!one) load(first);
+#pragma unroll
+                for (int k = 0; k < kHeld; ++k) c += v[k] <= top ? 1 : 0;
+            }
+            return c;
+        };
+        B cut = cut_at(tb);
+        int mine = count(cut);
+        // Candidates that crowd into few lanes leave the bound too high: halve the
+        // range for a lower one that still has take elements under it. (The ordered
+        // search that such lists fell back to takes 31 passes over 1089 places; as
+        // the last warp of a tile it held up the others.)
+        int pos = 0, M = 0;  // this lane's end among the compacted ones, and their number
+        auto scan = [&] {
+            pos = mine;
+#pragma unroll
+            for (int o = 1; o < kWarp; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, pos, o);
+                if (lane >= o) pos += u;
+            }
+            M = __shfl_sync(0xffffffffu, pos, kWarp - 1);
+        };
+        scan();
+        if (M > kCand) {
+            B lo = 0, hi = tb == none ? none - 1 : tb;
+            while (hi - lo > 1) {
+                const B mid = lo + (hi - lo) / 2;
+                if (__reduce_add_sync(0xffffffffu, count(mid)) < take) {
+                    lo = mid;
+                    continue;
+                }
+                hi = mid;
+                cut = cut_at(hi);
+                mine = count(cut);
+                if (__reduce_add_sync(0xffffffffu, mine) <= kCand) break;
+            }
+            scan();
         }
-        if constexpr (NEAR) {
+        if (NEAR && near) {
             if (!sure || limit < DB::kTiny) return -1;
             // a distance too close to the threshold to tell matters when it can be
             // kept, or when the group takes every accepted one; either way the cut
@@ -531,21 +633,8 @@ __device__ __forceinline__ int select_group(const StageArgs<T> &a, const typenam
             }
         }
         // Compact the elements at or under the cut into heap[] (any order).
-        int mine = 0;
-        for (int first = 0; first < nkeys; first += kHeld * kWarp) {
-            if (!one) load(first);
-#pragma unroll
-            for (int k = 0; k < kHeld; ++k) mine += v[k] <= cut ? 1 : 0;
-        }
-        int pos = mine;
-#pragma unroll
-        for (int o = 1; o < kWarp; o <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, pos, o);
-            if (lane >= o) pos += u;
-        }
-        const int M = __shfl_sync(0xffffffffu, pos, kWarp - 1);
-        if (NEAR && M > kCand) return -1;
-        if (NEAR || (sure && M <= kCand)) {
+        if (NEAR && near && M > kCand) return -1;
+        if (sure && M <= kCand) {
             pos -= mine;
             for (int first = 0; first < nkeys; first += kHeld * kWarp) {
                 if (!one) load(first);
@@ -559,7 +648,7 @@ __device__ __forceinline__ int select_group(const StageArgs<T> &a, const typenam
             K v0 = lane < M ? heap[lane] : K::invalid();  // distances for now, not keys
             K v1 = lane + kWarp < M ? heap[lane + kWarp] : K::invalid();
             bool ranked = false;
-            if constexpr (NEAR) {
+            if (NEAR && near) {
                 B *sorted = kb + kCand;
                 __syncwarp();
                 kb[lane] = v0.key_bits();
@@ -586,8 +675,8 @@ __device__ __forceinline__ int select_group(const StageArgs<T> &a, const typenam
                 if (__any_sync(0xffffffffu, v0.key_bits() < DB::kTiny || v1.key_bits() < DB::kTiny))
                     return -1;
                 if (!ranked) {
-                    if (lane < M) v0 = K::pack(exact(static_cast<int>(v0.idx())), v0.idx());
-                    if (lane + kWarp < M) v1 = K::pack(exact(static_cast<int>(v1.idx())), v1.idx());
+                    if (lane < M) v0 = K::pack(exact_dist(e, static_cast<int>(v0.idx())), v0.idx());
+                    if (lane + kWarp < M) v1 = K::pack(exact_dist(e, static_cast<int>(v1.idx())), v1.idx());
                 }
             }
             if (!ranked) {
@@ -626,7 +715,7 @@ __device__ __forceinline__ int select_group(const StageArgs<T> &a, const typenam
                     const bool t0 = lane < M && e0 && r0 < take;
                     const bool t1 = lane + kWarp < M && e1 && r1 < take;
                     tie = __any_sync(0xffffffffu, t0 || t1);
-                    if (NEAR && tie) return -1;
+                    if (NEAR && near && tie) return -1;
                 }
             }
             if (lane < M && r0 < take) put(r0, v0);
@@ -663,7 +752,7 @@ __device__ __forceinline__ int select_group(const StageArgs<T> &a, const typenam
     // with that exact algorithm when a tie touches the kept set: lane 0 works
     // the heap, the warp finds the entries that change it (the heap's top only
     // falls, so an entry not below it once is never below it).
-    if (!NEAR && accepted + 1 > GS && GS > 1 && tie) {
+    if (accepted + 1 > GS && GS > 1 && tie) {
         auto less = [](const K &p, const K &q) { return p.key() < q.key(); };
         auto adjust = [&](int hole, int len, K value) {
             const int top = hole;
@@ -742,22 +831,25 @@ __device__ __forceinline__ int select_group(const StageArgs<T> &a, const typenam
     return take + 1;
 }
 
-// A candidate's entry in the search list. Distances are sums of squares:
-// >= +0, or NaN, whose bits compare above any threshold. A zero distance (the
-// reference block itself, or an equal block) is rejected like one over the
-// threshold (include/Block.h:606): (bits - 1) wraps to the top for it.
-template <typename B>
-__device__ __forceinline__ B accept_dist(B bits, B limit, int &nvalid)
+// The same, the list made exact when its approximate distances do not decide
+// (one copy of the selection's code serves both: the stage kernels wait on
+// their instruction cache).
+template <typename T, bool NEAR>
+__device__ __forceinline__ int select_group(const Search<T> &e, bool near, int lane, int nvalid,
+                                            unsigned &n_fix)
 {
-    const bool ok = bits - 1 < limit;
-    nvalid += ok ? 1 : 0;
-    return ok ? bits : ~B(0);
-}
-
-// The matching threshold as distance bits: d <= thSSE is bits <= limit.
-template <typename T> __device__ __forceinline__ typename DistBits<T>::type dist_limit(T thSSE)
-{
-    return thSSE > T(0) ? DistBits<T>::of(thSSE) : typename DistBits<T>::type(0);
+    for (;;) {
+        if (NEAR && !near) {
+            __syncwarp();
+            nvalid = 0;
+            for (int i = lane; i <= e.ngrid; i += kWarp)
+                e.dist[i] = accept_dist(exact_dist(e, i), e.limit, nvalid);
+            __syncwarp();
+        }
+        const int n = select_once<T, NEAR>(e, near, lane, nvalid, n_fix);
+        if (n > 0) return n;
+        near = false;
+    }
 }
 
 // Which strip each lane takes in each round over a full window (KS = kStrip):
@@ -945,43 +1037,28 @@ __device__ int match_block(const StageArgs<T> &a, const Tile<T> &t, int j0, int 
     __syncwarp();
     n_cand += static_cast<unsigned>(ngrid);  // grid minus self, plus (0, 0)
 
-    // The exact distance of a list place, in the reference's order.
-    auto exact = [&](int i) -> B {
-        const T *cb;
-        int cp = t.pitch;
-        if (i < ngrid) {
-            const int rr = div_magic(i, nc_div);
-            cb = t.refw[0] + (tp + rr * st - t.ry0) * t.pitch + (l + (i - rr * nc) * st - t.rx0);
-        } else {
-            cb = block_ptr(t, t.refw[0], t.ref0[0], 0, 0, cp);
-        }
-        T acc = T(0);
-#pragma unroll 1
-        for (int y = 0; y < kBS; ++y) {
-            T r[kBS], c[kBS];
-#pragma unroll
-            for (int x = 0; x < kBS; ++x) {
-                r[x] = rb[y * t.pitch + x];
-                c[x] = cb[y * cp + x];
-            }
-            acc = ssd_row8(acc, r, c);
-        }
-        return DistBits<T>::of(acc);
-    };
-    if constexpr (kNearList) {
-        if (a.group_key == nullptr) {
-            const int n = select_group<T, true>(a, dist, limit, exact, ngrid, nc, nc_div, tp, l, st, j0,
-                                                i0, lane, nvalid, heap, list, lkeys, n_fix);
-            if (n > 0) return n;
-        }
-        // rare: the whole list exactly
-        __syncwarp();
-        nvalid = 0;
-        for (int i = lane; i <= ngrid; i += kWarp) dist[i] = accept_dist(exact(i), limit, nvalid);
-        __syncwarp();
-    }
-    return select_group<T, false>(a, dist, limit, exact, ngrid, nc, nc_div, tp, l, st, j0, i0, lane,
-                                  nvalid, heap, list, lkeys, n_fix);
+    Search<T> e;
+    e.win = win;
+    e.refb = rb;
+    e.slot = block_ptr(t, t.refw[0], t.ref0[0], 0, 0, e.slot_pitch);
+    e.pitch = t.pitch;
+    e.st = st;
+    e.ngrid = ngrid;
+    e.nc = nc;
+    e.nc_div = nc_div;
+    e.tp = tp;
+    e.l = l;
+    e.j0 = j0;
+    e.i0 = i0;
+    e.group_size = a.group_size;
+    e.dist_mul = a.distMul;
+    e.limit = limit;
+    e.dist = dist;
+    e.heap = heap;
+    e.list = list;
+    e.lkeys = lkeys;
+    // group dumps carry exact keys
+    return select_group<T, kNearList>(e, kNearList && a.group_key == nullptr, lane, nvalid, n_fix);
 }
 
 // ---------------------------------------------------------------------------
@@ -991,17 +1068,43 @@ __device__ int match_block(const StageArgs<T> &a, const Tile<T> &t, int j0, int 
 // column and pencil accesses below are all conflict-free.
 __device__ __forceinline__ int gidx(int y, int x) { return y * 8 + x + ((y >> 2) << 2); }
 
-// Forward 2-D transform (rows then columns) of the n blocks of a group, read
-// from a staged window and left in the warp's group buffer. Lane (z, h) =
-// (lane / 2, lane % 2) owns rows 4h..4h+3, then columns 4h..4h+3, of block z.
-template <typename T>
+// Columns of the forward or inverse 2-D transform, in place in the group buffer.
+template <typename T, int MAXN, bool INV>
+__device__ __forceinline__ void xy_cols(T *G, int n, int lane)
+{
+    const int h = lane & 1;
+#pragma unroll 1
+    for (int z = lane >> 1; z < (MAXN > kGSMax ? n : min(n, kGSMax)); z += kGSMax) {
+        T *gz = G + z * kGroupStride;
+        Pair<T> c01[8], c23[8];  // columns 4h, 4h + 1 and 4h + 2, 4h + 3
+#pragma unroll
+        for (int y = 0; y < 8; ++y) Vec4<T>::load4(gz + gidx(y, 4 * h), c01[y], c23[y]);
+        if (INV) {
+            redft01_8(c01);
+            redft01_8(c23);
+        } else {
+            redft10_8(c01);
+            redft10_8(c23);
+        }
+#pragma unroll
+        for (int y = 0; y < 8; ++y) Vec4<T>::store4(gz + gidx(y, 4 * h), c01[y], c23[y]);
+    }
+    __syncwarp();
+}
+
+// Forward 2-D transform (rows then columns) of the n <= MAXN blocks of a group,
+// read from a staged window and left in the warp's group buffer. Lane (z, h) =
+// (lane / 2, lane % 2) owns rows 4h..4h+3, then columns 4h..4h+3, of blocks z
+// and (MAXN 32) z + 16.
+template <typename T, int MAXN = kGSMax>
 __device__ __forceinline__ void gather_xy_forward(const Tile<T> &t, const T *win, const T *origin,
                                                   const BlockPos *list, int n, int lane, T *G,
                                                   unsigned &n_bad)
 {
-    const int z = lane >> 1, h = lane & 1;
-    T *gz = G + z * kGroupStride;
-    if (z < n) {
+    const int h = lane & 1;
+#pragma unroll 1
+    for (int z = lane >> 1; z < (MAXN > kGSMax ? n : min(n, kGSMax)); z += kGSMax) {
+        T *gz = G + z * kGroupStride;
         const BlockPos p = list[z];
         const bool ok = block_in_tile(t, p.y, p.x);
         n_bad += ok ? 0 : 1;
@@ -1019,34 +1122,7 @@ __device__ __forceinline__ void gather_xy_forward(const Tile<T> &t, const T *win
         }
     }
     __syncwarp();
-    if (z < n) {
-        Pair<T> c01[8], c23[8];  // columns 4h, 4h + 1 and 4h + 2, 4h + 3
-#pragma unroll
-        for (int y = 0; y < 8; ++y) Vec4<T>::load4(gz + gidx(y, 4 * h), c01[y], c23[y]);
-        redft10_8(c01);
-        redft10_8(c23);
-#pragma unroll
-        for (int y = 0; y < 8; ++y) Vec4<T>::store4(gz + gidx(y, 4 * h), c01[y], c23[y]);
-    }
-    __syncwarp();
-}
-
-// Columns of the inverse 2-D transform, in place in the group buffer.
-template <typename T>
-__device__ __forceinline__ void xy_inverse_cols(T *G, int n, int lane)
-{
-    const int z = lane >> 1, h = lane & 1;
-    T *gz = G + z * kGroupStride;
-    if (z < n) {
-        Pair<T> c01[8], c23[8];  // columns 4h, 4h + 1 and 4h + 2, 4h + 3
-#pragma unroll
-        for (int y = 0; y < 8; ++y) Vec4<T>::load4(gz + gidx(y, 4 * h), c01[y], c23[y]);
-        redft01_8(c01);
-        redft01_8(c23);
-#pragma unroll
-        for (int y = 0; y < 8; ++y) Vec4<T>::store4(gz + gidx(y, 4 * h), c01[y], c23[y]);
-    }
-    __syncwarp();
+    xy_cols<T, MAXN, false>(G, n, lane);
 }
 
 // Pencils along the group axis: lane owns positions p = 2 lane and 2 lane + 1,
@@ -1215,6 +1291,44 @@ __device__ __forceinline__ void aggregate_member_slow(const StageArgs<T> &a, con
     }
 }
 
+// Rows of the inverse 2-D transform of the n <= MAXN blocks in the group buffer,
+// each aggregated as soon as it is ready: BlockGroup::AddTo / CountTo
+// (include/Block.h:1240-1265, 1334-1357). The weight is the same over the block,
+// so it is added once, at the block's origin; the normalisation sums origins
+// over each pixel's covering blocks. Integer sums make that exactly the
+// per-pixel sum.
+template <typename T, int MAXN>
+__device__ __forceinline__ void aggregate_group(const StageArgs<T> &a, const Tile<T> &t, int p, int pt,
+                                                const BlockPos *list, int n, int lane, const T *G,
+                                                T numW, T denW, float scale, bool check)
+{
+    const int h = lane & 1;
+#pragma unroll 1
+    for (int z = lane >> 1; z < (MAXN > kGSMax ? n : min(n, kGSMax)); z += kGSMax) {
+        if (!block_in_tile(t, list[z].y, list[z].x)) continue;
+        const BlockPos q = list[z];
+        const T *gz = G + z * kGroupStride;
+        if (!check && (q.y >= kBS || q.x >= kBS)) {
+            int pitch;
+            const AccWin<T> dn = block_acc(t, p, q.y, q.x, pitch);
+#pragma unroll 1
+            for (int r = 0; r < 4; ++r) {
+                const int y = 4 * h + r;
+                T v[8];
+                Vec4<T>::load(gz + gidx(y, 0), v[0], v[1], v[2], v[3]);
+                Vec4<T>::load(gz + gidx(y, 4), v[4], v[5], v[6], v[7]);
+                redft01_8(v);
+#pragma unroll
+                for (int x = 0; x < 8; ++x) acc_add(dn + (y * pitch + x), v[x] * numW, scale);
+            }
+            if (h == 0) weight_add(a.den[pt], a.width, q.y, q.x, denW, scale);
+        } else {
+            aggregate_member_slow<T>(a, t, p, pt, q, gz, h, numW, denW, scale);
+        }
+    }
+    __syncwarp();
+}
+
 // Collaborative filtering of one group on plane p, aggregated into the CTA's
 // accumulator windows.
 // `check`: the plane holds non-finite pixels (poison_map is not null), so
@@ -1279,36 +1393,9 @@ __device__ void filter_group(const StageArgs<T> &a, const Tile<T> &t, int p, con
 
     group_inv(G, n, lane, sp);
     __syncwarp();
-    xy_inverse_cols(G, n, lane);
+    xy_cols<T, kGSMax, true>(G, n, lane);
 
-    // Rows of the inverse 2-D transform, each aggregated as soon as it is
-    // ready: BlockGroup::AddTo / CountTo (include/Block.h:1240-1265,
-    // 1334-1357). The weight is the same over the block, so it is added once,
-    // at the block's origin; the normalisation sums origins over each pixel's
-    // covering blocks. Integer sums make that exactly the per-pixel sum.
-    const int z = lane >> 1, h = lane & 1;
-    if (z < n && block_in_tile(t, list[z].y, list[z].x)) {
-        const BlockPos q = list[z];
-        const T *gz = G + z * kGroupStride;
-        if (!check && (q.y >= kBS || q.x >= kBS)) {
-            int pitch;
-            const AccWin<T> dn = block_acc(t, p, q.y, q.x, pitch);
-#pragma unroll 1
-            for (int r = 0; r < 4; ++r) {
-                const int y = 4 * h + r;
-                T v[8];
-                Vec4<T>::load(gz + gidx(y, 0), v[0], v[1], v[2], v[3]);
-                Vec4<T>::load(gz + gidx(y, 4), v[4], v[5], v[6], v[7]);
-                redft01_8(v);
-#pragma unroll
-                for (int x = 0; x < 8; ++x) acc_add(dn + (y * pitch + x), v[x] * numW, scale);
-            }
-            if (h == 0) weight_add(a.den[pt], a.width, q.y, q.x, denW, scale);
-        } else {
-            aggregate_member_slow<T>(a, t, p, pt, q, gz, h, numW, denW, scale);
-        }
-    }
-    __syncwarp();
+    aggregate_group<T, kGSMax>(a, t, p, pt, list, n, lane, G, numW, denW, scale, check);
 }
 
 // ---------------------------------------------------------------------------

@@ -58,3 +58,23 @@ def test_normalisation_tile_edges(bm3d_lib, oracle_mod, shape, block):
     want = oracle_mod.backend("port", np.float32).stage(False, p.as_dict(), noisy)
     want = want[1] if isinstance(want, tuple) else want
     assert np.abs(out - want).max() <= 1e-3
+
+
+@pytest.mark.parametrize("wiener", [False, True])
+@pytest.mark.parametrize("group_size,thmse", [(17, 1500.0), (24, 900.0), (31, 1e5), (32, 1200.0), (32, 1e5)])
+def test_groups_of_up_to_32(bm3d_lib, oracle_mod, group_size, thmse, wiener):
+    """Group lengths of the generic kernel's 8 x 8 path: full groups of 32 and
+    every shorter length that a tight threshold leaves, against the oracle."""
+    import isp_mw_b200
+    from isp_mw_b200 import synth
+    noisy = synth.pair(58, 67, 20.0, 9)[1]
+    guide = synth.pair(58, 67, 8.0, 9)[1] if wiener else noisy
+    p = isp_mw_b200.stage_params_default("np", wiener, [34.0] * 3)
+    p.group_size, p.thMSE = group_size, thmse * (0.2 if wiener and thmse < 1e4 else 1.0)
+    ctx = isp_mw_b200.Context(0)
+    out = np.empty_like(noisy)
+    ctx.stage(p, wiener, out, noisy, guide)
+    ctx.close()
+    want = oracle_mod.backend("port", np.float32).stage(wiener, p.as_dict(), noisy, guide)
+    want = want[1] if isinstance(want, tuple) else want
+    assert np.abs(out - want).max() <= 1e-3
