@@ -15,8 +15,9 @@ namespace bm3d {
 // shared-memory copy takes one address register and no global loads.
 constexpr int kBatchHeader = 16 + static_cast<int>((sizeof(StageArgs<float>) + 15) / 16 * 16);
 
-template <typename T, bool WIENER, int NPL, int KS, bool GENERIC>
-__global__ void __launch_bounds__(GENERIC ? (sizeof(T) == 4 ? 384 : 256) : stage_max_warps<T>() * kWarp, 1)
+// GEN: -1 for the register-resident body, else the generic body's BSC.
+template <typename T, bool WIENER, int NPL, int KS, int GEN>
+__global__ void __launch_bounds__((GEN >= 0 ? generic_max_warps(sizeof(T), GEN) : stage_max_warps<T>()) * kWarp, 1)
     batch_stage_kernel(const StageArgs<T> *__restrict__ args, const int *__restrict__ tile_base,
                        int nimg, int *counter)
 {
@@ -47,8 +48,8 @@ __global__ void __launch_bounds__(GENERIC ? (sizeof(T) == 4 ? 384 : 256) : stage
             __syncthreads();
         }
         unsigned char *body = smem + kBatchHeader;
-        if constexpr (GENERIC && NPL == 3) generic_tile_body_seq3<T, WIENER>(a, it - tile_base[lo], body, avail);
-        else if constexpr (GENERIC) generic_tile_body<T, WIENER, NPL>(a, it - tile_base[lo], body, avail);
+        if constexpr (GEN >= 0 && NPL == 3) generic_tile_body_seq3<T, WIENER, GEN>(a, it - tile_base[lo], body, avail);
+        else if constexpr (GEN >= 0) generic_tile_body<T, WIENER, NPL, GEN>(a, it - tile_base[lo], body, avail);
         else if constexpr (NPL == 3) stage_tile_body_seq3<T, WIENER, KS>(a, it - tile_base[lo], body, avail);
         else stage_tile_body<T, WIENER, NPL, KS>(a, it - tile_base[lo], body, avail);
         __syncthreads();  // every thread has read *item before it is replaced

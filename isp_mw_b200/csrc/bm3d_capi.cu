@@ -454,7 +454,12 @@ static int launch_ks(bm3d_ctx *ctx, StageArgs<T> &a, cudaStream_t s, int warps)
 template <typename T, bool W, int NPL>
 static int launch_generic(bm3d_ctx *ctx, StageArgs<T> &a, cudaStream_t s, int warps)
 {
-    const void *kern = generic_kernel_fn<T, W, NPL>();
+    const void *kern = generic_kernel_fn<T, W, NPL, 0>();
+    if constexpr (sizeof(T) == 4) {
+        const int bsc = generic_size_class(sizeof(T), a.block_size);
+        if (bsc == kBS) kern = generic_kernel_fn<T, W, NPL, kBS>();
+        else if (bsc == 11) kern = generic_kernel_fn<T, W, NPL, 11>();
+    }
     const SmemPlan sp = plan_smem<T>(NPL, W, a.ref_alias_src, a.region_h, a.region_pitch,
                                      a.span, warps, true, a.block_size, a.group_size,
                                      a.tile_x * a.tile_y);
@@ -546,7 +551,7 @@ static double tile_cost(const bm3d_ctx *ctx, const StageArgs<T> &a, const SmemPl
                         const TileShape &t, int nplanes, bool generic)
 {
     const size_t sm_smem = ctx->smem_optin + 1024;  // an SM's share; 1 KB of it per CTA is reserved
-    const int regs = sizeof(T) == 8 ? 256 : generic ? 168 : 128;
+    const int regs = sizeof(T) == 8 || (generic && a.block_size == 11) ? 256 : generic ? 168 : 128;
     const int by_smem = static_cast<int>(sm_smem / (sp.total + 1024));
     const int by_regs = 65536 / (t.warps * kWarp * regs);
     const int per_sm = std::max(1, std::min(by_smem, by_regs));
@@ -583,13 +588,14 @@ static int plan_geometry(bm3d_ctx *ctx, StageArgs<T> &a, const bm3d_stage_params
     a.ny = ref_count(height - BS, a.step);
     a.span = 2 * (a.range / a.bm_step) + 1;
     // The launch bounds (register-resident 512 threads in FP32, 256 in FP64;
-    // generic 384 and 256) limit the warps; the small shapes are for windows
-    // that leave no room for more.
+    // generic 384, and 256 in FP64 and for BlockSize 11) limit the warps; the
+    // small shapes are for windows that leave no room for more.
     static const TileShape fast[] = {{2, 2, 4}, {4, 2, 8}, {4, 4, 8}, {4, 8, 8}, {6, 4, 8}, {8, 8, 16}};
     static const TileShape gen[] = {{6, 6, 12}, {6, 4, 12}, {4, 3, 12}, {3, 2, 6}, {2, 2, 4},
                                     {4, 4, 8},  {4, 2, 8},  {5, 2, 5},  {4, 4, 4}};
     static const TileShape gen_small[] = {{2, 2, 4}, {2, 2, 2}, {1, 1, 2}, {1, 1, 1}};
-    const int max_warps = generic ? (sizeof(T) == 4 ? 12 : 8) : stage_max_warps<T>();
+    const int max_warps = generic ? generic_max_warps(sizeof(T), generic_size_class(sizeof(T), BS))
+                                  : stage_max_warps<T>();
     if (generic || !ctx->tiling_set) {
         TileShape best{0, 0, 0};
         double least = 1e300;

@@ -170,6 +170,11 @@ int build_stage(bm3d_batch *B, bool wiener, int tx, int ty, int warps, StageBuil
     std::vector<int> base(1, 0);
     size_t smem = 0;
     bool generic = false;
+    {
+        const bm3d_stage_params &p = wiener ? B->pf[0] : B->pb[0];
+        if (!fast_args(p.block_size, p.group_size))
+            warps = std::min(warps, generic_max_warps(sizeof(float), generic_size_class(sizeof(float), p.block_size)));
+    }
     for (int i = 0; i < B->n; ++i) {
         const bm3d_stage_params *p = wiener ? &B->pf[i] : &B->pb[i];
         if ((wiener ? B->gf[i] : B->gb[i]) != Guard::Run) continue;
@@ -269,12 +274,19 @@ int launch_batch_stage(bm3d_batch *B, StageBuild &sbd, cudaStream_t s)
         return BM3D_OK;
     };
     const bool ks4 = (W ? B->pf[0].bm_step : B->pb[0].bm_step) == 1;
+    const int bsc = generic_size_class(sizeof(float), (W ? B->pf[0] : B->pb[0]).block_size);
     if (B->npl == 3) {
-        if (sbd.generic) return go(batch_kernel_fn<W, 3, 1, true>());
-        return go(ks4 ? batch_kernel_fn<W, 3, 4, false>() : batch_kernel_fn<W, 3, 1, false>());
+        if (sbd.generic)
+            return go(bsc == 11    ? batch_kernel_fn<W, 3, 1, 11>()
+                      : bsc == kBS ? batch_kernel_fn<W, 3, 1, kBS>()
+                                   : batch_kernel_fn<W, 3, 1, 0>());
+        return go(ks4 ? batch_kernel_fn<W, 3, 4, -1>() : batch_kernel_fn<W, 3, 1, -1>());
     }
-    if (sbd.generic) return go(batch_kernel_fn<W, 1, 1, true>());
-    return go(ks4 ? batch_kernel_fn<W, 1, 4, false>() : batch_kernel_fn<W, 1, 1, false>());
+    if (sbd.generic)
+        return go(bsc == 11    ? batch_kernel_fn<W, 1, 1, 11>()
+                  : bsc == kBS ? batch_kernel_fn<W, 1, 1, kBS>()
+                               : batch_kernel_fn<W, 1, 1, 0>());
+    return go(ks4 ? batch_kernel_fn<W, 1, 4, -1>() : batch_kernel_fn<W, 1, 1, -1>());
 }
 
 int launch_planes(bm3d_batch *B, const DevBuf &planes, bool prep, cudaStream_t s)
@@ -378,12 +390,16 @@ int tune_stage(bm3d_batch *B, StageBuild &sbd, const DevBuf &planes, bool autotu
                                        {6, 8, 16}, {8, 6, 12}, {4, 2, 8}, {2, 2, 4}, {4, 4, 4},
                                        {2, 2, 1}};
     static const int gen_cand[][3] = {{6, 6, 12}, {6, 4, 12}, {4, 3, 12}, {4, 4, 8},
-                                      {4, 4, 4},  {2, 2, 4},  {2, 2, 2},  {1, 1, 2}, {1, 1, 1}};
+                                      {5, 2, 5},  {4, 4, 4},  {2, 2, 4},  {2, 2, 2},
+                                      {1, 1, 2},  {1, 1, 1}};
     const int (*cand)[3] = generic ? gen_cand : fast_cand;
-    const int ncand = generic ? 9 : 11;
+    const int ncand = generic ? 10 : 11;
     int best = -1;
     float best_ms = 1e30f;
+    const int max_warps = generic ? generic_max_warps(sizeof(float), generic_size_class(sizeof(float), p.block_size))
+                                  : stage_max_warps<float>();
     for (int c = 0; c < ncand; ++c) {
+        if (cand[c][2] > max_warps) continue;  // a smaller shape comes below
         int rc = build_stage(B, W, cand[c][0], cand[c][1], cand[c][2], sbd);
         if (rc == BM3D_ERR_UNSUPPORTED) continue;
         if (rc != BM3D_OK) return rc;

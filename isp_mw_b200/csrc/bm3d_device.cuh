@@ -54,22 +54,6 @@ __device__ __forceinline__ float ssd_row8(float acc, const float (&r)[8], const 
     }
     return acc;
 }
-// The same sum up to rounding, in a third fewer operations: squares and sums
-// fused, even and odd columns in the two halves of acc. All terms are >= 0, so
-// it is within 98 * 2^-24 (relative) of the ordered sum -- 65 roundings there,
-// 33 here -- as long as neither is near the subnormal range.
-__device__ __forceinline__ unsigned long long ssd_row8_near(unsigned long long acc,
-                                                            const unsigned long long (&r)[4],
-                                                            const unsigned long long (&c)[4])
-{
-#pragma unroll
-    for (int x = 0; x < 4; ++x) {
-        unsigned long long d;
-        asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(r[x]), "l"(c[x]));
-        asm("fma.rn.f32x2 %0, %1, %1, %0;" : "+l"(acc) : "l"(d));
-    }
-    return acc;
-}
 __device__ __forceinline__ double ssd_row8(double acc, const double (&r)[8], const double (&c)[8])
 {
 #pragma unroll
@@ -366,9 +350,11 @@ __host__ __device__ constexpr bool generic_one_buffer(bool wiener, int bs)
 // displacement is 5 pixels or more ((3, 1) for 21, the residue many windows
 // had: on planes whose texture runs that way a 4K YUV frame took 6.1 instead
 // of 5.4 ms). They also give 4 * pitch = 20 or 12, which spreads block
-// matching's strips over the banks (build_tasks).
+// matching's strips over the banks (build_tasks). Windows of 252 and 253, the
+// widest a three-plane tile's group lists hold, take 253.
 __host__ __device__ inline int window_pitch(int w)
 {
+    if (w == 252 || w == 253) return 253;
     for (;; ++w) {
         const int r = w & 31;
         if (r == 5 || r == 13 || r == 19 || r == 27) return w;
@@ -405,14 +391,14 @@ __host__ __device__ inline SmemPlan plan_smem(int nplanes, bool wiener, int alia
     // block (0, 0) copies: T per staged window, then (16-byte aligned) Acc per accumulator
     s.off_origin_acc = s.off_origin + (sizeof(T) * bsq * s.n_stage + 15) / 16 * 16;
     s.off_tasks = (s.off_origin_acc + sizeof(Acc) * bsq * nplanes + 15) / 16 * 16;
-    s.off_warps = s.off_tasks + (bs == kBS ? sizeof(unsigned) * kWarp * task_rounds(span) : 0);
+    s.off_warps = s.off_tasks + (bs == kBS || bs == 11 ? sizeof(unsigned) * kWarp * task_rounds(span) : 0);
     const size_t group_bytes = generic
         ? sizeof(T) * static_cast<size_t>(gs) * generic_block_stride(bs) *
               (wiener && !generic_one_buffer<T>(wiener, bs) ? 2 : 1)
         : sizeof(T) * kGSMax * kGroupStride;
     const size_t key_bytes = sizeof(T) * (static_cast<size_t>(span) * span + 1);  // distance bits
     const auto up = [](size_t v) { return (v + 15) / 16 * 16; };
-    const size_t heap_bytes = sizeof(SortKey<T>) * kCand, ref_bytes = sizeof(T) * bsq;
+    const size_t heap_bytes = sizeof(SortKey<T>) * kCand, ref_bytes = sizeof(T) * bs * ((bs + 3) / 4 * 4);
     s.off_ref = s.off_heap = up(key_bytes);
     s.off_keys = s.off_heap + up(heap_bytes > ref_bytes ? heap_bytes : ref_bytes);
     const size_t match_bytes = s.off_keys + sizeof(T) * kGSTab;

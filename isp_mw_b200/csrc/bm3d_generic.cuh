@@ -4,8 +4,8 @@
 // and the separable 3-D transforms run one line per lane: 8-point butterflies
 // for BlockSize 8, recursive even/odd splits for full GroupSize-32 groups,
 // cosine matrices from global memory otherwise. Block matching keeps the
-// reference's exact distance order (BlockSize 8 with step 1 uses the
-// register-resident kernel's strips); selection, aggregation and the staged
+// reference's exact distance order (BlockSize 8, and 11 in FP32, with step 1 use
+// the register-resident kernel's strips); selection, aggregation and the staged
 // windows are shared with the register-resident kernel.
 //
 // Reference: as bm3d_stage.cuh (source/BM3D.cpp:80-457, include/Block.h:578-751).
@@ -70,7 +70,7 @@ __device__ __forceinline__ void dct_line11(T *base, int stride, bool inverse)
 }
 
 template <typename T>
-__device__ void dct_z_generic(T *G, int n, int bs, int lane, const T *tab, bool inverse);
+__device__ void dct_z_generic(T *G, int n, int bs, int lane, const T *tab, const float *pad, bool inverse);
 
 // Separable 3-D transform of an n x bs x bs group (row-major [z][y][x]) with
 // the concatenated matrices `tab` (forward REDFT10 or backward REDFT01, as
@@ -79,7 +79,7 @@ __device__ void dct_z_generic(T *G, int n, int bs, int lane, const T *tab, bool 
 // gathered or aggregated, their other passes in dct_cols_z_fwd /
 // dct_z_cols_inv.
 template <typename T>
-__device__ void dct3_generic(T *G, int n, int bs, int lane, const T *tab, bool inverse)
+__device__ void dct3_generic(T *G, int n, int bs, int lane, const T *tab, const float *pad, bool inverse)
 {
     const int bsq = bs * bs;
     if (sizeof(T) == 4 && bs == 11) {
@@ -101,7 +101,7 @@ __device__ void dct3_generic(T *G, int n, int bs, int lane, const T *tab, bool i
         }
     }
     __syncwarp();
-    dct_z_generic(G, n, bs, lane, tab, inverse);
+    dct_z_generic(G, n, bs, lane, tab, pad, inverse);
 }
 
 // Row-fused block sizes: 8 (both precisions) and 11 (FP32, the "vn" final
@@ -124,7 +124,7 @@ __device__ __forceinline__ void dct_line_bs(T *base, int stride, bool inverse)
 // Forward, after gather_rows (which transformed the rows): the columns, then
 // the group axis -- the passes and order of dct3_generic.
 template <typename T, int BS>
-__device__ void dct_cols_z_fwd(T *G, int n, int lane, const T *tab)
+__device__ void dct_cols_z_fwd(T *G, int n, int lane, const T *tab, const float *pad)
 {
     constexpr int ZS = BS == 8 ? 72 : BS * BS, RS = BS == 8 ? 9 : BS;
     for (int line = lane; line < n * BS; line += kWarp) {  // along y
@@ -132,17 +132,17 @@ __device__ void dct_cols_z_fwd(T *G, int n, int lane, const T *tab)
         dct_line_bs<T, BS>(G + z * ZS + x, RS, false);
     }
     __syncwarp();
-    dct_z_generic(G, n, BS, lane, tab, false);
+    dct_z_generic(G, n, BS, lane, tab, pad, false);
 }
 
 // Inverse: the group axis, then the columns; the rows are transformed by
 // aggregate_rows as it adds them (the register-resident kernel's inverse
 // order).
 template <typename T, int BS>
-__device__ void dct_z_cols_inv(T *G, int n, int lane, const T *tab)
+__device__ void dct_z_cols_inv(T *G, int n, int lane, const T *tab, const float *pad)
 {
     constexpr int ZS = BS == 8 ? 72 : BS * BS, RS = BS == 8 ? 9 : BS;
-    dct_z_generic(G, n, BS, lane, tab, true);
+    dct_z_generic(G, n, BS, lane, tab, pad, true);
     for (int line = lane; line < n * BS; line += kWarp) {  // along y
         const int z = line / BS, x = line - z * BS;
         dct_line_bs<T, BS>(G + z * ZS + x, RS, true);
@@ -150,34 +150,81 @@ __device__ void dct_z_cols_inv(T *G, int n, int lane, const T *tab)
     __syncwarp();
 }
 
-// The group-axis pass of a separable 3-D transform (see dct3_generic).
+// Group-axis transform of pencils g0 and g1 (length n < 32, stride zs)
+// by matrix columns m of 32 rows: y_k = sum_j m[k][j] x_j, j in order, from the
+// buffer into registers. ROWS (16 or 32) bounds n. Sums of all rows advance
+// together, so a step is independent loads and multiply-adds; row by row, each
+// output waited for its own chain of loads and adds, and one short group could
+// take longer than the rest of a tile.
+template <int ROWS>
+__device__ __forceinline__ void pencils_by_columns(const float *g0, const float *g1, int zs, int n,
+                                                   const float *m, Pair<float> (&out)[kGSTab])
+{
+    float a[ROWS], b[ROWS];
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) a[k] = b[k] = 0.0f;
+#pragma unroll 1
+    for (int j = 0; j < n; ++j) {
+        const float x0 = g0[j * zs], x1 = g1[j * zs];
+        const float4 *c = reinterpret_cast<const float4 *>(m + 32 * j);
+#pragma unroll
+        for (int k = 0; k < ROWS; k += 4) {
+            const float4 q = __ldg(c + k / 4);
+            const float r[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                a[k + i] = fmaf(r[i], x0, a[k + i]);
+                b[k + i] = fmaf(r[i], x1, b[k + i]);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kGSTab; ++k)
+        out[k] = k < ROWS ? Pair<float>::make(a[k < ROWS ? k : 0], b[k < ROWS ? k : 0])
+                          : Pair<float>::make(0.0f, 0.0f);
+}
+
+// The group-axis pass of a separable 3-D transform (see dct3_generic). FP32: two
+// pencils at a time as the halves of pairs, recursive even/odd splits for full
+// groups of 32 (dct.cuh), matrix columns for shorter ones.
 template <typename T>
-__device__ void dct_z_generic(T *G, int n, int bs, int lane, const T *tab, bool inverse)
+__device__ void dct_z_generic(T *G, int n, int bs, int lane, const T *tab, const float *pad, bool inverse)
 {
     // along the group: pencil p = (y, x) of every block
     const int bsq = bs * bs;
     const int zs = generic_block_stride(bs), rs = generic_row_stride(bs);
-    if constexpr (sizeof(T) == 4) {
-        if (n == 32) {  // full GroupSize-32 groups: recursive even/odd splits (dct.cuh)
-            for (int line = lane; line < bsq; line += kWarp) {
-                const int py = line / bs;
-                T *g = G + py * rs + (line - py * bs);
-                T v[32];
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = g[j * zs];
-                if (inverse) redft01_pow2<T, 32>(v);
-                else redft10_pow2<T, 32>(v);
-#pragma unroll
-                for (int k = 0; k < 32; ++k) g[k * zs] = v[k];
-            }
-            __syncwarp();
-            return;
-        }
-    }
-    const T *mz = tab + dct_table_offset(n);
-    for (int line = lane; line < bsq; line += kWarp) {
+    auto pencil = [&](int line) {
         const int py = line / bs;
-        dct_line(G + py * rs + (line - py * bs), zs, n, mz);
+        return G + py * rs + (line - py * bs);
+    };
+    if constexpr (sizeof(T) == 4) {
+        using P = Pair<float>;
+        const float *m = pad + pad32_offset(n < 32 ? n : 1);
+        for (int line = lane; line < bsq; line += 2 * kWarp) {
+            float *g0 = pencil(line);
+            const bool both = line + kWarp < bsq;
+            float *g1 = both ? pencil(line + kWarp) : g0;
+            P v[kGSTab];
+            if (n == 32) {
+#pragma unroll
+                for (int j = 0; j < kGSTab; ++j) v[j] = P::make(g0[j * zs], g1[j * zs]);
+                if (inverse) redft01_pow2<P, kGSTab>(v);
+                else redft10_pow2<P, kGSTab>(v);
+            } else if (n <= 16) {
+                pencils_by_columns<16>(g0, g1, zs, n, m, v);
+            } else {
+                pencils_by_columns<32>(g0, g1, zs, n, m, v);
+            }
+#pragma unroll
+            for (int k = 0; k < kGSTab; ++k)
+                if (k < n) {
+                    g0[k * zs] = v[k].lo();
+                    if (both) g1[k * zs] = v[k].hi();
+                }
+        }
+    } else {
+        const T *mz = tab + dct_table_offset(n);
+        for (int line = lane; line < bsq; line += kWarp) dct_line(pencil(line), zs, n, mz);
     }
     __syncwarp();
 }
@@ -264,7 +311,28 @@ __device__ int match_generic(const StageArgs<T> &a, const Tile<T> &t, int j0, in
     e.heap = heap;
     e.list = list;
     e.lkeys = lkeys;
-    return select_group<T, false>(e, false, lane, nvalid, n_fix);
+    return select_group<T, false, kBS>(e, false, lane, nvalid, n_fix);
+}
+
+// Whether blocks of size bs match by strips of candidates (with BMstep 1).
+template <typename T, int BSC> __device__ __forceinline__ bool strip_blocks(int bs)
+{
+    return BSC == kBS || BSC == 11 || (sizeof(T) == 8 && BSC == 0 && bs == kBS);
+}
+
+// Block matching by strips where they apply, else one lane per candidate.
+template <typename T, int BSC>
+__device__ __forceinline__ int match_any(const StageArgs<T> &a, const Tile<T> &t, bool strips, int j0,
+                                         int i0, int lane, const unsigned *tasks,
+                                         typename DistBits<T>::type *dist, T *refblk, SortKey<T> *heap,
+                                         BlockPos *list, T *lkeys, unsigned &n_cand, unsigned &n_fix)
+{
+    if constexpr (BSC > 0 || sizeof(T) == 8) {
+        if (strips)
+            return match_block<T, kStrip, (BSC > 0 ? BSC : kBS)>(a, t, j0, i0, lane, tasks, dist, refblk,
+                                                                  heap, list, lkeys, n_cand, n_fix);
+    }
+    return match_generic<T>(a, t, j0, i0, lane, dist, refblk, heap, list, lkeys, n_cand, n_fix);
 }
 
 // Element e of a group stored [z][y][x]: shifts for BlockSize 8, divisions
@@ -374,40 +442,6 @@ __device__ __forceinline__ void aggregate_rows(const StageArgs<T> &a, const Tile
     }
 }
 
-// Group-axis transform of pencils g0 and g1 (length n < 32, stride kGroupStride)
-// by matrix columns m of 32 rows: y_k = sum_j m[k][j] x_j, j in order, from the
-// buffer into registers. ROWS (16 or 32) bounds n. Sums of all rows advance
-// together, so a step is independent loads and multiply-adds; row by row, each
-// output waited for its own chain of loads and adds, and one short group could
-// take longer than the rest of a tile.
-template <int ROWS>
-__device__ __forceinline__ void pencils_by_columns(const float *g0, const float *g1, int n,
-                                                   const float *m, Pair<float> (&out)[kGSTab])
-{
-    float a[ROWS], b[ROWS];
-#pragma unroll
-    for (int k = 0; k < ROWS; ++k) a[k] = b[k] = 0.0f;
-#pragma unroll 1
-    for (int j = 0; j < n; ++j) {
-        const float x0 = g0[j * kGroupStride], x1 = g1[j * kGroupStride];
-        const float4 *c = reinterpret_cast<const float4 *>(m + 32 * j);
-#pragma unroll
-        for (int k = 0; k < ROWS; k += 4) {
-            const float4 q = __ldg(c + k / 4);
-            const float r[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                a[k + i] = fmaf(r[i], x0, a[k + i]);
-                b[k + i] = fmaf(r[i], x1, b[k + i]);
-            }
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < kGSTab; ++k)
-        out[k] = k < ROWS ? Pair<float>::make(a[k < ROWS ? k : 0], b[k < ROWS ? k : 0])
-                          : Pair<float>::make(0.0f, 0.0f);
-}
-
 // Collaborative filtering of an FP32 group of 8 x 8 blocks, up to 32 of them, in
 // one group buffer of the register-resident kernel's layout and passes (16-byte
 // rows, columns in packed pairs). Each lane owns pencils lane and lane + 32 of
@@ -427,8 +461,8 @@ __device__ void filter_group32(const StageArgs<float> &a, const Tile<float> &t, 
     float *const g0 = G + gidx(lane >> 3, lane & 7);        // pencil lane
     float *const g1 = G + gidx((lane >> 3) + 4, lane & 7);  // pencil lane + 32
     auto by_columns = [&](const float *m, P (&v)[kGSTab]) {
-        if (n <= 16) pencils_by_columns<16>(g0, g1, n, m + pad32_offset(n), v);
-        else pencils_by_columns<32>(g0, g1, n, m + pad32_offset(n), v);
+        if (n <= 16) pencils_by_columns<16>(g0, g1, kGroupStride, n, m + pad32_offset(n), v);
+        else pencils_by_columns<32>(g0, g1, kGroupStride, n, m + pad32_offset(n), v);
     };
     auto forward = [&](P (&v)[kGSTab]) {
         if (n == kGSTab) {
@@ -508,8 +542,9 @@ __device__ void filter_group32(const StageArgs<float> &a, const Tile<float> &t, 
     aggregate_group<float, kGSTab>(a, t, p, pt, list, n, lane, G, numW, denW, scale, check);
 }
 
-// Collaborative filtering of one group on plane p (generic sizes).
-template <typename T, bool WIENER>
+// Collaborative filtering of one group on plane p (generic sizes; BSC as in
+// generic_stage_kernel).
+template <typename T, bool WIENER, int BSC>
 __device__ void filter_generic(const StageArgs<T> &a, const Tile<T> &t, int p, const BlockPos *list,
                                int n, int lane, T *Gs, T *Gr, float scale,
                                unsigned &n_bad, int pt = -1, bool check = false)
@@ -517,13 +552,11 @@ __device__ void filter_generic(const StageArgs<T> &a, const Tile<T> &t, int p, c
     // p indexes the tile's windows; pt (default p) the plane's threshold /
     // Wiener tables, which differ when planes share one set of windows
     if (pt < 0) pt = p;
-    if constexpr (sizeof(T) == 4) {
-        if (t.bs == kBS) {
-            filter_group32<WIENER>(a, t, p, list, n, lane, Gs, scale, n_bad, pt, check);
-            return;
-        }
+    if constexpr (BSC == kBS) {
+        filter_group32<WIENER>(a, t, p, list, n, lane, Gs, scale, n_bad, pt, check);
+        return;
     }
-    const int bs = t.bs, bsq = bs * bs, total = n * bsq;
+    const int bs = BSC > 0 ? BSC : t.bs, bsq = bs * bs, total = n * bsq;
     const int zs = generic_block_stride(bs), rs = generic_row_stride(bs);
     T denW;
     if (bs == 8) {
@@ -532,7 +565,7 @@ __device__ void filter_generic(const StageArgs<T> &a, const Tile<T> &t, int p, c
             gather_rows<T, 8>(t, t.refw[p], t.ref0[p], list, n, lane, Gr,
                               static_cast<unsigned *>(nullptr));
         __syncwarp();
-        dct_cols_z_fwd<T, 8>(Gs, n, lane, a.dct_fwd);
+        dct_cols_z_fwd<T, 8>(Gs, n, lane, a.dct_fwd, a.pad_fwd);
     } else if (rows_fused<T>(bs)) {  // 11, FP32
         if constexpr (sizeof(T) == 4) {
             gather_rows<T, 11>(t, t.srcw[p], t.src0[p], list, n, lane, Gs, &n_bad);
@@ -540,7 +573,7 @@ __device__ void filter_generic(const StageArgs<T> &a, const Tile<T> &t, int p, c
                 gather_rows<T, 11>(t, t.refw[p], t.ref0[p], list, n, lane, Gr,
                                    static_cast<unsigned *>(nullptr));
             __syncwarp();
-            dct_cols_z_fwd<T, 11>(Gs, n, lane, a.dct_fwd);
+            dct_cols_z_fwd<T, 11>(Gs, n, lane, a.dct_fwd, a.pad_fwd);
         }
     } else {
         for (int e = lane; e < total; e += kWarp) {
@@ -561,7 +594,7 @@ __device__ void filter_generic(const StageArgs<T> &a, const Tile<T> &t, int p, c
             }
         }
         __syncwarp();
-        dct3_generic(Gs, n, bs, lane, a.dct_fwd, false);
+        dct3_generic(Gs, n, bs, lane, a.dct_fwd, a.pad_fwd, false);
     }
     if (!WIENER) {
         // hard threshold (source/BM3D.cpp:361-371) with thr by #zero indices
@@ -579,11 +612,11 @@ __device__ void filter_generic(const StageArgs<T> &a, const Tile<T> &t, int p, c
         const int retained = __reduce_add_sync(0xffffffffu, kept);
         denW = retained < 1 ? T(1) : T(1) / static_cast<T>(retained);
     } else {
-        if (bs == 8) dct_cols_z_fwd<T, 8>(Gr, n, lane, a.dct_fwd);
+        if (bs == 8) dct_cols_z_fwd<T, 8>(Gr, n, lane, a.dct_fwd, a.pad_fwd);
         else if (rows_fused<T>(bs)) {
-            if constexpr (sizeof(T) == 4) dct_cols_z_fwd<T, 11>(Gr, n, lane, a.dct_fwd);
+            if constexpr (sizeof(T) == 4) dct_cols_z_fwd<T, 11>(Gr, n, lane, a.dct_fwd, a.pad_fwd);
         } else {
-            dct3_generic(Gr, n, bs, lane, a.dct_fwd, false);
+            dct3_generic(Gr, n, bs, lane, a.dct_fwd, a.pad_fwd, false);
         }
         const T s2 = a.wss[pt][n - 1];
         T l2 = T(0);
@@ -601,20 +634,20 @@ __device__ void filter_generic(const StageArgs<T> &a, const Tile<T> &t, int p, c
     const T numW = static_cast<T>(static_cast<double>(denW) / a.finalAMP[n - 1]);
     __syncwarp();
     if (bs == 8) {
-        dct_z_cols_inv<T, 8>(Gs, n, lane, a.dct_inv);
+        dct_z_cols_inv<T, 8>(Gs, n, lane, a.dct_inv, a.pad_inv);
         aggregate_rows<T, 8>(a, t, p, pt, list, n, lane, Gs, numW, denW, scale, check);
         __syncwarp();
         return;
     }
     if constexpr (sizeof(T) == 4) {
         if (bs == 11) {
-            dct_z_cols_inv<T, 11>(Gs, n, lane, a.dct_inv);
+            dct_z_cols_inv<T, 11>(Gs, n, lane, a.dct_inv, a.pad_inv);
             aggregate_rows<T, 11>(a, t, p, pt, list, n, lane, Gs, numW, denW, scale, check);
             __syncwarp();
             return;
         }
     }
-    dct3_generic(Gs, n, bs, lane, a.dct_inv, true);
+    dct3_generic(Gs, n, bs, lane, a.dct_inv, a.pad_inv, true);
     // the block weight once per block, at its origin (as the register-resident kernel)
     for (int e = lane; e < total; e += kWarp) {
         int z, y, x;
@@ -651,13 +684,13 @@ __device__ void filter_generic(const StageArgs<T> &a, const Tile<T> &t, int p, c
     __syncwarp();
 }
 
-template <typename T, bool WIENER, int NPL>
+template <typename T, bool WIENER, int NPL, int BSC>
 __device__ __forceinline__ void generic_tile_body(const StageArgs<T> &a, int tile, unsigned char *smem,
                                                   unsigned avail)
 {
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-    const int bs = a.block_size;
+    const int bs = BSC > 0 ? BSC : a.block_size;
     const int right = a.width - bs, bottom = a.height - bs;
 
     Tile<T> t;
@@ -672,7 +705,7 @@ __device__ __forceinline__ void generic_tile_body(const StageArgs<T> &a, int til
     carve_tile<T, WIENER, NPL>(a, sp, smem, t);
     unsigned *tasks = reinterpret_cast<unsigned *>(smem + sp.off_tasks);
     unsigned char *wbase = smem + sp.off_warps + sp.warp_bytes * warp;
-    const bool strips = bs == kBS && a.bm_step == 1;
+    const bool strips = strip_blocks<T, BSC>(bs) && a.bm_step == 1;
     if (strips && warp == 0)
         build_tasks(tasks, reinterpret_cast<unsigned *>(wbase), a.span, t.pitch, lane);
     stage_tile<T, WIENER, NPL>(a, t);
@@ -701,11 +734,8 @@ __device__ __forceinline__ void generic_tile_body(const StageArgs<T> &a, int til
         const int j0 = ref_pos(ky, a.step, bottom), i0 = ref_pos(kx, a.step, right);
         // BlockSize 8 with step 1: the register-resident kernel's strips of
         // four candidates; otherwise one lane per candidate
-        const int n = strips
-                          ? match_block<T, kStrip>(a, t, j0, i0, lane, tasks, dist, refblk, heap, list, lkeys, n_cand,
-                                              n_fix)
-                          : match_generic<T>(a, t, j0, i0, lane, dist, refblk, heap, list, lkeys,
-                                             n_cand, n_fix);
+        const int n = match_any<T, BSC>(a, t, strips, j0, i0, lane, tasks, dist, refblk, heap, list,
+                                        lkeys, n_cand, n_fix);
         n_sum += n;
         n_sq += static_cast<unsigned>(n * n);
         dump_group(a, ky, kx, n, lane, list, lkeys);
@@ -713,7 +743,7 @@ __device__ __forceinline__ void generic_tile_body(const StageArgs<T> &a, int til
 #pragma unroll
             for (int p = 0; p < NPL; ++p)
                 if (a.active & (1 << p))
-                    filter_generic<T, WIENER>(a, t, p, list, n, lane, Gs, Gr, scale[p], n_bad,
+                    filter_generic<T, WIENER, BSC>(a, t, p, list, n, lane, Gs, Gr, scale[p], n_bad,
                                               -1, check[p]);
         }
         __syncwarp();
@@ -728,13 +758,13 @@ __device__ __forceinline__ void generic_tile_body(const StageArgs<T> &a, int til
 // through a single plane's windows (as stage_tile_body_seq3): plane 0 matches
 // and keeps each reference block's group list in shared memory, planes 1 and
 // 2 re-stage their windows and filter with those lists.
-template <typename T, bool WIENER>
+template <typename T, bool WIENER, int BSC>
 __device__ __forceinline__ void generic_tile_body_seq3(const StageArgs<T> &a, int tile,
                                                        unsigned char *smem, unsigned avail)
 {
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-    const int bs = a.block_size, GS = a.group_size;
+    const int bs = BSC > 0 ? BSC : a.block_size, GS = a.group_size;
     const int right = a.width - bs, bottom = a.height - bs;
 
     Tile<T> t;
@@ -754,7 +784,7 @@ __device__ __forceinline__ void generic_tile_body_seq3(const StageArgs<T> &a, in
 
     unsigned *tasks = reinterpret_cast<unsigned *>(smem + sp.off_tasks);
     unsigned char *wbase = smem + sp.off_warps + sp.warp_bytes * warp;
-    const bool strips = bs == kBS && a.bm_step == 1;
+    const bool strips = strip_blocks<T, BSC>(bs) && a.bm_step == 1;
     if (strips && warp == 0)
         build_tasks(tasks, reinterpret_cast<unsigned *>(wbase), a.span, t.pitch, lane);
     T *Gs = reinterpret_cast<T *>(wbase);
@@ -779,11 +809,8 @@ __device__ __forceinline__ void generic_tile_body_seq3(const StageArgs<T> &a, in
             if (c == 0) {
                 const int ky = ky0 + r / tw, kx = kx0 + r % tw;
                 const int j0 = ref_pos(ky, a.step, bottom), i0 = ref_pos(kx, a.step, right);
-                n = strips
-                        ? match_block<T, kStrip>(a, t, j0, i0, lane, tasks, dist, refblk, heap, list, lkeys, n_cand,
-                                            n_fix)
-                        : match_generic<T>(a, t, j0, i0, lane, dist, refblk, heap, list, lkeys,
-                                           n_cand, n_fix);
+                n = match_any<T, BSC>(a, t, strips, j0, i0, lane, tasks, dist, refblk, heap, list,
+                                      lkeys, n_cand, n_fix);
                 n_sum += n;
                 n_sq += static_cast<unsigned>(n * n);
                 dump_group(a, ky, kx, n, lane, list, lkeys);
@@ -806,7 +833,7 @@ __device__ __forceinline__ void generic_tile_body_seq3(const StageArgs<T> &a, in
             }
             __syncwarp();
             if (filt)
-                filter_generic<T, WIENER>(a, t, 0, list, n, lane, Gs, Gr, scale, n_bad, c, check);
+                filter_generic<T, WIENER, BSC>(a, t, 0, list, n, lane, Gs, Gr, scale, n_bad, c, check);
             __syncwarp();
         }
         __syncthreads();
@@ -816,13 +843,28 @@ __device__ __forceinline__ void generic_tile_body_seq3(const StageArgs<T> &a, in
     flush_stats(a, lane, n_sum, n_sq, n_cand, n_fix, n_bad);
 }
 
-template <typename T, bool WIENER, int NPL>
-__global__ void __launch_bounds__(sizeof(T) == 4 ? 384 : 256, 1)
+// BSC: BlockSize 8 (groups of up to 32) and 11 in FP32 have kernels of their own,
+// so that neither's registers and code are the other's: 11 x 11 groups of 32
+// leave shared memory for five warps, and that kernel takes up to 255 registers
+// a thread. 0 is any size. Against one kernel for all (168 registers, 240 bytes
+// of them spilled): np's final stage on 1283 x 717 2.05 -> 1.93 ms, vn's (11 x 11,
+// with strips) on 960 x 540 1.47 -> 1.13 ms.
+__host__ __device__ constexpr int generic_max_warps(int elem_bytes, int bsc)
+{
+    return elem_bytes == 8 || bsc == 11 ? 8 : 12;
+}
+__host__ __device__ constexpr int generic_size_class(int elem_bytes, int bs)
+{
+    return elem_bytes == 4 && (bs == kBS || bs == 11) ? bs : 0;
+}
+
+template <typename T, bool WIENER, int NPL, int BSC>
+__global__ void __launch_bounds__(generic_max_warps(sizeof(T), BSC) * kWarp, 1)
     generic_stage_kernel(const StageArgs<T> a)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    if constexpr (NPL == 3) generic_tile_body_seq3<T, WIENER>(a, blockIdx.x, smem, dynamic_smem_bytes());
-    else generic_tile_body<T, WIENER, NPL>(a, blockIdx.x, smem, dynamic_smem_bytes());
+    if constexpr (NPL == 3) generic_tile_body_seq3<T, WIENER, BSC>(a, blockIdx.x, smem, dynamic_smem_bytes());
+    else generic_tile_body<T, WIENER, NPL, BSC>(a, blockIdx.x, smem, dynamic_smem_bytes());
 }
 
 }  // namespace bm3d

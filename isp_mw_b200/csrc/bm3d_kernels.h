@@ -11,10 +11,10 @@ namespace bm3d {
 
 // stage_kernel<T, W, NPL, KS> (bm3d_stage.cuh)
 template <typename T, bool W, int NPL, int KS> const void *stage_kernel_fn();
-// generic_stage_kernel<T, W, NPL> (bm3d_generic.cuh)
-template <typename T, bool W, int NPL> const void *generic_kernel_fn();
-// batch_stage_kernel<float, W, NPL, KS, GENERIC> (bm3d_batch.cuh)
-template <bool W, int NPL, int KS, bool GENERIC> const void *batch_kernel_fn();
+// generic_stage_kernel<T, W, NPL, BSC> (bm3d_generic.cuh)
+template <typename T, bool W, int NPL, int BSC> const void *generic_kernel_fn();
+// batch_stage_kernel<float, W, NPL, KS, GEN> (bm3d_batch.cuh)
+template <bool W, int NPL, int KS, int GEN> const void *batch_kernel_fn();
 
 // Cosine matrices for group lengths 1..16, concatenated (1496 entries each).
 struct DctTableData {
@@ -36,4 +36,6 @@ cudaError_t upload_dct_tables_all(const DctTableData &t);
     X(generic_f32)           \
     X(generic_f64)           \
     X(batch_basic)           \
-    X(batch_final)
+    X(batch_final)          \
+    X(batch_generic_basic)  \
+    X(batch_generic_final)

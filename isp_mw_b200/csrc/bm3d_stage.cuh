@@ -280,12 +280,13 @@ template <> struct DistBits<float> {
     static __device__ __forceinline__ float value(unsigned b) { return __uint_as_float(b); }
     // keys between 2^-124 and 2^127: normal, with room for the rounding slack
     static constexpr unsigned kLow = 0x01800000u, kHigh = 0x7f000000u;
-    // approximate distances (ssd_row8_near): two that differ by more than kNear
-    // units in the last place are in the order of the exact keys. kNear of them
-    // are at least 256 * 2^-24 of the value; the bounds need 2 (65 + 33) 2^-24
-    // for the two sums and 4 * 2^-24 for keys that round together. All of it
-    // holds above kTiny = 2^-100, far from the subnormal range.
-    static constexpr unsigned kNear = 256u, kTiny = 0x0d800000u;
+    // approximate distances (ssd_row_near): two that differ by more than near_ulps
+    // units in the last place are in the order of the exact keys. A unit is at least
+    // 2^-24 of the value; the bounds need twice the two sums' roundings (8 x 8
+    // blocks: 65 + 33, 11 x 11: 122 + 67) and 4 for keys that round together. All
+    // of it holds above kTiny = 2^-100, far from the subnormal range.
+    static constexpr unsigned near_ulps(int bs) { return bs <= 8 ? 256u : 512u; }
+    static constexpr unsigned kTiny = 0x0d800000u;
     static __device__ __forceinline__ unsigned warp_max(unsigned v)
     {
         return __reduce_max_sync(0xffffffffu, v);
@@ -302,7 +303,8 @@ template <> struct DistBits<double> {
         return __longlong_as_double(static_cast<long long>(b));
     }
     static constexpr unsigned long long kLow = 0x0040000000000000ull, kHigh = 0x7fe0000000000000ull;
-    static constexpr unsigned long long kNear = 0, kTiny = 0;
+    static constexpr unsigned long long near_ulps(int) { return 0; }
+    static constexpr unsigned long long kTiny = 0;
     static __device__ __forceinline__ unsigned long long warp_max(unsigned long long v)
     {
 #pragma unroll
@@ -430,8 +432,8 @@ template <typename T> struct Search {
     T *lkeys;
 };
 
-// The exact distance of a list place, in the reference's order (BlockSize 8).
-template <typename T>
+// The exact distance of a list place, in the reference's order.
+template <typename T, int BS>
 __device__ __forceinline__ typename DistBits<T>::type exact_dist(const Search<T> &e, int i)
 {
     const T *cb = e.slot;
@@ -443,14 +445,12 @@ __device__ __forceinline__ typename DistBits<T>::type exact_dist(const Search<T>
     }
     T acc = T(0);
 #pragma unroll 1
-    for (int y = 0; y < kBS; ++y) {
-        T r[kBS], c[kBS];
+    for (int y = 0; y < BS; ++y) {
 #pragma unroll
-        for (int x = 0; x < kBS; ++x) {
-            r[x] = e.refb[y * e.pitch + x];
-            c[x] = cb[y * cp + x];
+        for (int x = 0; x < BS; ++x) {
+            const T d = sub_rn(e.refb[y * e.pitch + x], cb[y * cp + x]);
+            acc = add_rn(acc, mul_rn(d, d));
         }
-        acc = ssd_row8(acc, r, c);
     }
     return DistBits<T>::of(acc);
 }
@@ -490,12 +490,12 @@ template <typename T> __device__ __forceinline__ typename DistBits<T>::type dist
 // final 0.355 / 0.461 -> 0.333 / 0.438 ms, np 2.82 / 6.27 -> 2.00 / 5.86 ms
 // (the smaller list also lets np's basic stage keep 16 warps).
 //
-// NEAR, near: the list holds approximate distances (ssd_row8_near), accepted up to
+// NEAR, near: the list holds approximate distances (ssd_row_near), accepted up to
 // kNear above `limit`. The cut then leaves that much more room, and the
 // approximate order stands when no kept distance is within kNear of the next;
 // else exact_dist gives the compacted ones'. Returns -1 where the whole list has to be exact: a distance
 // at the matching threshold, ties, ranges where the bounds do not hold.
-template <typename T, bool NEAR>
+template <typename T, bool NEAR, int BS>
 __device__ __forceinline__ int select_once(const Search<T> &e, bool near, int lane, int nvalid,
                                            unsigned &n_fix)
 {
@@ -503,6 +503,7 @@ __device__ __forceinline__ int select_once(const Search<T> &e, bool near, int la
     using DB = DistBits<T>;
     using B = typename DB::type;
     const B none = ~B(0);
+    constexpr B kNear = NEAR ? DB::near_ulps(BS) : B(0);
     const int GS = e.group_size, nkeys = e.ngrid + 1;
     const B limit = e.limit;
     const B *const dist = e.dist;
@@ -571,7 +572,7 @@ __device__ __forceinline__ int select_once(const Search<T> &e, bool near, int la
         tb = DB::warp_max(tb);
         // The cut leaves slack for distances that share the bound's key. With
         // fewer than take lanes holding a candidate it keeps them all.
-        const B slack = 3 + (NEAR && near ? DB::kNear : 0);
+        const B slack = 3 + (NEAR && near ? kNear : 0);
         bool sure = true;  // the slack holds (keys are normal)
         auto cut_at = [&](B bound) {
             if (bound >= none - slack) return static_cast<B>(none - 1);
@@ -625,10 +626,10 @@ __device__ __forceinline__ int select_once(const Search<T> &e, bool near, int la
             // a distance too close to the threshold to tell matters when it can be
             // kept, or when the group takes every accepted one; either way the cut
             // is up there
-            if (cut >= limit - DB::kNear) {
+            if (cut >= limit - kNear) {
                 bool edge = false;
                 for (int i = lane; i < nkeys; i += kWarp)
-                    edge |= dist[i] - (limit - DB::kNear) <= 2 * DB::kNear;
+                    edge |= dist[i] - (limit - kNear) <= 2 * kNear;
                 if (__any_sync(0xffffffffu, edge)) return -1;
             }
         }
@@ -664,19 +665,19 @@ __device__ __forceinline__ int select_once(const Search<T> &e, bool near, int la
                 if (lane + kWarp < M) sorted[r1] = v1.key_bits();
                 __syncwarp();
                 const B s0 = sorted[lane], n0 = lane + 1 < kCand ? sorted[lane + 1] : none;
-                bool close = lane < take && lane + 1 < M && (s0 == none || n0 == none || n0 - s0 <= DB::kNear);
+                bool close = lane < take && lane + 1 < M && (s0 == none || n0 == none || n0 - s0 <= kNear);
                 if (more) {
                     const B s1 = sorted[lane + kWarp];
                     const B n1 = lane + kWarp + 1 < kCand ? sorted[lane + kWarp + 1] : none;
                     close |= lane + kWarp < take && lane + kWarp + 1 < M &&
-                             (s1 == none || n1 == none || n1 - s1 <= DB::kNear);
+                             (s1 == none || n1 == none || n1 - s1 <= kNear);
                 }
                 ranked = !__any_sync(0xffffffffu, close);
                 if (__any_sync(0xffffffffu, v0.key_bits() < DB::kTiny || v1.key_bits() < DB::kTiny))
                     return -1;
                 if (!ranked) {
-                    if (lane < M) v0 = K::pack(exact_dist(e, static_cast<int>(v0.idx())), v0.idx());
-                    if (lane + kWarp < M) v1 = K::pack(exact_dist(e, static_cast<int>(v1.idx())), v1.idx());
+                    if (lane < M) v0 = K::pack(exact_dist<T, BS>(e, static_cast<int>(v0.idx())), v0.idx());
+                    if (lane + kWarp < M) v1 = K::pack(exact_dist<T, BS>(e, static_cast<int>(v1.idx())), v1.idx());
                 }
             }
             if (!ranked) {
@@ -834,7 +835,7 @@ __device__ __forceinline__ int select_once(const Search<T> &e, bool near, int la
 // The same, the list made exact when its approximate distances do not decide
 // (one copy of the selection's code serves both: the stage kernels wait on
 // their instruction cache).
-template <typename T, bool NEAR>
+template <typename T, bool NEAR, int BS>
 __device__ __forceinline__ int select_group(const Search<T> &e, bool near, int lane, int nvalid,
                                             unsigned &n_fix)
 {
@@ -842,14 +843,40 @@ __device__ __forceinline__ int select_group(const Search<T> &e, bool near, int l
         if (NEAR && !near) {
             __syncwarp();
             nvalid = 0;
-            for (int i = lane; i <= e.ngrid; i += kWarp)
-                e.dist[i] = accept_dist(exact_dist(e, i), e.limit, nvalid);
+            if constexpr (NEAR)
+                for (int i = lane; i <= e.ngrid; i += kWarp)
+                    e.dist[i] = accept_dist(exact_dist<T, BS>(e, i), e.limit, nvalid);
             __syncwarp();
         }
-        const int n = select_once<T, NEAR>(e, near, lane, nvalid, n_fix);
+        const int n = select_once<T, NEAR, BS>(e, near, lane, nvalid, n_fix);
         if (n > 0) return n;
         near = false;
     }
+}
+
+// Row stride of the reference block's copy: rows of 8 or, for 11, of 12 values
+// are whole 16-byte words.
+__host__ __device__ constexpr int ref_row_stride(int bs) { return (bs + 3) / 4 * 4; }
+
+// acc += (r - c)^2 over one row of BS values, even columns in the low half, odd
+// ones in the high half, squares and sums fused: the ordered, unfused sum of
+// ssd_row8 up to rounding, in a third fewer operations. All terms are >= 0, so
+// the halves' sum is within (65 + 33) * 2^-24 of the ordered one for 8 x 8 blocks
+// and (122 + 67) * 2^-24 for 11 x 11.
+template <int BS>
+__device__ __forceinline__ Pair<float> ssd_row_near(Pair<float> acc, const Pair<float> (&r)[ref_row_stride(BS) / 2],
+                                                    const Pair<float> (&c)[(BS + 1) / 2])
+{
+#pragma unroll
+    for (int x = 0; x < BS / 2; ++x) {
+        const Pair<float> d = vsub(r[x], c[x]);
+        asm("fma.rn.f32x2 %0, %1, %1, %0;" : "+l"(acc.v) : "l"(d.v));
+    }
+    if (BS & 1) {
+        const float d = __fsub_rn(r[BS / 2].lo(), c[BS / 2].lo());
+        acc = Pair<float>::make(__fmaf_rn(d, d, acc.lo()), acc.hi());
+    }
+    return acc;
 }
 
 // Which strip each lane takes in each round over a full window (KS = kStrip):
@@ -903,10 +930,10 @@ __device__ __forceinline__ void build_tasks(unsigned *tab, unsigned *spill, int 
 // taken with fused squares and sums (128 cycles) and strips go to the lanes of
 // their banks (build_tasks); either alone gains nothing, both together take the
 // 1080p basic / final stage from 0.241 / 0.346 to 0.225 / 0.329 ms (4 x 8 tiles)
-// and np on 1283 x 717 from 3.66 to 3.45 ms.
-// Fills list[0..n)
-// with (y, x) in the reference's group order and returns n.
-template <typename T, int KS>
+// and np on 1283 x 717 from 3.66 to 3.45 ms. The same for 11 x 11 blocks, against
+// one candidate a lane: vn's final stage on 960 x 540 1.47 -> 1.13 ms.
+// Fills list[0..n) with (y, x) in the reference's group order and returns n.
+template <typename T, int KS, int BS = kBS>
 __device__ int match_block(const StageArgs<T> &a, const Tile<T> &t, int j0, int i0, int lane,
                            const unsigned *tasks, typename DistBits<T>::type *dist, T *refblk, SortKey<T> *heap,
                            BlockPos *list, T *lkeys, unsigned &n_cand, unsigned &n_fix)
@@ -921,7 +948,7 @@ __device__ int match_block(const StageArgs<T> &a, const Tile<T> &t, int j0, int 
         return 1;
     }
     const int st = a.bm_step, R = a.range;
-    const int right = a.width - kBS, bottom = a.height - kBS;
+    const int right = a.width - BS, bottom = a.height - BS;
     const int l = search_boundary(i0, 0, R, st), r = search_boundary(i0, right, R, st);
     const int tp = search_boundary(j0, 0, R, st), b = search_boundary(j0, bottom, R, st);
     // KS > 1 only with BMstep == 1
@@ -935,8 +962,9 @@ __device__ int match_block(const StageArgs<T> &a, const Tile<T> &t, int j0, int 
     // final 0.374 -> 0.368 ms: fewer registers to shuffle, not more warps -- 20
     // and 24 warps a multiprocessor, at 96 and 80 registers, are no faster).
     const T *rb = t.refw[0] + (j0 - t.ry0) * t.pitch + (i0 - t.rx0);
-    refblk[lane] = rb[(lane >> 3) * t.pitch + (lane & 7)];
-    refblk[lane + kWarp] = rb[((lane >> 3) + 4) * t.pitch + (lane & 7)];
+    constexpr int RS = ref_row_stride(BS);
+    for (int k = lane; k < BS * BS; k += kWarp)
+        refblk[k / BS * RS + k % BS] = rb[k / BS * t.pitch + k % BS];
     __syncwarp();
 
     // Candidates: column strips of KS consecutive grid rows per task, plus one
@@ -946,9 +974,9 @@ __device__ int match_block(const StageArgs<T> &a, const Tile<T> &t, int j0, int 
     // FP32 lists hold approximate distances first (select_group, NEAR)
     constexpr bool kNearList = sizeof(T) == 4;
     const B limit = dist_limit(a.thSSE);
-    const B accept = kNearList && limit < static_cast<B>(0x7f800000u) ? limit + DistBits<T>::kNear : limit;
+    const B accept = kNearList && limit < static_cast<B>(0x7f800000u) ? limit + DistBits<T>::near_ulps(BS) : limit;
     int nvalid = 0;
-    constexpr int ROWS = (KS - 1) + kBS;
+    constexpr int ROWS = (KS - 1) + BS;
     // a window that the plane's border clips takes its strips in raster order
     const bool full = KS == kStrip && nr == a.span && nc == a.span;
     const T *const win = t.refw[0] + (tp - t.ry0) * t.pitch + (l - t.rx0);
@@ -982,50 +1010,48 @@ __device__ int match_block(const StageArgs<T> &a, const Tile<T> &t, int j0, int 
         // other parts of the CTA's shared memory.
         T d[KS];
         if constexpr (kNearList) {
-            unsigned long long acc[KS], refv[KS][4];  // row y of the reference block in refv[y % KS]
+            Pair<float> acc[KS], refv[KS][RS / 2];  // row y of the reference block in refv[y % KS]
 #pragma unroll
-            for (int q = 0; q < KS; ++q) acc[q] = 0;
+            for (int q = 0; q < KS; ++q) acc[q] = Pair<float>{0};
 #pragma unroll
             for (int w = 0; w < ROWS; ++w) {
-                unsigned long long row[4];
-                if (w < kBS) {
-                    unsigned long long (&r)[4] = refv[w % KS];
-                    const ulonglong2 *rr = reinterpret_cast<const ulonglong2 *>(refblk + w * kBS);
-                    const ulonglong2 r01 = rr[0], r23 = rr[1];
-                    r[0] = r01.x; r[1] = r01.y; r[2] = r23.x; r[3] = r23.y;
-                }
+                if (w < BS) {
 #pragma unroll
-                for (int x = 0; x < 4; ++x)
-                    row[x] = Pair<float>::make(base[w * bp + 2 * x], base[w * bp + 2 * x + 1]).v;
+                    for (int x = 0; x < RS / 4; ++x)
+                        Vec4<float>::load4(refblk + w * RS + 4 * x, refv[w % KS][2 * x],
+                                           refv[w % KS][2 * x + 1]);
+                }
+                Pair<float> row[(BS + 1) / 2];
+#pragma unroll
+                for (int x = 0; x < (BS + 1) / 2; ++x)
+                    row[x] = Pair<float>::make(base[w * bp + 2 * x],
+                                               2 * x + 1 < BS ? base[w * bp + 2 * x + 1] : 0.0f);
 #pragma unroll
                 for (int q = 0; q < KS; ++q) {
                     const int y = w - q;
-                    if (y >= 0 && y < kBS) acc[q] = ssd_row8_near(acc[q], refv[y % KS], row);
+                    if (y >= 0 && y < BS) acc[q] = ssd_row_near<BS>(acc[q], refv[y % KS], row);
                 }
             }
 #pragma unroll
-            for (int q = 0; q < KS; ++q) {
-                const Pair<float> s{acc[q]};
-                d[q] = s.lo() + s.hi();
-            }
+            for (int q = 0; q < KS; ++q) d[q] = acc[q].lo() + acc[q].hi();
         } else {
-            T refv[KS][kBS];
+            T refv[KS][BS];
 #pragma unroll
             for (int q = 0; q < KS; ++q) d[q] = T(0);
 #pragma unroll
             for (int w = 0; w < ROWS; ++w) {
-                T row[kBS];
-                if (w < kBS) {
-                    T (&r)[kBS] = refv[w % KS];
-                    Vec4<T>::load(refblk + w * kBS, r[0], r[1], r[2], r[3]);
-                    Vec4<T>::load(refblk + w * kBS + 4, r[4], r[5], r[6], r[7]);
+                T row[BS];
+                if (w < BS) {
+                    T (&r)[BS] = refv[w % KS];
+                    Vec4<T>::load(refblk + w * BS, r[0], r[1], r[2], r[3]);
+                    Vec4<T>::load(refblk + w * BS + 4, r[4], r[5], r[6], r[7]);
                 }
 #pragma unroll
-                for (int x = 0; x < kBS; ++x) row[x] = base[w * bp + x];
+                for (int x = 0; x < BS; ++x) row[x] = base[w * bp + x];
 #pragma unroll
                 for (int q = 0; q < KS; ++q) {
                     const int y = w - q;
-                    if (y >= 0 && y < kBS) d[q] = ssd_row8(d[q], refv[y % KS], row);
+                    if (y >= 0 && y < BS) d[q] = ssd_row8(d[q], refv[y % KS], row);
                 }
             }
         }
@@ -1058,7 +1084,7 @@ __device__ int match_block(const StageArgs<T> &a, const Tile<T> &t, int j0, int 
     e.list = list;
     e.lkeys = lkeys;
     // group dumps carry exact keys
-    return select_group<T, kNearList>(e, kNearList && a.group_key == nullptr, lane, nvalid, n_fix);
+    return select_group<T, kNearList, BS>(e, kNearList && a.group_key == nullptr, lane, nvalid, n_fix);
 }
 
 // ---------------------------------------------------------------------------

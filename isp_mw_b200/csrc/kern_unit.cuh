@@ -12,14 +12,14 @@ template <typename T, bool W, int NPL, int KS> const void *stage_kernel_fn()
     return reinterpret_cast<const void *>(&stage_kernel<T, W, NPL, KS>);
 }
 
-template <typename T, bool W, int NPL> const void *generic_kernel_fn()
+template <typename T, bool W, int NPL, int BSC> const void *generic_kernel_fn()
 {
-    return reinterpret_cast<const void *>(&generic_stage_kernel<T, W, NPL>);
+    return reinterpret_cast<const void *>(&generic_stage_kernel<T, W, NPL, BSC>);
 }
 
-template <bool W, int NPL, int KS, bool GENERIC> const void *batch_kernel_fn()
+template <bool W, int NPL, int KS, int GEN> const void *batch_kernel_fn()
 {
-    return reinterpret_cast<const void *>(&batch_stage_kernel<float, W, NPL, KS, GENERIC>);
+    return reinterpret_cast<const void *>(&batch_stage_kernel<float, W, NPL, KS, GEN>);
 }
 
 static cudaError_t upload_dct_tables_here(const DctTableData &t)

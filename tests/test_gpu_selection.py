@@ -90,3 +90,29 @@ def test_approximate_order_equals_exact(ctx, bm_range, group_size, shape, wiener
         assert stats[0] > 0
     assert torch.equal(out[0], out[1])
     assert not torch.equal(out[0], plane)
+
+
+# 11 x 11 blocks match by the same strips and approximate distances (BMstep 1);
+# BMstep 2 takes one candidate a lane.
+@pytest.mark.parametrize("bm_range,bm_step,group_size,shape", [(1, 1, 2, (40, 41)), (3, 1, 8, (24, 71)),
+                                                               (9, 1, 16, (11, 11)), (9, 2, 16, (60, 53)),
+                                                               (9, 1, 17, (75, 91)), (16, 1, 32, (70, 83))])
+@pytest.mark.parametrize("kind", ["noisy", "quantised", "flat"])
+def test_groups_of_11x11_blocks(ctx, oracle_mod, kind, bm_range, bm_step, group_size, shape):
+    import torch
+    import isp_mw_b200
+    rng = np.random.default_rng(bm_range * 100 + group_size)
+    plane = torch.from_numpy((0.5 + 0.09 * rng.standard_normal(shape)).astype(np.float32)).cuda()
+    out = []
+    for k in (0, 67):  # approximate and exact distances, as above
+        p = isp_mw_b200.stage_params_default("vn", False, [40.0] * 3)
+        p.block_size, p.block_step, p.group_size = 11, 4, group_size
+        p.bm_range, p.bm_step = bm_range, bm_step
+        if k == 0:
+            _check(ctx, oracle_mod, p, _plane(kind), 1.0)
+        p.thMSE = 1e4 * 2.0 ** (-2 * k)
+        dst = torch.zeros_like(plane)
+        ctx.stage(p, False, dst, plane, None, 2.0 ** k)
+        out.append(dst)
+    assert torch.equal(out[0], out[1])
+    assert not torch.equal(out[0], plane)
