@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(kConvThreads, kConvCtasPerSm) conv48_kernel(co
     int it = 0, prev = -1;
     for (int tile = blockIdx.x; tile < a.tiles; tile += gridDim.x, ++it) {
         const int b = it % kConvStages;
-        cp_async_wait_1();
+        cp_async_wait<1>();
         fence_async_smem();
         tc_fence_before();
         __syncthreads();
@@ -742,17 +742,38 @@ __global__ void __launch_bounds__(kT3Threads, 1)
 // Weight gradient of a 48 -> 48 layer on the tensor cores:
 //   dW[co][ci][ky][kx] = sum over pixels p of G[p][co] * X[p + (ky - 1, kx - 1)][ci]
 // One MMA per K-step of 16 pixels (two tile columns) and input-row shift dy:
-// A = G (MN-major, M = 128 rows of which co 0..47 are real; the rest read the
-// next columns and are discarded), B = the halo tile of X starting dy rows
-// down, read as N = 144 = (dx, ci) (MN-major: 18 channel groups 160 bytes
-// apart across the three dx shifts), D[dy] = 128 x 144 FP32 in TMEM. Each CTA accumulates over
-// its tiles and writes a partial dW (and the bias gradient from G) that
-// reduce_partials_kernel sums.
-constexpr int kGTileBytes = kCopyBytes;  // 16 columns of G plus two columns of slack
+// A = G (MN-major, M = 64 rows of which co 0..47 are real; the rest read the
+// bytes that follow and are discarded), B = the halo tile of X starting dy rows
+// down, read as N = 144 = (dx, ci) (MN-major: 18 channel groups 160 bytes apart
+// across the three dx shifts), D[dy] = 64 x 144 FP32 in TMEM. Each CTA
+// accumulates over its tiles and writes a partial dW (and the bias gradient from
+// G) that reduce_partials_kernel sums.
+//
+// What bounds it: the tensor core's operand fetch, 2.3 cycles per 8 x 8 core
+// matrix of these layouts: 52 of them an MMA (68 with M = 128, as it was: 61 us
+// where this takes 47). Under that stay: tiles read in the order of global memory,
+// 16-byte chunks of whole rows of pixels, G's channel groups 144 bytes apart so
+// that a row's chunks land on distinct banks; kWgStages - 1 tiles on their way;
+// chunk addresses worked out once; the bias summed by six warps. One tile ahead,
+// with G gathered 16 bytes at a time down its columns, addresses divided out per
+// chunk, 48 threads summing the bias and dW written element by element 1728
+// bytes apart, a layer of 32 crops of 128 x 128 took 124 us; now 47.
+constexpr int kWgGroupBytes = kTY * 16 + 16;        // 144: one 8-channel group of a G column
+constexpr int kWgColBytes = 6 * kWgGroupBytes;      // 864
+constexpr int kGTileBytes = kTX * kWgColBytes;      // 13824
 constexpr int kWgBuf = kGTileBytes + kTileBytes;
-constexpr int kWgSmem = 2 * kWgBuf + 64;
-constexpr uint32_t kIdescWg = instr_desc_bf16(128, 3 * kC, true, true);
-constexpr int kWgPartial = kWmid + kC;  // per CTA: dW (PyTorch layout) then db
+constexpr int kWgStages = 4;
+constexpr int kWgThreads = 512;
+constexpr int kWgBiasThreads = 2 * kTX * 6;         // the last six warps: (rows, column, group)
+constexpr int kWgGChunks = (kTX * kTY * 6 + kWgThreads - 1) / kWgThreads;
+constexpr int kWgXChunks = (kTileChunks + kWgThreads - 1) / kWgThreads;
+constexpr int kWgOffRed = kWgStages * kWgBuf;       // bias sums, [rows, column][channel]
+constexpr int kWgOffBar = kWgOffRed + 2 * kTX * kC * 4;
+constexpr int kWgSmem = kWgOffBar + 8 * kWgStages + 16;
+constexpr uint32_t kIdescWg = instr_desc_bf16(64, 3 * kC, true, true);
+constexpr int kWgPartial = kWmid + kC;  // per CTA: dW as [dy][dx][ci][co], then db
+static_assert(15 * kWgColBytes + 8 * kWgGroupBytes <= kWgBuf, "the discarded rows' reads stay in the buffer");
+static_assert(kWgThreads >= kWgBiasThreads + 32, "the issuing warp sums no bias");
 
 struct WgradArgs {
     const __nv_bfloat16 *x;  // layer input [n][h][w][48]
@@ -763,56 +784,82 @@ struct WgradArgs {
     unsigned *err;
 };
 
-__device__ __forceinline__ void load_g_tile(const __nv_bfloat16 *g, int h, int w, int img, int y0,
-                                            int x0, unsigned char *buf)
-{
-    // 16 columns x 6 channel groups x 8 rows; the two slack columns stay zero
-    for (int i = threadIdx.x; i < kTX * 48; i += blockDim.x) {
-        const int yy = i & 7;
-        int r = i >> 3;
-        const int ch = r % 6;
-        const int col = r / 6;
-        const int gy = y0 + yy, gx = x0 + col;
-        const bool ok = gy < h && gx < w;
-        const __nv_bfloat16 *src =
-            ok ? g + ((static_cast<long long>(img) * h + gy) * w + gx) * kC + ch * 8 : g;
-        cp_async16(buf + i * 16, src, ok);
+// The chunks a thread copies of every tile: where each lies in the buffer, its
+// row and column, and its elements from the tile's first pixel. Worked out once
+// (redone per chunk, the divisions were most of the kernel's instructions).
+template <int N> struct WgradChunks {
+    int at[N], rc[N], off[N];
+    // rows x cols x 6 chunks; `halo` pixels before the tile in both directions
+    __device__ __forceinline__ void init(int rows, int cols, int halo, int col_bytes, int group_bytes, int w)
+    {
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const int i = threadIdx.x + k * kWgThreads;
+            const int yy = i / (cols * 6), r = i - yy * (cols * 6);
+            const int col = r / 6, ch = r - col * 6;
+            at[k] = yy < rows ? col * col_bytes + ch * group_bytes + yy * 16 : -1;
+            rc[k] = (yy - halo) << 16 | ((col - halo) & 0xffff);
+            off[k] = ((yy - halo) * w + col - halo) * kC + ch * 8;
+        }
     }
-}
+    // the tile whose first pixel is (y0, x0) of the h x w image at img
+    __device__ __forceinline__ void load(const __nv_bfloat16 *img, int y0, int x0, int h, int w,
+                                         uint32_t buf) const
+    {
+        const __nv_bfloat16 *const first = img + (static_cast<long long>(y0) * w + x0) * kC;
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            if (at[k] < 0) continue;
+            const int gy = y0 + (rc[k] >> 16), gx = x0 + static_cast<short>(rc[k]);
+            const bool ok = static_cast<unsigned>(gy) < static_cast<unsigned>(h) &&
+                            static_cast<unsigned>(gx) < static_cast<unsigned>(w);
+            cp_async16(buf + at[k], ok ? first + off[k] : img, ok);
+        }
+    }
+};
 
-__global__ void __launch_bounds__(kConvThreads, 1) wgrad48_kernel(const WgradArgs a)
+__global__ void __launch_bounds__(kWgThreads, 1) wgrad48_kernel(const WgradArgs a)
 {
     extern __shared__ __align__(128) unsigned char smem[];
-    // operand buffer b (G tile, then the three X copies) at smem + b * kWgBuf
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + 2 * kWgBuf);
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(mbar + 2);
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + kWgOffBar);  // one per buffer
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(mbar + kWgStages);
+    float *red = reinterpret_cast<float *>(smem + kWgOffRed);
     __shared__ int abort_flag;
 
     const int tid = threadIdx.x;
-    // zero both buffers once: the G tiles' slack columns are read as discarded rows
-    for (int i = tid; i < 2 * kWgBuf / 16; i += blockDim.x)
-        reinterpret_cast<uint4 *>(smem)[i] = make_uint4(0, 0, 0, 0);
     if (tid == 0) {
         abort_flag = 0;
-        mbar_init(&mbar[0], 1);
-        mbar_init(&mbar[1], 1);
+        for (int k = 0; k < kWgStages; ++k) mbar_init(&mbar[k], 1);
         fence_mbar_init();
     }
     if ((tid >> 5) == 0) tmem_alloc(tslot, 512);
+    tc_fence_before();
     __syncthreads();
+    tc_fence_after();
     const uint32_t tbase = *tslot;
 
-    int img, y0, x0;
-    float bsum = 0.0f;  // thread tid < 48: bias gradient of channel tid
+    WgradChunks<kWgGChunks> gc;
+    WgradChunks<kWgXChunks> xc;
+    gc.init(kTY, kTX, 0, kWgColBytes, kWgGroupBytes, a.w);
+    xc.init(kHaloRows, kCols, 1, kHaloColBytes, kGroupBytes, a.w);
+    const uint32_t buf0 = smem_u32(smem);
+    auto load_tile = [&](int tile, int buf) {  // (an empty group past the end)
+        if (tile < a.tiles) {
+            int img, y0, x0;
+            tile_origin(tile, a.tiles_x, a.tiles_y, img, y0, x0);
+            const long long plane = static_cast<long long>(img) * a.h * a.w * kC;
+            gc.load(a.g + plane, y0, x0, a.h, a.w, buf0 + buf * kWgBuf);
+            xc.load(a.x + plane, y0, x0, a.h, a.w, buf0 + buf * kWgBuf + kGTileBytes);
+        }
+        cp_async_commit();
+    };
+    for (int k = 0; k < kWgStages - 1; ++k) load_tile(blockIdx.x + k * gridDim.x, k);
+    const int bt = tid - (kWgThreads - kWgBiasThreads);  // bias thread, or negative
+    float bsum[8] = {};
     int it = 0;
-    if (blockIdx.x < a.tiles) {
-        tile_origin(blockIdx.x, a.tiles_x, a.tiles_y, img, y0, x0);
-        load_g_tile(a.g, a.h, a.w, img, y0, x0, smem);
-        load_conv_tile(a.x, a.h, a.w, img, y0, x0, smem + kGTileBytes);
-    }
     for (int tile = blockIdx.x; tile < a.tiles; tile += gridDim.x, ++it) {
-        const int b = it & 1;
-        cp_async_wait_all();
+        const int b = it % kWgStages;
+        cp_async_wait<kWgStages - 2>();  // this tile has landed
         fence_async_smem();
         tc_fence_before();
         __syncthreads();
@@ -821,13 +868,13 @@ __global__ void __launch_bounds__(kConvThreads, 1) wgrad48_kernel(const WgradArg
             tc_fence_after();
             const uint32_t gb = smem_u32(smem + b * kWgBuf), xb = gb + kGTileBytes;
             // base descriptors plus compile-time offsets (as issue_tile_mmas)
-            const uint64_t ad0 = smem_desc(gb, 768, 128);
+            const uint64_t ad0 = smem_desc(gb, kWgColBytes, kWgGroupBytes);
             const uint64_t bd0 = smem_desc(xb, kHaloColBytes, kGroupBytes);
 #pragma unroll
             for (int s = 0; s < kTX / 2; ++s) {
 #pragma unroll
                 for (int dy = 0; dy < 3; ++dy) {
-                    const uint64_t ad = ad0 + static_cast<uint64_t>((s * 2 * kColBytes) >> 4);
+                    const uint64_t ad = ad0 + static_cast<uint64_t>((s * 2 * kWgColBytes) >> 4);
                     const uint64_t bd =
                         bd0 + static_cast<uint64_t>((dy * 16 + s * 2 * kHaloColBytes) >> 4);
                     mma_bf16(tbase + dy * 3 * kC, ad, bd, kIdescWg, it > 0 || s > 0);
@@ -835,59 +882,66 @@ __global__ void __launch_bounds__(kConvThreads, 1) wgrad48_kernel(const WgradArg
             }
             mma_commit(&mbar[b]);
         }
-        if (tid < kC) {  // bias gradient from the staged G tile
-            const __nv_bfloat16 *gs = reinterpret_cast<const __nv_bfloat16 *>(smem + b * kWgBuf);
-            const int ch = tid >> 3, c8 = tid & 7;
-            for (int col = 0; col < kTX; ++col)
+        if (bt >= 0) {  // bias gradient from the staged G tile: four rows of a column's group
+            const uint4 *gs = reinterpret_cast<const uint4 *>(
+                smem + b * kWgBuf + (bt >> 1) * kWgGroupBytes + (bt & 1) * 64);
 #pragma unroll
-                for (int yy = 0; yy < 8; ++yy)
-                    bsum += __bfloat162float(gs[((col * 6 + ch) * 8 + yy) * 8 + c8]);
-        }
-        // the other buffer is free once the previous tile's MMAs completed
-        const int next = tile + gridDim.x;
-        if (it > 0) {
-            if (!mbar_wait(&mbar[b ^ 1], ((it - 1) >> 1) & 1, kWaitLimit)) {
-                abort_flag = 1;
-                if (a.err) atomicOr(a.err, 1u);
+            for (int yy = 0; yy < kTY / 2; ++yy) {
+                const uint4 u = gs[yy];
+                const unsigned wd[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    bsum[2 * k] += __uint_as_float(wd[k] << 16);
+                    bsum[2 * k + 1] += __uint_as_float(wd[k] & 0xffff0000u);
+                }
             }
         }
-        __syncthreads();  // bias reads of this buffer done; wait results published
-        if (abort_flag) break;
-        if (next < a.tiles) {
-            tile_origin(next, a.tiles_x, a.tiles_y, img, y0, x0);
-            load_g_tile(a.g, a.h, a.w, img, y0, x0, smem + (b ^ 1) * kWgBuf);
-            load_conv_tile(a.x, a.h, a.w, img, y0, x0, smem + (b ^ 1) * kWgBuf + kGTileBytes);
+        // the previous tile's buffer is free once its MMAs completed (its bias
+        // reads ended before this iteration's barrier)
+        const int f = (it + kWgStages - 1) % kWgStages;
+        bool free = true;
+        if (it > 0 && !mbar_wait(&mbar[f], ((it - 1) / kWgStages) & 1, kWaitLimit)) {
+            free = false;
+            abort_flag = 1;
+            if (a.err) atomicOr(a.err, 1u);
         }
+        load_tile(free ? tile + (kWgStages - 1) * gridDim.x : a.tiles, f);
+    }
+    if (bt >= 0) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            red[((bt >> 1) / 6 * 2 + (bt & 1)) * kC + (bt >> 1) % 6 * 8 + k] = bsum[k];
     }
     __syncthreads();
     float *out = a.partial + static_cast<long long>(blockIdx.x) * kWgPartial;
     const bool ok = !abort_flag && it > 0 &&
-                    mbar_wait(&mbar[(it - 1) & 1], ((it - 1) >> 1) & 1, kWaitLimit);
+                    mbar_wait(&mbar[(it - 1) % kWgStages], ((it - 1) / kWgStages) & 1, kWaitLimit);
     if (!ok && !abort_flag && it > 0 && a.err) atomicOr(a.err, 1u);
     tc_fence_after();
     const int warp = tid >> 5, lane = tid & 31;
-    if (ok && warp < 2) {  // TMEM lanes 0..63 hold co = lane (rows >= 48 discarded)
-        const int co = 32 * warp + lane;
-        const uint32_t ta = tbase + (static_cast<uint32_t>(32 * warp) << 16);
+    // an M = 64 accumulator's row co is TMEM lane co % 16 of quadrant co / 16 (rows
+    // >= 48 discarded): the warps of quadrants 0..2 share the 27 column groups
+    if (ok && (warp & 3) < kC / 16) {
+        const int co = 16 * (warp & 3) + lane;
+        const uint32_t ta = tbase + (static_cast<uint32_t>(32 * (warp & 3)) << 16);
 #pragma unroll 1
-        for (int c16 = 0; c16 < 27; ++c16) {  // 432 columns: (dy, dx, ci)
+        for (int c16 = warp >> 2; c16 < 27; c16 += kWgThreads / 128) {  // 432 columns: (dy, dx, ci)
             float v[16];
             tmem_ld16(ta + c16 * 16, v);
             tmem_wait_ld();
-            if (co < kC) {
+            if (lane < 16) {
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const int col = c16 * 16 + i;
-                    const int dy = col / 144, rem = col - 144 * dy;
-                    const int dx = rem / kC, ci = rem - kC * dx;
-                    out[((co * kC + ci) * 3 + dy) * 3 + dx] = v[i];
-                }
+                for (int i = 0; i < 16; ++i) out[(c16 * 16 + i) * kC + co] = v[i];
             }
         }
     } else if (!ok && tid < kC) {
         for (int i = tid; i < kWmid; i += kC) out[i] = 0.0f;
     }
-    if (tid < kC) out[kWmid + tid] = (ok || it == 0) ? bsum : 0.0f;
+    if (tid < kC) {
+        float sum = 0.0f;
+        for (int k = 0; k < 2 * kTX; ++k) sum += red[k * kC + tid];
+        out[kWmid + tid] = (ok || it == 0) ? sum : 0.0f;
+    }
     cp_async_wait_all();
     tc_fence_before();
     __syncthreads();
@@ -897,16 +951,60 @@ __global__ void __launch_bounds__(kConvThreads, 1) wgrad48_kernel(const WgradArg
     }
 }
 
-// out[i] = sum over the `parts` partial vectors (`stride` floats apart) of element i < len;
-// a fixed order, so the sums are reproducible
-__global__ void reduce_partials_kernel(const float *partial, int parts, int len, int stride,
-                                       float *out)
+// Sums of a layer's partial gradients, in double and in a fixed order
+// (reproducible), and Adam on its FP32 master parameters (bias-corrected step
+// size precomputed). `len` sums over `parts` vectors `len` floats apart, the first
+// `wlen` the weights; `mid` weights come as [dy][dx][ci][co]. A block takes 32
+// neighbouring sums and its eight warps each an eighth of the parts, so that
+// loads are whole lines and no thread waits for a chain of 148 (296) of them:
+// with Adam, 7.5 us a layer for 32 crops of 128 x 128 (12 MB of partials) where
+// one thread a sum took 17, and a launch of its own for Adam 3.
+constexpr int kReduceSums = 32, kReduceThreads = 256;
+struct ReduceArgs {
+    const float *partial;
+    float *w, *b;  // results
+    int parts, len, wlen;
+    bool mid;
+    const float *grad;      // Adam: w and b point into it
+    float *param, *m, *v;   // null: sums only
+    float lr_t, beta1, beta2, eps;
+};
+
+__global__ void __launch_bounds__(kReduceThreads) reduce_partials_kernel(const ReduceArgs a)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < len; i += gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (int p = 0; p < parts; ++p) s += partial[static_cast<long long>(p) * stride + i];
-        out[i] = static_cast<float>(s);
+    __shared__ double part[kReduceThreads / 32][kReduceSums];
+    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5, nslices = kReduceThreads / 32;
+    const int i = blockIdx.x * kReduceSums + lane;
+    double s = 0.0;
+    if (i < a.len) {
+        const float *p = a.partial + i;
+        const int from = a.parts * slice / nslices, to = a.parts * (slice + 1) / nslices;
+#pragma unroll 8
+        for (int q = from; q < to; ++q) s += p[static_cast<long long>(q) * a.len];
     }
+    part[slice][lane] = s;
+    __syncthreads();
+    if (slice != 0 || i >= a.len) return;
+    for (int q = 1; q < nslices; ++q) s += part[q][lane];
+    float *out;
+    if (i >= a.wlen) {
+        out = a.b + (i - a.wlen);
+    } else if (a.mid) {
+        const int col = i / kC, co = i - col * kC;  // col = (dy * 3 + dx) * 48 + ci
+        const int tap = col / kC, ci = col - tap * kC;
+        out = a.w + (co * kC + ci) * 9 + tap;
+    } else {
+        out = a.w + i;
+    }
+    const float g = static_cast<float>(s);
+    *out = g;
+    if (a.param == nullptr) return;
+    const long long e = out - a.grad;
+    const float mi = a.beta1 * a.m[e] + (1.0f - a.beta1) * g;
+    const float vi = a.beta2 * a.v[e] + (1.0f - a.beta2) * g * g;
+    a.m[e] = mi;
+    a.v[e] = vi;
+    a.param[e] -= a.lr_t * mi / (sqrtf(vi) + a.eps);
 }
 
 // ---------------------------------------------------------------------------
@@ -1318,20 +1416,6 @@ __global__ void __launch_bounds__(240) wgrad_in_kernel(const InArgs a, const __n
     __syncthreads();
     for (int i = threadIdx.x; i < kW1Partial; i += blockDim.x)
         partial[static_cast<long long>(blockIdx.x) * kW1Partial + i] = red[i];
-}
-
-// Adam on the FP32 master parameters (bias-corrected step size precomputed).
-__global__ void adam_kernel(float *param, const float *grad, float *m, float *v, int count,
-                            float lr_t, float beta1, float beta2, float eps)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        const float g = grad[i];
-        const float mi = beta1 * m[i] + (1.0f - beta1) * g;
-        const float vi = beta2 * v[i] + (1.0f - beta2) * g * g;
-        m[i] = mi;
-        v[i] = vi;
-        param[i] -= lr_t * mi / (sqrtf(vi) + eps);
-    }
 }
 
 // Packs the six 48 -> 48 layers' FP32 weights [co][ci][ky][kx] into the

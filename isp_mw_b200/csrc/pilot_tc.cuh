@@ -145,16 +145,23 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *mbar, uint32_t parity, uint3
 // --- asynchronous global -> shared copies --------------------------------------
 // 16 bytes, or 16 zero bytes when `valid` is false (src-size 0; src must still
 // be a mapped address).
+__device__ __forceinline__ void cp_async16(uint32_t smem_dst, const void *gsrc, bool valid)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_dst), "l"(gsrc),
+                 "r"(valid ? 16 : 0)
+                 : "memory");
+}
 __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc, bool valid)
 {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)),
-                 "l"(gsrc), "r"(valid ? 16 : 0)
-                 : "memory");
+    cp_async16(smem_u32(smem_dst), gsrc, valid);
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-// All but the most recently committed group have landed.
-__device__ __forceinline__ void cp_async_wait_1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+// All but the N most recently committed groups have landed.
+template <int N> __device__ __forceinline__ void cp_async_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 
 // --- tensor memory access (TMA) ------------------------------------------------
 // Tiled copies through a tensor map (a __grid_constant__ kernel parameter,

@@ -328,3 +328,24 @@ def test_pilot_full_is_final_stage_on_pilot_estimate(ctx):
     ctx.stage(f, True, want, noisy, est)
     assert np.array_equal(full, want)
     p.close()
+
+
+# tiles of 16 x 8 on more and fewer CTAs than there are, at and past their edges;
+# both gradients are exact sums of BF16 products up to FP32 accumulation
+@pytest.mark.parametrize("shape", [(1, 1, 1), (1, 8, 16), (1, 9, 17), (2, 7, 15), (5, 40, 130),
+                                   (9, 121, 129)])
+def test_wgrad48_tile_edges(ctx, shape):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(11)
+    n, h, w = shape
+    x = torch.randn(n, h, w, C, device="cuda", generator=g).bfloat16()
+    gr = torch.randn(n, h, w, C, device="cuda", generator=g).bfloat16()
+    dw = torch.empty(C, C, 3, 3, device="cuda")
+    db = torch.empty(C, device="cuda")
+    ctx._check(ctx.lib.bm3d_pilot_wgrad48(ctx.h, n, h, w, x.data_ptr(), gr.data_ptr(),
+                                          dw.data_ptr(), db.data_ptr(), _stream()))
+    ref_w = torch.nn.grad.conv2d_weight(x.double().permute(0, 3, 1, 2), (C, C, 3, 3),
+                                        gr.double().permute(0, 3, 1, 2), padding=1)
+    ref_b = gr.double().sum(dim=(0, 1, 2))
+    for got, ref in ((dw.double(), ref_w), (db.double(), ref_b)):
+        assert float((got - ref).abs().max()) <= 1e-5 * max(1.0, float(ref.abs().max()))
