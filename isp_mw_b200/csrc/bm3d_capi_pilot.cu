@@ -70,11 +70,12 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
 
 // The TMA pipelines' two views of n images of h x w x 48 BF16 (NHWC): the
 // input as (channel % 8, x, channel / 8, y, image), box {8, in_cols, 6,
-// in_rows, 1}, and the output as (channel, x, y, image), box {48, out_cols,
-// 4, 1}: {8, 10, 6, 18, 1} / {48, 8, 4, 1} for conv48_tma_kernel,
+// in_rows, 1}, and the output as (channel, x, y, image), box {out_ch, out_cols,
+// 4, 1}: {8, 10, 6, 18, 1} / {16, 8, 4, 1} for conv48_tma_kernel,
 // {8, 8, 6, 18, 1} / {48, 6, 4, 1} for conv48_n144_kernel.
 bool encode_conv_maps(const void *x, void *y, int n, int h, int w, CUtensorMap &in, CUtensorMap &out,
-                      int in_cols = kT2X + 2, int out_cols = kT2X, int in_rows = kT2Y + 2)
+                      int in_cols = kT2X + 2, int out_cols = kT2X, int in_rows = kT2Y + 2,
+                      int out_ch = 16)
 {
     auto enc = tensor_map_encoder();
     if (!enc) return false;
@@ -92,7 +93,7 @@ bool encode_conv_maps(const void *x, void *y, int n, int h, int w, CUtensorMap &
     const cuuint64_t odim[4] = {static_cast<cuuint64_t>(kC), static_cast<cuuint64_t>(w),
                                 static_cast<cuuint64_t>(h), static_cast<cuuint64_t>(n)};
     const cuuint64_t ostride[3] = {px, px * w, px * w * h};
-    const cuuint32_t obox[4] = {kC, static_cast<cuuint32_t>(out_cols), 4, 1};
+    const cuuint32_t obox[4] = {static_cast<cuuint32_t>(out_ch), static_cast<cuuint32_t>(out_cols), 4, 1};
     return enc(&out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, y, odim, ostride, obox, ones,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
@@ -117,7 +118,7 @@ int run_conv48(bm3d_ctx *ctx, const __nv_bfloat16 *x, __nv_bfloat16 *y, const __
     const int choice = g_conv_choice.load();
     CUtensorMap tin, tout;
     if (w3 != nullptr && mode != kMaskPrev && (choice == 0 || choice == 3) &&
-        encode_conv_maps(x, y, n, h, wd, tin, tout, kIn3X, kT3X, kT3Y + 2)) {
+        encode_conv_maps(x, y, n, h, wd, tin, tout, kIn3X, kT3X, kT3Y + 2, kC)) {
         a.wt = reinterpret_cast<const uint4 *>(w3);
         a.tiles_x = (wd + kT3X - 1) / kT3X;
         a.tiles_y = (h + kT3Y - 1) / kT3Y;

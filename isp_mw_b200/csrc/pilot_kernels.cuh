@@ -327,22 +327,28 @@ __global__ void __launch_bounds__(kConvThreads, kConvCtasPerSm) conv48_kernel(co
 // rows, so tap (dy, dx) starts dy * 960 + dx * 16 bytes in. The copy
 // zero-fills the halo outside the image.
 //
-// Warps: 0 loads (lane 0), 1 issues the MMAs (lane 0), 2-5 drain the
-// accumulators -- warp w reads TMEM lanes 32 (w % 4) .. + 31, pixel rows
-// 4 (w % 4) .. + 3 -- and store their 4 x 8 pixels with a TMA store of a 4-D
-// view (channel, x, y, image) from a per-warp staging buffer (the store clips
-// at the image edges). kTmaStages operand buffers and two accumulators are
-// handed on by mbarriers (full / empty for each); no CTA-wide barrier runs
-// inside the tile loop.
+// Warps: 0 loads (lane 0), 1 issues the MMAs (lane 0), the others drain: kSets
+// accumulators, each with four warps per 16 channels -- warp w reads TMEM lanes
+// 32 (w % 4) .. + 31, pixel rows 4 (w % 4) .. + 3 -- which store their 4 x 8
+// pixels with a TMA store of a 4-D view (channel, x, y, image) from a per-warp
+// staging buffer (the store clips at the image edges). kTmaStages operand buffers
+// and the accumulators are handed on by mbarriers (full / empty for each); no
+// CTA-wide barrier runs inside the tile loop. What bounds it: the tensor core's
+// operand fetch, 2.3 cycles per 8 x 8 core matrix, 44 of them an MMA. (Four warps
+// draining whole pixels of both accumulators, with the mask read after the MMAs,
+// were slower than that: data gradient of 32 crops of 128 x 128 52 -> 43 us.)
 constexpr int kT2X = 8, kT2Y = 16;
 constexpr int kTmaStages = 4;
-constexpr int kTmaThreads = 192;
-constexpr int kStoreBytes = 32 * kC * 2;  // one warp's 4 x 8 output pixels
+constexpr int kSets = 2;    // accumulators, each with its own set of draining warps
+constexpr int kSplit = 3;   // 16-channel parts of an accumulator
+constexpr int kSetWarps = 4 * kSplit;
+constexpr int kTmaThreads = 64 + 32 * kSets * kSetWarps;  // producer, MMA issuer, the draining sets
+constexpr int kStoreBytes = 32 * 16 * 2;  // one warp's 16 channels of 4 x 8 output pixels
 constexpr int kTmaOffStage = kWeightBytes;
 constexpr int kTmaOffStore = kTmaOffStage + kTmaStages * kTileBytes;
-constexpr int kTmaOffBias = kTmaOffStore + 4 * 2 * kStoreBytes;
+constexpr int kTmaOffBias = kTmaOffStore + kSets * kSetWarps * 2 * kStoreBytes;
 constexpr int kTmaOffBar = kTmaOffBias + kC * 4;
-constexpr int kTmaSmem = kTmaOffBar + 8 * (2 * kTmaStages + 4) + 16;
+constexpr int kTmaSmem = kTmaOffBar + 8 * (2 * kTmaStages + 2 * kSets) + 16;
 static_assert(kTmaOffStage % 128 == 0 && kTmaOffStore % 128 == 0 && kTileBytes % 128 == 0,
               "TMA buffers 128-byte aligned");
 
@@ -368,6 +374,15 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi, bool relu)
     return d;
 }
 
+// All ones in each half of a BF16 pair that is positive: sign bit clear and nonzero.
+__device__ __forceinline__ uint32_t bf16x2_positive(uint32_t x)
+{
+    const uint32_t t = ((x & 0x7fff7fffu) + 0x7fff7fffu) & ~x;  // bit 15: nonzero and not negative
+    uint32_t m;  // the sign bits of bytes 1 and 3, spread
+    asm("prmt.b32 %0, %1, 0, 0xbb99;" : "=r"(m) : "r"(t));
+    return m;
+}
+
 __global__ void __launch_bounds__(kTmaThreads, 1)
     conv48_tma_kernel(const __grid_constant__ CUtensorMap tm_in,
                       const __grid_constant__ CUtensorMap tm_out, const ConvArgs a)
@@ -376,8 +391,8 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + kTmaOffBar);
     uint64_t *empty = full + kTmaStages;
     uint64_t *accf = empty + kTmaStages;
-    uint64_t *acce = accf + 2;
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(acce + 2);
+    uint64_t *acce = accf + kSets;
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(acce + kSets);
     float *bias_s = reinterpret_cast<float *>(smem + kTmaOffBias);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (blockIdx.x >= a.tiles) return;
@@ -390,9 +405,9 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
-        for (int k = 0; k < 2; ++k) {
+        for (int k = 0; k < kSets; ++k) {
             mbar_init(&accf[k], 1);
-            mbar_init(&acce[k], 4);  // one arrival per draining warp
+            mbar_init(&acce[k], kSetWarps);  // one arrival per draining warp of set k
         }
         fence_mbar_init();
     }
@@ -439,85 +454,69 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
                 mma_commit(&accf[k]);
             }
         }
-    } else {  // drain: warps 2..5
-        const int q = warp & 3;
+    } else {  // drain: set (warp - 2) / 12, TMEM lanes 32 (warp % 4) .. + 31, 16 channels
+        const int q = warp & 3, set = (warp - 2) / kSetWarps;
+        const int c0 = (warp - 2 - set * kSetWarps) / 4 * 16;  // the first channel
         unsigned char *const stage0 = smem + kTmaOffStore + (warp - 2) * 2 * kStoreBytes;
-        const uint32_t lane_base = static_cast<uint32_t>(32 * q) << 16;
-        int it = 0;
-        for (int tile = blockIdx.x; tile < a.tiles; tile += gridDim.x, ++it) {
-            const int k = it & 1;
-            if (!__all_sync(0xffffffffu, mbar_wait(&accf[k], (it >> 1) & 1, kWaitLimit))) {
+        const uint32_t ta = tbase + set * kAccCols + c0 + (static_cast<uint32_t>(32 * q) << 16);
+        const bool relu = a.mode == kBiasRelu;
+        int use = 0;  // times this set's accumulator was filled
+        for (int tile = blockIdx.x + set * gridDim.x; tile < a.tiles;
+             tile += kSets * gridDim.x, ++use) {
+            int img, y0, x0;
+            tile_origin_8x16(tile, a.tiles_x, a.tiles_y, img, y0, x0);
+            // the mask's loads return while the tile's MMAs run
+            uint4 mk[2] = {};
+            if (a.mode == kMaskPrev) {
+                const int gy = y0 + 4 * q + (lane >> 3), gx = x0 + (lane & 7);
+                if (gy < a.h && gx < a.w) {
+                    const uint4 *mp = reinterpret_cast<const uint4 *>(
+                        a.aux + ((static_cast<long long>(img) * a.h + gy) * a.w + gx) * kC + c0);
+                    mk[0] = __ldg(mp);
+                    mk[1] = __ldg(mp + 1);
+                }
+            }
+            if (!__all_sync(0xffffffffu, mbar_wait(&accf[set], use & 1, kWaitLimit))) {
                 ok = false;
                 break;
             }
             tc_fence_after();
-            float v[48];
-            {
-                float t0[16], t1[16], t2[16];
-                const uint32_t ta = tbase + k * kAccCols + lane_base;
-                tmem_ld16(ta, t0);
-                tmem_ld16(ta + 16, t1);
-                tmem_ld16(ta + 32, t2);
-                tmem_wait_ld();
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    v[i] = t0[i];
-                    v[16 + i] = t1[i];
-                    v[32 + i] = t2[i];
-                }
-            }
+            float v[16];
+            tmem_ld16(ta, v);
+            tmem_wait_ld();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&acce[k]);  // the accumulator may be overwritten
+            if (lane == 0) mbar_arrive(&acce[set]);  // the accumulator may be overwritten
 
-            int img, y0, x0;
-            tile_origin_8x16(tile, a.tiles_x, a.tiles_y, img, y0, x0);
-            uint32_t pk[24];
+            uint32_t pk[8];
             if (a.mode == kMaskPrev) {
-                const int gy = y0 + 4 * q + (lane >> 3), gx = x0 + (lane & 7);
-                uint4 mk[6] = {};
-                if (gy < a.h && gx < a.w) {
-                    const uint4 *mp = reinterpret_cast<const uint4 *>(
-                        a.aux + ((static_cast<long long>(img) * a.h + gy) * a.w + gx) * kC);
+                const unsigned mw[8] = {mk[0].x, mk[0].y, mk[0].z, mk[0].w,
+                                        mk[1].x, mk[1].y, mk[1].z, mk[1].w};
 #pragma unroll
-                    for (int j = 0; j < 6; ++j) mk[j] = __ldg(mp + j);
-                }
-#pragma unroll
-                for (int j = 0; j < 6; ++j) {
-                    const unsigned mw[4] = {mk[j].x, mk[j].y, mk[j].z, mk[j].w};
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        // bf16 > 0: sign bit clear and nonzero
-                        uint32_t p = pack_bf16(v[8 * j + 2 * e], v[8 * j + 2 * e + 1], false);
-                        if ((mw[e] & 0x8000u) || (mw[e] & 0xffffu) == 0) p &= 0xffff0000u;
-                        if ((mw[e] >> 31) || (mw[e] >> 16) == 0) p &= 0x0000ffffu;
-                        pk[4 * j + e] = p;
-                    }
-                }
+                for (int e = 0; e < 8; ++e)
+                    pk[e] = pack_bf16(v[2 * e], v[2 * e + 1], false) & bf16x2_positive(mw[e]);
             } else {
-                const bool relu = a.mode == kBiasRelu;
-                const float4 *b4 = reinterpret_cast<const float4 *>(bias_s);
+                const float4 *b4 = reinterpret_cast<const float4 *>(bias_s + c0);
 #pragma unroll
-                for (int j = 0; j < 12; ++j) {
+                for (int j = 0; j < 4; ++j) {
                     const float4 b = b4[j];
                     pk[2 * j] = pack_bf16(v[4 * j] + b.x, v[4 * j + 1] + b.y, relu);
                     pk[2 * j + 1] = pack_bf16(v[4 * j + 2] + b.z, v[4 * j + 3] + b.w, relu);
                 }
             }
-            unsigned char *const stg = stage0 + (it & 1) * kStoreBytes;
-            if (lane == 0) bulk_wait_read_1();  // the store two tiles back has read this buffer
+            unsigned char *const stg = stage0 + (use & 1) * kStoreBytes;
+            if (lane == 0) bulk_wait_read_1();  // this warp's store two tiles back has read it
             __syncwarp();
-            uint4 *dst = reinterpret_cast<uint4 *>(stg + lane * kC * 2);
-#pragma unroll
-            for (int j = 0; j < 6; ++j)
-                dst[j] = make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
+            uint4 *dst = reinterpret_cast<uint4 *>(stg + lane * 32);
+            dst[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            dst[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
             fence_async_smem();
             __syncwarp();
             if (lane == 0) {
                 // rows wholly below the image store nothing; the (then empty)
                 // group is still committed, so wait_group.read 1 keeps pairing
                 // each buffer with the store two tiles back
-                if (y0 + 4 * q < a.h) tma_store_4d(&tm_out, stg, 0, x0, y0 + 4 * q, img);
+                if (y0 + 4 * q < a.h) tma_store_4d(&tm_out, stg, c0, x0, y0 + 4 * q, img);
                 bulk_commit();
             }
         }
@@ -548,10 +547,10 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
 // input tile, 8 columns x 18 rows, arrives by one TMA load of the 5-D view
 // (box {8, 8, 6, 18, 1}) as [row][channel / 8][column][channel % 8]: K-major,
 // LBO = 128 bytes, SBO = 768 bytes (one input row). Warp roles, mbarriers and
-// stores as conv48_tma_kernel, except that there are kT3Sets accumulators
+// stores as conv48_tma_kernel, except that there are kSets accumulators
 // (144 of 160 TMEM columns each) and as many sets of four draining warps: set
 // k (warps 2 + 4k .. 5 + 4k) takes the tiles of accumulator k, so each tile's
-// epilogue (nine TMEM loads, 96 shuffles per lane) has kT3Sets MMA tiles'
+// epilogue (nine TMEM loads, 96 shuffles per lane) has kSets MMA tiles'
 // time. Forward modes (bias, ReLU) only.
 constexpr int kT3X = 6, kT3Y = 16;
 constexpr int kIn3X = 8;
