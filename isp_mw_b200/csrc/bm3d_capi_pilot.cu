@@ -33,6 +33,7 @@ struct bm3d_pilot {
 namespace {
 
 constexpr int kPackElems = 9 * kC * kC;  // per layer
+constexpr int kPackTotal = 12 * kPackElems + 6 * kPack3Elems;
 
 int pilot_fail(bm3d_ctx *ctx, int code, const char *msg)
 {
@@ -68,35 +69,41 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
     return fn;
 }
 
-// The TMA pipelines' two views of n images of h x w x 48 BF16 (NHWC): the
-// input as (channel % 8, x, channel / 8, y, image), box {8, in_cols, 6,
-// in_rows, 1}, and the output as (channel, x, y, image), box {out_ch, out_cols,
-// 4, 1}: {8, 10, 6, 18, 1} / {16, 8, 4, 1} for conv48_tma_kernel,
-// {8, 8, 6, 18, 1} / {48, 6, 4, 1} for conv48_n144_kernel.
-bool encode_conv_maps(const void *x, void *y, int n, int h, int w, CUtensorMap &in, CUtensorMap &out,
-                      int in_cols = kT2X + 2, int out_cols = kT2X, int in_rows = kT2Y + 2,
-                      int out_ch = 16)
+// The TMA pipelines' views of n images of h x w x 48 BF16 (NHWC): the output as
+// (channel, x, y, image), the N = 48 pipeline's input as (channel % 8, x,
+// channel / 8, y, image) and the N = 144 one's as (channel, x, y, image) in
+// 128-byte swizzled rows of 64 channels, of which the last 16 lie outside the
+// tensor and are filled with zeros.
+bool encode_map(CUtensorMap &m, const void *p, int rank, const cuuint64_t *dim, const cuuint64_t *stride,
+                const cuuint32_t *box, CUtensorMapSwizzle swizzle)
 {
     auto enc = tensor_map_encoder();
-    if (!enc) return false;
-    const cuuint64_t px = 2ull * kC;  // bytes per pixel
-    const cuuint64_t gdim[5] = {8, static_cast<cuuint64_t>(w), 6, static_cast<cuuint64_t>(h),
-                                static_cast<cuuint64_t>(n)};
-    const cuuint64_t gstride[4] = {px, 16, px * w, px * w * h};
-    const cuuint32_t box[5] = {8, static_cast<cuuint32_t>(in_cols), 6,
-                               static_cast<cuuint32_t>(in_rows), 1};
     const cuuint32_t ones[5] = {1, 1, 1, 1, 1};
-    if (enc(&in, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void *>(x), gdim, gstride, box, ones,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return false;
-    const cuuint64_t odim[4] = {static_cast<cuuint64_t>(kC), static_cast<cuuint64_t>(w),
-                                static_cast<cuuint64_t>(h), static_cast<cuuint64_t>(n)};
-    const cuuint64_t ostride[3] = {px, px * w, px * w * h};
-    const cuuint32_t obox[4] = {static_cast<cuuint32_t>(out_ch), static_cast<cuuint32_t>(out_cols), 4, 1};
-    return enc(&out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, y, odim, ostride, obox, ones,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return enc && enc(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, static_cast<cuuint32_t>(rank),
+                      const_cast<void *>(p), dim, stride, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                      swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+bool encode_pixels(CUtensorMap &m, const void *p, int n, int h, int w, cuuint32_t ch, cuuint32_t cols,
+                   cuuint32_t rows, CUtensorMapSwizzle swizzle)
+{
+    const cuuint64_t px = 2ull * kC;  // bytes per pixel
+    const cuuint64_t dim[4] = {kC, static_cast<cuuint64_t>(w), static_cast<cuuint64_t>(h),
+                               static_cast<cuuint64_t>(n)};
+    const cuuint64_t stride[3] = {px, px * w, px * w * h};
+    const cuuint32_t box[4] = {ch, cols, rows, 1};
+    return encode_map(m, p, 4, dim, stride, box, swizzle);
+}
+
+bool encode_groups(CUtensorMap &m, const void *p, int n, int h, int w, cuuint32_t cols, cuuint32_t rows)
+{
+    const cuuint64_t px = 2ull * kC;
+    const cuuint64_t dim[5] = {8, static_cast<cuuint64_t>(w), 6, static_cast<cuuint64_t>(h),
+                               static_cast<cuuint64_t>(n)};
+    const cuuint64_t stride[4] = {px, 16, px * w, px * w * h};
+    const cuuint32_t box[5] = {8, cols, 6, rows, 1};
+    return encode_map(m, p, 5, dim, stride, box, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 // One 48 -> 48 layer on the tensor cores.
@@ -118,16 +125,17 @@ int run_conv48(bm3d_ctx *ctx, const __nv_bfloat16 *x, __nv_bfloat16 *y, const __
     const int choice = g_conv_choice.load();
     CUtensorMap tin, tout;
     if (w3 != nullptr && mode != kMaskPrev && (choice == 0 || choice == 3) &&
-        encode_conv_maps(x, y, n, h, wd, tin, tout, kIn3X, kT3X, kT3Y + 2, kC)) {
+        encode_pixels(tin, x, n, h, wd, 64, kIn3X, kT3Y + 2, CU_TENSOR_MAP_SWIZZLE_128B) &&
+        encode_pixels(tout, y, n, h, wd, kC, kT3X, 4, CU_TENSOR_MAP_SWIZZLE_NONE)) {
         a.wt = reinterpret_cast<const uint4 *>(w3);
         a.tiles_x = (wd + kT3X - 1) / kT3X;
         a.tiles_y = (h + kT3Y - 1) / kT3Y;
         a.tiles = n * a.tiles_x * a.tiles_y;
         // more than half an SM's shared memory keeps one CTA (and its 512
         // TMEM columns) per SM, so no CTA's allocation waits on another's
-        const int smem3 = std::max(kT3Smem, 120 * 1024);
-        CK(ctx, raise_smem_limit(reinterpret_cast<const void *>(conv48_n144_kernel), smem3));
-        conv48_n144_kernel<<<std::max(1, std::min(a.tiles, ctx->sm_count)), kT3Threads, smem3,
+        static_assert(kT3Smem > 120 * 1024, "one CTA per SM");
+        CK(ctx, raise_smem_limit(reinterpret_cast<const void *>(conv48_n144_kernel), kT3Smem));
+        conv48_n144_kernel<<<std::max(1, std::min(a.tiles, ctx->sm_count)), kT3Threads, kT3Smem,
                              s>>>(tin, tout, a);
         CK(ctx, cudaGetLastError());
         g_conv_last.store(3);
@@ -136,7 +144,8 @@ int run_conv48(bm3d_ctx *ctx, const __nv_bfloat16 *x, __nv_bfloat16 *y, const __
     if (choice == 3 && mode != kMaskPrev)
         return pilot_fail(ctx, BM3D_ERR_CUDA,
                           "pilot: the N = 144 convolution's tensor maps did not encode");
-    if (choice != 1 && encode_conv_maps(x, y, n, h, wd, tin, tout)) {
+    if (choice != 1 && encode_groups(tin, x, n, h, wd, kT2X + 2, kT2Y + 2) &&
+        encode_pixels(tout, y, n, h, wd, 16, kT2X, 4, CU_TENSOR_MAP_SWIZZLE_NONE)) {
         a.tiles_x = (wd + kT2X - 1) / kT2X;
         a.tiles_y = (h + kT2Y - 1) / kT2Y;
         a.tiles = n * a.tiles_x * a.tiles_y;
@@ -232,7 +241,7 @@ const __nv_bfloat16 *wbwd(const bm3d_pilot *p, int layer)
 }
 const __nv_bfloat16 *wfwd3(const bm3d_pilot *p, int layer)
 {
-    return static_cast<const __nv_bfloat16 *>(p->wpack.ptr) + (12 + layer - 2) * kPackElems;
+    return static_cast<const __nv_bfloat16 *>(p->wpack.ptr) + 12 * kPackElems + (layer - 2) * kPack3Elems;
 }
 const float *param(const bm3d_pilot *p, int offset)
 {
@@ -332,7 +341,7 @@ extern "C" int bm3d_pilot_create(bm3d_ctx *ctx, unsigned long long seed, bm3d_pi
             bm3d_pilot_destroy(p);
             return rc;
         }
-    if ((rc = ensure(ctx, p->wpack, 18 * kPackElems * sizeof(__nv_bfloat16))) != BM3D_OK) {
+    if ((rc = ensure(ctx, p->wpack, kPackTotal * sizeof(__nv_bfloat16))) != BM3D_OK) {
         bm3d_pilot_destroy(p);
         return rc;
     }
@@ -672,7 +681,7 @@ extern "C" int bm3d_pilot_conv48(bm3d_ctx *ctx, int n, int h, int w, const void 
     // weight: FP32 [48][48][3][3] (device); packed here into the operand layout
     DevBuf &wp = ctx->groups[0], &pp = ctx->groups[1], &eb = ctx->groups[2];
     int rc;
-    if ((rc = ensure(ctx, wp, 18 * kPackElems * sizeof(__nv_bfloat16))) != BM3D_OK) return rc;
+    if ((rc = ensure(ctx, wp, kPackTotal * sizeof(__nv_bfloat16))) != BM3D_OK) return rc;
     if ((rc = ensure(ctx, pp, kParams * sizeof(float))) != BM3D_OK) return rc;
     if ((rc = ensure(ctx, eb, sizeof(unsigned))) != BM3D_OK) return rc;
     float *params = static_cast<float *>(pp.ptr);

@@ -333,8 +333,8 @@ __global__ void __launch_bounds__(kConvThreads, kConvCtasPerSm) conv48_kernel(co
 // pixels with a TMA store of a 4-D view (channel, x, y, image) from a per-warp
 // staging buffer (the store clips at the image edges). kTmaStages operand buffers
 // and the accumulators are handed on by mbarriers (full / empty for each); no
-// CTA-wide barrier runs inside the tile loop. What bounds it: the tensor core's
-// operand fetch, 2.3 cycles per 8 x 8 core matrix, 44 of them an MMA. (Four warps
+// CTA-wide barrier runs inside the tile loop. What bounds it: operand fetch from
+// shared memory, 101 cycles an MMA (see conv48_n144_kernel). (Four warps
 // draining whole pixels of both accumulators, with the mask read after the MMAs,
 // were slower than that: data gradient of 32 crops of 128 x 128 52 -> 43 us.)
 constexpr int kT2X = 8, kT2Y = 16;
@@ -532,9 +532,7 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
 }
 
 // ---------------------------------------------------------------------------
-// Forward 48 -> 48 convolution with the three column taps in N: the N = 48
-// form is bound by the tensor core's operand fetch (an M = 128, N = 48,
-// K = 16 MMA fetches 5.5 KB for 24 cycles of math). Here an MMA is
+// Forward 48 -> 48 convolution with the three column taps in N. Here an MMA is
 // M = 128 input pixels (16 rows x 8 columns, m = row * 8 + column) by
 // N = 144 = (column tap dx, output channel) by K = 16 input channels:
 //   D[(r, c)][dx][co] = sum over row taps dy and channels of
@@ -544,34 +542,44 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
 // D[(r, j + 2)][2]: TMEM lanes m, m + 1, m + 2 of the same warp, added with
 // two shuffles per channel in the epilogue. Each tile yields 16 rows x 6
 // columns (the input's 8 columns minus the two the taps reach past). The
-// input tile, 8 columns x 18 rows, arrives by one TMA load of the 5-D view
-// (box {8, 8, 6, 18, 1}) as [row][channel / 8][column][channel % 8]: K-major,
-// LBO = 128 bytes, SBO = 768 bytes (one input row). Warp roles, mbarriers and
-// stores as conv48_tma_kernel, except that there are kSets accumulators
-// (144 of 160 TMEM columns each) and as many sets of four draining warps: set
-// k (warps 2 + 4k .. 5 + 4k) takes the tiles of accumulator k, so each tile's
-// epilogue (nine TMEM loads, 96 shuffles per lane) has kSets MMA tiles'
-// time. Forward modes (bias, ReLU) only.
+// input tile, 8 columns x 18 rows, arrives by one TMA load as 128-byte swizzled
+// rows of one pixel (48 channels and 16 zeros from outside the tensor): a tile row
+// is one 1024-byte swizzle atom. Warp roles, mbarriers and stores as
+// conv48_tma_kernel, except that there are kT3Sets accumulators (144 of 160
+// TMEM columns each) and as many sets of four draining warps, each warp with all
+// 48 channels: set k (warps 2 + 4k .. 5 + 4k) takes the tiles of accumulator k,
+// so each tile's epilogue (nine TMEM loads, 96 shuffles per lane) has kT3Sets MMA
+// tiles' time. Forward modes (bias, ReLU) only.
+//
+// What bounds it: operand fetch from shared memory, 55 bytes a cycle whatever
+// the layout -- an MMA takes 0.56 M + 0.59 N cycles, 158 here where its
+// arithmetic takes 72, and M = 128, N = 48 with nine taps takes 101 for a third of
+// the products. On a 1080p plane a layer takes 110 us; with a third of the MMAs
+// 82, without the stores 102, without the shuffles 106. Tiles of 16-byte chunks
+// (the unswizzled core-matrix layout, six times the TMA's requests) took 115,
+// 32-byte swizzled ones 110, twelve warps draining 16 channels each 125.
 constexpr int kT3X = 6, kT3Y = 16;
 constexpr int kIn3X = 8;
-constexpr int kRow3Bytes = 6 * kIn3X * 16;          // 768
-constexpr int kTile3Bytes = (kT3Y + 2) * kRow3Bytes;  // 13824
+constexpr int kRow3Bytes = kIn3X * 128;               // 1024: one input row
+constexpr int kTile3Bytes = (kT3Y + 2) * kRow3Bytes;  // 18432
 constexpr int kN3 = 3 * kC;                          // 144
 constexpr int kAcc3Cols = 160;                       // TMEM column stride of the accumulators (144 used)
 constexpr int kStore3Bytes = 4 * kT3X * kC * 2;      // one warp's 4 x 6 output pixels: 2304
 constexpr int kT3Stages = 4;
 constexpr int kT3Sets = 3;  // accumulators, each with its own set of four draining warps
 constexpr int kT3Threads = 64 + 128 * kT3Sets;  // producer, MMA issuer, the draining sets
-constexpr int kT3OffStage = kWeightBytes;
+constexpr int kTap3Elems = kN3 * 64;                  // one row tap's weights: [n][64], 48 used
+constexpr int kPack3Elems = 3 * kTap3Elems;
+constexpr int kT3OffStage = kPack3Elems * 2;
 constexpr int kT3OffStore = kT3OffStage + kT3Stages * kTile3Bytes;
 constexpr int kT3OffBias = kT3OffStore + 4 * kT3Sets * 2 * kStore3Bytes;
 constexpr int kT3OffBar = kT3OffBias + kC * 4;
-constexpr int kT3Smem = kT3OffBar + 8 * (2 * kT3Stages + 2 * kT3Sets) + 16;
+constexpr int kT3Smem = kT3OffBar + 8 * (2 * kT3Stages + 2 * kT3Sets) + 16 + 1024;  // to align to 1024
 static_assert(kT3Sets * kAcc3Cols <= 512 && kAcc3Cols % 32 == 0, "accumulators fit TMEM");
 constexpr uint32_t kIdesc3 = instr_desc_bf16(128, kN3, false, false);
-static_assert(kT3OffStage % 128 == 0 && kT3OffStore % 128 == 0 && kTile3Bytes % 128 == 0 &&
-                  kStore3Bytes % 128 == 0,
-              "TMA buffers 128-byte aligned");
+static_assert(kTap3Elems * 2 % 1024 == 0 && kT3OffStage % 1024 == 0 && kTile3Bytes % 1024 == 0,
+              "swizzled rows repeat every 1024 bytes");
+static_assert(kT3OffStore % 128 == 0 && kStore3Bytes % 128 == 0, "TMA buffers 128-byte aligned");
 
 __device__ __forceinline__ void tile_origin_6x16(int tile, int tiles_x, int tiles_y, int &img,
                                                  int &y0, int &x0)
@@ -588,7 +596,8 @@ __global__ void __launch_bounds__(kT3Threads, 1)
     conv48_n144_kernel(const __grid_constant__ CUtensorMap tm_in,
                        const __grid_constant__ CUtensorMap tm_out, const ConvArgs a)
 {
-    extern __shared__ __align__(128) unsigned char smem[];
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char *const smem = smem_raw + (1024 - (smem_u32(smem_raw) & 1023)) % 1024;
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + kT3OffBar);
     uint64_t *empty = full + kT3Stages;
     uint64_t *accf = empty + kT3Stages;
@@ -598,7 +607,7 @@ __global__ void __launch_bounds__(kT3Threads, 1)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (blockIdx.x >= a.tiles) return;
 
-    for (int i = tid; i < kWeightBytes / 16; i += blockDim.x)
+    for (int i = tid; i < kPack3Elems * 2 / 16; i += blockDim.x)
         reinterpret_cast<uint4 *>(smem)[i] = __ldg(a.wt + i);
     if (tid < kC) bias_s[tid] = __ldg(a.bias + tid);
     if (tid == 0) {
@@ -632,7 +641,7 @@ __global__ void __launch_bounds__(kT3Threads, 1)
                 int img, y0, x0;
                 tile_origin_6x16(tile, a.tiles_x, a.tiles_y, img, y0, x0);
                 mbar_arrive_expect_tx(&full[st], kTile3Bytes);
-                tma_load_5d(smem + kT3OffStage + st * kTile3Bytes, &tm_in, &full[st], 0, x0 - 1, 0,
+                tma_load_4d(smem + kT3OffStage + st * kTile3Bytes, &tm_in, &full[st], 0, x0 - 1,
                             y0 - 1, img);
             }
         }
@@ -648,16 +657,16 @@ __global__ void __launch_bounds__(kT3Threads, 1)
                 }
                 tc_fence_after();
                 const uint64_t ad0 =
-                    smem_desc(smem_u32(smem + kT3OffStage + st * kTile3Bytes), 128, kRow3Bytes);
-                const uint64_t bd0 = smem_desc(smem_u32(smem), 128, 256);
+                    smem_desc_sw128(smem_u32(smem + kT3OffStage + st * kTile3Bytes), kRow3Bytes);
+                const uint64_t bd0 = smem_desc_sw128(smem_u32(smem), 1024);
 #pragma unroll
                 for (int dy = 0; dy < 3; ++dy) {
 #pragma unroll
                     for (int s3 = 0; s3 < 3; ++s3) {
                         const uint64_t ad =
-                            ad0 + static_cast<uint64_t>((dy * kRow3Bytes + s3 * 256) >> 4);
+                            ad0 + static_cast<uint64_t>((dy * kRow3Bytes + s3 * 32) >> 4);
                         const uint64_t bd =
-                            bd0 + static_cast<uint64_t>(((dy * 3 + s3) * kN3 * 16 * 2) >> 4);
+                            bd0 + static_cast<uint64_t>((dy * kTap3Elems * 2 + s3 * 32) >> 4);
                         mma_bf16(tbase + k * kAcc3Cols, ad, bd, kIdesc3, dy > 0 || s3 > 0);
                     }
                 }
@@ -748,9 +757,8 @@ __global__ void __launch_bounds__(kT3Threads, 1)
 // accumulates over its tiles and writes a partial dW (and the bias gradient from
 // G) that reduce_partials_kernel sums.
 //
-// What bounds it: the tensor core's operand fetch, 2.3 cycles per 8 x 8 core
-// matrix of these layouts: 52 of them an MMA (68 with M = 128, as it was: 61 us
-// where this takes 47). Under that stay: tiles read in the order of global memory,
+// What bounds it: operand fetch from shared memory, 121 cycles an MMA (see
+// conv48_n144_kernel; 158 with M = 128, as it was: 61 us where this takes 47). Under that stay: tiles read in the order of global memory,
 // 16-byte chunks of whole rows of pixels, G's channel groups 144 bytes apart so
 // that a row's chunks land on distinct banks; kWgStages - 1 tiles on their way;
 // chunk addresses worked out once; the bias summed by six warps. One tile ahead,
@@ -1423,9 +1431,9 @@ __global__ void __launch_bounds__(240) wgrad_in_kernel(const InArgs a, const __n
 // with N = ci, K = co.
 // BF16 copies of the six 48 -> 48 layers' weights in the MMA operand
 // layouts: `fwd` and `bwd` (flipped, transposed: the data gradient) per tap
-// as [co / 8][ci / 8][co % 8][ci % 8] (N = 48); `fwd3` (may be null) for the
-// N = 144 forward kernel, per (row tap dy, 16-channel step s) as
-// [n / 8][k / 8][n % 8][k % 8] with n = column tap * 48 + co, k = ci - 16 s.
+// as [co / 8][ci / 8][co % 8][ci % 8] (N = 48); `fwd3` for the N = 144 forward
+// kernel, per row tap dy as 144 rows n = column tap * 48 + co of 64 channels ci
+// (48 used), 128-byte swizzled (smem_desc_sw128).
 __global__ void pack_weights_kernel(const float *params, __nv_bfloat16 *fwd, __nv_bfloat16 *bwd,
                                     __nv_bfloat16 *fwd3)
 {
@@ -1434,14 +1442,6 @@ __global__ void pack_weights_kernel(const float *params, __nv_bfloat16 *fwd, __n
         const int layer = i / per;
         int r = i - layer * per;
         const float *w = params + off_w(layer + 2);
-        if (fwd3 != nullptr) {
-            const int blk = r / (3 * kC * 16), e = r - blk * (3 * kC * 16);
-            const int dy = blk / 3, st = blk % 3;
-            const int nb = e / 128, kb = (e / 64) % 2, n8 = (e / 8) % 8, k8 = e % 8;
-            const int n = nb * 8 + n8, k = kb * 8 + k8;
-            const int dx = n / kC, co = n % kC, ci = st * 16 + k;
-            fwd3[i] = __float2bfloat16_rn(w[((co * kC + ci) * 3 + dy) * 3 + dx]);
-        }
         const int tap = r / (kC * kC);
         r -= tap * kC * kC;
         // r = element of the packed tap: [n / 8][k / 8][n % 8][k % 8]
@@ -1449,6 +1449,8 @@ __global__ void pack_weights_kernel(const float *params, __nv_bfloat16 *fwd, __n
         const int n = ng * 8 + n8, k = kg * 8 + k8;
         const int ky = tap / 3, kx = tap % 3;
         fwd[i] = __float2bfloat16_rn(w[((n * kC + k) * 3 + ky) * 3 + kx]);
+        const int n3 = kx * kC + n;
+        fwd3[layer * kPack3Elems + ky * kTap3Elems + n3 * 64 + ((k / 8) ^ (n3 & 7)) * 8 + k8] = fwd[i];
         bwd[i] = __float2bfloat16_rn(w[((k * kC + n) * 3 + (2 - ky)) * 3 + (2 - kx)]);
     }
 }

@@ -28,6 +28,15 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t smem_addr, uint32_t lbo, 
     return d;
 }
 
+// The same for a K-major operand in 128-byte swizzled rows (layout type 2):
+// element (r, k) in row (r % 8) * 128 + (r / 8) * SBO, its 16-byte chunk k / 8
+// exchanged with chunk (k / 8) ^ (r % 8), as TMA writes it. Rows repeat every
+// 1024 bytes, to which operands align; a K-step of 16 starts 32 bytes further.
+__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t smem_addr, uint32_t sbo)
+{
+    return smem_desc(smem_addr, 16, sbo) | static_cast<uint64_t>(2) << 61;
+}
+
 // Instruction descriptor of tcgen05.mma.kind::f16 with BF16 A and B and an
 // FP32 accumulator: D format F32 at [4, 6), A format BF16 at [7, 10), B format
 // BF16 at [10, 13), A / B major at bits 15 / 16 (0 = K-major, 1 = MN-major),
@@ -189,6 +198,17 @@ __device__ __forceinline__ void tma_load_5d(void *smem_dst, const void *tmap, ui
         " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];" ::"r"(smem_u32(smem_dst)),
         "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(mbar)), "r"(c0), "r"(c1), "r"(c2),
         "r"(c3), "r"(c4)
+        : "memory");
+}
+
+__device__ __forceinline__ void tma_load_4d(void *smem_dst, const void *tmap, uint64_t *mbar, int c0,
+                                            int c1, int c2, int c3)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(smem_u32(smem_dst)),
+        "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(mbar)), "r"(c0), "r"(c1), "r"(c2),
+        "r"(c3)
         : "memory");
 }
 
