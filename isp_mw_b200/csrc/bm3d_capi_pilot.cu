@@ -43,6 +43,12 @@ int pilot_fail(bm3d_ctx *ctx, int code, const char *msg)
 
 int grid_for(const bm3d_ctx *ctx, int tiles) { return std::max(1, std::min(tiles, ctx->sm_count)); }
 
+// CTAs of layers 1 and 8's pixel kernels.
+int px_grid(const bm3d_ctx *ctx, long long pixels)
+{
+    return static_cast<int>(std::min<long long>((pixels + kPxPerCta - 1) / kPxPerCta, 6LL * ctx->sm_count));
+}
+
 // Which 48 -> 48 convolution kernel runs: 0 = the N = 144 TMA pipeline for
 // forward layers and the N = 48 one for data gradients, when their tensor
 // maps encode (else the cp.async kernel); 1 = the cp.async kernel; 2 = the
@@ -284,7 +290,7 @@ int forward(bm3d_pilot *p, const float *in, long long stride, long long img_stri
     ia.h = h;
     ia.w = w;
     if (p->timing) CK(ctx, cudaEventRecord(p->ev[0], s));
-    conv_in_kernel<<<blocks, 256, 0, s>>>(ia);
+    conv_in_kernel<<<px_grid(ctx, pixels), kPxThreads, 0, s>>>(ia);
     CK(ctx, cudaGetLastError());
     if (p->timing) CK(ctx, cudaEventRecord(p->ev[1], s));
     int rc;
@@ -550,7 +556,6 @@ extern "C" int bm3d_pilot_train_step(bm3d_pilot *p, int count, int height, int w
     float *grad = static_cast<float *>(p->grad.ptr);
     float *part = static_cast<float *>(p->partial.ptr);
     const float *dout = static_cast<const float *>(p->dout.ptr);
-    const int blocks = static_cast<int>(std::min<long long>((pixels + 255) / 256, 8LL * ctx->sm_count));
     const int rblocks = 2 * ctx->sm_count;
     // Adam's bias-corrected step size. Each layer is summed and updated as soon as
     // its partials are written (while they are in L2; 75 MB of all layers' read
@@ -582,7 +587,7 @@ extern "C" int bm3d_pilot_train_step(bm3d_pilot *p, int count, int height, int w
     ob.n = count;
     ob.h = height;
     ob.w = width;
-    out_backward_kernel<<<blocks, 256, 0, s>>>(ob);
+    out_backward_kernel<<<px_grid(ctx, pixels), kPxThreads, 0, s>>>(ob);
     CK(ctx, cudaGetLastError());
     if ((rc = update(rblocks, kW8Partial, kW8, kOffW8, false)) != BM3D_OK) return rc;
     // layers 7 .. 2: weight gradient (tensor cores), data gradient (tensor cores)

@@ -1049,81 +1049,129 @@ __device__ __forceinline__ unsigned long long ffma2(unsigned long long a, unsign
     return d;
 }
 
-// Layer 1, one pixel per thread. The noise-level input is constant inside the
-// image, so for a pixel whose 3 x 3 neighbourhood is inside, its part is
-// sigma * sum_t W1[c][1][t] (one constant per channel); border pixels sum it
-// over their inside taps. Channel pairs run as packed FMAs on weights kept
-// [tap][channel] in shared memory (128-bit broadcast reads).
-__global__ void __launch_bounds__(256) conv_in_kernel(const InArgs a)
+// Layers 1 and 8's pixel kernels give each thread two pixels, 32 apart, of its
+// warp's 64: every weight read serves both. Results go through shared memory
+// (pixels kPxPitch apart: distinct banks) so that a warp writes its 64 pixels as
+// whole lines; straight from the registers, a store's lanes lie 96 bytes apart.
+constexpr int kPxThreads = 128, kPxWarps = kPxThreads / 32, kPxPerWarp = 64;
+constexpr int kPxPitch = 112;
+constexpr int kPxPerCta = kPxWarps * kPxPerWarp;
+
+// Chunk j (16 bytes) of a warp's staged pixels.
+__device__ __forceinline__ uint4 staged_chunk(const unsigned char *stage, int j)
+{
+    return *reinterpret_cast<const uint4 *>(stage + j / 6 * kPxPitch + j % 6 * 16);
+}
+
+// acc += x * w. (Scalar: a packed FMA takes the FP32 pipe as long as two and its
+// operand (x, x) two moves each time.)
+__device__ __forceinline__ void fma4(float4 &acc, float x, const float4 w)
+{
+    acc.x = fmaf(x, w.x, acc.x);
+    acc.y = fmaf(x, w.y, acc.y);
+    acc.z = fmaf(x, w.z, acc.z);
+    acc.w = fmaf(x, w.w, acc.w);
+}
+
+// Layer 1. The noise-level input is constant inside the image, so for a pixel
+// whose 3 x 3 neighbourhood is inside, its part is sigma * sum_t W1[c][1][t] (one
+// constant per channel); border pixels sum it over their inside taps. Weights are
+// kept [tap][channel] in shared memory (128-bit broadcast reads). What bounds it: the FP32
+// pipe (28 us of a 1080p plane) and latency. A 1080p plane 101 -> 80 us against one
+// pixel a thread, packed FMAs and 16-byte stores from registers (84 with these
+// FMAs packed); 32 crops of 128 x 128, where its 2048 units fill 888 CTAs
+// unevenly, 35 -> 38.
+__global__ void __launch_bounds__(kPxThreads, 6) conv_in_kernel(const InArgs a)
 {
     __shared__ __align__(16) float wn[9][kC];  // W1[c][0][t] at [t][c]
     __shared__ __align__(16) float wsg[9][kC]; // W1[c][1][t] at [t][c]
     __shared__ __align__(16) float bias[kC], stot[kC];
-    for (int i = threadIdx.x; i < 9 * kC; i += blockDim.x) {
-        const int t = i / kC, c = i - t * kC;
-        wn[t][c] = a.wb[(c * 2 + 0) * 9 + t];
-        wsg[t][c] = a.wb[(c * 2 + 1) * 9 + t];
+    __shared__ __align__(16) unsigned char staging[kPxWarps][kPxPerWarp * kPxPitch];
+#pragma unroll
+    for (int k = 0; k < (kW1 + kPxThreads - 1) / kPxThreads; ++k) {
+        const int i = threadIdx.x + k * kPxThreads;  // W1[c][cin][t]
+        const int c = i / 18, r = i - c * 18;
+        if (i < kW1) (r < 9 ? wn[r][c] : wsg[r - 9][c]) = a.wb[i];
     }
+    for (int c = threadIdx.x; c < kC; c += blockDim.x) bias[c] = a.wb[kW1 + c];
+    __syncthreads();
     for (int c = threadIdx.x; c < kC; c += blockDim.x) {
-        bias[c] = a.wb[kW1 + c];
         float st = 0.0f;
-        for (int t = 0; t < 9; ++t) st += a.wb[(c * 2 + 1) * 9 + t];
+        for (int t = 0; t < 9; ++t) st += wsg[t][c];
         stot[c] = st;
     }
     __syncthreads();
-    const long long total = static_cast<long long>(a.n) * a.h * a.w;
-    for (long long p = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; p < total;
-         p += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const int img = static_cast<int>(p / (static_cast<long long>(a.h) * a.w));
-        const int r = static_cast<int>(p - static_cast<long long>(img) * a.h * a.w);
-        const int y = r / a.w, x = r - y * a.w;
-        const float s = a.sigma[img];
-        const bool interior = y > 0 && y < a.h - 1 && x > 0 && x < a.w - 1;
-        unsigned long long nd[9];  // (noisy, noisy) of each tap, 0 outside
-        unsigned inside = 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned char *const stage = staging[warp];
+    // (pixels of activations that fit in memory count below 2^31)
+    const unsigned plane = static_cast<unsigned>(a.h) * a.w, total = plane * a.n;
+    for (unsigned base = (blockIdx.x * kPxWarps + warp) * kPxPerWarp; base < total;
+         base += gridDim.x * kPxPerCta) {
+        float nd[2][9], sd[2];  // noisy at each tap, 0 outside; sigma
+        unsigned inside[2];
 #pragma unroll
-        for (int t = 0; t < 9; ++t) {
-            const int yy = y + t / 3 - 1, xx = x + t % 3 - 1;
-            const bool ok = yy >= 0 && yy < a.h && xx >= 0 && xx < a.w;
-            const float v = ok ? __ldg(a.in + img * a.img_stride + yy * a.stride + xx) : 0.0f;
-            nd[t] = f2pack(v, v);
-            inside |= (ok ? 1u : 0u) << t;
-        }
-        const unsigned long long sd = f2pack(s, s);
-        uint32_t packed[24];
-#pragma unroll
-        for (int c = 0; c < kC; c += 4) {
-            const float4 b4 = *reinterpret_cast<const float4 *>(&bias[c]);
-            unsigned long long acc0 = f2pack(b4.x, b4.y), acc1 = f2pack(b4.z, b4.w);
-            if (interior) {
-                const float4 s4 = *reinterpret_cast<const float4 *>(&stot[c]);
-                acc0 = ffma2(sd, f2pack(s4.x, s4.y), acc0);
-                acc1 = ffma2(sd, f2pack(s4.z, s4.w), acc1);
-            } else {
-#pragma unroll
-                for (int t = 0; t < 9; ++t)
-                    if (inside & (1u << t)) {
-                        const float4 s4 = *reinterpret_cast<const float4 *>(&wsg[t][c]);
-                        acc0 = ffma2(sd, f2pack(s4.x, s4.y), acc0);
-                        acc1 = ffma2(sd, f2pack(s4.z, s4.w), acc1);
-                    }
-            }
+        for (int k = 0; k < 2; ++k) {
+            const unsigned p = min(base + 32 * k + lane, total - 1);
+            const unsigned img = p / plane, r = p - img * plane;
+            const int y = r / a.w, x = r - y * a.w;
+            const float *at = a.in + img * a.img_stride + y * a.stride + x;
+            sd[k] = a.sigma[img];
+            inside[k] = 0;
 #pragma unroll
             for (int t = 0; t < 9; ++t) {
-                const float4 w4 = *reinterpret_cast<const float4 *>(&wn[t][c]);
-                acc0 = ffma2(nd[t], f2pack(w4.x, w4.y), acc0);
-                acc1 = ffma2(nd[t], f2pack(w4.z, w4.w), acc1);
+                const int yy = y + t / 3 - 1, xx = x + t % 3 - 1;
+                const bool ok = yy >= 0 && yy < a.h && xx >= 0 && xx < a.w;
+                nd[k][t] = ok ? __ldg(at + (t / 3 - 1) * a.stride + (t % 3 - 1)) : 0.0f;
+                inside[k] |= (ok ? 1u : 0u) << t;
             }
-            float v0, v1, v2, v3;
-            f2unpack(acc0, v0, v1);
-            f2unpack(acc1, v2, v3);
-            packed[c / 2] = pack_bf16(v0, v1, true);
-            packed[c / 2 + 1] = pack_bf16(v2, v3, true);
         }
-        uint4 *dst = reinterpret_cast<uint4 *>(a.y + p * kC);
+#pragma unroll 2
+        for (int q = 0; q < 6; ++q) {
+            uint32_t packed[2][4];
 #pragma unroll
-        for (int q = 0; q < 6; ++q)
-            dst[q] = make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
+            for (int hf = 0; hf < 2; ++hf) {
+                const int c = 8 * q + 4 * hf;
+                const float4 b4 = *reinterpret_cast<const float4 *>(&bias[c]);
+                const float4 s4 = *reinterpret_cast<const float4 *>(&stot[c]);
+                float4 acc[2];
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    acc[k] = b4;
+                    if (inside[k] == 0x1ffu) {
+                        fma4(acc[k], sd[k], s4);
+                    } else {
+#pragma unroll 1
+                        for (int t = 0; t < 9; ++t)
+                            if (inside[k] & (1u << t))
+                                fma4(acc[k], sd[k], *reinterpret_cast<const float4 *>(&wsg[t][c]));
+                    }
+                }
+#pragma unroll
+                for (int t = 0; t < 9; ++t) {
+                    const float4 w4 = *reinterpret_cast<const float4 *>(&wn[t][c]);
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) fma4(acc[k], nd[k][t], w4);
+                }
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    packed[k][2 * hf] = pack_bf16(acc[k].x, acc[k].y, true);
+                    packed[k][2 * hf + 1] = pack_bf16(acc[k].z, acc[k].w, true);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+                *reinterpret_cast<uint4 *>(stage + (32 * k + lane) * kPxPitch + q * 16) =
+                    make_uint4(packed[k][0], packed[k][1], packed[k][2], packed[k][3]);
+        }
+        __syncwarp();
+        uint4 *const dst = reinterpret_cast<uint4 *>(a.y + static_cast<size_t>(base) * kC);
+        const int chunks = static_cast<int>(min(total - base, static_cast<unsigned>(kPxPerWarp))) * 6;
+#pragma unroll
+        for (int i = 0; i < kPxPerWarp * 6 / 32; ++i) {
+            const int j = lane + 32 * i;
+            if (j < chunks) dst[j] = staged_chunk(stage, j);
+        }
+        __syncwarp();
     }
 }
 
@@ -1274,48 +1322,85 @@ struct OutBackArgs {
     int n, h, w;
 };
 
-__global__ void __launch_bounds__(256) out_backward_kernel(const OutBackArgs a)
+// What bounds it: latency; then the lines of X7 and G7 (100 MB for 32 crops of
+// 128 x 128: 15 us). Those crops 38 -> 29 us against one pixel a thread, scalar
+// weight reads and strided 16-byte accesses (32 with scalar FMAs).
+__global__ void __launch_bounds__(kPxThreads, 6) out_backward_kernel(const OutBackArgs a)
 {
-    __shared__ float ws[kW8];
-    for (int i = threadIdx.x; i < kW8; i += blockDim.x) ws[i] = a.wb[i];
+    __shared__ __align__(16) float wt[9][kC];  // W8[c][t] at [t][c]
+    __shared__ __align__(16) unsigned char staging[kPxWarps][kPxPerWarp * kPxPitch];
+    for (int i = threadIdx.x; i < 9 * kC; i += blockDim.x) {
+        const int t = i / kC, c = i - t * kC;
+        wt[t][c] = a.wb[c * 9 + t];
+    }
     __syncthreads();
-    const long long total = static_cast<long long>(a.n) * a.h * a.w;
-    for (long long p = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; p < total;
-         p += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const int img = static_cast<int>(p / (static_cast<long long>(a.h) * a.w));
-        const int r = static_cast<int>(p - static_cast<long long>(img) * a.h * a.w);
-        const int y = r / a.w, x = r - y * a.w;
-        float d[9];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned char *const stage = staging[warp];
+    const unsigned plane = static_cast<unsigned>(a.h) * a.w, total = plane * a.n;
+    for (unsigned base = (blockIdx.x * kPxWarps + warp) * kPxPerWarp; base < total;
+         base += gridDim.x * kPxPerCta) {
+        unsigned long long d[2][9];
 #pragma unroll
-        for (int t = 0; t < 9; ++t) {
-            // out(q) uses x(q + t - 1): x(p) reaches out(p - (t - 1))
-            const int yy = y - (t / 3 - 1), xx = x - (t % 3 - 1);
-            const bool ok = yy >= 0 && yy < a.h && xx >= 0 && xx < a.w;
-            d[t] = ok ? a.dout[(static_cast<long long>(img) * a.h + yy) * a.w + xx] : 0.0f;
+        for (int k = 0; k < 2; ++k) {
+            const unsigned p = min(base + 32 * k + lane, total - 1);
+            const unsigned r = p % plane;
+            const int y = r / a.w, x = r - y * a.w;
+#pragma unroll
+            for (int t = 0; t < 9; ++t) {
+                // out(q) uses x(q + t - 1): x(p) reaches out(p - (t - 1))
+                const int yy = y - (t / 3 - 1), xx = x - (t % 3 - 1);
+                const bool ok = yy >= 0 && yy < a.h && xx >= 0 && xx < a.w;
+                const float v =
+                    ok ? a.dout[static_cast<long long>(p) - (t / 3 - 1) * a.w - (t % 3 - 1)] : 0.0f;
+                d[k][t] = f2pack(v, v);
+            }
         }
-        const uint4 *xs = reinterpret_cast<const uint4 *>(a.x7 + p * kC);
-        uint4 *gd = reinterpret_cast<uint4 *>(a.g + p * kC);
-#pragma unroll
+#pragma unroll 2
         for (int q = 0; q < 6; ++q) {
-            const uint4 u = xs[q];
-            const unsigned wd[4] = {u.x, u.y, u.z, u.w};
-            uint32_t o[4];
+            uint32_t packed[2][4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int c = q * 8 + 2 * k;
-                float g0 = 0.0f, g1 = 0.0f;
+            for (int hf = 0; hf < 2; ++hf) {
+                unsigned long long g0[2] = {}, g1[2] = {};
 #pragma unroll
                 for (int t = 0; t < 9; ++t) {
-                    g0 += ws[c * 9 + t] * d[t];
-                    g1 += ws[(c + 1) * 9 + t] * d[t];
+                    const float4 w4 = *reinterpret_cast<const float4 *>(&wt[t][8 * q + 4 * hf]);
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        g0[k] = ffma2(f2pack(w4.x, w4.y), d[k][t], g0[k]);
+                        g1[k] = ffma2(f2pack(w4.z, w4.w), d[k][t], g1[k]);
+                    }
                 }
-                if (!(__uint_as_float(wd[k] << 16) > 0.0f)) g0 = 0.0f;
-                if (!(__uint_as_float(wd[k] & 0xffff0000u) > 0.0f)) g1 = 0.0f;
-                const __nv_bfloat162 b2 = __floats2bfloat162_rn(g0, g1);
-                o[k] = *reinterpret_cast<const uint32_t *>(&b2);
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    float v0, v1, v2, v3;
+                    f2unpack(g0[k], v0, v1);
+                    f2unpack(g1[k], v2, v3);
+                    packed[k][2 * hf] = pack_bf16(v0, v1, false);
+                    packed[k][2 * hf + 1] = pack_bf16(v2, v3, false);
+                }
             }
-            gd[q] = make_uint4(o[0], o[1], o[2], o[3]);
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+                *reinterpret_cast<uint4 *>(stage + (32 * k + lane) * kPxPitch + q * 16) =
+                    make_uint4(packed[k][0], packed[k][1], packed[k][2], packed[k][3]);
         }
+        __syncwarp();
+        const uint4 *const xs = reinterpret_cast<const uint4 *>(a.x7 + static_cast<size_t>(base) * kC);
+        uint4 *const gd = reinterpret_cast<uint4 *>(a.g + static_cast<size_t>(base) * kC);
+        const int chunks = static_cast<int>(min(total - base, static_cast<unsigned>(kPxPerWarp))) * 6;
+#pragma unroll
+        for (int i = 0; i < kPxPerWarp * 6 / 32; ++i) {
+            const int j = lane + 32 * i;
+            if (j >= chunks) break;
+            const uint4 u = xs[j], g = staged_chunk(stage, j);
+            auto positive = [](unsigned v) {  // all ones in each half that is > 0
+                return __hgt2_mask(*reinterpret_cast<const __nv_bfloat162 *>(&v),
+                                   __float2bfloat162_rn(0.0f));
+            };
+            gd[j] = make_uint4(g.x & positive(u.x), g.y & positive(u.y), g.z & positive(u.z),
+                               g.w & positive(u.w));
+        }
+        __syncwarp();
     }
 }
 

@@ -349,3 +349,29 @@ def test_wgrad48_tile_edges(ctx, shape):
     ref_b = gr.double().sum(dim=(0, 1, 2))
     for got, ref in ((dw.double(), ref_w), (db.double(), ref_b)):
         assert float((got - ref).abs().max()) <= 1e-5 * max(1.0, float(ref.abs().max()))
+
+
+# layers 1 and 8 forward and backward at sizes around their units of 64 pixels and
+# columns of 5 x 16: every FP32 gradient within the BF16 chain's tolerance
+@pytest.mark.parametrize("shape", [(1, 1, 1), (3, 1, 70), (2, 17, 5), (1, 63, 1), (4, 33, 31)])
+def test_pilot_edge_layers_at_ragged_sizes(ctx, shape):
+    import torch
+    import isp_mw_b200
+    n, h, w = shape
+    noisy, clean, sigma = _data(n, max(h, 16), max(w, 16), 5)
+    noisy, clean = noisy[:, :h, :w].contiguous(), clean[:, :h, :w].contiguous()
+    pilot = isp_mw_b200.Pilot(ctx, seed=3)
+    params = torch.from_numpy(pilot.params()).cuda().double().requires_grad_(True)
+    err = (_emulate(params, noisy.double(), sigma.double()) - clean.double()).square()
+    q = ((25.0 / 255.0) / sigma.double()).square().view(-1, 1, 1)
+    loss = (err * q).mean()
+    loss.backward()
+    loss = loss.item()
+    got = pilot.train_step(noisy, clean, sigma, 1e-4)
+    grad = torch.from_numpy(pilot.grad()).cuda().double()
+    pilot.close()
+    assert abs(got - loss) <= 1e-2 * loss + 1e-9
+    ref = params.grad
+    for part in (slice(0, 912), slice(-433, None)):  # layer 1, layer 8
+        d = (grad[part] - ref[part]).norm()
+        assert float(d) <= 0.05 * float(ref[part].norm()) + 1e-7, (part, float(d))
