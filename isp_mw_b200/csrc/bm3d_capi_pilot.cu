@@ -556,7 +556,7 @@ extern "C" int bm3d_pilot_train_step(bm3d_pilot *p, int count, int height, int w
     float *grad = static_cast<float *>(p->grad.ptr);
     float *part = static_cast<float *>(p->partial.ptr);
     const float *dout = static_cast<const float *>(p->dout.ptr);
-    const int rblocks = 2 * ctx->sm_count;
+    const int rblocks = 2 * ctx->sm_count;  // even: wgrad_in_kernel's two planes
     // Adam's bias-corrected step size. Each layer is summed and updated as soon as
     // its partials are written (while they are in L2; 75 MB of all layers' read
     // back together took 54 us) and its FP32 weights have been read.
@@ -575,7 +575,7 @@ extern "C" int bm3d_pilot_train_step(bm3d_pilot *p, int count, int height, int w
         return run_reduce(ctx, ra, s);
     };
     // layer 8: weight gradient, then the gradient into layer 7's pre-activation
-    wgrad_out_kernel<<<rblocks, 256, 0, s>>>(X(7), dout, count, height, width, part);
+    wgrad_out_kernel<<<rblocks, kEdgeThreads, 0, s>>>(X(7), dout, count, height, width, part);
     CK(ctx, cudaGetLastError());
     __nv_bfloat16 *G[2] = {static_cast<__nv_bfloat16 *>(p->gbuf[0].ptr),
                            static_cast<__nv_bfloat16 *>(p->gbuf[1].ptr)};
@@ -614,7 +614,7 @@ extern "C" int bm3d_pilot_train_step(bm3d_pilot *p, int count, int height, int w
     ia.n = count;
     ia.h = height;
     ia.w = width;
-    wgrad_in_kernel<<<rblocks, 240, 0, s>>>(ia, G[cur], part);
+    wgrad_in_kernel<<<rblocks, kEdgeThreads, 0, s>>>(ia, G[cur], part);
     CK(ctx, cudaGetLastError());
     if ((rc = update(rblocks, kW1Partial, kW1, 0, false)) != BM3D_OK) return rc;
     // the packed BF16 copies of the updated weights

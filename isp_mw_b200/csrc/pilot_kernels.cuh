@@ -1404,110 +1404,184 @@ __global__ void __launch_bounds__(kPxThreads, 6) out_backward_kernel(const OutBa
     }
 }
 
-// Weight and bias gradients of layer 8: dW8[ci][t] = sum_p dOut[p] X7[p + t - 1][ci],
-// db8 = sum_p dOut[p]. One thread per (pixel, 8-channel group); per-CTA partials.
+// Weight and bias gradients of layers 8 and 1, FP32 products and sums:
+//   dW8[ci][t] = sum_p dOut[p] X7[p + t - 1][ci], db8 = sum_p dOut[p];
+//   dW1[co][cin][t] = sum_p G1[p][co] In_cin[p + t - 1], db1[co] = sum_p G1[p][co].
+// Both are sums, per 8-channel group of a 48-channel image V (X7, G1), of V times
+// the nine neighbours of a plane u; X7[q] meets dOut[q - (t - 1)], the neighbours
+// in reverse. 30 lanes of a warp take five columns of six groups -- V's rows are
+// read as 480 contiguous bytes -- and walk kEdgeRows pixels down them, the 3 x 3
+// window of u sliding in registers, kEdgeAhead rows of loads at a time, products
+// in packed pairs. Layer 1's two planes have blocks of their own. What bounds it:
+// latency of the loads and the FP32 pipe. One pixel and 4 (8) channels a thread
+// and iteration, each with its nine loads and 64-bit divisions, took 126 (layer 1)
+// and 69 us (layer 8) for 32 crops of 128 x 128; this takes 52 and 26 (56 and 27
+// with scalar FMAs).
 constexpr int kW8Partial = kW8 + 1;
+constexpr int kW1Partial = kW1 + kC;
+constexpr int kEdgeThreads = 192, kEdgeRows = 16, kEdgeAhead = 4, kEdgeCols = 5;
 
-__global__ void __launch_bounds__(256) wgrad_out_kernel(const __nv_bfloat16 *x7, const float *dout,
-                                                         int n, int h, int w, float *partial)
+struct EdgeSums {
+    unsigned long long dw[9][4];  // per tap, channel pairs
+    unsigned long long v[4];      // sums of V
+    float u;                      // sum of u
+};
+
+// This warp's share (of `warps`) of the sums; u is sigma[image] everywhere inside
+// the image where `constant`.
+template <bool REVERSE>
+__device__ __forceinline__ void edge_sums(const __nv_bfloat16 *v, const float *u, long long stride,
+                                          long long img_stride, const float *sigma, bool constant, int n,
+                                          int h, int w, int warp, int warps, int grp, int col, EdgeSums &e)
 {
-    __shared__ float red[kW8Partial];
-    for (int i = threadIdx.x; i < kW8Partial; i += blockDim.x) red[i] = 0.0f;
-    __syncthreads();
-    const long long total = static_cast<long long>(n) * h * w;
-    const int grp = threadIdx.x % 6;  // 8-channel group
-    float acc[72];
+    const int ux = (w + kEdgeCols - 1) / kEdgeCols, uy = (h + kEdgeRows - 1) / kEdgeRows;
+    const unsigned long long one = f2pack(1.0f, 1.0f);
+    for (long long unit = warp; unit < static_cast<long long>(n) * uy * ux; unit += warps) {
+        const int img = static_cast<int>(unit / (uy * ux));
+        const int r0 = static_cast<int>(unit - static_cast<long long>(img) * uy * ux);
+        const int y0 = r0 / ux * kEdgeRows, x = r0 % ux * kEdgeCols + col;
+        if (x >= w) continue;
+        const float *const ui = u + img * img_stride;
+        const __nv_bfloat16 *const vi = v + (static_cast<long long>(img) * h * w + x) * kC + grp * 8;
+        const float sg = constant ? sigma[img] : 0.0f;
+        auto at = [&](int yy, int xx) {
+            const bool ok = yy >= 0 && yy < h && xx >= 0 && xx < w;
+            return !ok ? 0.0f : constant ? sg : __ldg(ui + yy * stride + xx);
+        };
+        unsigned long long win[3][3];  // rows y - 1 .. y + 1, columns x - 1 .. x + 1
 #pragma unroll
-    for (int i = 0; i < 72; ++i) acc[i] = 0.0f;
-    float bacc = 0.0f;
-    const int per_block = blockDim.x / 6;
-    if (static_cast<int>(threadIdx.x) < per_block * 6) {
-        for (long long q = blockIdx.x * static_cast<long long>(per_block) + threadIdx.x / 6; q < total;
-             q += static_cast<long long>(gridDim.x) * per_block) {
-            // X7[q] reaches dOut[q - (t - 1)] through tap t
-            const int img = static_cast<int>(q / (static_cast<long long>(h) * w));
-            const int r = static_cast<int>(q - static_cast<long long>(img) * h * w);
-            const int y = r / w, x = r - y * w;
-            const uint4 u = reinterpret_cast<const uint4 *>(x7 + q * kC)[grp];
-            float xv[8];
-            const unsigned wd[4] = {u.x, u.y, u.z, u.w};
+        for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                xv[2 * k] = __uint_as_float(wd[k] << 16);
-                xv[2 * k + 1] = __uint_as_float(wd[k] & 0xffff0000u);
+            for (int i = 0; i < 3; ++i) {
+                const float f = at(y0 - 1 + j, x - 1 + i);
+                win[j][i] = f2pack(f, f);
+            }
+        const int yend = min(y0 + kEdgeRows, h);
+        for (int y = y0; y < yend; y += kEdgeAhead) {
+            uint4 rows[kEdgeAhead];
+            float below[kEdgeAhead][3];
+#pragma unroll
+            for (int r = 0; r < kEdgeAhead; ++r) {
+                rows[r] = y + r < yend ? __ldg(reinterpret_cast<const uint4 *>(
+                                             vi + static_cast<long long>(y + r) * w * kC))
+                                       : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) below[r][i] = at(y + r + 1, x - 1 + i);
             }
 #pragma unroll
-            for (int t = 0; t < 9; ++t) {
-                const int yy = y - (t / 3 - 1), xx = x - (t % 3 - 1);
-                const bool ok = yy >= 0 && yy < h && xx >= 0 && xx < w;
-                const float d = ok ? dout[(static_cast<long long>(img) * h + yy) * w + xx] : 0.0f;
+            for (int r = 0; r < kEdgeAhead; ++r) {
+                if (y + r >= yend) break;
 #pragma unroll
-                for (int k = 0; k < 8; ++k) acc[t * 8 + k] += d * xv[k];
+                for (int i = 0; i < 3; ++i) win[2][i] = f2pack(below[r][i], below[r][i]);
+                unsigned long long xv[4];
+                unpack_bf16x8(rows[r], xv);
+#pragma unroll
+                for (int t = 0; t < 9; ++t) {
+                    const unsigned long long ut = REVERSE ? win[2 - t / 3][2 - t % 3] : win[t / 3][t % 3];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) e.dw[t][k] = ffma2(xv[k], ut, e.dw[t][k]);
+                }
+                if (REVERSE) {
+                    float lo, hi;
+                    f2unpack(win[1][1], lo, hi);
+                    e.u += lo;
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) e.v[k] = ffma2(xv[k], one, e.v[k]);
+                }
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) win[j][i] = win[j + 1][i];
             }
-            if (grp == 0) bacc += dout[q];
         }
-#pragma unroll
-        for (int t = 0; t < 9; ++t)
-#pragma unroll
-            for (int k = 0; k < 8; ++k) atomicAdd(&red[(grp * 8 + k) * 9 + t], acc[t * 8 + k]);
-        if (grp == 0) atomicAdd(&red[kW8], bacc);
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < kW8Partial; i += blockDim.x)
-        partial[static_cast<long long>(blockIdx.x) * kW8Partial + i] = red[i];
 }
 
-// Weight and bias gradients of layer 1: dW1[co][cin][t] = sum_p G1[p][co] In_cin[p + t - 1],
-// db1[co] = sum_p G1[p][co]; one thread per (pixel, 4-channel group).
-constexpr int kW1Partial = kW1 + kC;
-
-__global__ void __launch_bounds__(240) wgrad_in_kernel(const InArgs a, const __nv_bfloat16 *g1,
-                                                        float *partial)
+// Sum over a warp's five columns, in lanes 0..5 (lanes 30, 31 hold none; with
+// shared atomics for the block's sums the kernels took 73 and 44 us).
+__device__ __forceinline__ float column_sum(float v)
 {
-    __shared__ float red[kW1Partial];
-    for (int i = threadIdx.x; i < kW1Partial; i += blockDim.x) red[i] = 0.0f;
-    __syncthreads();
-    const long long total = static_cast<long long>(a.n) * a.h * a.w;
-    const int grp = threadIdx.x % 12;  // 4-channel group
-    float acc[72], bacc[4];
+    return v + __shfl_down_sync(0xffffffffu, v, 6) + __shfl_down_sync(0xffffffffu, v, 12) +
+           __shfl_down_sync(0xffffffffu, v, 18) + __shfl_down_sync(0xffffffffu, v, 24);
+}
+
+constexpr int kEdgeWarps = kEdgeThreads / 32;
+
+__global__ void __launch_bounds__(kEdgeThreads, 2) wgrad_out_kernel(const __nv_bfloat16 *x7,
+                                                                    const float *dout, int n, int h,
+                                                                    int w, float *partial)
+{
+    __shared__ float red[kEdgeWarps][kW8Partial];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane % 6, col = lane / 6;
+    EdgeSums e = {};
+    if (col < kEdgeCols)
+        edge_sums<true>(x7, dout, w, static_cast<long long>(h) * w, nullptr, false, n, h, w,
+                        blockIdx.x * kEdgeWarps + warp, gridDim.x * kEdgeWarps, grp, col, e);
+    __syncwarp();
 #pragma unroll
-    for (int i = 0; i < 72; ++i) acc[i] = 0.0f;
+    for (int t = 0; t < 9; ++t)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) bacc[i] = 0.0f;
-    const int per_block = blockDim.x / 12;
-    for (long long p = blockIdx.x * static_cast<long long>(per_block) + threadIdx.x / 12; p < total;
-         p += static_cast<long long>(gridDim.x) * per_block) {
-        const int img = static_cast<int>(p / (static_cast<long long>(a.h) * a.w));
-        const int r = static_cast<int>(p - static_cast<long long>(img) * a.h * a.w);
-        const int y = r / a.w, x = r - y * a.w;
-        const uint2 u = reinterpret_cast<const uint2 *>(g1 + p * kC)[grp];
-        const float gv[4] = {__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u),
-                             __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u)};
-        const float s = a.sigma[img];
-#pragma unroll
-        for (int t = 0; t < 9; ++t) {
-            const int yy = y + t / 3 - 1, xx = x + t % 3 - 1;
-            const bool ok = yy >= 0 && yy < a.h && xx >= 0 && xx < a.w;
-            const float nv = ok ? __ldg(a.in + img * a.img_stride + yy * a.stride + xx) : 0.0f;
-            const float sv = ok ? s : 0.0f;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                acc[(k * 2 + 0) * 9 + t] += gv[k] * nv;
-                acc[(k * 2 + 1) * 9 + t] += gv[k] * sv;
+        for (int k = 0; k < 4; ++k) {
+            float lo, hi;
+            f2unpack(e.dw[t][k], lo, hi);
+            lo = column_sum(lo);
+            hi = column_sum(hi);
+            if (lane < 6) {
+                red[warp][(grp * 8 + 2 * k) * 9 + t] = lo;
+                red[warp][(grp * 8 + 2 * k + 1) * 9 + t] = hi;
             }
         }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) bacc[k] += gv[k];
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-#pragma unroll
-        for (int i = 0; i < 18; ++i) atomicAdd(&red[(grp * 4 + k) * 18 + i], acc[k * 18 + i]);
-        atomicAdd(&red[kW1 + grp * 4 + k], bacc[k]);
-    }
+    const float db = column_sum(e.u);
+    if (lane == 0) red[warp][kW8] = db;
     __syncthreads();
-    for (int i = threadIdx.x; i < kW1Partial; i += blockDim.x)
-        partial[static_cast<long long>(blockIdx.x) * kW1Partial + i] = red[i];
+    for (int i = threadIdx.x; i < kW8Partial; i += blockDim.x) {
+        float sum = 0.0f;
+#pragma unroll
+        for (int q = 0; q < kEdgeWarps; ++q) sum += red[q][i];
+        partial[static_cast<long long>(blockIdx.x) * kW8Partial + i] = sum;
+    }
+}
+
+// Even blocks take the noisy plane (and the bias), odd ones the noise-level plane.
+__global__ void __launch_bounds__(kEdgeThreads, 2) wgrad_in_kernel(const InArgs a, const __nv_bfloat16 *g1,
+                                                                   float *partial)
+{
+    __shared__ float red[kEdgeWarps][kC * 10];  // [channel][nine taps, V]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane % 6, col = lane / 6;
+    const int cin = blockIdx.x & 1;
+    EdgeSums e = {};
+    if (col < kEdgeCols)
+        edge_sums<false>(g1, a.in, a.stride, a.img_stride, a.sigma, cin == 1, a.n, a.h, a.w,
+                         (blockIdx.x >> 1) * kEdgeWarps + warp, (gridDim.x >> 1) * kEdgeWarps, grp, col, e);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int t = 0; t < 10; ++t) {
+            float lo, hi;
+            f2unpack(t < 9 ? e.dw[t < 9 ? t : 0][k] : e.v[k], lo, hi);
+            lo = column_sum(lo);
+            hi = column_sum(hi);
+            if (lane < 6) {
+                red[warp][(grp * 8 + 2 * k) * 10 + t] = lo;
+                red[warp][(grp * 8 + 2 * k + 1) * 10 + t] = hi;
+            }
+        }
+    __syncthreads();
+    float *const out = partial + static_cast<long long>(blockIdx.x) * kW1Partial;
+    for (int i = threadIdx.x; i < kC * 10; i += blockDim.x) {
+        const int c = i / 10, t = i - c * 10;
+        float sum = 0.0f;
+#pragma unroll
+        for (int q = 0; q < kEdgeWarps; ++q) sum += red[q][i];
+        if (t < 9) {
+            out[(c * 2 + cin) * 9 + t] = sum;
+            out[(c * 2 + (cin ^ 1)) * 9 + t] = 0.0f;
+        } else {
+            out[kW1 + c] = cin == 0 ? sum : 0.0f;
+        }
+    }
 }
 
 // Packs the six 48 -> 48 layers' FP32 weights [co][ci][ky][kx] into the
