@@ -534,6 +534,18 @@ static SmemPlan plan_tile(StageArgs<T> &a, const bm3d_stage_params *p, bool wien
                         !fast_args(BS, p->group_size), BS, p->group_size, a.tile_x * a.tile_y);
 }
 
+// Whether a stage is over the limit on window and list sizes (stage_limit_bytes)
+// at its smallest tile.
+template <typename T>
+static bool over_limit(const bm3d_ctx *ctx, const StageArgs<T> &a, const bm3d_stage_params *p, bool wiener,
+                       int nplanes)
+{
+    const int reach = a.match ? a.range : 0, BS = p->block_size;
+    return stage_limit_bytes<T>(nplanes, wiener, a.ref_alias_src, std::min(a.height, 2 * reach + BS),
+                                std::min(a.width, 2 * reach + BS), a.span,
+                                !fast_args(BS, p->group_size), BS, p->group_size, 1) > ctx->smem_optin;
+}
+
 // Predicted time of a stage at one tile shape (microseconds; only the order
 // matters). Fast profile: a warp takes 8.5 us for a reference block when its SM
 // runs few warps and 12 us with 16; about a third of it is matching, the rest
@@ -587,6 +599,10 @@ static int plan_geometry(bm3d_ctx *ctx, StageArgs<T> &a, const bm3d_stage_params
     a.nx = ref_count(width - BS, a.step);
     a.ny = ref_count(height - BS, a.step);
     a.span = 2 * (a.range / a.bm_step) + 1;
+    if (over_limit(ctx, a, p, wiener, nplanes)) {
+        ctx->err = "stage does not fit in shared memory";
+        return BM3D_ERR_UNSUPPORTED;
+    }
     // The launch bounds (register-resident 512 threads in FP32, 256 in FP64;
     // generic 384, and 256 in FP64 and for BlockSize 11) limit the warps; the
     // small shapes are for windows that leave no room for more.

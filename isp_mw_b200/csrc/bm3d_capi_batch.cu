@@ -197,6 +197,13 @@ int build_stage(bm3d_batch *B, bool wiener, int tx, int ty, int warps, StageBuil
         a.ny = ref_count(a.height - BS, a.step);
         a.span = 2 * (a.range / a.bm_step) + 1;
         const int reach = a.match ? a.range : 0;
+        const int least = generic ? 1 : 2;  // reference blocks of the smallest tile, each way
+        const int limit_w = (least - 1) * a.step + 2 * reach + BS;
+        if (stage_limit_bytes<float>(npl, wiener, wiener ? 0 : (1 << npl) - 1, std::min(a.height, limit_w),
+                                     std::min(a.width, limit_w), a.span, generic, BS, p->group_size,
+                                     std::min(least, a.nx) * std::min(least, a.ny)) + 16 >
+            ctx->smem_optin)
+            return BM3D_ERR_UNSUPPORTED;
         a.region_w = std::min(a.width, (tx - 1) * a.step + 2 * reach + BS);
         a.region_h = std::min(a.height, (ty - 1) * a.step + 2 * reach + BS);
         a.region_pitch = window_pitch(a.region_w);

@@ -409,10 +409,43 @@ __host__ __device__ inline SmemPlan plan_smem(int nplanes, bool wiener, int alia
     s.total = seq3 ? s.off_groups + static_cast<size_t>(tile_refs) * (2 * glist + 1)
                    : s.off_warps + s.warp_bytes * nwarps;
     // the task table's list places and offsets have 16 bits (a list of 256 x 256
-    // would not fit anyway)
+    // is over stage_limit_bytes)
     if (span > 255) s.total = ~size_t(0) >> 1;
     if (seq3 && (region_h > 255 || region_pitch > 255)) s.total = ~size_t(0) >> 1;  // too wide
     return s;
+}
+
+// Which stages are taken at all: those whose smallest tile (tile_refs reference
+// blocks in a region_h x region_w window, one warp) counts no more bytes here than
+// a CTA may have. Per window pixel and plane 16 bytes and those of the staged
+// windows, per list place 8 (FP64: 16), the group buffers and 1 KB a warp. The
+// kernels use less (plan_smem); the limit on BMrange, BlockSize and GroupSize is
+// part of the interface and does not move with their layouts.
+template <typename T>
+inline size_t stage_limit_bytes(int nplanes, bool wiener, int alias_mask, int region_h, int region_w,
+                                int span, bool generic, int bs, int gs, int tile_refs)
+{
+    const size_t refuse = ~size_t(0) >> 1;
+    const bool seq3 = nplanes == 3;
+    int windows = wiener ? 0 : (alias_mask & 1 ? 0 : 1);
+    if (seq3) nplanes = 1;
+    if (wiener)
+        for (int p = 0; p < nplanes; ++p) windows += (alias_mask >> p & 1) ? 0 : 1;
+    windows += nplanes;
+    const auto up = [](size_t v) { return (v + 15) / 16 * 16; };
+    const size_t pitch = region_w + (5 - region_w % 8 + 8) % 8, px = region_h * pitch;
+    const size_t bsq = static_cast<size_t>(bs) * bs, key = 2 * sizeof(T);
+    if (seq3 && (region_h > 255 || pitch > 255)) return refuse;
+    size_t bytes = up(px * sizeof(T)) * windows + up(px * 8) * 2 * nplanes;
+    bytes += up(sizeof(T) * bsq * windows);
+    bytes = up(bytes + 16 * bsq * nplanes);
+    const size_t group = generic ? sizeof(T) * gs * generic_block_stride(bs) *
+                                       (wiener && !generic_one_buffer<T>(wiener, bs) ? 2 : 1)
+                                 : sizeof(T) * kGSMax * kGroupStride;
+    const size_t list = key * (static_cast<size_t>(span) * span + 1);
+    bytes = up(bytes + up(up(group > list ? group : list) + (generic ? up(sizeof(T) * bsq) : 0) +
+                          key * kCand + (sizeof(BlockPos) + sizeof(T)) * kGSTab));
+    return seq3 ? bytes + static_cast<size_t>(tile_refs) * (2 * (generic ? gs : kGSMax) + 1) : bytes;
 }
 
 }  // namespace bm3d

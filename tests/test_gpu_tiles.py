@@ -78,3 +78,30 @@ def test_groups_of_up_to_32(bm3d_lib, oracle_mod, group_size, thmse, wiener):
     want = oracle_mod.backend("port", np.float32).stage(wiener, p.as_dict(), noisy, guide)
     want = want[1] if isinstance(want, tuple) else want
     assert np.abs(out - want).max() <= 1e-3
+
+
+# The limit on the search range does not move with the kernels' layouts: the
+# largest range taken and the next, by stage_limit_bytes' sum for these parameters
+# (one plane, fast profile, 1 x 1 tile: 20 B a window pixel and 8 B a list place;
+# batches: 2 x 2 tile). Whole images smaller than the window leave room for more.
+@pytest.mark.parametrize("shape,bm_range,ok", [((300, 310), 42, True), ((300, 310), 43, False),
+                                               ((40, 300), 60, True), ((40, 300), 90, False)])
+def test_search_range_limit(bm3d_lib, shape, bm_range, ok):
+    import torch
+    import isp_mw_b200
+    from isp_mw_b200 import synth
+    h, w = shape
+    src = torch.from_numpy(synth.pair(h, w, 20.0, 3)[1]).cuda()
+    p = isp_mw_b200.stage_params_default("fast", False, [30.0] * 3)
+    p.bm_range, p.block_step = bm_range, 32
+    dst = torch.zeros_like(src)
+    ctx = isp_mw_b200.Context(0)
+    if ok:
+        ctx.stage(p, False, dst, src)
+        ctx.check()
+        assert not torch.equal(dst, torch.zeros_like(dst))
+    else:
+        with pytest.raises(isp_mw_b200.BM3DError) as e:
+            ctx.stage(p, False, dst, src)
+        assert e.value.code == isp_mw_b200.BM3D_ERR_UNSUPPORTED
+    ctx.close()
