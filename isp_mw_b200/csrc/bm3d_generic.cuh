@@ -75,7 +75,7 @@ __device__ void dct_z_generic(T *G, int n, int bs, int lane, const T *tab, const
 // Separable 3-D transform of an n x bs x bs group (row-major [z][y][x]) with
 // the concatenated matrices `tab` (forward REDFT10 or backward REDFT01, as
 // `inverse` says): rows, columns, then the group axis. The row-fused block
-// sizes (rows_fused) do not come here: their rows are transformed as they are
+// sizes (8, and 11 in FP32) do not come here: their rows are transformed as they are
 // gathered or aggregated, their other passes in dct_cols_z_fwd /
 // dct_z_cols_inv.
 template <typename T>
@@ -104,13 +104,9 @@ __device__ void dct3_generic(T *G, int n, int bs, int lane, const T *tab, const 
     dct_z_generic(G, n, bs, lane, tab, pad, inverse);
 }
 
-// Row-fused block sizes: 8 (both precisions) and 11 (FP32, the "vn" final
-// stage). Rows are transformed in registers as they are gathered
-// (gather_rows) or aggregated (aggregate_rows); these run the other passes.
-template <typename T> __host__ __device__ constexpr bool rows_fused(int bs)
-{
-    return bs == 8 || (bs == 11 && sizeof(T) == 4);
-}
+// Row-fused block sizes: 8 and 11 (FP32, the "vn" final stage). Rows are
+// transformed in registers as they are gathered (gather_rows) or aggregated
+// (aggregate_rows); these run the other passes.
 
 // One line of BS points, in place, by the block size's butterflies or
 // constant-bank symmetric form.
@@ -558,16 +554,19 @@ __device__ void filter_generic(const StageArgs<T> &a, const Tile<T> &t, int p, c
     }
     const int bs = BSC > 0 ? BSC : t.bs, bsq = bs * bs, total = n * bsq;
     const int zs = generic_block_stride(bs), rs = generic_row_stride(bs);
+    // FP32's 8 and 11 have kernels of their own; FP64's 8 shares this one
+    const bool eight = sizeof(T) == 8 && bs == 8;
+    constexpr bool kEleven = BSC == 11;
     T denW;
-    if (bs == 8) {
+    if (eight) {
         gather_rows<T, 8>(t, t.srcw[p], t.src0[p], list, n, lane, Gs, &n_bad);
         if (WIENER)
             gather_rows<T, 8>(t, t.refw[p], t.ref0[p], list, n, lane, Gr,
                               static_cast<unsigned *>(nullptr));
         __syncwarp();
         dct_cols_z_fwd<T, 8>(Gs, n, lane, a.dct_fwd, a.pad_fwd);
-    } else if (rows_fused<T>(bs)) {  // 11, FP32
-        if constexpr (sizeof(T) == 4) {
+    } else if (kEleven) {
+        if constexpr (kEleven) {
             gather_rows<T, 11>(t, t.srcw[p], t.src0[p], list, n, lane, Gs, &n_bad);
             if (WIENER)
                 gather_rows<T, 11>(t, t.refw[p], t.ref0[p], list, n, lane, Gr,
@@ -612,9 +611,9 @@ __device__ void filter_generic(const StageArgs<T> &a, const Tile<T> &t, int p, c
         const int retained = __reduce_add_sync(0xffffffffu, kept);
         denW = retained < 1 ? T(1) : T(1) / static_cast<T>(retained);
     } else {
-        if (bs == 8) dct_cols_z_fwd<T, 8>(Gr, n, lane, a.dct_fwd, a.pad_fwd);
-        else if (rows_fused<T>(bs)) {
-            if constexpr (sizeof(T) == 4) dct_cols_z_fwd<T, 11>(Gr, n, lane, a.dct_fwd, a.pad_fwd);
+        if (eight) dct_cols_z_fwd<T, 8>(Gr, n, lane, a.dct_fwd, a.pad_fwd);
+        else if (kEleven) {
+            if constexpr (kEleven) dct_cols_z_fwd<T, 11>(Gr, n, lane, a.dct_fwd, a.pad_fwd);
         } else {
             dct3_generic(Gr, n, bs, lane, a.dct_fwd, a.pad_fwd, false);
         }
@@ -622,7 +621,7 @@ __device__ void filter_generic(const StageArgs<T> &a, const Tile<T> &t, int p, c
         T l2 = T(0);
         for (int e = lane; e < total; e += kWarp) {
             // any one-to-one order works here; the padded layout needs its address
-            const int g = bs == 8 ? (e >> 6) * 72 + ((e >> 3) & 7) * 9 + (e & 7) : e;
+            const int g = eight ? (e >> 6) * 72 + ((e >> 3) & 7) * 9 + (e & 7) : e;
             const T y2 = Gr[g] * Gr[g];
             const T w = wiener_weight(y2, s2);
             Gs[g] *= w;
@@ -633,19 +632,17 @@ __device__ void filter_generic(const StageArgs<T> &a, const Tile<T> &t, int p, c
     }
     const T numW = static_cast<T>(static_cast<double>(denW) / a.finalAMP[n - 1]);
     __syncwarp();
-    if (bs == 8) {
+    if (eight) {
         dct_z_cols_inv<T, 8>(Gs, n, lane, a.dct_inv, a.pad_inv);
         aggregate_rows<T, 8>(a, t, p, pt, list, n, lane, Gs, numW, denW, scale, check);
         __syncwarp();
         return;
     }
-    if constexpr (sizeof(T) == 4) {
-        if (bs == 11) {
-            dct_z_cols_inv<T, 11>(Gs, n, lane, a.dct_inv, a.pad_inv);
-            aggregate_rows<T, 11>(a, t, p, pt, list, n, lane, Gs, numW, denW, scale, check);
-            __syncwarp();
-            return;
-        }
+    if constexpr (kEleven) {
+        dct_z_cols_inv<T, 11>(Gs, n, lane, a.dct_inv, a.pad_inv);
+        aggregate_rows<T, 11>(a, t, p, pt, list, n, lane, Gs, numW, denW, scale, check);
+        __syncwarp();
+        return;
     }
     dct3_generic(Gs, n, bs, lane, a.dct_inv, a.pad_inv, true);
     // the block weight once per block, at its origin (as the register-resident kernel)

@@ -31,12 +31,10 @@ namespace pilot {
 
 constexpr int kC = 48;                          // hidden channels
 constexpr int kTX = 16, kTY = 8;                // output tile (128 pixels)
-constexpr int kColBytes = kTY * kC * 2;         // 768: one column of 8 rows (gradient tile)
 constexpr int kHaloRows = kTY + 2;              // 10 input rows per column
 constexpr int kGroupBytes = kHaloRows * 16;     // 160: one 8-channel group of a halo column
 constexpr int kHaloColBytes = 6 * kGroupBytes;  // 960: one halo column
 constexpr int kCols = kTX + 2;                  // 18 input columns
-constexpr int kCopyBytes = kCols * kColBytes;   // 13824: gradient tile incl. two slack columns
 constexpr int kTileBytes = kCols * kHaloColBytes;  // 17280: the input tile with its halo
 constexpr int kTileChunks = kTileBytes / 16;    // 1080 16-byte chunks
 constexpr int kTapBytes = kC * kC * 2;          // 4608: one tap, [co / 8][ci / 8][co % 8][ci % 8]
