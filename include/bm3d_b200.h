@@ -37,8 +37,8 @@ enum {
      * copied to dst unchanged, as source/BM3D.cpp:82-87 and 143-151 do. */
     BM3D_COPIED = 1,
     BM3D_ERR_INVALID = -1,     /* null pointer, width/height < BlockSize, stride < width, ... */
-    BM3D_ERR_UNSUPPORTED = -2, /* valid in the reference but not built here: BlockSize > 16 or
-                                  GroupSize > 32 */
+    BM3D_ERR_UNSUPPORTED = -2, /* valid in the reference but not built here: BlockSize > 16,
+                                  GroupSize > 32, or a search window over a CTA's shared memory */
     BM3D_ERR_CUDA = -3,        /* CUDA runtime error (message via bm3d_last_error) */
     BM3D_ERR_NOMEM = -4,       /* device allocation failed */
     BM3D_ERR_TOO_LARGE = -5    /* plane exceeds bm3d_stage_noalloc's static scratch */
@@ -285,7 +285,7 @@ int bm3d_noalloc_check(void *stream);
  * with width[i] x height[i] and row pitch stride[i]. With `autotune` the
  * tile shape and warps per CTA of each stage are picked by timing candidate
  * configurations on this batch. Results equal per-plane bm3d_full bit for bit.
- * The batch keeps its own device buffers (16 B per pixel of accumulators and
+ * The batch keeps its own device buffers (24 B per pixel of accumulators and
  * the basic estimates) until bm3d_batch_destroy. Replaces looping the
  * reference's BM3D over images (no batched form exists there). */
 typedef struct bm3d_batch bm3d_batch;
@@ -482,8 +482,9 @@ int bm3d_pilot_wgrad48(bm3d_ctx *ctx, int n, int h, int w, const void *x, const 
  * counterpart in the reference, which exits on allocation failure. */
 int bm3d_inject_alloc_failures(int count);
 
-/* Tile shape used by the stage kernels: reference blocks per CTA tile
- * (tile_x x tile_y) and warps per CTA. 0 keeps the current value. */
+/* Fixes the tile shape of the stage kernels (BlockSize 8, GroupSize <= 16):
+ * reference blocks per CTA tile (tile_x x tile_y) and warps per CTA. 0 keeps the
+ * current value. Without it each call picks the shape from its sizes. */
 int bm3d_set_tiling(bm3d_ctx *ctx, int tile_x, int tile_y, int warps);
 
 #ifdef __cplusplus
