@@ -403,9 +403,10 @@ __host__ __device__ inline SmemPlan plan_smem(int nplanes, bool wiener, int alia
     s.off_keys = s.off_heap + up(heap_bytes > ref_bytes ? heap_bytes : ref_bytes);
     const size_t match_bytes = s.off_keys + sizeof(T) * kGSTab;
     s.off_list = up(group_bytes > match_bytes ? group_bytes : match_bytes);
-    s.warp_bytes = s.off_list + up(sizeof(BlockPos) * (gs > 1 ? gs : 1));
+    // (the register-resident layout is one for every GroupSize: its kernel does not pass gs)
+    const int glist = generic ? (gs > 1 ? gs : 1) : kGSMax;  // group-list entries
+    s.warp_bytes = s.off_list + up(sizeof(BlockPos) * glist);
     s.off_groups = (s.off_warps + s.warp_bytes * nwarps + 15) / 16 * 16;
-    const int glist = generic ? gs : kGSMax;  // group-list entries per reference block
     s.total = seq3 ? s.off_groups + static_cast<size_t>(tile_refs) * (2 * glist + 1)
                    : s.off_warps + s.warp_bytes * nwarps;
     // the task table's list places and offsets have 16 bits (a list of 256 x 256
