@@ -216,6 +216,12 @@ long long bm3d_ref_block_count(const bm3d_stage_params *params, int width, int h
 int bm3d_debug_groups(bm3d_ctx *ctx, const bm3d_stage_params *params, int wiener, const float *ref,
                       int width, int height, size_t stride, float value_range, int *counts,
                       int *pos_yx, float *keys);
+/* The same without the keys, by the matching that the stages themselves run:
+ * FP32 stages decide by approximate distances where these are enough, and the
+ * keys of bm3d_debug_groups need exact ones throughout. */
+int bm3d_debug_positions(bm3d_ctx *ctx, const bm3d_stage_params *params, int wiener,
+                         const float *ref, int width, int height, size_t stride,
+                         float value_range, int *counts, int *pos_yx);
 
 /* Counters of the last stage run on this context: out[0] = sum of group
  * sizes, out[1] = sum of squared group sizes, out[2] = candidate blocks

@@ -37,6 +37,7 @@ EXPORTS = [
     "bm3d_stage_params_default", "bm3d_stage_params_thmse_default", "bm3d_ctx_create",
     "bm3d_ctx_destroy", "bm3d_last_error", "bm3d_stage", "bm3d_stage3", "bm3d_full",
     "bm3d_full3", "bm3d_stage_f64", "bm3d_ref_block_count", "bm3d_debug_groups",
+    "bm3d_debug_positions",
     "bm3d_last_stats", "bm3d_check", "bm3d_batch_check", "bm3d_set_tiling", "bm3d_set_kernel_timing", "bm3d_kernel_time",
     "bm3d_stage_noalloc", "bm3d_noalloc_check", "bm3d_batch_create", "bm3d_batch_run", "bm3d_batch_tuning",
     "bm3d_batch_destroy", "bm3d_plane_int", "bm3d_stage_int", "bm3d_frame", "bm3d_stage_frame",
@@ -122,6 +123,8 @@ def load_library(path: str = LIB_PATH) -> ctypes.CDLL:
                                    ctypes.c_double, ip, vp]
     lib.bm3d_ref_block_count.argtypes = [sp, ip, ip]
     lib.bm3d_ref_block_count.restype = ctypes.c_longlong
+    lib.bm3d_debug_positions.argtypes = [vp, sp, ip, vp, ip, ip, ctypes.c_size_t, ctypes.c_float,
+                                         vp, vp]
     lib.bm3d_debug_groups.argtypes = [vp, sp, ip, vp, ip, ip, ctypes.c_size_t, ctypes.c_float,
                                       vp, vp, vp]
     lib.bm3d_last_stats.argtypes = [vp, ctypes.POINTER(ctypes.c_ulonglong)]
@@ -416,6 +419,20 @@ class Context:
                                         counts.ctypes.data, pos.ctypes.data, keys.ctypes.data)
         self._check(rc, allow_copied=False)
         return counts, pos, keys
+
+    def debug_positions(self, params: StageParams, wiener: bool, ref: np.ndarray,
+                        value_range: float = 1.0):
+        """(counts[R], pos[R, 32, 2]) as the stages themselves match (``bm3d_debug_positions``)."""
+        ref = np.ascontiguousarray(ref, dtype=np.float32)
+        h, w = ref.shape
+        n = self.ref_block_count(params, w, h)
+        counts = np.zeros(n, np.int32)
+        pos = np.full((n, GROUP_STRIDE, 2), -1, np.int32)
+        rc = self.lib.bm3d_debug_positions(self.h, ctypes.byref(params), int(wiener),
+                                           ref.ctypes.data, w, h, w, value_range,
+                                           counts.ctypes.data, pos.ctypes.data)
+        self._check(rc, allow_copied=False)
+        return counts, pos
 
     def set_kernel_timing(self, on: bool):
         self._check(self.lib.bm3d_set_kernel_timing(self.h, int(on)))

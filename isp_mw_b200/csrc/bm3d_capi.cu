@@ -384,6 +384,30 @@ Guard bm3d::check_params(const bm3d_stage_params *p, int nplanes)
     return Guard::Run;
 }
 
+// The distances whose keys (key_from_dist) are normal, as bits: the least and the
+// greatest that approximate matching may rank (DistBits, select_once); keys grow
+// with the distance. None: low above high.
+static void near_range(double mul, unsigned &low, unsigned &high)
+{
+    using DB = DistBits<float>;
+    auto value = [](unsigned bits) {
+        float f;
+        std::memcpy(&f, &bits, sizeof(f));
+        return f;
+    };
+    auto first = [&](auto reached) {  // the first distance that `reached` holds for
+        unsigned lo = 0, hi = 0x7f800000u;
+        while (lo < hi) {
+            const unsigned mid = lo + (hi - lo) / 2;
+            if (reached(static_cast<float>(static_cast<double>(value(mid)) * mul))) hi = mid;
+            else lo = mid + 1;
+        }
+        return lo;
+    };
+    low = std::max(DB::kTiny, first([&](float key) { return key >= value(DB::kLow); }));
+    high = first([&](float key) { return key > value(DB::kHigh); }) - 1;
+}
+
 template <typename T>
 void bm3d::fill_tables(StageArgs<T> &a, const bm3d_stage_params *p, bool wiener, int nplanes,
                        double value_range)
@@ -417,6 +441,7 @@ void bm3d::fill_tables(StageArgs<T> &a, const bm3d_stage_params *p, bool wiener,
     const double MSE2SSE = static_cast<double>(BS * BS) * range * range / double(255 * 255);
     a.distMul = double(1) / MSE2SSE;
     a.thSSE = static_cast<T>(thMSE * MSE2SSE);
+    near_range(a.distMul, a.near_low, a.near_high);
     a.match = (GS == 1 || thMSE <= 0) ? 0 : 1;
 }
 
@@ -1039,11 +1064,12 @@ template int bm3d::full_any<float>(bm3d_ctx *, const bm3d_stage_params *, const 
                              int, float *const[], const float *const[], const float *const[],
                              int, int, size_t, double, int, void *);
 
-extern "C" int bm3d_debug_groups(bm3d_ctx *ctx, const bm3d_stage_params *p, int wiener,
-                                 const float *ref, int width, int height, size_t stride,
-                                 float value_range, int *counts, int *pos_yx, float *keys)
+// The groups of every reference block; keys may be null.
+static int dump_groups(bm3d_ctx *ctx, const bm3d_stage_params *p, int wiener, const float *ref,
+                       int width, int height, size_t stride, float value_range, int *counts,
+                       int *pos_yx, float *keys)
 {
-    if (!ctx || !p || !ref || !counts || !pos_yx || !keys) return BM3D_ERR_INVALID;
+    if (!ctx || !p || !ref || !counts || !pos_yx) return BM3D_ERR_INVALID;
     const Guard g = check_params(p, 1);
     if (g == Guard::Invalid || g == Guard::Copy) return BM3D_ERR_INVALID;
     if (g == Guard::Unsupported) return BM3D_ERR_UNSUPPORTED;
@@ -1056,7 +1082,7 @@ extern "C" int bm3d_debug_groups(bm3d_ctx *ctx, const bm3d_stage_params *p, int 
     if ((rc = ensure(ctx, ctx->stage_in[0], plane_bytes)) != BM3D_OK) return rc;
     if ((rc = ensure(ctx, ctx->groups[0], sizeof(int) * nref)) != BM3D_OK) return rc;
     if ((rc = ensure(ctx, ctx->groups[1], sizeof(int) * nref * kGSTab * 2)) != BM3D_OK) return rc;
-    if ((rc = ensure(ctx, ctx->groups[2], sizeof(float) * nref * kGSTab)) != BM3D_OK) return rc;
+    if (keys && (rc = ensure(ctx, ctx->groups[2], sizeof(float) * nref * kGSTab)) != BM3D_OK) return rc;
     cudaStream_t s = nullptr;
     float *in = static_cast<float *>(ctx->stage_in[0].ptr);
     if ((rc = copy_plane(ctx, in, width, ref, stride, width, height, cudaMemcpyHostToDevice, s)) !=
@@ -1067,15 +1093,31 @@ extern "C" int bm3d_debug_groups(bm3d_ctx *ctx, const bm3d_stage_params *p, int 
     rc = run_stage_device<float>(ctx, p, wiener != 0, 1, d, sp, sp, width, height, width,
                                  value_range, s, Chain::None, static_cast<int *>(ctx->groups[0].ptr),
                                  static_cast<int *>(ctx->groups[1].ptr),
-                                 static_cast<float *>(ctx->groups[2].ptr), true);
+                                 keys ? static_cast<float *>(ctx->groups[2].ptr) : nullptr, true);
     if (rc != BM3D_OK) return rc;
     CK(ctx, cudaMemcpyAsync(counts, ctx->groups[0].ptr, sizeof(int) * nref, cudaMemcpyDeviceToHost, s));
     CK(ctx, cudaMemcpyAsync(pos_yx, ctx->groups[1].ptr, sizeof(int) * nref * kGSTab * 2,
                             cudaMemcpyDeviceToHost, s));
-    CK(ctx, cudaMemcpyAsync(keys, ctx->groups[2].ptr, sizeof(float) * nref * kGSTab,
-                            cudaMemcpyDeviceToHost, s));
+    if (keys)
+        CK(ctx, cudaMemcpyAsync(keys, ctx->groups[2].ptr, sizeof(float) * nref * kGSTab,
+                                cudaMemcpyDeviceToHost, s));
     CK(ctx, cudaStreamSynchronize(s));
     return BM3D_OK;
+}
+
+extern "C" int bm3d_debug_groups(bm3d_ctx *ctx, const bm3d_stage_params *p, int wiener,
+                                 const float *ref, int width, int height, size_t stride,
+                                 float value_range, int *counts, int *pos_yx, float *keys)
+{
+    if (!keys) return BM3D_ERR_INVALID;
+    return dump_groups(ctx, p, wiener, ref, width, height, stride, value_range, counts, pos_yx, keys);
+}
+
+extern "C" int bm3d_debug_positions(bm3d_ctx *ctx, const bm3d_stage_params *p, int wiener,
+                                    const float *ref, int width, int height, size_t stride,
+                                    float value_range, int *counts, int *pos_yx)
+{
+    return dump_groups(ctx, p, wiener, ref, width, height, stride, value_range, counts, pos_yx, nullptr);
 }
 
 extern "C" int bm3d_set_kernel_timing(bm3d_ctx *ctx, int on)

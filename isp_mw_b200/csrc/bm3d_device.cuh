@@ -270,6 +270,7 @@ template <typename T> struct StageArgs {
     int ref_alias_src;          // bit p set: ref[p] == src[p], stage once
     T thSSE;                    // FLType(thMSE * MSE2SSE)      (include/Block.h:582-584)
     double distMul;             // 1 / MSE2SSE
+    unsigned near_low, near_high;  // FP32 distances (bits) that approximate matching may rank
     T thr[kMaxPlanes][kGSTab][4];  // hard thresholds by (#zero indices) (source/BM3D.cpp:35-68)
     T wss[kMaxPlanes][kGSTab];     // wienerSigmaSqr                     (source/BM3D.cpp:31)
     double finalAMP[kGSTab];       // 2n * 2BS * 2BS                     (source/BM3D.cpp:26)

@@ -426,6 +426,7 @@ template <typename T> struct Search {
     int group_size;
     double dist_mul;
     typename DistBits<T>::type limit;  // the matching threshold (dist_limit)
+    unsigned near_low, near_high;      // StageArgs'
     typename DistBits<T>::type *dist;
     SortKey<T> *heap;
     BlockPos *list;
@@ -494,7 +495,9 @@ template <typename T> __device__ __forceinline__ typename DistBits<T>::type dist
 // kNear above `limit`. The cut then leaves that much more room, and the
 // approximate order stands when no kept distance is within kNear of the next;
 // else exact_dist gives the compacted ones'. Returns -1 where the whole list has to be exact: a distance
-// at the matching threshold, ties, ranges where the bounds do not hold.
+// at the matching threshold, ties, ranges where the bounds do not hold -- keys that
+// are subnormal or zero tie at distances far apart, so every compacted distance has
+// to lie in near_low .. near_high, not the cut's bound alone.
 template <typename T, bool NEAR, int BS>
 __device__ __forceinline__ int select_once(const Search<T> &e, bool near, int lane, int nvalid,
                                            unsigned &n_fix)
@@ -622,7 +625,8 @@ __device__ __forceinline__ int select_once(const Search<T> &e, bool near, int la
             scan();
         }
         if (NEAR && near) {
-            if (!sure || limit < DB::kTiny) return -1;
+            // (a cut that keeps all of them leaves them below the threshold)
+            if (!sure || limit < DB::kTiny || (cut == none - 1 && limit > e.near_high)) return -1;
             // a distance too close to the threshold to tell matters when it can be
             // kept, or when the group takes every accepted one; either way the cut
             // is up there
@@ -673,7 +677,7 @@ __device__ __forceinline__ int select_once(const Search<T> &e, bool near, int la
                              (s1 == none || n1 == none || n1 - s1 <= kNear);
                 }
                 ranked = !__any_sync(0xffffffffu, close);
-                if (__any_sync(0xffffffffu, v0.key_bits() < DB::kTiny || v1.key_bits() < DB::kTiny))
+                if (__any_sync(0xffffffffu, v0.key_bits() < e.near_low || v1.key_bits() < e.near_low))
                     return -1;
                 if (!ranked) {
                     if (lane < M) v0 = K::pack(exact_dist<T, BS>(e, static_cast<int>(v0.idx())), v0.idx());
@@ -1079,6 +1083,8 @@ __device__ int match_block(const StageArgs<T> &a, const Tile<T> &t, int j0, int 
     e.group_size = a.group_size;
     e.dist_mul = a.distMul;
     e.limit = limit;
+    e.near_low = a.near_low;
+    e.near_high = a.near_high;
     e.dist = dist;
     e.heap = heap;
     e.list = list;
@@ -1582,7 +1588,7 @@ __device__ __forceinline__ void dump_group(const StageArgs<T> &a, int ky, int kx
     for (int k = lane; k < n; k += kWarp) {
         a.group_pos[(ridx * kGSTab + k) * 2 + 0] = list[k].y;
         a.group_pos[(ridx * kGSTab + k) * 2 + 1] = list[k].x;
-        a.group_key[ridx * kGSTab + k] = lkeys[k];
+        if (a.group_key != nullptr) a.group_key[ridx * kGSTab + k] = lkeys[k];
     }
     __syncwarp();  // the keys' bytes become the group buffer
 }
