@@ -771,7 +771,8 @@ static int run_stage_device(bm3d_ctx *ctx, const bm3d_stage_params *p, bool wien
             if (njobs == 1) q.stats = ctx->stats;
         }
     }
-    if (!bm_only && !follows) {
+    // (njobs 0: noise levels that are not numbers pass the guard and select no plane)
+    if (!bm_only && !follows && njobs > 0) {
         prep_kernel<T><<<dim3(std::min(height, blocks), njobs), threads, 0, s>>>(jobs);
         CK(ctx, cudaGetLastError());
     }
@@ -781,7 +782,7 @@ static int run_stage_device(bm3d_ctx *ctx, const bm3d_stage_params *p, bool wien
     a.bm_only = bm_only ? 1 : 0;
     if ((rc = launch_stage(ctx, a, wiener, nplanes, s, warps)) != BM3D_OK) return rc;
     ctx->last_stream = s;
-    if (bm_only) return BM3D_OK;
+    if (bm_only || njobs == 0) return BM3D_OK;
     normalize_kernel<T><<<dim3(normalize_tiles<T>(width, height), njobs), 256, 0, s>>>(jobs);
     CK(ctx, cudaGetLastError());
     return BM3D_OK;
@@ -1005,8 +1006,12 @@ int bm3d::full_any(bm3d_ctx *ctx, const bm3d_stage_params *basic, const bm3d_sta
     // passes prepare the final stage
     bool chained = std::is_same<typename AccOf<T>::type, long long>::value && gb == Guard::Run &&
                    gf == Guard::Run;
-    for (int c = 0; c < nplanes; ++c)
+    bool any = false;  // (the passes that prepare run on planes that are filtered)
+    for (int c = 0; c < nplanes; ++c) {
         chained = chained && filtered(basic, gb, c) == filtered(fin, gf, c);
+        any = any || filtered(basic, gb, c);
+    }
+    chained = chained && any;
     if ((rc = refused(gb)) != BM3D_OK) return rc;
     if (gb == Guard::Run) {
         rc = run_stage_device(ctx, basic, false, nplanes, tmp, ds, dr, width, height, dpitch,

@@ -48,3 +48,31 @@ def test_combined_equals_stages(bm3d_lib, profile, kind, sigma):
             ctx.stage(f, True, want1, src[0], est1)
             assert same(got1, want1)
     ctx.close()
+
+
+def test_no_plane_to_filter(bm3d_lib):
+    """Noise levels that are no numbers pass the parameter guard and select no
+    plane: the combined call copies, a stage leaves dst alone, in batches too."""
+    import torch
+    import isp_mw_b200
+    ctx = isp_mw_b200.Context(0)
+    b = isp_mw_b200.stage_params_default("fast", False, [30.0] * 3)
+    f = isp_mw_b200.stage_params_default("fast", True, [30.0] * 3)
+    for p in (b, f):
+        p.sigma[0], p.sigma[1], p.sigma[2] = float("nan"), 0.0, float("nan")
+    src = _planes(3, 40, 61, "plain")
+    dst = [torch.full_like(p, -1.0) for p in src]
+    for wiener, p in ((False, b), (True, f)):
+        ctx.stage3(p, wiener, dst, src)
+        assert all(bool((d == -1.0).all()) for d in dst)
+    counts = ctx.last_stats()  # the final stage's alone, as after a combined call
+    ctx.full3(b, f, dst, src)
+    ctx.check()
+    assert all(torch.equal(d, s) for d, s in zip(dst, src)) and ctx.last_stats() == counts
+    dst = [torch.full_like(p, -1.0) for p in src]
+    batch = isp_mw_b200.Batch(ctx, [b], [f], [dst], [src])
+    batch.run()
+    batch.check()
+    batch.close()
+    assert all(torch.equal(d, s) for d, s in zip(dst, src))
+    ctx.close()
