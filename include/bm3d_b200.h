@@ -487,6 +487,8 @@ int bm3d_pilot_wgrad48(bm3d_ctx *ctx, int n, int h, int w, const void *x, const 
  * later calls allocate normally); 0 turns it off. Process-wide. No
  * counterpart in the reference, which exits on allocation failure. */
 int bm3d_inject_alloc_failures(int count);
+/* The same after `skip` allocations that succeed. */
+int bm3d_inject_alloc_failures_after(int skip, int count);
 
 /* Fixes the tile shape of the stage kernels (BlockSize 8, GroupSize <= 16):
  * reference blocks per CTA tile (tile_x x tile_y) and warps per CTA. 0 keeps the

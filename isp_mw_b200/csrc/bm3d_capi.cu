@@ -35,14 +35,26 @@ int bm3d::cuda_fail(bm3d_ctx *ctx, cudaError_t e, const char *what)
     return e == cudaErrorMemoryAllocation ? BM3D_ERR_NOMEM : BM3D_ERR_CUDA;
 }
 
-// Allocations still to fail on purpose (bm3d_inject_alloc_failures).
-static std::atomic<int> g_fail_allocs{0};
+// Allocations still to fail on purpose (bm3d_inject_alloc_failures), and those
+// that succeed before them.
+static std::atomic<int> g_fail_allocs{0}, g_skip_allocs{0};
 
-extern "C" int bm3d_inject_alloc_failures(int count)
+extern "C" int bm3d_inject_alloc_failures(int count) { return bm3d_inject_alloc_failures_after(0, count); }
+
+extern "C" int bm3d_inject_alloc_failures_after(int skip, int count)
 {
-    if (count < 0) return BM3D_ERR_INVALID;
+    if (skip < 0 || count < 0) return BM3D_ERR_INVALID;
+    g_skip_allocs.store(skip);
     g_fail_allocs.store(count);
     return BM3D_OK;
+}
+
+// Takes one from a counter above zero.
+static bool take_one(std::atomic<int> &counter)
+{
+    for (int left = counter.load(); left > 0; left = counter.load())
+        if (counter.compare_exchange_weak(left, left - 1)) return true;
+    return false;
 }
 
 int bm3d::ensure(bm3d_ctx *ctx, DevBuf &b, size_t bytes)
@@ -51,11 +63,30 @@ int bm3d::ensure(bm3d_ctx *ctx, DevBuf &b, size_t bytes)
     if (b.ptr) cudaFree(b.ptr);
     b.ptr = nullptr;
     b.bytes = 0;
-    for (int left = g_fail_allocs.load(); left > 0; left = g_fail_allocs.load())
-        if (g_fail_allocs.compare_exchange_weak(left, left - 1))
-            return cuda_fail(ctx, cudaErrorMemoryAllocation, "cudaMalloc (injected failure)");
-    CK(ctx, cudaMalloc(&b.ptr, bytes));
+    if (!take_one(g_skip_allocs) && take_one(g_fail_allocs))
+        return cuda_fail(ctx, cudaErrorMemoryAllocation, "cudaMalloc (injected failure)");
+    const cudaError_t e = cudaMalloc(&b.ptr, bytes);
+    if (e != cudaSuccess) {
+        b.ptr = nullptr;
+        cudaGetLastError();  // the next launch check is not about this
+        return cuda_fail(ctx, e, "cudaMalloc");
+    }
     b.bytes = bytes;
+    return BM3D_OK;
+}
+
+int bm3d::ensure_optional(bm3d_ctx *ctx, DevBuf &b, size_t bytes, cudaStream_t s, bool &got)
+{
+    got = b.bytes >= bytes;
+    if (got) return BM3D_OK;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (s != nullptr) CK(ctx, cudaStreamIsCapturing(s, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone) return BM3D_OK;  // an allocation would end it
+    const std::string err = ctx->err;
+    const int rc = ensure(ctx, b, bytes);
+    got = rc == BM3D_OK;
+    if (rc != BM3D_ERR_NOMEM) return rc;
+    ctx->err = err;
     return BM3D_OK;
 }
 
@@ -688,7 +719,9 @@ static int plan_geometry(bm3d_ctx *ctx, StageArgs<T> &a, const bm3d_stage_params
 
 // How a stage call relates to another one: a basic stage that also prepares
 // the final stage that follows on the same planes, and that final stage
-// (PlaneJob's *_next). Saves the final stage's preparation pass and resets.
+// (PlaneJob's *_next). Saves the final stage's preparation pass and resets. A
+// leading stage that finds no room for the final stage's weight sums (8 B per
+// pixel) sets None: the stages then run one after the other, with the same results.
 enum class Chain { None, Leads, Follows };
 
 // One stage over device-resident planes (all with row pitch `stride`).
@@ -696,7 +729,7 @@ template <typename T>
 static int run_stage_device(bm3d_ctx *ctx, const bm3d_stage_params *p, bool wiener, int nplanes,
                             T *const dst[], const T *const src[], const T *const ref[], int width,
                             int height, size_t stride, double value_range, cudaStream_t s,
-                            Chain chain = Chain::None, int *gcount = nullptr, int *gpos = nullptr,
+                            Chain &chain, int *gcount = nullptr, int *gpos = nullptr,
                             T *gkey = nullptr, bool bm_only = false)
 {
     StageArgs<T> a;
@@ -727,7 +760,7 @@ static int run_stage_device(bm3d_ctx *ctx, const bm3d_stage_params *p, bool wien
     // FP32 sums are fixed point: planes with NaN / Inf pixels take the checking
     // aggregation (FP64 sums are doubles and carry them like the reference's)
     constexpr bool kFixed = std::is_same<Acc, long long>::value;
-    const bool follows = chain == Chain::Follows, leads = chain == Chain::Leads;
+    const bool follows = chain == Chain::Follows;
     a.nonfinite = !kFixed ? nullptr : follows ? ctx->nonfinite_next : ctx->nonfinite;
     a.stats = ctx->stats;
     a.bad = ctx->stats + 4;
@@ -735,13 +768,12 @@ static int run_stage_device(bm3d_ctx *ctx, const bm3d_stage_params *p, bool wien
     if (!follows) CK(ctx, cudaMemsetAsync(ctx->head, 0, kHeadClear, s));
     PlaneJobs<T> jobs;
     std::memset(&jobs, 0, sizeof(jobs));
-    int njobs = 0;
+    int njobs = 0, plane_of[kMaxPlanes];
     for (int c = 0; c < nplanes; ++c) {
         if (!(a.active & (1 << c)) && !bm_only) continue;
         DevBuf &den = follows ? ctx->den_next[c] : ctx->acc[2 * c + 1];
         if ((rc = ensure(ctx, ctx->acc[2 * c], acc_bytes)) != BM3D_OK) return rc;
         if ((rc = ensure(ctx, den, acc_bytes)) != BM3D_OK) return rc;
-        if (leads && (rc = ensure(ctx, ctx->den_next[c], acc_bytes)) != BM3D_OK) return rc;
         a.num[c] = static_cast<Acc *>(ctx->acc[2 * c].ptr);
         a.den[c] = static_cast<Acc *>(den.ptr);
         if (kFixed) {  // starts zeroed; normalisation leaves it zero
@@ -750,6 +782,7 @@ static int run_stage_device(bm3d_ctx *ctx, const bm3d_stage_params *p, bool wien
             if (grow) CK(ctx, cudaMemsetAsync(ctx->poison[c].ptr, 0, ctx->poison[c].bytes, s));
             a.poison[c] = static_cast<unsigned char *>(ctx->poison[c].ptr);
         }
+        plane_of[njobs] = c;
         PlaneJob<T> &q = jobs.job[njobs++];
         q.num = a.num[c];
         q.den = a.den[c];
@@ -765,11 +798,17 @@ static int run_stage_device(bm3d_ctx *ctx, const bm3d_stage_params *p, bool wien
         q.log2_corner = a.log2_corner;
         q.nonfinite = kFixed ? const_cast<unsigned *>(a.nonfinite) + c : nullptr;
         q.poison = a.poison[c];
-        if (leads) {
-            q.den_next = static_cast<long long *>(ctx->den_next[c].ptr);
-            q.nonfinite_next = ctx->nonfinite_next + c;
-            if (njobs == 1) q.stats = ctx->stats;
-        }
+    }
+    for (int j = 0; j < njobs && chain == Chain::Leads; ++j) {
+        bool got;
+        if ((rc = ensure_optional(ctx, ctx->den_next[plane_of[j]], acc_bytes, s, got)) != BM3D_OK) return rc;
+        if (!got) chain = Chain::None;
+    }
+    for (int j = 0; j < njobs && chain == Chain::Leads; ++j) {
+        PlaneJob<T> &q = jobs.job[j];
+        q.den_next = static_cast<long long *>(ctx->den_next[plane_of[j]].ptr);
+        q.nonfinite_next = ctx->nonfinite_next + plane_of[j];
+        if (j == 0) q.stats = ctx->stats;
     }
     // (njobs 0: noise levels that are not numbers pass the guard and select no plane)
     if (!bm_only && !follows && njobs > 0) {
@@ -849,9 +888,10 @@ int bm3d::stage_any(bm3d_ctx *ctx, const bm3d_stage_params *p, int wiener, int n
         ctx->err = "parameters outside this build (BlockSize <= 16, GroupSize <= 32)";
         return BM3D_ERR_UNSUPPORTED;
     }
+    Chain alone = Chain::None;
     if (mem == BM3D_MEM_DEVICE)
         return run_stage_device(ctx, p, wiener != 0, nplanes, dst, src, ref, width, height, stride,
-                                value_range, s);
+                                value_range, s, alone);
     const size_t plane_bytes = sizeof(T) * static_cast<size_t>(width) * height;
     T *dd[kMaxPlanes];
     const T *ds[kMaxPlanes], *dr[kMaxPlanes];
@@ -881,7 +921,7 @@ int bm3d::stage_any(bm3d_ctx *ctx, const bm3d_stage_params *p, int wiener, int n
                 return rc;
     }
     rc = run_stage_device(ctx, p, wiener != 0, nplanes, dd, ds, dr, width, height, width,
-                          value_range, s);
+                          value_range, s, alone);
     if (rc != BM3D_OK) return rc;
     for (int c = 0; c < nplanes; ++c)
         if ((rc = copy_plane(ctx, dst[c], stride, static_cast<const T *>(dd[c]), width, width,
@@ -1013,17 +1053,19 @@ int bm3d::full_any(bm3d_ctx *ctx, const bm3d_stage_params *basic, const bm3d_sta
     }
     chained = chained && any;
     if ((rc = refused(gb)) != BM3D_OK) return rc;
+    Chain chain = chained ? Chain::Leads : Chain::None;
     if (gb == Guard::Run) {
         rc = run_stage_device(ctx, basic, false, nplanes, tmp, ds, dr, width, height, dpitch,
-                              value_range, s, chained ? Chain::Leads : Chain::None);
+                              value_range, s, chain);
         if (rc != BM3D_OK) return rc;
     }
     if ((rc = refused(gf)) != BM3D_OK) return rc;
     if (gf == Guard::Run) {
         const T *tr[kMaxPlanes];
         for (int c = 0; c < nplanes; ++c) tr[c] = tmp[c];
+        if (chain == Chain::Leads) chain = Chain::Follows;
         rc = run_stage_device(ctx, fin, true, nplanes, dd, ds, tr, width, height, dpitch,
-                              value_range, s, chained ? Chain::Follows : Chain::None);
+                              value_range, s, chain);
         if (rc != BM3D_OK) return rc;
     }
     if (mem == BM3D_MEM_HOST) {
@@ -1095,8 +1137,9 @@ static int dump_groups(bm3d_ctx *ctx, const bm3d_stage_params *p, int wiener, co
         return rc;
     float *d[1] = {in};
     const float *sp[1] = {in};
+    Chain alone = Chain::None;
     rc = run_stage_device<float>(ctx, p, wiener != 0, 1, d, sp, sp, width, height, width,
-                                 value_range, s, Chain::None, static_cast<int *>(ctx->groups[0].ptr),
+                                 value_range, s, alone, static_cast<int *>(ctx->groups[0].ptr),
                                  static_cast<int *>(ctx->groups[1].ptr),
                                  keys ? static_cast<float *>(ctx->groups[2].ptr) : nullptr, true);
     if (rc != BM3D_OK) return rc;

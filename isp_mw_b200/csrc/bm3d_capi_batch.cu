@@ -506,13 +506,15 @@ static int batch_create_any(bm3d_ctx *ctx, int npl, int count, const bm3d_stage_
         for (int c = 0; npl > 1 && c < npl; ++c)
             B->chained = B->chained && (basic[i].sigma[c] > 0) == (final_[i].sigma[c] > 0);
     }
-    if (B->chained && (rc = ensure(ctx, B->den_next, sizeof(long long) * next_total)) != BM3D_OK)
-        return fail(rc);
     if ((rc = ensure(ctx, B->poison, acc_total / 2)) != BM3D_OK) return fail(rc);
     // all zero between stages: the normalisation clears what it reads
     CK(ctx, cudaMemset(B->poison.ptr, 0, acc_total / 2));
     if ((rc = ensure(ctx, B->bad, sizeof(unsigned long long))) != BM3D_OK) return fail(rc);
     CK(ctx, cudaMemset(B->bad.ptr, 0, sizeof(unsigned long long)));
+    // without room for the final stage's own weight sums the stages run one after the other
+    if (B->chained && (rc = ensure_optional(ctx, B->den_next, sizeof(long long) * next_total, nullptr,
+                                            B->chained)) != BM3D_OK)
+        return fail(rc);
     // per-pixel kernels' plane tables, active planes of each stage in batch order
     for (int st = 0; st < 2; ++st) {
         std::vector<PlaneJob<float>> q;

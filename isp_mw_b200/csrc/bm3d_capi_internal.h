@@ -93,6 +93,9 @@ int cuda_fail(bm3d_ctx *ctx, cudaError_t e, const char *what);
 
 // Grow a context buffer to at least `bytes`.
 int ensure(bm3d_ctx *ctx, DevBuf &b, size_t bytes);
+// The same for a buffer that the caller can do without: no room for it, or a
+// stream that is being captured, is no error and leaves `got` false.
+int ensure_optional(bm3d_ctx *ctx, DevBuf &b, size_t bytes, cudaStream_t s, bool &got);
 
 // Raise a kernel's dynamic shared memory limit to at least `bytes`; never
 // lower it. The limit belongs to the kernel function and is shared by every

@@ -76,3 +76,57 @@ def test_no_plane_to_filter(bm3d_lib):
     batch.close()
     assert all(torch.equal(d, s) for d, s in zip(dst, src))
     ctx.close()
+
+
+@pytest.mark.parametrize("planes", [1, 3])
+def test_no_room_for_the_next_stage_sums(bm3d_lib, planes):
+    """Without room for the final stage's own weight sums the stages run one
+    after the other: same results, no error, in single calls and batches."""
+    import torch
+    import isp_mw_b200
+    b = isp_mw_b200.stage_params_default("fast", False, [30.0, 20.0, 20.0])
+    f = isp_mw_b200.stage_params_default("fast", True, [30.0, 20.0, 20.0])
+    src = _planes(planes, 90, 128, "nan")
+    same = lambda x, y: all(np.array_equal(p.cpu().numpy(), q.cpu().numpy(), equal_nan=True)
+                            for p, q in zip(x, y))
+    one = (lambda x: x) if planes == 3 else (lambda x: x[0])
+    call = lambda c, *args: (c.full3 if planes == 3 else c.full)(*args)
+    ctx = isp_mw_b200.Context(0)
+    want = [torch.zeros_like(p) for p in src]
+    call(ctx, b, f, one(want), one(src))
+    copied = isp_mw_b200.stage_params_default("fast", True, [0.0] * 3)
+    short = isp_mw_b200.Context(0)
+    got = [torch.zeros_like(p) for p in src]
+    call(short, b, copied, one(got), one(src))  # every buffer but those sums
+    try:
+        for skip in range(planes):
+            bm3d_lib.bm3d_inject_alloc_failures_after(skip, 1)
+            got = [torch.zeros_like(p) for p in src]
+            call(short, b, f, one(got), one(src))
+            assert same(got, want)
+            bm3d_lib.bm3d_inject_alloc_failures(0)
+            short.close()
+            short = isp_mw_b200.Context(0)
+            call(short, b, copied, one(got), one(src))
+        # captured with those sums missing: nothing to allocate
+        stream = torch.cuda.Stream()
+        got = [torch.zeros_like(p) for p in src]
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            call(short, b, f, one(got), one(src))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert same(got, want)
+        # a batch: sums, estimates, state, marks and consistency counter come first
+        got = [torch.zeros_like(p) for p in src]
+        bm3d_lib.bm3d_inject_alloc_failures_after(5, 1)
+        batch = isp_mw_b200.Batch(ctx, [b], [f], [one(got)], [one(src)])
+        batch.run()
+        batch.check()
+        batch.close()
+        assert same(got, want)
+    finally:
+        bm3d_lib.bm3d_inject_alloc_failures(0)
+        short.close()
+        ctx.close()
