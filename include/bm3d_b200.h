@@ -489,6 +489,9 @@ int bm3d_pilot_wgrad48(bm3d_ctx *ctx, int n, int h, int w, const void *x, const 
 int bm3d_inject_alloc_failures(int count);
 /* The same after `skip` allocations that succeed. */
 int bm3d_inject_alloc_failures_after(int skip, int count);
+/* Likewise for kernel launches of the pilot: after `skip` launches one is
+ * reported as failed (BM3D_ERR_CUDA); a negative skip turns it off. */
+int bm3d_inject_launch_failure_after(int skip);
 
 /* Fixes the tile shape of the stage kernels (BlockSize 8, GroupSize <= 16):
  * reference blocks per CTA tile (tile_x x tile_y) and warps per CTA. 0 keeps the

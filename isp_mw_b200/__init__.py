@@ -43,7 +43,8 @@ EXPORTS = [
     "bm3d_batch_destroy", "bm3d_plane_int", "bm3d_stage_int", "bm3d_frame", "bm3d_stage_frame",
     "bm3d_full_many", "bm3d_batch3_create", "bm3d_host_batch_create", "bm3d_host_batch3_create",
     "bm3d_host_batch_run", "bm3d_host_batch_join", "bm3d_host_batch_destroy",
-    "bm3d_inject_alloc_failures", "bm3d_inject_alloc_failures_after", "bm3d_batch_stage_times", "bm3d_batch_final_create",
+    "bm3d_inject_alloc_failures", "bm3d_inject_alloc_failures_after",
+    "bm3d_inject_launch_failure_after", "bm3d_batch_stage_times", "bm3d_batch_final_create",
     "bm3d_batch3_final_create",
     "bm3d_pilot_param_count", "bm3d_pilot_set_conv_kernel", "bm3d_pilot_conv_kernel",
     "bm3d_pilot_set_timing", "bm3d_pilot_layer_ms",
@@ -136,6 +137,7 @@ def load_library(path: str = LIB_PATH) -> ctypes.CDLL:
     lib.bm3d_noalloc_check.argtypes = [vp]
     lib.bm3d_inject_alloc_failures.argtypes = [ip]
     lib.bm3d_inject_alloc_failures_after.argtypes = [ip, ip]
+    lib.bm3d_inject_launch_failure_after.argtypes = [ip]
     lib.bm3d_pilot_param_count.argtypes = []
     lib.bm3d_pilot_set_conv_kernel.argtypes = [ip]
     lib.bm3d_pilot_conv_kernel.argtypes = []

@@ -57,6 +57,22 @@ static bool take_one(std::atomic<int> &counter)
     return false;
 }
 
+// Pilot launches until one is reported as failed; negative: none is.
+static std::atomic<int> g_fail_launch{-1};
+
+extern "C" int bm3d_inject_launch_failure_after(int skip)
+{
+    g_fail_launch.store(skip < 0 ? -1 : skip);
+    return BM3D_OK;
+}
+
+cudaError_t bm3d::launch_error()
+{
+    const cudaError_t e = cudaGetLastError();
+    if (g_fail_launch.load() < 0 || g_fail_launch.fetch_sub(1) != 0) return e;
+    return cudaErrorInvalidConfiguration;
+}
+
 int bm3d::ensure(bm3d_ctx *ctx, DevBuf &b, size_t bytes)
 {
     if (b.bytes >= bytes) return BM3D_OK;

@@ -93,6 +93,8 @@ int cuda_fail(bm3d_ctx *ctx, cudaError_t e, const char *what);
 
 // Grow a context buffer to at least `bytes`.
 int ensure(bm3d_ctx *ctx, DevBuf &b, size_t bytes);
+// The error of the launch before it, or one injected (bm3d_inject_launch_failure_after).
+cudaError_t launch_error();
 // The same for a buffer that the caller can do without: no room for it, or a
 // stream that is being captured, is no error and leaves `got` false.
 int ensure_optional(bm3d_ctx *ctx, DevBuf &b, size_t bytes, cudaStream_t s, bool &got);

@@ -143,7 +143,7 @@ int run_conv48(bm3d_ctx *ctx, const __nv_bfloat16 *x, __nv_bfloat16 *y, const __
         CK(ctx, raise_smem_limit(reinterpret_cast<const void *>(conv48_n144_kernel), kT3Smem));
         conv48_n144_kernel<<<std::max(1, std::min(a.tiles, ctx->sm_count)), kT3Threads, kT3Smem,
                              s>>>(tin, tout, a);
-        CK(ctx, cudaGetLastError());
+        CK(ctx, launch_error());
         g_conv_last.store(3);
         return BM3D_OK;
     }
@@ -158,7 +158,7 @@ int run_conv48(bm3d_ctx *ctx, const __nv_bfloat16 *x, __nv_bfloat16 *y, const __
         CK(ctx, raise_smem_limit(reinterpret_cast<const void *>(conv48_tma_kernel), kTmaSmem));
         conv48_tma_kernel<<<std::max(1, std::min(a.tiles, ctx->sm_count)), kTmaThreads, kTmaSmem,
                             s>>>(tin, tout, a);
-        CK(ctx, cudaGetLastError());
+        CK(ctx, launch_error());
         g_conv_last.store(2);
         return BM3D_OK;
     }
@@ -170,7 +170,7 @@ int run_conv48(bm3d_ctx *ctx, const __nv_bfloat16 *x, __nv_bfloat16 *y, const __
     CK(ctx, raise_smem_limit(reinterpret_cast<const void *>(conv48_kernel), kConvSmem));
     conv48_kernel<<<std::max(1, std::min(a.tiles, kConvCtasPerSm * ctx->sm_count)), kConvThreads,
                     kConvSmem, s>>>(a);
-    CK(ctx, cudaGetLastError());
+    CK(ctx, launch_error());
     g_conv_last.store(1);
     return BM3D_OK;
 }
@@ -194,15 +194,15 @@ int run_wgrad48(bm3d_ctx *ctx, const __nv_bfloat16 *x, const __nv_bfloat16 *g, f
     static_assert(kWgSmem > 120 * 1024, "one CTA per SM");
     CK(ctx, raise_smem_limit(reinterpret_cast<const void *>(wgrad48_kernel), kWgSmem));
     wgrad48_kernel<<<parts, kWgThreads, kWgSmem, s>>>(a);
-    CK(ctx, cudaGetLastError());
+    CK(ctx, launch_error());
     return BM3D_OK;
 }
 
-// Sums a layer's partial gradients; with Adam's state set in a, updates too.
+// Sums a layer's partial gradients.
 int run_reduce(bm3d_ctx *ctx, const ReduceArgs &a, cudaStream_t s)
 {
     reduce_partials_kernel<<<(a.len + kReduceSums - 1) / kReduceSums, kReduceThreads, 0, s>>>(a);
-    CK(ctx, cudaGetLastError());
+    CK(ctx, launch_error());
     return BM3D_OK;
 }
 
@@ -259,7 +259,7 @@ int pack(bm3d_pilot *p, cudaStream_t s)
     __nv_bfloat16 *w = static_cast<__nv_bfloat16 *>(p->wpack.ptr);
     pack_weights_kernel<<<216, 256, 0, s>>>(static_cast<const float *>(p->params.ptr), w,
                                             w + 6 * kPackElems, w + 12 * kPackElems);
-    CK(p->ctx, cudaGetLastError());
+    CK(p->ctx, launch_error());
     return BM3D_OK;
 }
 
@@ -291,7 +291,7 @@ int forward(bm3d_pilot *p, const float *in, long long stride, long long img_stri
     ia.w = w;
     if (p->timing) CK(ctx, cudaEventRecord(p->ev[0], s));
     conv_in_kernel<<<px_grid(ctx, pixels), kPxThreads, 0, s>>>(ia);
-    CK(ctx, cudaGetLastError());
+    CK(ctx, launch_error());
     if (p->timing) CK(ctx, cudaEventRecord(p->ev[1], s));
     int rc;
     for (int layer = 2; layer <= 7; ++layer) {
@@ -316,7 +316,7 @@ int forward(bm3d_pilot *p, const float *in, long long stride, long long img_stri
     oa.h = h;
     oa.w = w;
     conv_out_kernel<<<blocks, 256, 0, s>>>(oa);
-    CK(ctx, cudaGetLastError());
+    CK(ctx, launch_error());
     if (p->timing) CK(ctx, cudaEventRecord(p->ev[8], s));
     return BM3D_OK;
 }
@@ -557,26 +557,14 @@ extern "C" int bm3d_pilot_train_step(bm3d_pilot *p, int count, int height, int w
     float *part = static_cast<float *>(p->partial.ptr);
     const float *dout = static_cast<const float *>(p->dout.ptr);
     const int rblocks = 2 * ctx->sm_count;  // even: wgrad_in_kernel's two planes
-    // Adam's bias-corrected step size. Each layer is summed and updated as soon as
-    // its partials are written (while they are in L2; 75 MB of all layers' read
-    // back together took 54 us) and its FP32 weights have been read.
-    p->step += 1;
-    const float b1 = 0.9f, b2 = 0.999f;
-    const double c1 = 1.0 - std::pow(b1, static_cast<double>(p->step));
-    const double c2 = 1.0 - std::pow(b2, static_cast<double>(p->step));
-    const float lr_t = static_cast<float>(lr * std::sqrt(c2) / c1);
-    auto update = [&](int parts, int len, int wlen, int offset, bool mid) {
-        ReduceArgs ra = {part, grad + offset, grad + offset + wlen, parts, len, wlen, mid,
-                         grad,
-                         static_cast<float *>(p->params.ptr),
-                         static_cast<float *>(p->adam_m.ptr),
-                         static_cast<float *>(p->adam_v.ptr),
-                         lr_t, b1, b2, 1e-8f};
-        return run_reduce(ctx, ra, s);
+    // each layer's partials are summed as soon as they are written, while they are
+    // in L2 (75 MB of all layers' read back together took 54 us)
+    auto sum = [&](int parts, int len, int wlen, int offset, bool mid) {
+        return run_reduce(ctx, {part, grad + offset, grad + offset + wlen, parts, len, wlen, mid}, s);
     };
     // layer 8: weight gradient, then the gradient into layer 7's pre-activation
     wgrad_out_kernel<<<rblocks, kEdgeThreads, 0, s>>>(X(7), dout, count, height, width, part);
-    CK(ctx, cudaGetLastError());
+    CK(ctx, launch_error());
     __nv_bfloat16 *G[2] = {static_cast<__nv_bfloat16 *>(p->gbuf[0].ptr),
                            static_cast<__nv_bfloat16 *>(p->gbuf[1].ptr)};
     OutBackArgs ob;
@@ -588,8 +576,8 @@ extern "C" int bm3d_pilot_train_step(bm3d_pilot *p, int count, int height, int w
     ob.h = height;
     ob.w = width;
     out_backward_kernel<<<px_grid(ctx, pixels), kPxThreads, 0, s>>>(ob);
-    CK(ctx, cudaGetLastError());
-    if ((rc = update(rblocks, kW8Partial, kW8, kOffW8, false)) != BM3D_OK) return rc;
+    CK(ctx, launch_error());
+    if ((rc = sum(rblocks, kW8Partial, kW8, kOffW8, false)) != BM3D_OK) return rc;
     // layers 7 .. 2: weight gradient (tensor cores), data gradient (tensor cores)
     int cur = 1;
     for (int layer = 7; layer >= 2; --layer) {
@@ -597,7 +585,7 @@ extern "C" int bm3d_pilot_train_step(bm3d_pilot *p, int count, int height, int w
         if ((rc = run_wgrad48(ctx, X(layer - 1), G[cur], part, count, height, width, err, s,
                               parts)) != BM3D_OK)
             return rc;
-        if ((rc = update(parts, kWgPartial, kWmid, off_w(layer), true)) != BM3D_OK) return rc;
+        if ((rc = sum(parts, kWgPartial, kWmid, off_w(layer), true)) != BM3D_OK) return rc;
         if ((rc = run_conv48(ctx, G[cur], G[cur ^ 1], wbwd(p, layer), nullptr, nullptr, X(layer - 1),
                              kMaskPrev, count, height, width, err, s)) != BM3D_OK)
             return rc;
@@ -615,9 +603,18 @@ extern "C" int bm3d_pilot_train_step(bm3d_pilot *p, int count, int height, int w
     ia.h = height;
     ia.w = width;
     wgrad_in_kernel<<<rblocks, kEdgeThreads, 0, s>>>(ia, G[cur], part);
-    CK(ctx, cudaGetLastError());
-    if ((rc = update(rblocks, kW1Partial, kW1, 0, false)) != BM3D_OK) return rc;
-    // the packed BF16 copies of the updated weights
+    CK(ctx, launch_error());
+    if ((rc = sum(rblocks, kW1Partial, kW1, 0, false)) != BM3D_OK) return rc;
+    // Adam, then the packed BF16 copies of the updated weights
+    const float b1 = 0.9f, b2 = 0.999f;
+    const double c1 = 1.0 - std::pow(b1, static_cast<double>(p->step + 1));
+    const double c2 = 1.0 - std::pow(b2, static_cast<double>(p->step + 1));
+    adam_kernel<<<(kParams + 255) / 256, 256, 0, s>>>(
+        static_cast<float *>(p->params.ptr), grad, static_cast<float *>(p->adam_m.ptr),
+        static_cast<float *>(p->adam_v.ptr), kParams, static_cast<float>(lr * std::sqrt(c2) / c1), b1, b2,
+        1e-8f);
+    CK(ctx, launch_error());
+    p->step += 1;
     if ((rc = pack(p, s)) != BM3D_OK) return rc;
     if (loss) {
         double l = 0.0;
@@ -696,7 +693,7 @@ extern "C" int bm3d_pilot_conv48(bm3d_ctx *ctx, int n, int h, int w, const void 
     __nv_bfloat16 *packed = static_cast<__nv_bfloat16 *>(wp.ptr);
     pack_weights_kernel<<<216, 256, 0, s>>>(params, packed, packed + 6 * kPackElems,
                                             packed + 12 * kPackElems);
-    CK(ctx, cudaGetLastError());
+    CK(ctx, launch_error());
     unsigned *err = static_cast<unsigned *>(eb.ptr);
     CK(ctx, cudaMemsetAsync(err, 0, sizeof(unsigned), s));
     if ((rc = run_conv48(ctx, static_cast<const __nv_bfloat16 *>(x), static_cast<__nv_bfloat16 *>(y),

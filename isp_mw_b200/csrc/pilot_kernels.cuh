@@ -957,8 +957,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) wgrad48_kernel(const WgradArgs 
 }
 
 // Sums of a layer's partial gradients, in double and in a fixed order
-// (reproducible), and Adam on its FP32 master parameters (bias-corrected step
-// size precomputed). `len` sums over `parts` vectors `len` floats apart, the first
+// (reproducible). `len` sums over `parts` vectors `len` floats apart, the first
 // `wlen` the weights; `mid` weights come as [dy][dx][ci][co]. A block takes 32
 // neighbouring sums and its eight warps each an eighth of the parts, so that
 // loads are whole lines and no thread waits for a chain of 148 (296) of them:
@@ -970,9 +969,6 @@ struct ReduceArgs {
     float *w, *b;  // results
     int parts, len, wlen;
     bool mid;
-    const float *grad;      // Adam: w and b point into it
-    float *param, *m, *v;   // null: sums only
-    float lr_t, beta1, beta2, eps;
 };
 
 __global__ void __launch_bounds__(kReduceThreads) reduce_partials_kernel(const ReduceArgs a)
@@ -1001,15 +997,23 @@ __global__ void __launch_bounds__(kReduceThreads) reduce_partials_kernel(const R
     } else {
         out = a.w + i;
     }
-    const float g = static_cast<float>(s);
-    *out = g;
-    if (a.param == nullptr) return;
-    const long long e = out - a.grad;
-    const float mi = a.beta1 * a.m[e] + (1.0f - a.beta1) * g;
-    const float vi = a.beta2 * a.v[e] + (1.0f - a.beta2) * g * g;
-    a.m[e] = mi;
-    a.v[e] = vi;
-    a.param[e] -= a.lr_t * mi / (sqrtf(vi) + a.eps);
+    *out = static_cast<float>(s);
+}
+
+// Adam on the FP32 master parameters (bias-corrected step size precomputed). One
+// launch for all layers once every gradient is there: a step that fails before it
+// leaves parameters and moments as they were.
+__global__ void adam_kernel(float *param, const float *grad, float *m, float *v, int count, float lr_t,
+                            float beta1, float beta2, float eps)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+        const float g = grad[i];
+        const float mi = beta1 * m[i] + (1.0f - beta1) * g;
+        const float vi = beta2 * v[i] + (1.0f - beta2) * g * g;
+        m[i] = mi;
+        v[i] = vi;
+        param[i] -= lr_t * mi / (sqrtf(vi) + eps);
+    }
 }
 
 // ---------------------------------------------------------------------------

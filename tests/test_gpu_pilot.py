@@ -375,3 +375,33 @@ def test_pilot_edge_layers_at_ragged_sizes(ctx, shape):
     for part in (slice(0, 912), slice(-433, None)):  # layer 1, layer 8
         d = (grad[part] - ref[part]).norm()
         assert float(d) <= 0.05 * float(ref[part].norm()) + 1e-7, (part, float(d))
+
+
+def test_failed_step_leaves_the_training_state(ctx, tmp_path):
+    """A step whose launch fails, anywhere in its forward or backward pass,
+    changes neither parameters nor moments nor the step count; the next step is
+    what it would have been."""
+    import isp_mw_b200
+    noisy, clean, sigma = _data(2, 24, 32, 9)
+    a, b = isp_mw_b200.Pilot(ctx, seed=4), isp_mw_b200.Pilot(ctx, seed=4)
+    state = lambda p: (p.save(str(tmp_path / "s")), (tmp_path / "s").read_bytes())[1]
+    for p in (a, b):
+        p.train_step(noisy, clean, sigma, 1e-3)
+    assert state(a) == state(b)
+    before = state(a)
+    failed = 0
+    for skip in range(31):  # forward 8, layer 8 3, layers 7 .. 2 18, layer 1 2
+        ctx.lib.bm3d_inject_launch_failure_after(skip)
+        try:
+            with pytest.raises(isp_mw_b200.BM3DError):
+                a.train_step(noisy, clean, sigma, 1e-3)
+            failed += 1
+        finally:
+            ctx.lib.bm3d_inject_launch_failure_after(-1)
+        assert state(a) == before, skip
+    assert failed == 31
+    for p in (a, b):
+        p.train_step(noisy, clean, sigma, 1e-3)
+    assert state(a) == state(b) != before
+    a.close()
+    b.close()
