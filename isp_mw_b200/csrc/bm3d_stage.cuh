@@ -495,7 +495,7 @@ template <typename T> __device__ __forceinline__ typename DistBits<T>::type dist
 // kNear above `limit`. The cut then leaves that much more room, and the
 // approximate order stands when no kept distance is within kNear of the next;
 // else exact_dist gives the compacted ones'. Returns -1 where the whole list has to be exact: a distance
-// at the matching threshold, ties, ranges where the bounds do not hold -- keys that
+// at the matching threshold, ties in a full group, ranges where the bounds do not hold -- keys that
 // are subnormal or zero tie at distances far apart, so every compacted distance has
 // to lie in near_low .. near_high, not the cut's bound alone.
 template <typename T, bool NEAR, int BS>
@@ -720,7 +720,8 @@ __device__ __forceinline__ int select_once(const Search<T> &e, bool near, int la
                     const bool t0 = lane < M && e0 && r0 < take;
                     const bool t1 = lane + kWarp < M && e1 && r1 < take;
                     tie = __any_sync(0xffffffffu, t0 || t1);
-                    if (NEAR && near && tie) return -1;
+                    // (a list that the group takes whole keeps its order among equal keys)
+                    if (NEAR && near && tie && accepted >= GS) return -1;
                 }
             }
             if (lane < M && r0 < take) put(r0, v0);
