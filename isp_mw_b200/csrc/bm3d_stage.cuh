@@ -976,8 +976,12 @@ __device__ int match_block(const StageArgs<T> &a, const Tile<T> &t, int j0, int 
     // task for the trailing (0, 0) slot of the reference's search list.
     const int nstrips = (nr + KS - 1) / KS;
     const int ntasks = nstrips * nc;
-    // FP32 lists hold approximate distances first (select_group, NEAR)
-    constexpr bool kNearList = sizeof(T) == 4;
+    // FP32 lists hold approximate distances first (select_group, NEAR). With BMstep
+    // over 1 a list is a quarter as long or less, and what its distances save does not
+    // pay for the lists that have to be made exact: final stage of a 1080p plane with
+    // BMstep 2 in ordered against approximate distances 266 / 268 us (noise), 360 / 426
+    // (computer graphics), 460 / 546 (8-bit values).
+    constexpr bool kNearList = sizeof(T) == 4 && KS > 1;
     const B limit = dist_limit(a.thSSE);
     const B accept = kNearList && limit < static_cast<B>(0x7f800000u) ? limit + DistBits<T>::near_ulps(BS) : limit;
     int nvalid = 0;
