@@ -1127,6 +1127,10 @@ __global__ void __launch_bounds__(kPxThreads, 6) conv_in_kernel(const InArgs a)
                 inside[k] |= (ok ? 1u : 0u) << t;
             }
         }
+        // taps of border pixels, for both pixels and all lanes in step (one tap at a
+        // time of one pixel at a time took 7 of 18 us on one 128 x 128 image)
+        const unsigned edge[2] = {inside[0] == 0x1ffu ? 0u : inside[0], inside[1] == 0x1ffu ? 0u : inside[1]};
+        const bool border = __any_sync(0xffffffffu, (edge[0] | edge[1]) != 0);
 #pragma unroll 2
         for (int q = 0; q < 6; ++q) {
             uint32_t packed[2][4];
@@ -1139,13 +1143,15 @@ __global__ void __launch_bounds__(kPxThreads, 6) conv_in_kernel(const InArgs a)
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
                     acc[k] = b4;
-                    if (inside[k] == 0x1ffu) {
-                        fma4(acc[k], sd[k], s4);
-                    } else {
-#pragma unroll 1
-                        for (int t = 0; t < 9; ++t)
-                            if (inside[k] & (1u << t))
-                                fma4(acc[k], sd[k], *reinterpret_cast<const float4 *>(&wsg[t][c]));
+                    if (edge[k] == 0) fma4(acc[k], sd[k], s4);
+                }
+                if (border) {
+#pragma unroll
+                    for (int t = 0; t < 9; ++t) {
+                        const float4 w4 = *reinterpret_cast<const float4 *>(&wsg[t][c]);
+#pragma unroll
+                        for (int k = 0; k < 2; ++k)
+                            if (edge[k] >> t & 1) fma4(acc[k], sd[k], w4);
                     }
                 }
 #pragma unroll
