@@ -283,8 +283,31 @@ def set_f32_transform_mode(kind: str, mode: int) -> int:
     return old
 
 
+# Profile defaults restated (include/BM3D.h:27-151): BlockSize, BlockStep,
+# GroupSize, BMrange, lambda, and thMSE's constant and factor of sigma[0].
+_DEFAULTS = {
+    False: {"fast": (8, 8, 16, 9, 2.7, 400, 80), "lc": (8, 6, 16, 9, 2.7, 400, 80),
+            "np": (8, 4, 16, 16, 2.7, 400, 80), "high": (8, 3, 16, 16, 2.7, 400, 80),
+            "vn": (8, 4, 32, 16, 2.8, 1000, 150)},
+    True: {"fast": (8, 7, 16, 9, 0.0, 200, 10), "lc": (8, 5, 16, 9, 0.0, 200, 10),
+           "np": (8, 3, 32, 16, 0.0, 200, 10), "high": (8, 2, 32, 16, 0.0, 200, 10),
+           "vn": (11, 6, 32, 16, 0.0, 400, 40)},
+}
+
+
+def stage_default(profile: str, wiener: bool, sigma: Sequence[float]) -> dict:
+    """Profile defaults from the table above (pinned by the golden fixtures'
+    parameters, which the compiled reference gave)."""
+    bs, step, gs, rng, lam, c0, c1 = _DEFAULTS[bool(wiener)][profile]
+    return {"block_size": bs, "block_step": step, "group_size": gs, "bm_range": rng, "bm_step": 1,
+            "thMSE": c0 + float(sigma[0]) * c1, "lambda": lam, "sigma": [float(v) for v in sigma]}
+
+
 def reference_stage_default(profile: str, wiener: bool, sigma: Sequence[float]) -> dict:
-    """Profile defaults from the compiled reference's own parameter classes."""
+    """Profile defaults from the compiled reference's own parameter classes, or
+    the restated ones where the reference is not built."""
+    if not reference_available():
+        return stage_default(profile, wiener, sigma)
     lib = _load(os.path.join(REF_DIR, "libbm3d_ref_f32.so"))
     out = StageParams()
     s = (ctypes.c_double * 3)(*sigma)
