@@ -82,23 +82,13 @@ template <typename T>
 __device__ void dct3_generic(T *G, int n, int bs, int lane, const T *tab, const float *pad, bool inverse)
 {
     const int bsq = bs * bs;
-    if (sizeof(T) == 4 && bs == 11) {
-        for (int line = lane; line < n * 11; line += kWarp)  // along x
-            dct_line11(G + line * 11, 1, inverse);
-        __syncwarp();
-        for (int line = lane; line < n * 11; line += kWarp) {  // along y
-            const int z = line / 11, x = line - z * 11;
-            dct_line11(G + z * 121 + x, 11, inverse);
-        }
-    } else {
-        const T *mb = tab + dct_table_offset(bs);
-        for (int line = lane; line < n * bs; line += kWarp)  // along x
-            dct_line(G + line * bs, 1, bs, mb);
-        __syncwarp();
-        for (int line = lane; line < n * bs; line += kWarp) {  // along y
-            const int z = line / bs, x = line - z * bs;
-            dct_line(G + z * bsq + x, bs, bs, mb);
-        }
+    const T *mb = tab + dct_table_offset(bs);
+    for (int line = lane; line < n * bs; line += kWarp)  // along x
+        dct_line(G + line * bs, 1, bs, mb);
+    __syncwarp();
+    for (int line = lane; line < n * bs; line += kWarp) {  // along y
+        const int z = line / bs, x = line - z * bs;
+        dct_line(G + z * bsq + x, bs, bs, mb);
     }
     __syncwarp();
     dct_z_generic(G, n, bs, lane, tab, pad, inverse);

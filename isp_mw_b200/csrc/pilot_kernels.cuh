@@ -1592,12 +1592,8 @@ __global__ void __launch_bounds__(kEdgeThreads, 2) wgrad_in_kernel(const InArgs 
     }
 }
 
-// Packs the six 48 -> 48 layers' FP32 weights [co][ci][ky][kx] into the
-// shared-memory operand layout, BF16: forward taps (dy, dx) = (ky, kx) with
-// N = co, K = ci; and the data-gradient form, taps flipped (2 - ky, 2 - kx)
-// with N = ci, K = co.
-// BF16 copies of the six 48 -> 48 layers' weights in the MMA operand
-// layouts: `fwd` and `bwd` (flipped, transposed: the data gradient) per tap
+// BF16 copies of the six 48 -> 48 layers' FP32 weights [co][ci][ky][kx] in the MMA
+// operand layouts: `fwd` and `bwd` (flipped, transposed: the data gradient) per tap
 // as [co / 8][ci / 8][co % 8][ci % 8] (N = 48); `fwd3` for the N = 144 forward
 // kernel, per row tap dy as 144 rows n = column tap * 48 + co of 64 channels ci
 // (48 used), 128-byte swizzled (smem_desc_sw128).
