@@ -291,6 +291,10 @@ template <> struct DistBits<float> {
     {
         return __reduce_max_sync(0xffffffffu, v);
     }
+    static __device__ __forceinline__ unsigned warp_min(unsigned v)
+    {
+        return __reduce_min_sync(0xffffffffu, v);
+    }
 };
 template <> struct DistBits<double> {
     using type = unsigned long long;
@@ -313,6 +317,10 @@ template <> struct DistBits<double> {
             v = o > v ? o : v;
         }
         return v;
+    }
+    static __device__ __forceinline__ unsigned long long warp_min(unsigned long long v)
+    {
+        return ~warp_max(~v);
     }
 };
 
@@ -433,17 +441,25 @@ template <typename T> struct Search {
     T *lkeys;
 };
 
+// Where a list place's pixels are.
+template <typename T>
+__device__ __forceinline__ const T *list_block(const Search<T> &e, int i, int &pitch)
+{
+    if (i >= e.ngrid) {
+        pitch = e.slot_pitch;
+        return e.slot;
+    }
+    const int rr = div_magic(i, e.nc_div);
+    pitch = e.pitch;
+    return e.win + rr * e.st * e.pitch + (i - rr * e.nc) * e.st;
+}
+
 // The exact distance of a list place, in the reference's order.
 template <typename T, int BS>
 __device__ __forceinline__ typename DistBits<T>::type exact_dist(const Search<T> &e, int i)
 {
-    const T *cb = e.slot;
-    int cp = e.slot_pitch;
-    if (i < e.ngrid) {
-        const int rr = div_magic(i, e.nc_div);
-        cb = e.win + rr * e.st * e.pitch + (i - rr * e.nc) * e.st;
-        cp = e.pitch;
-    }
+    int cp;
+    const T *cb = list_block(e, i, cp);
     T acc = T(0);
 #pragma unroll 1
     for (int y = 0; y < BS; ++y) {
@@ -454,6 +470,29 @@ __device__ __forceinline__ typename DistBits<T>::type exact_dist(const Search<T>
         }
     }
     return DistBits<T>::of(acc);
+}
+
+// The same of two places, which may be one: they share the reference block's
+// loads, and neither waits for the other's chain of sums.
+template <typename T, int BS>
+__device__ __forceinline__ void exact_dists(const Search<T> &e, int i, int j, typename DistBits<T>::type &di,
+                                            typename DistBits<T>::type &dj)
+{
+    int pi, pj;
+    const T *ci = list_block(e, i, pi), *cj = list_block(e, j, pj);
+    T si = T(0), sj = T(0);
+#pragma unroll 1
+    for (int y = 0; y < BS; ++y) {
+#pragma unroll
+        for (int x = 0; x < BS; ++x) {
+            const T r = e.refb[y * e.pitch + x];
+            const T u = sub_rn(r, ci[y * pi + x]), w = sub_rn(r, cj[y * pj + x]);
+            si = add_rn(si, mul_rn(u, u));
+            sj = add_rn(sj, mul_rn(w, w));
+        }
+    }
+    di = DistBits<T>::of(si);
+    dj = DistBits<T>::of(sj);
 }
 
 // A candidate's entry in the search list. Distances are sums of squares:
@@ -493,11 +532,11 @@ template <typename T> __device__ __forceinline__ typename DistBits<T>::type dist
 //
 // NEAR, near: the list holds approximate distances (ssd_row_near), accepted up to
 // kNear above `limit`. The cut then leaves that much more room, and the
-// approximate order stands when no kept distance is within kNear of the next;
-// else exact_dist gives the compacted ones'. Returns -1 where the whole list has to be exact: a distance
-// at the matching threshold, ties in a full group, ranges where the bounds do not hold -- keys that
-// are subnormal or zero tie at distances far apart, so every compacted distance has
-// to lie in near_low .. near_high, not the cut's bound alone.
+// approximate order stands when no kept distance is within kNear of the next; else
+// exact_dist gives the compacted ones'. Returns -1 where the whole list has to be
+// exact: a distance at the matching threshold, ties in a full group, ranges where the
+// bounds do not hold -- keys that are subnormal or zero tie at distances far apart, so
+// every compacted distance has to lie in near_low .. near_high, not the cut's bound alone.
 template <typename T, bool NEAR, int BS>
 __device__ __forceinline__ int select_once(const Search<T> &e, bool near, int lane, int nvalid,
                                            unsigned &n_fix)
@@ -597,7 +636,9 @@ __device__ __forceinline__ int select_once(const Search<T> &e, bool near, int la
         // Candidates that crowd into few lanes leave the bound too high: halve the
         // range for a lower one that still has take elements under it. (The ordered
         // search that such lists fell back to takes 31 passes over 1089 places; as
-        // the last warp of a tile it held up the others.)
+        // the last warp of a tile it held up the others.) Both ends move to elements
+        // of the list, so that lists of few different distances -- computer graphics --
+        // take a step or two instead of 20 to 60.
         int pos = 0, M = 0;  // this lane's end among the compacted ones, and their number
         auto scan = [&] {
             pos = mine;
@@ -611,13 +652,25 @@ __device__ __forceinline__ int select_once(const Search<T> &e, bool near, int la
         scan();
         if (M > kCand) {
             B lo = 0, hi = tb == none ? none - 1 : tb;
-            while (hi - lo > 1) {
+            while (hi - lo > (NEAR && near ? kNear : B(1))) {
                 const B mid = lo + (hi - lo) / 2;
-                if (__reduce_add_sync(0xffffffffu, count(mid)) < take) {
-                    lo = mid;
+                B under = 0, over = none;  // the elements next to mid
+                int c = 0;
+                for (int first = 0; first < nkeys; first += kHeld * kWarp) {
+                    if (!one) load(first);
+#pragma unroll
+                    for (int k = 0; k < kHeld; ++k) {
+                        const bool low = v[k] <= mid;
+                        c += low ? 1 : 0;
+                        if (low && v[k] > under) under = v[k];
+                        if (!low && v[k] < over) over = v[k];
+                    }
+                }
+                if (__reduce_add_sync(0xffffffffu, c) < take) {
+                    lo = DB::warp_min(over) - 1;
                     continue;
                 }
-                hi = mid;
+                hi = DB::warp_max(under);
                 cut = cut_at(hi);
                 mine = count(cut);
                 if (__reduce_add_sync(0xffffffffu, mine) <= kCand) break;
@@ -726,10 +779,14 @@ __device__ __forceinline__ int select_once(const Search<T> &e, bool near, int la
             }
             if (lane < M && r0 < take) put(r0, v0);
             if (lane + kWarp < M && r1 < take) put(r1, v1);
+        } else if (sure) {
+            // Many candidates share the cut, so more than the group holds: in all but
+            // contrived lists equal keys touch the kept set, and the exact algorithm
+            // below places any keys.
+            tie = true;
         } else {
-            // Rare (many candidates share the cut, or keys outside the normal
-            // range): repeated warp minimum, whose owner lane advances to the
-            // next key of its elements.
+            // Rare (keys outside the normal range): repeated warp minimum, whose
+            // owner lane advances to the next key of its elements.
             auto next_after = [&](const K &m, bool any) {
                 K nxt = K::invalid();
                 for (int i = lane; i < nkeys; i += kWarp) {
@@ -848,9 +905,25 @@ __device__ __forceinline__ int select_group(const Search<T> &e, bool near, int l
         if (NEAR && !near) {
             __syncwarp();
             nvalid = 0;
-            if constexpr (NEAR)
-                for (int i = lane; i <= e.ngrid; i += kWarp)
-                    e.dist[i] = accept_dist(exact_dist<T, BS>(e, i), e.limit, nvalid);
+            if constexpr (NEAR) {
+                // What the approximate pass rejected is past the limit, equal to the
+                // reference block or no number either way (bounds that hold above kTiny).
+                const bool skip = e.limit >= DistBits<T>::kTiny;
+                auto next = [&](int i) {
+                    while (i <= e.ngrid && skip && e.dist[i] == ~typename DistBits<T>::type(0)) i += kWarp;
+                    return i;
+                };
+                for (int i = next(lane); __any_sync(0xffffffffu, i <= e.ngrid);) {
+                    const int j = i <= e.ngrid ? next(i + kWarp) : i;
+                    if (i <= e.ngrid) {
+                        typename DistBits<T>::type di, dj;
+                        exact_dists<T, BS>(e, i, j <= e.ngrid ? j : i, di, dj);
+                        e.dist[i] = accept_dist(di, e.limit, nvalid);
+                        if (j <= e.ngrid) e.dist[j] = accept_dist(dj, e.limit, nvalid);
+                        i = next(j + kWarp);
+                    }
+                }
+            }
             __syncwarp();
         }
         const int n = select_once<T, NEAR, BS>(e, near, lane, nvalid, n_fix);
