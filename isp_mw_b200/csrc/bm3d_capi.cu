@@ -675,6 +675,7 @@ static int plan_geometry(bm3d_ctx *ctx, StageArgs<T> &a, const bm3d_stage_params
         ctx->err = "stage does not fit in shared memory";
         return BM3D_ERR_UNSUPPORTED;
     }
+    if (!a.match) a.span = 1;  // no search list (past the limit, which counts one)
     // The launch bounds (register-resident 512 threads in FP32, 256 in FP64;
     // generic 384, and 256 in FP64 and for BlockSize 11) limit the warps; the
     // small shapes are for windows that leave no room for more.

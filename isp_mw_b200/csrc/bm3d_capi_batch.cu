@@ -204,6 +204,7 @@ int build_stage(bm3d_batch *B, bool wiener, int tx, int ty, int warps, StageBuil
                                      std::min(least, a.nx) * std::min(least, a.ny)) + 16 >
             ctx->smem_optin)
             return BM3D_ERR_UNSUPPORTED;
+        if (!a.match) a.span = 1;  // no search list (past the limit, which counts one)
         a.region_w = std::min(a.width, (tx - 1) * a.step + 2 * reach + BS);
         a.region_h = std::min(a.height, (ty - 1) * a.step + 2 * reach + BS);
         a.region_pitch = window_pitch(a.region_w);

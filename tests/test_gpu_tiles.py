@@ -105,3 +105,35 @@ def test_search_range_limit(bm3d_lib, shape, bm_range, ok):
             ctx.stage(p, False, dst, src)
         assert e.value.code == isp_mw_b200.BM3D_ERR_UNSUPPORTED
     ctx.close()
+
+
+@pytest.mark.parametrize("planes", [1, 3])
+@pytest.mark.parametrize("block,bm_range", [(8, 1), (8, 32), (11, 9), (11, 30), (5, 1), (5, 32)])
+def test_groups_of_one_have_no_search_list(bm3d_lib, oracle_mod, block, bm_range, planes):
+    """Groups of one match nothing, at any BMrange within the limit: single calls
+    and batches agree bit for bit, and with the oracle."""
+    import torch
+    import isp_mw_b200
+    from isp_mw_b200 import synth
+    noisy = [synth.pair(83, 97, 20.0, 3 + c)[1] for c in range(planes)]
+    src = [torch.from_numpy(p).cuda() for p in noisy]
+    ctx = isp_mw_b200.Context(0)
+    b, f = (isp_mw_b200.stage_params_default("fast", w, [30.0] * 3) for w in (False, True))
+    for p in (b, f):
+        p.block_size, p.group_size, p.bm_range, p.block_step = block, 1, bm_range, block - 1
+    dst = [torch.zeros_like(p) for p in src]
+    if planes == 1:
+        ctx.full(b, f, dst[0], src[0])
+    else:
+        ctx.full3(b, f, dst, src)
+    ctx.check()
+    other = [torch.zeros_like(p) for p in src]
+    batch = isp_mw_b200.Batch(ctx, [b], [f], other if planes == 1 else [other], src if planes == 1 else [src])
+    batch.run()
+    batch.check()
+    batch.close()
+    assert all(torch.equal(p, q) for p, q in zip(dst, other))
+    if planes == 1:
+        _, want = oracle_mod.backend("port", np.float32).full(b.as_dict(), f.as_dict(), noisy[0])
+        assert np.abs(dst[0].cpu().numpy() - want).max() <= 1e-3
+    ctx.close()
