@@ -624,7 +624,9 @@ static bool over_limit(const bm3d_ctx *ctx, const StageArgs<T> &a, const bm3d_st
 // follows the group's size. A tile adds staging, flushing and the wait for its last
 // warp: about 10 us where other CTAs of the SM overlap it, or by its window in the
 // generic kernel, whose 12 warps fill an SM. CTAs run in waves, whose rounding up
-// fades once there are several. Measured at 64 x 64 .. 3840 x 2160, one shape for all
+// fades once there are several: the sooner in the generic kernels, where a CTA of
+// few warps starts as soon as another of its SM ends. Blocks under 8 x 8 take no
+// less time than those of 8 x 8. Measured at 64 x 64 .. 3840 x 2160, one shape for all
 // sizes (8 x 8, 16 warps) against the shapes this picks, basic / final stage:
 // 64 x 64 60 / 67 -> 20 / 23 us, 512 x 512 72 / 88 -> 49 / 65 us, 1280 x 720
 // 128 / 197 -> 113 / 177 us, 1920 x 1080 245 / 343 -> 225 / 329 us; generic kernel
@@ -642,13 +644,13 @@ static double tile_cost(const bm3d_ctx *ctx, const StageArgs<T> &a, const SmemPl
     const double tiles = static_cast<double>(a.tiles_x) * ((a.ny + a.tile_y - 1) / a.tile_y);
     const double share = tiles / ctx->sm_count;  // tiles per SM
     const int ctas = std::min(per_sm, std::max(1, static_cast<int>(std::ceil(share))));
-    const double px = a.block_size * a.block_size / 64.0;
+    const double px = std::max(1.0, a.block_size * a.block_size / 64.0);
     const double work = px * (0.65 * std::max(16, a.group_size) / 16.0 +
                               0.35 * a.span * a.span / 361.0) * (nplanes == 3 ? 1.9 : 1.0);
     const double round = (8.5 + 0.22 * ctas * t.warps) * work;
     const int rounds = (a.tile_x * a.tile_y + t.warps - 1) / t.warps;
     const double x = share / per_sm;
-    const double waves = x < 4.0 ? std::ceil(x) : x + 0.5;
+    const double waves = generic && per_sm > 1 ? std::max(1.0, x + 0.3) : x < 4.0 ? std::ceil(x) : x + 0.5;
     const double window = static_cast<double>(a.region_w) * a.region_h * ctas;
     const double edge = generic ? 3.0 + 1.05e-3 * window : 8.0 + rounds + 0.1 * t.warps;
     return waves * (rounds * round + edge * nplanes);
@@ -682,34 +684,45 @@ static int plan_geometry(bm3d_ctx *ctx, StageArgs<T> &a, const bm3d_stage_params
     static const TileShape fast[] = {{2, 2, 4}, {4, 2, 8}, {4, 4, 8}, {4, 8, 8}, {6, 4, 8}, {8, 8, 16}};
     static const TileShape gen[] = {{6, 6, 12}, {6, 4, 12}, {4, 3, 12}, {3, 2, 6}, {2, 2, 4},
                                     {4, 4, 8},  {4, 2, 8},  {5, 2, 5},  {4, 4, 4}};
+    static const TileShape gen_tiny[] = {{6, 4, 12}, {2, 2, 4}};
     static const TileShape gen_small[] = {{2, 2, 4}, {2, 2, 2}, {1, 1, 2}, {1, 1, 1}};
     const int max_warps = generic ? generic_max_warps(sizeof(T), generic_size_class(sizeof(T), BS))
                                   : stage_max_warps<T>();
     if (generic || !ctx->tiling_set) {
         TileShape best{0, 0, 0};
         double least = 1e300, within = 0;
-        // Blocks over 8 x 8 without a kernel of their own: rounds are several times
-        // longer than the model's, so even work counts for more than it says, and the
-        // smallest tile within a tenth is taken. (16 x 16 blocks in groups of 32, 330 x
-        // 250, basic stage: 2 x 2 against 4 x 4 tiles on 4 warps 2.34 / 2.37 ms on noise,
-        // 2.05 / 2.65 on computer graphics; 4 x 4 blocks lose up to a fifth by it.)
-        const bool even = generic && BS > kBS && generic_size_class(sizeof(T), BS) == 0;
+        // The model is made for 8 x 8 and (FP32) 11 x 11 blocks in FP32; elsewhere the
+        // smallest tile not much above the least cost is taken, because its warps wait
+        // least for one another where groups differ in size. FP32 blocks under 8 x 8
+        // choose between two shapes that fill the registers with 12 warps (4 x 4 tiles
+        // on 4 warps, which cost least, took 2486 us where 6 x 4 on 12 took 1876 and
+        // 2 x 2 on 4 2225: 2 x 2 blocks, groups of 32, noise, 320 x 256). Over 198 stages
+        // of BlockSize 2 to 16 on 64 x 64, 333 x 200 and 700 x 540, noise and computer
+        // graphics, the geometric mean over the best of the shapes is 1.02 (FP32 under
+        // 8 x 8; by the least cost 1.12), 1.01 (over; 1.06) and 1.02 (FP64; 1.07).
+        const bool plain = generic && generic_size_class(sizeof(T), BS) == 0;
+        const bool small = plain && sizeof(T) == 4 && BS < kBS;
         auto offer = [&](const TileShape &t) {
             if (t.warps > max_warps) return;
             const SmemPlan sp = plan_tile(a, p, wiener, nplanes, t);
             if (sp.total > ctx->smem_optin) return;
             const double c = tile_cost(ctx, a, sp, t, nplanes, generic);
-            if (within > 0 ? c <= within && (best.warps == 0 || t.tx * t.ty < best.tx * best.ty) : c < least) {
+            const int size = t.tx * t.ty - best.tx * best.ty;
+            if (within > 0 ? c <= within && (best.warps == 0 || size < 0 || (size == 0 && c < least)) : c < least) {
                 least = c;
                 best = t;
             }
         };
-        if (generic) for (const TileShape &t : gen) offer(t);
-        else for (const TileShape &t : fast) offer(t);
-        if (even && best.warps != 0) {
-            within = 1.1 * least;
+        auto offer_all = [&] {
+            if (!generic) for (const TileShape &t : fast) offer(t);
+            else if (small) for (const TileShape &t : gen_tiny) offer(t);
+            else for (const TileShape &t : gen) offer(t);
+        };
+        offer_all();
+        if (plain && best.warps != 0) {
+            within = (small ? 1.06 : 1.2) * least;
             best = TileShape{0, 0, 0};
-            for (const TileShape &t : gen) offer(t);
+            offer_all();
         }
         if (generic && best.warps == 0)
             for (const TileShape &t : gen_small)

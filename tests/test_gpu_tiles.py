@@ -137,3 +137,25 @@ def test_groups_of_one_have_no_search_list(bm3d_lib, oracle_mod, block, bm_range
         _, want = oracle_mod.backend("port", np.float32).full(b.as_dict(), f.as_dict(), noisy[0])
         assert np.abs(dst[0].cpu().numpy() - want).max() <= 1e-3
     ctx.close()
+
+
+# block sizes without a kernel of their own: one tile of 2 x 2 reference blocks,
+# some, and enough for the shape of 6 x 4 on 12 warps; FP64 to the 9th digit
+@pytest.mark.parametrize("shape", [(19, 20), (60, 49), (150, 161)])
+@pytest.mark.parametrize("block,step,group_size", [(1, 1, 4), (2, 1, 32), (4, 3, 17), (7, 4, 16), (9, 5, 8), (16, 9, 32)])
+@pytest.mark.parametrize("wiener", [False, True])
+def test_block_sizes_at_picked_shapes(bm3d_lib, oracle_mod, shape, block, step, group_size, wiener):
+    import isp_mw_b200
+    from isp_mw_b200 import synth
+    p = isp_mw_b200.stage_params_default("fast", wiener, [30.0] * 3)
+    p.block_size, p.block_step, p.group_size, p.bm_range = block, step, group_size, 3
+    noisy = synth.pair(*shape, 20.0, 5)[1]
+    ctx = isp_mw_b200.Context(0)
+    for dtype, tol in ((np.float32, 1e-3), (np.float64, 1e-9)):
+        src = noisy.astype(dtype)
+        out = np.empty_like(src)
+        ctx.stage(p, wiener, out, src)
+        want = oracle_mod.backend("port", dtype).stage(wiener, p.as_dict(), src)
+        want = want[1] if isinstance(want, tuple) else want
+        assert np.abs(out - want).max() <= tol
+    ctx.close()
