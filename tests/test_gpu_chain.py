@@ -118,9 +118,9 @@ def test_no_room_for_the_next_stage_sums(bm3d_lib, planes):
         graph.replay()
         torch.cuda.synchronize()
         assert same(got, want)
-        # a batch: sums, estimates, state, marks and consistency counter come first
+        # a batch: estimates, state, marks and consistency counter come first
         got = [torch.zeros_like(p) for p in src]
-        bm3d_lib.bm3d_inject_alloc_failures_after(5, 1)
+        bm3d_lib.bm3d_inject_alloc_failures_after(4, 1)
         batch = isp_mw_b200.Batch(ctx, [b], [f], [one(got)], [one(src)])
         batch.run()
         batch.check()
