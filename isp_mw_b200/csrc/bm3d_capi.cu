@@ -120,13 +120,13 @@ cudaError_t bm3d::raise_smem_limit(const void *kern, size_t bytes)
                                 static_cast<int>(bytes));
 }
 
-#define BM3D_DECLARE_UNIT(name) cudaError_t bm3d_upload_dct_tables_##name(const bm3d::DctTableData &);
+#define BM3D_DECLARE_UNIT(name) cudaError_t bm3d_upload_dct_tables_##name(const bm3d::DctTables &);
 BM3D_KERNEL_UNITS(BM3D_DECLARE_UNIT)
 #undef BM3D_DECLARE_UNIT
 
 namespace bm3d {
 
-cudaError_t upload_dct_tables_all(const DctTableData &t)
+cudaError_t upload_dct_tables_all(const DctTables &t)
 {
     cudaError_t e = cudaSuccess;
 #define BM3D_UPLOAD_UNIT(name) \
@@ -158,20 +158,17 @@ static void make_dct_tables(float *ff, float *fi, double *df, double *di)
     }
 }
 
-static float g_tab_ff[1496], g_tab_fi[1496];
-static float g_pad_f[bm3d::kPadTable], g_pad_i[bm3d::kPadTable];
-static float g_d11_f[11 * 11], g_d11_i[11 * 11];
-static double g_tab_df[1496], g_tab_di[1496];
+static bm3d::DctTables g_tab;
 static std::once_flag g_tab_once;
 
 static void init_dct_tables()
 {
-    make_dct_tables(g_tab_ff, g_tab_fi, g_tab_df, g_tab_di);
+    make_dct_tables(g_tab.fwd_f, g_tab.inv_f, g_tab.fwd_d, g_tab.inv_d);
     const long double pi = 3.141592653589793238462643383279502884L;
     for (int k = 0; k < 11; ++k)
         for (int j = 0; j < 11; ++j) {
-            g_d11_f[k * 11 + j] = static_cast<float>(2.0L * cosl(pi * (2 * j + 1) * k / 22.0L));
-            g_d11_i[k * 11 + j] =
+            g_tab.d11_fwd[k * 11 + j] = static_cast<float>(2.0L * cosl(pi * (2 * j + 1) * k / 22.0L));
+            g_tab.d11_inv[k * 11 + j] =
                 static_cast<float>(j == 0 ? 1.0L : 2.0L * cosl(pi * j * (2 * k + 1) / 22.0L));
         }
     // column-major, 16 rows, zero past row n: the same FP32 values
@@ -180,8 +177,8 @@ static void init_dct_tables()
         const int src = (n - 1) * n * (2 * n - 1) / 6, dst = bm3d::pad_table_offset(n);
         for (int j = 0; j < n; ++j)
             for (int k = 0; k < 16; ++k) {
-                g_pad_f[dst + 16 * j + k] = k < n ? g_tab_ff[src + k * n + j] : 0.0f;
-                g_pad_i[dst + 16 * j + k] = k < n ? g_tab_fi[src + k * n + j] : 0.0f;
+                g_tab.pad_fwd[dst + 16 * j + k] = k < n ? g_tab.fwd_f[src + k * n + j] : 0.0f;
+                g_tab.pad_inv[dst + 16 * j + k] = k < n ? g_tab.inv_f[src + k * n + j] : 0.0f;
             }
     }
 }
@@ -189,8 +186,7 @@ static void init_dct_tables()
 static cudaError_t upload_dct_tables()
 {
     std::call_once(g_tab_once, init_dct_tables);
-    return upload_dct_tables_all(
-        DctTableData{g_tab_ff, g_tab_fi, g_tab_df, g_tab_di, g_pad_f, g_pad_i, g_d11_f, g_d11_i});
+    return upload_dct_tables_all(g_tab);
 }
 
 extern "C" int bm3d_ctx_create(bm3d_ctx **out, int device)
@@ -247,11 +243,14 @@ extern "C" int bm3d_ctx_create(bm3d_ctx **out, int device)
                     tf[kDctTableSize + o + k * n + j] = static_cast<float>(ci);
                     td[o + k * n + j] = static_cast<double>(cf);
                     td[kDctTableSize + o + k * n + j] = static_cast<double>(ci);
-                    if (n < kGSTab) {
-                        const int q = 2 * kDctTableSize + pad32_offset(n) + 32 * j + k;
-                        tf[q] = static_cast<float>(cf);
-                        tf[q + kPad32Table] = static_cast<float>(ci);
-                    }
+                }
+        }
+        for (int n = 1; n < kGSTab; ++n) {  // the same, column by column in 32 rows
+            const int o = dct_table_offset(n), q = 2 * kDctTableSize + pad32_offset(n);
+            for (int k = 0; k < n; ++k)
+                for (int j = 0; j < n; ++j) {
+                    tf[q + 32 * j + k] = tf[o + k * n + j];
+                    tf[q + kPad32Table + 32 * j + k] = tf[kDctTableSize + o + k * n + j];
                 }
         }
         e = cudaMalloc(&ctx->gtab_f, tf.size() * sizeof(float));

@@ -22,6 +22,18 @@ __host__ __device__ constexpr int pad_table_offset(int n)
     return 16 * ((n - 1) * n / 2 - (n > 8 ? 8 : 0));
 }
 
+// The constant cosine tables of a kernel unit. One block, because making a context
+// fills every unit's: 80 copies of single arrays took 0.5 to 0.7 ms, ten take 0.13.
+struct DctTables {
+    // lengths 1..16 (row k = output k), concatenated: n starts at (n-1) n (2n-1) / 6
+    float fwd_f[1496], inv_f[1496];
+    double fwd_d[1496], inv_d[1496];
+    // FP32, lengths other than 8 and 16, column by column: n starts at
+    // pad_table_offset(n), entry (row k, column j) at + 16 j + k, zero for k >= n
+    float pad_fwd[kPadTable], pad_inv[kPadTable];
+    float d11_fwd[11 * 11], d11_inv[11 * 11];  // length 11, for blocks of 11
+};
+
 // ---------------------------------------------------------------------------
 // Arithmetic that must not be contracted into FMA: the reference accumulates
 // block distances as dist += temp * temp with separate rounding of the product

@@ -15,13 +15,6 @@
 
 namespace bm3d {
 
-// FP32 cosine matrices of length 11 (row k = output k) for BlockSize 11 rows
-// and columns (the "vn" final stage): every coefficient a constant-bank
-// operand. Each translation unit has its own copy, filled by the host when a
-// context is made.
-static __constant__ float c_dct11_fwd[11 * 11];
-static __constant__ float c_dct11_inv[11 * 11];
-
 // In-place length-n transform of one strided line, by one lane: out[k] =
 // sum_j mat[k n + j] in[j] (row k = output k), n <= kGSTab.
 template <typename T>
@@ -62,8 +55,8 @@ __device__ __forceinline__ void dct_line11(T *base, int stride, bool inverse)
         T v[11];
 #pragma unroll
         for (int j = 0; j < 11; ++j) v[j] = base[j * stride];
-        if (inverse) redft01_line<T, 11>(v, c_dct11_inv);
-        else redft10_line<T, 11>(v, c_dct11_fwd);
+        if (inverse) redft01_line<T, 11>(v, c_dct.d11_inv);
+        else redft10_line<T, 11>(v, c_dct.d11_fwd);
 #pragma unroll
         for (int j = 0; j < 11; ++j) base[j * stride] = v[j];
     }
@@ -370,7 +363,7 @@ __device__ __forceinline__ void gather_rows(const Tile<T> &t, const T *win, cons
             for (int x = 0; x < BS; ++x) v[x] = T(0);
         }
         if constexpr (BS == 8) redft10_8(v);
-        else redft10_line<T, BS>(v, c_dct11_fwd);
+        else redft10_line<T, BS>(v, c_dct.d11_fwd);
         T *g = G + line * RS;
 #pragma unroll
         for (int x = 0; x < BS; ++x) g[x] = v[x];
@@ -398,7 +391,7 @@ __device__ __forceinline__ void aggregate_rows(const StageArgs<T> &a, const Tile
 #pragma unroll
         for (int x = 0; x < BS; ++x) v[x] = g[x];
         if constexpr (BS == 8) redft01_8(v);
-        else redft01_line<T, BS>(v, c_dct11_inv);
+        else redft01_line<T, BS>(v, c_dct.d11_inv);
         int pitch;
         AccWin<T> dn = block_acc(t, p, q.y, q.x, pitch);
         dn = dn + y * pitch;

@@ -16,14 +16,9 @@ template <typename T, bool W, int NPL, int BSC> const void *generic_kernel_fn();
 // batch_stage_kernel<float, W, NPL, KS, GEN> (bm3d_batch.cuh)
 template <bool W, int NPL, int KS, int GEN> const void *batch_kernel_fn();
 
-// Cosine matrices for group lengths 1..16, concatenated (1496 entries each).
-struct DctTableData {
-    const float *fwd_f, *inv_f;
-    const double *fwd_d, *inv_d;
-    const float *pad_fwd, *pad_inv;  // kPadTable entries each (bm3d_device.cuh)
-    const float *d11_fwd, *d11_inv;  // length-11 matrices, 121 entries each
-};
-cudaError_t upload_dct_tables_all(const DctTableData &t);
+// Every unit's constant tables on the current device.
+struct DctTables;  // bm3d_device.cuh
+cudaError_t upload_dct_tables_all(const DctTables &t);
 
 }  // namespace bm3d
 

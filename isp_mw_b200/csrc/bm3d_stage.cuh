@@ -16,27 +16,18 @@
 
 namespace bm3d {
 
-// Cosine matrices for group lengths 1..16 (row k = output k), concatenated;
-// length n starts at (n-1) n (2n-1) / 6. Every translation unit that launches
-// these kernels has its own copy, filled by the host when a context is made.
-static __constant__ float c_dct_fwd_f[1496];
-static __constant__ float c_dct_inv_f[1496];
-static __constant__ double c_dct_fwd_d[1496];
-static __constant__ double c_dct_inv_d[1496];
-// FP32 cosine matrices of the lengths other than 8 and 16, column by column:
-// length n starts at 16 * (sum of the lengths m < n, m != 8), and entry
-// (row k, column j) sits at + 16 j + k, zero for k >= n.
-static __constant__ float c_dct_pad_fwd[kPadTable];
-static __constant__ float c_dct_pad_inv[kPadTable];
+// Every translation unit that launches these kernels has its own copy, filled by
+// the host when a context is made.
+static __constant__ DctTables c_dct;
 
 template <typename T> struct DctTab;
 template <> struct DctTab<float> {
-    static __device__ __forceinline__ const float *fwd() { return c_dct_fwd_f; }
-    static __device__ __forceinline__ const float *inv() { return c_dct_inv_f; }
+    static __device__ __forceinline__ const float *fwd() { return c_dct.fwd_f; }
+    static __device__ __forceinline__ const float *inv() { return c_dct.inv_f; }
 };
 template <> struct DctTab<double> {
-    static __device__ __forceinline__ const double *fwd() { return c_dct_fwd_d; }
-    static __device__ __forceinline__ const double *inv() { return c_dct_inv_d; }
+    static __device__ __forceinline__ const double *fwd() { return c_dct.fwd_d; }
+    static __device__ __forceinline__ const double *inv() { return c_dct.inv_d; }
 };
 
 // Transforms along the group axis for two pencils at once. Lengths 8 and 16
@@ -1314,7 +1305,7 @@ __device__ __forceinline__ void group_fwd(T *G, int n, int lane, Pair<T> (&p)[kG
             load_pencils(G, 8, lane, p);
             zbfly8(p, false);
         } else {
-            zgen(G, n, lane, c_dct_pad_fwd + pad_table_offset(n), p);
+            zgen(G, n, lane, c_dct.pad_fwd + pad_table_offset(n), p);
         }
     } else {
         load_pencils(G, n, lane, p);
@@ -1338,7 +1329,7 @@ __device__ __forceinline__ void group_inv(T *G, int n, int lane, Pair<T> (&p)[kG
         } else {
             store_pencils(G, n, lane, p);
             __syncwarp();
-            zgen(G, n, lane, c_dct_pad_inv + pad_table_offset(n), p);
+            zgen(G, n, lane, c_dct.pad_inv + pad_table_offset(n), p);
         }
     } else {
         zdct2<true>(p, n);

@@ -22,23 +22,12 @@ template <bool W, int NPL, int KS, int GEN> const void *batch_kernel_fn()
     return reinterpret_cast<const void *>(&batch_stage_kernel<float, W, NPL, KS, GEN>);
 }
 
-static cudaError_t upload_dct_tables_here(const DctTableData &t)
-{
-    cudaError_t e;
-    if ((e = cudaMemcpyToSymbol(c_dct_fwd_f, t.fwd_f, sizeof(c_dct_fwd_f))) != cudaSuccess) return e;
-    if ((e = cudaMemcpyToSymbol(c_dct_inv_f, t.inv_f, sizeof(c_dct_inv_f))) != cudaSuccess) return e;
-    if ((e = cudaMemcpyToSymbol(c_dct_fwd_d, t.fwd_d, sizeof(c_dct_fwd_d))) != cudaSuccess) return e;
-    if ((e = cudaMemcpyToSymbol(c_dct_pad_fwd, t.pad_fwd, sizeof(c_dct_pad_fwd))) != cudaSuccess) return e;
-    if ((e = cudaMemcpyToSymbol(c_dct_pad_inv, t.pad_inv, sizeof(c_dct_pad_inv))) != cudaSuccess) return e;
-    if ((e = cudaMemcpyToSymbol(c_dct11_fwd, t.d11_fwd, sizeof(c_dct11_fwd))) != cudaSuccess) return e;
-    if ((e = cudaMemcpyToSymbol(c_dct11_inv, t.d11_inv, sizeof(c_dct11_inv))) != cudaSuccess) return e;
-    return cudaMemcpyToSymbol(c_dct_inv_d, t.inv_d, sizeof(c_dct_inv_d));
-}
+static cudaError_t upload_dct_tables_here(const DctTables &t) { return cudaMemcpyToSymbol(c_dct, &t, sizeof(t)); }
 
 }  // namespace bm3d
 
 #define BM3D_KERNEL_UNIT(name)                                                      \
-    cudaError_t bm3d_upload_dct_tables_##name(const bm3d::DctTableData &t)         \
+    cudaError_t bm3d_upload_dct_tables_##name(const bm3d::DctTables &t)            \
     {                                                                               \
         return bm3d::upload_dct_tables_here(t);                                     \
     }
