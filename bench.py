@@ -487,8 +487,8 @@ def run_batch(args):
 # batch kernel itself is committed these are four times the per-plane
 # stage_kernel captures (profiles/stage_kernel_{final,basic}_1080p_full.txt):
 # the batch kernel runs the same per-tile body over the same tiles.
-TRAFFIC_FINAL_1080P = 46.487e6 + 0.0e6
-TRAFFIC_BASIC_1080P = 37.286e6 + 0.004e6
+TRAFFIC_FINAL_1080P = 46.649e6 + 0.025e6
+TRAFFIC_BASIC_1080P = 37.340e6 + 0.027e6
 TRAFFIC_BATCH_FINAL_4X1080P = 4 * TRAFFIC_FINAL_1080P
 TRAFFIC_BATCH_BASIC_4X1080P = 4 * TRAFFIC_BASIC_1080P
 TRAFFIC_SOURCE = ("4 x the per-plane stage_kernel capture on one 1920x1080 plane, sigma 25 "
