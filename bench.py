@@ -985,7 +985,7 @@ def run_pilot_yuv(args):
 # DRAM bytes (read + write) of one 48 -> 48 layer launch on one 1920x1080
 # plane, per forward kernel, from the ncu captures named beside them
 PILOT_CONV_TRAFFIC_PER_PLANE = {
-    "conv48_n144_kernel": (199_203_328 + 158_855_680,
+    "conv48_n144_kernel": (199_243_776 + 159_338_752,
                            "profiles/conv48_n144_kernel_1080p_full.txt"),
     "conv48_tma_kernel": (199_160_576 + 156_573_952,
                           "profiles/conv48_tma_kernel_1080p_full.txt"),
