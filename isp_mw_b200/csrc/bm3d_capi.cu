@@ -649,7 +649,8 @@ static double tile_cost(const bm3d_ctx *ctx, const StageArgs<T> &a, const SmemPl
     const double round = (8.5 + 0.22 * ctas * t.warps) * work;
     const int rounds = (a.tile_x * a.tile_y + t.warps - 1) / t.warps;
     const double x = share / per_sm;
-    const double waves = generic && per_sm > 1 ? std::max(1.0, x + 0.3) : x < 4.0 ? std::ceil(x) : x + 0.5;
+    const double tail = generic_size_class(sizeof(T), a.block_size) != 0 ? 0.15 : 0.3;  // of a wave
+    const double waves = generic && per_sm > 1 ? std::max(1.0, x + tail) : x < 4.0 ? std::ceil(x) : x + 0.5;
     const double window = static_cast<double>(a.region_w) * a.region_h * ctas;
     const double edge = generic ? 3.0 + 1.05e-3 * window : 8.0 + rounds + 0.1 * t.warps;
     return waves * (rounds * round + edge * nplanes);
@@ -701,8 +702,11 @@ static int plan_geometry(bm3d_ctx *ctx, StageArgs<T> &a, const bm3d_stage_params
         // 8 x 8; by the least cost 1.12), 1.01 (over; 1.06) and 1.02 (FP64; 1.07).
         const bool plain = generic && generic_size_class(sizeof(T), BS) == 0;
         const bool small = plain && sizeof(T) == 4 && BS < kBS;
+        // (FP32 8 x 8 blocks lose by 4 x 4 tiles on 4 warps: four rounds, whose spread
+        // nothing evens out; np final stage 700 x 540, computer graphics, up to 1.5 times)
+        const bool no_rounds = generic && !plain && BS == kBS;
         auto offer = [&](const TileShape &t) {
-            if (t.warps > max_warps) return;
+            if (t.warps > max_warps || (no_rounds && t.tx * t.ty == 4 * t.warps)) return;
             const SmemPlan sp = plan_tile(a, p, wiener, nplanes, t);
             if (sp.total > ctx->smem_optin) return;
             const double c = tile_cost(ctx, a, sp, t, nplanes, generic);
